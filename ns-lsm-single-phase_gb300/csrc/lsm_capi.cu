@@ -153,6 +153,8 @@ int check_grid(lsm_context* c, const lsm_grid* g, DevGrid* dg) {
     dg->pl = g->physical_face[2] != 0; dg->pr = g->physical_face[3] != 0;
     dg->pd = g->physical_face[4] != 0; dg->pu = g->physical_face[5] != 0;
     dg->dc = g->dc; dg->de = g->de; dg->dz = g->dz;
+    dg->unit = g->dc == 1.0 && g->de == 1.0 && g->dz == 1.0;
+    dg->vc = 1.0 / g->dc * (1.0 / g->de) * (1.0 / g->dz);
     return LSM_OK;
 }
 

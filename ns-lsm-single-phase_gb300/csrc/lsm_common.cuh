@@ -20,6 +20,8 @@ struct DevGrid {
     int ia, ib, ja, jb, ka, kb;  // non-ghost range (0-based, inclusive)
     int pb, pf, pl, pr, pd, pu;  // physical faces i1, im, j1, jm, k1, km
     double dc, de, dz;       // 1/dxi, 1/deta, 1/dzeta
+    int unit;                // dc = de = dz = 1: products with them are exact and left out
+    double vc;               // 1/dc * (1/de) * (1/dz)
 };
 
 __host__ __device__ inline long long gid(const DevGrid& g, int i, int j, int k) {

@@ -5,13 +5,14 @@
 // x86-64 code does.  Division and square root are IEEE-rounded in CUDA FP64;
 // sin/cos are CUDA's (a few ulp from glibc's).
 //
-// Roofline: these kernels are FP64-issue bound on GB300, not HBM bound (the
-// WENO3 stage alone spends 24 FP64 divisions per node); they are the
-// "plain FP64 GPU path" that the FP32 batched kernels are measured against.
+// Roofline: these kernels are bound by the FP64 pipe of GB300, not by HBM:
+// products, quotients, roots and comparisons therefore run on the integer
+// pipes where they are many (lsm_soft64.cuh), bit for bit as CUDA's operators.
 #include <cuda_runtime.h>
 
 #include "lsm_common.cuh"
 #include "lsm_kernels.h"
+#include "lsm_soft64.cuh"
 
 namespace lsm {
 
@@ -23,22 +24,44 @@ inline dim3 box_grid(int ni, int nj, int nk) {
     return dim3((ni + BX - 1) / BX, (nj + BY - 1) / BY, (nk + BZ - 1) / BZ);
 }
 
-// GetWENO3Reconstruction, src/AdvectionMethods.F90:195-245
-__device__ __forceinline__ double weno3(double f0, double f1, double f2, double f3, double ws) {
+// a b in a call: an inlined product would be predicated, and predicated-off
+// operations occupy the FP64 pipe too
+__device__ __noinline__ double product_ieee(double a, double b) { return a * b; }
+
+// GetWENO3Reconstruction, src/AdvectionMethods.F90:195-245, on the stencil
+// oriented by the upwind choice
+__device__ __noinline__ double weno3_ieee(double fL, double fC, double fR) {
     const double d0 = 2.0 / 3.0, d1 = 1.0 / 3.0, epsw = 0.000001;
-    double fL, fC, fR;
-    if (ws > 0.0) { fL = f0; fC = f1; fR = f2; }
-    else          { fL = f3; fC = f2; fR = f1; }
-    double b0 = (fC - fR) * (fC - fR);
-    double b1 = (fL - fC) * (fL - fC);
-    double t0 = b0 + epsw, t1 = b1 + epsw;
-    double a0 = d0 / (t0 * t0);
-    double a1 = d1 / (t1 * t1);
-    double w0 = a0 / (a0 + a1);
-    double w1 = a1 / (a0 + a1);
-    double u0 = 0.5 * fC + 0.5 * fR;
-    double u1 = -0.5 * fL + 1.5 * fC;
+    const double b0 = (fC - fR) * (fC - fR);
+    const double b1 = (fL - fC) * (fL - fC);
+    const double t0 = b0 + epsw, t1 = b1 + epsw;
+    const double a0 = d0 / (t0 * t0);
+    const double a1 = d1 / (t1 * t1);
+    const double w0 = a0 / (a0 + a1), w1 = a1 / (a0 + a1);
+    const double u0 = 0.5 * fC + 0.5 * fR;
+    const double u1 = -0.5 * fL + 1.5 * fC;
     return u0 * w0 + u1 * w1;
+}
+// The same value with the products, quotients and halvings on the integer
+// pipes, beside the 9 operations left to the FP64 pipe: valid while the
+// differences stay below 2^60 (t, a and w then lie in 2^-20 .. 2^121,
+// 2^-243 .. 2^40 and 2^-300 .. 1; a square below 2^-1000 does not change
+// t) and the two candidates u are normal.
+__device__ __forceinline__ double weno3(double fL, double fC, double fR) {
+    const double d0 = 2.0 / 3.0, d1 = 1.0 / 3.0, epsw = 0.000001;
+    const double eR = fC - fR, eL = fL - fC;
+    const double t0 = usqr(eR) + epsw, t1 = usqr(eL) + epsw;
+    const double a0 = udiv(d0, usqr(t0));
+    const double a1 = udiv(d1, usqr(t1));
+    double w0, w1;
+    udiv2(a0, a1, a0 + a1, &w0, &w1);
+    const double s0 = fC + fR;
+    const double u0 = u2d(d2u(s0) - kOne52);   // 0.5 fC + 0.5 fR: halving is exact
+    const double u1 = 1.5 * fC - u2d(d2u(fL) - kOne52);
+    const bool ok = biased_exp(eR) < 1083u && biased_exp(eL) < 1083u && biased_exp(s0) - 523u < 600u &&
+                    biased_exp(u1) - 523u < 600u && biased_exp(fL) - 2u < 1121u;
+    if (!ok) return weno3_ieee(fL, fC, fR);
+    return umul(u0, w0) + umul(u1, w1);
 }
 
 __device__ __forceinline__ bool in_weno_range(const DevGrid& g, int i, int j, int k) {
@@ -48,34 +71,6 @@ __device__ __forceinline__ bool in_weno_range(const DevGrid& g, int i, int j, in
 
 __device__ __forceinline__ bool non_ghost(const DevGrid& g, int i, int j, int k) {
     return i >= g.ia && i <= g.ib && j >= g.ja && j <= g.jb && k >= g.ka && k <= g.kb;
-}
-
-// calc_RH_AD_WENO3 body for one node, src/calc_RH_AD_WENO3.F90:132-399
-__device__ double weno3_rhs_node(const DevGrid& g, const double* __restrict__ phi,
-                                 const double* __restrict__ ucn, long long l, int i, int j, int k) {
-    const int i0 = g.ia + g.pb, i1 = g.ib - g.pf;
-    const int j0 = g.ja + g.pl, j1 = g.jb - g.pr;
-    const int k0 = g.ka + g.pd, k1 = g.kb - g.pu;
-    const bool lo[3] = {g.pb && i == i0, g.pl && j == j0, g.pd && k == k0};
-    const bool hi[3] = {g.pf && i == i1, g.pr && j == j1, g.pu && k == k1};
-    const long long st[3] = {1, g.sj, g.sk};
-    const double dd[3] = {g.dc, g.de, g.dz};
-    double L[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const long long s = st[d];
-        const double U = __ldg(ucn + 3 * l + d);
-        double ws = U;
-        double p0 = __ldg(phi + l - s), p1 = __ldg(phi + l), p2 = __ldg(phi + l + s), p3;
-        if (hi[d]) { ws = 1.0; p3 = 0.0; } else p3 = __ldg(phi + l + 2 * s);
-        const double fp = weno3(p0, p1, p2, p3, ws);
-        ws = U;
-        if (lo[d]) { ws = -1.0; p0 = 0.0; } else p0 = __ldg(phi + l - 2 * s);
-        p1 = __ldg(phi + l - s); p2 = __ldg(phi + l); p3 = __ldg(phi + l + s);
-        const double fm = weno3(p0, p1, p2, p3, ws);
-        L[d] = U * (dd[d] * (fp - fm));
-    }
-    return L[0] + L[1] + L[2];
 }
 
 // calc_RH_AD (orderAD == 0) for one non-ghost node, src/calc_RH_AD.F90:1-273
@@ -123,7 +118,7 @@ __global__ void contra_kernel(DevGrid g, const double* __restrict__ q, const dou
         ucn[3 * l] = 0.0; ucn[3 * l + 1] = 0.0; ucn[3 * l + 2] = 0.0;
         return;
     }
-    const double tmp = 1.0 / aj[l];
+    const double tmp = sdiv(1.0, aj[l]);
     const double u = q[4 * l + 1], v = q[4 * l + 2], w = q[4 * l + 3];
     ucn[3 * l + 0] = tmp * (csi[3 * l] * u + csi[3 * l + 1] * v + csi[3 * l + 2] * w);
     ucn[3 * l + 1] = tmp * (eta[3 * l] * u + eta[3 * l + 1] * v + eta[3 * l + 2] * w);
@@ -131,43 +126,154 @@ __global__ void contra_kernel(DevGrid g, const double* __restrict__ q, const dou
 }
 
 // ------------------------------------------------------------ A2 / A7 ----
-__global__ void rh_ad_kernel(DevGrid g, int orderAD, const double* __restrict__ phi,
-                             const double* __restrict__ ucn, const int* __restrict__ mask,
-                             double* __restrict__ rh) {
+__global__ void rh_upwind_kernel(DevGrid g, const double* __restrict__ phi, const double* __restrict__ ucn,
+                                 const int* __restrict__ mask, double* __restrict__ rh) {
     const int i = blockIdx.x * BX + threadIdx.x, j = blockIdx.y * BY + threadIdx.y,
               k = blockIdx.z * BZ + threadIdx.z;
     if (i >= g.ni || j >= g.nj || k >= g.nk) return;
     const long long l = gid(g, i, j, k);
-    double r = 0.0;
-    if (orderAD == 1) {
-        if (in_weno_range(g, i, j, k) && !(mask && mask[l] == 0)) r = weno3_rhs_node(g, phi, ucn, l, i, j, k);
-    } else {
-        if (non_ghost(g, i, j, k) && !(mask && mask[l] <= 0)) r = upwind_rhs_node(g, phi, ucn, l, i, j, k);
-    }
-    rh[l] = r;
+    rh[l] = non_ghost(g, i, j, k) && !(mask && mask[l] <= 0) ? upwind_rhs_node(g, phi, ucn, l, i, j, k) : 0.0;
 }
 
 // ---------------------------------------------------------------- A4 ----
 // One TVD-RK3 stage, src/ad_RKTVD3.F90:53-81, written to `out` (ping-pong):
 // out = c1*phin + c2*phi1 - c3*aj*dt*rh on advected non-ghost nodes, phi1
 // elsewhere.  rh is 0 on physical-boundary nodes under WENO3.
-__global__ void rk_stage_kernel(DevGrid g, int orderAD, const double* __restrict__ phin,
-                                const double* __restrict__ phi1, const double* __restrict__ ucn,
-                                const double* __restrict__ aj, const int* __restrict__ mask, double c1,
-                                double c2, double c3, double dt, double* __restrict__ out) {
+struct StageArgs {
+    const double *phin, *phi1, *ucn, *aj;
+    const int* mask;
+    double c1, c2, c3, dt;
+    int first;   // c1 = 1, c2 = 0, c3 = 1 and phi1 is phin
+    double* out;
+};
+
+__device__ __forceinline__ double stage_value(const StageArgs& a, long long l, double p1, double rh) {
+    // first stage: 1 phin + 0 phi1 = phin and 1 aj = aj, exactly
+    if (a.first && finite64(p1)) return p1 - a.aj[l] * a.dt * rh;
+    return a.c1 * a.phin[l] + a.c2 * p1 - a.c3 * a.aj[l] * a.dt * rh;
+}
+
+__global__ void rk_upwind_kernel(DevGrid g, StageArgs a) {
     const int i = blockIdx.x * BX + threadIdx.x, j = blockIdx.y * BY + threadIdx.y,
               k = blockIdx.z * BZ + threadIdx.z;
     if (i >= g.ni || j >= g.nj || k >= g.nk) return;
     const long long l = gid(g, i, j, k);
-    const double p1 = phi1[l];
-    if (!non_ghost(g, i, j, k) || (mask && mask[l] <= 0)) { out[l] = p1; return; }
-    double rh = 0.0;
-    if (orderAD == 1) {
-        if (in_weno_range(g, i, j, k)) rh = weno3_rhs_node(g, phi1, ucn, l, i, j, k);
-    } else {
-        rh = upwind_rhs_node(g, phi1, ucn, l, i, j, k);
+    const double p1 = a.phi1[l];
+    if (!non_ghost(g, i, j, k) || (a.mask && a.mask[l] <= 0)) { a.out[l] = p1; return; }
+    a.out[l] = stage_value(a, l, p1, upwind_rhs_node(g, a.phi1, a.ucn, l, i, j, k));
+}
+
+// calc_RH_AD_WENO3 (src/calc_RH_AD_WENO3.F90:132-399) and, with RH false,
+// the stage built on it, for the 32 x TY x TZ nodes of a block of NT threads.
+//
+// The reconstruction of the face between two nodes is the lower node's
+// (f+) and the upper node's (f-); both evaluate the same expression on the
+// same values whenever they choose the same upwind side.  So a block
+// evaluates each face once into shared memory (the choice of the lower
+// node where that is advected, else the upper's), then each node takes its
+// six faces from there and evaluates for itself only an f- whose stored
+// choice is not its own (a sign change of the contravariant velocity).
+//
+// Bounded by the FP64 pipe (one warp operation in 16 clocks of an SM: 51 of
+// them a node here, six reconstructions with CUDA's divisions took 360) and,
+// nearly as much, by the issue of the integer work beside it: 1.81 ms before,
+// 0.33 ms now on 256 x 128 x 96 nodes.  A tile of 32 x 8 x 4 evaluates 3.4
+// faces a node, 32 x 2 x 2 4.0.
+template <int TY, int TZ, int NT, bool RH>
+__global__ void __launch_bounds__(NT, 1280 / NT) weno_kernel(DevGrid g, StageArgs a) {
+    constexpr int RZ = (TZ + 1) * TY, RY = TZ * (TY + 1), RX = TZ * TY;   // rows of 32 faces per direction
+    constexpr int NF = 32 * (RZ + RY + RX) + RX;                          // and the rows' lower x faces
+    __shared__ double F[NF];
+    __shared__ bool up_of[NF];
+    const int t = threadIdx.x, lane = t & 31;
+    const int bi = blockIdx.x * 32, bj = blockIdx.y * TY, bk = blockIdx.z * TZ;
+    const int c0[3] = {g.ia + g.pb, g.ja + g.pl, g.ka + g.pd}, c1[3] = {g.ib - g.pf, g.jb - g.pr, g.kb - g.pu};
+    const int plo[3] = {g.pb, g.pl, g.pd};
+    const double* __restrict__ phi = a.phi1;
+    const double* __restrict__ ucn = a.ucn;
+    const int* __restrict__ mask = a.mask;
+    auto advected = [&](int i, int j, int k, long long l) {
+        if (!in_weno_range(g, i, j, k)) return false;
+        if (!mask) return true;
+        const int m = __ldg(mask + l);
+        return RH ? m != 0 : m > 0;
+    };
+    auto rec = [&](long long l, long long s, bool up) {
+        return weno3(__ldg(phi + (up ? l - s : l + 2 * s)), __ldg(phi + (up ? l : l + s)),
+                     __ldg(phi + (up ? l + s : l)));
+    };
+    for (int w = t; w < NF; w += NT) {
+        int d, i = bi + lane, j = bj, k = bk;   // the face's lower node
+        int r = w >> 5;
+        if (r < RZ) {
+            d = 2; j += r % TY; k += r / TY - 1;
+        } else if (r < RZ + RY) {
+            r -= RZ; d = 1; j += r % (TY + 1) - 1; k += r / (TY + 1);
+        } else if (r < RZ + RY + RX) {
+            r -= RZ + RY; d = 0; j += r % TY; k += r / TY;
+        } else {
+            r = w - 32 * (RZ + RY + RX); d = 0; i = bi - 1; j += r % TY; k += r / TY;
+        }
+        if (i < 0 || j < 0 || k < 0) continue;
+        const long long s = d == 0 ? 1 : (d == 1 ? g.sj : g.sk), l = gid(g, i, j, k);
+        const int c = d == 0 ? i : (d == 1 ? j : k);
+        const bool last = d == 0 ? g.pf && c == c1[0] : (d == 1 ? g.pr && c == c1[1] : g.pu && c == c1[2]);
+        const bool first = d == 0 ? g.pb && c + 1 == c0[0] : (d == 1 ? g.pl && c + 1 == c0[1] : g.pd && c + 1 == c0[2]);
+        const bool own = advected(i, j, k, l);
+        if (!own && !advected(i + (d == 0), j + (d == 1), k + (d == 2), l + s)) continue;
+        const bool pos = gt0(__ldg(ucn + 3 * (own ? l : l + s) + d));
+        // the one-sided stencils next to a physical face
+        const bool up = own ? pos || last : pos && !first;
+        F[w] = rec(l, s, up);
+        up_of[w] = up;
     }
-    out[l] = c1 * phin[l] + c2 * p1 - c3 * aj[l] * dt * rh;
+    __syncthreads();
+    for (int row = t >> 5; row < TY * TZ; row += NT / 32) {
+        const int ty = row % TY, tz = row / TY;
+        const int i = bi + lane, j = bj + ty, k = bk + tz;
+        if (i >= g.ni || j >= g.nj || k >= g.nk) continue;
+        const long long l = gid(g, i, j, k);
+        double rh = 0.0;
+        if (advected(i, j, k, l)) {
+            const int xr = 32 * (RZ + RY + row);
+            const int lo[3] = {lane ? xr + lane - 1 : 32 * (RZ + RY + RX) + row, 32 * (RZ + tz * (TY + 1) + ty) + lane,
+                               32 * row + lane};
+            const int hi[3] = {xr + lane, lo[1] + 32, lo[2] + 32 * TY};
+            const int c[3] = {i, j, k};
+            const long long st[3] = {1, g.sj, g.sk};
+            const double dd[3] = {g.dc, g.de, g.dz};
+            double L[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const double U = __ldg(ucn + 3 * l + d);
+                const bool up = gt0(U) && !(plo[d] && c[d] == c0[d]);
+                double fm = F[lo[d]];
+                if (up_of[lo[d]] != up) fm = rec(l - st[d], st[d], up);
+                const double D = F[hi[d]] - fm;
+                L[d] = U * (g.unit ? D : product_ieee(dd[d], D));
+            }
+            rh = L[0] + L[1] + L[2];
+        }
+        if (RH) {
+            a.out[l] = rh;
+        } else {
+            const double p1 = phi[l];
+            a.out[l] = non_ghost(g, i, j, k) && (!mask || mask[l] > 0) ? stage_value(a, l, p1, rh) : p1;
+        }
+    }
+}
+
+// The largest tile that still fills the GPU: 32 x 8 x 4 from one full wave of
+// blocks on (5 on each of 152 SMs), 32 x 4 x 2 from two blocks per SM on,
+// 32 x 2 x 2 below.  Measured: 256 x 128 x 96 nodes 332 / 377 us with 8 x 4 /
+// 4 x 2, 64^3 49 / 42 us.
+template <bool RH>
+void launch_weno(const DevGrid& g, const StageArgs& a, cudaStream_t s) {
+    auto grid = [&](int ty, int tz) { return dim3((g.ni + 31) / 32, (g.nj + ty - 1) / ty, (g.nk + tz - 1) / tz); };
+    auto blocks = [](const dim3& d) { return (long long)d.x * d.y * d.z; };
+    if (blocks(grid(8, 4)) >= 5 * 152) weno_kernel<8, 4, 256, RH><<<grid(8, 4), 256, 0, s>>>(g, a);
+    else if (blocks(grid(4, 2)) >= 2 * 152) weno_kernel<4, 2, 256, RH><<<grid(4, 2), 256, 0, s>>>(g, a);
+    else weno_kernel<2, 2, 128, RH><<<grid(2, 2), 128, 0, s>>>(g, a);
 }
 
 // ---------------------------------------------------------------- A5 ----
@@ -518,14 +624,18 @@ void launch_contra(const DevGrid& g, const double* q, const double* csi, const d
 void launch_rh_ad(const DevGrid& g, int orderAD, const double* phi, const double* ucn, const int* mask,
                   double* rh, cudaStream_t s) {
     ProfScope ps_("rh_ad_kernel", s);
-    rh_ad_kernel<<<LSM_BOX(g)>>>(g, orderAD, phi, ucn, mask, rh);
+    if (orderAD == 1) launch_weno<true>(g, StageArgs{nullptr, phi, ucn, nullptr, mask, 0.0, 0.0, 0.0, 0.0, 0, rh}, s);
+    else rh_upwind_kernel<<<LSM_BOX(g)>>>(g, phi, ucn, mask, rh);
 }
 
 void launch_rk_stage(const DevGrid& g, int orderAD, const double* phin, const double* phi1, const double* ucn,
                      const double* aj, const int* mask, double c1, double c2, double c3, double dt, double* out,
                      cudaStream_t s) {
     ProfScope ps_("rk_stage_kernel", s);
-    rk_stage_kernel<<<LSM_BOX(g)>>>(g, orderAD, phin, phi1, ucn, aj, mask, c1, c2, c3, dt, out);
+    const int first = c1 == 1.0 && c2 == 0.0 && c3 == 1.0 && phin == phi1;
+    const StageArgs a{phin, phi1, ucn, aj, mask, c1, c2, c3, dt, first, out};
+    if (orderAD == 1) launch_weno<false>(g, a, s);
+    else rk_upwind_kernel<<<LSM_BOX(g)>>>(g, a);
 }
 
 void launch_bc_rk(const DevGrid& g, const DevBC& bc, int orderAD, const double* phin, const double* phi1,
