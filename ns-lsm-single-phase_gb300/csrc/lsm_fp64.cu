@@ -408,50 +408,80 @@ __global__ void bc_full_kernel(DevGrid g, DevBC bc, const double* __restrict__ s
 }
 
 // ------------------------------------------------------------ R1 / R2 ----
-// One-sided differences of src/calc_sign_ini.F90:42-176 (= calc_RH_RN.F90:36-170)
-// and the Godunov norms of calc_sign_ini.F90:204-242, for one node.
-__device__ __forceinline__ void godunov_node(const DevGrid& g, const double* __restrict__ f,
-                                             const double* __restrict__ csi, const double* __restrict__ eta,
-                                             const double* __restrict__ zet, long long l, int i, int j, int k,
-                                             double* gplus, double* gminus) {
+// The Godunov norm of calc_sign_ini.F90:190-242 as written there, from the
+// metrics and the backward / forward differences
+__device__ __noinline__ double godunov_norm_ieee(bool plus, double m0, double m1, double m2, double m3, double m4,
+                                                 double m5, double m6, double m7, double m8, double q0, double q1,
+                                                 double q2, double p0, double p1, double p2) {
+    const double M[9] = {m0, m1, m2, m3, m4, m5, m6, m7, m8};
+    double m[3];
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        const double ab = (M[x] * q0 + M[3 + x] * q1 + M[6 + x] * q2) / 2.0;
+        const double af = (M[x] * p0 + M[3 + x] * p1 + M[6 + x] * p2) / 2.0;
+        const double p = plus ? ab + fabs(ab) : ab - fabs(ab), q = plus ? af - fabs(af) : af + fabs(af);
+        m[x] = fmax(p * p, q * q);
+    }
+    return sqrt(m[0] + m[1] + m[2]);
+}
+
+// The norm G+ (plus) or G- of one node: the one-sided differences of
+// src/calc_sign_ini.F90:42-176 (= calc_RH_RN.F90:36-170), the gradients on
+// them and the Godunov choice.
+//
+// Of each pair b/2 +- |b/2| one is b and the other 0, and the larger of two
+// squares is the square of the larger magnitude: both are chosen on the
+// integer pipes, and only the norm that is used is formed, with one square
+// per direction.  The products and the root run on the integer pipes too,
+// beside the 20 additions left to the FP64 pipe (134 clocked operations
+// where both norms were formed with CUDA's root).  Each is exactly the value
+// of the written-out expression while every factor is 0 or within 2^+-240;
+// others take that expression, in a call (as in product_ieee).  0.79 ms a
+// pseudo-step before, 0.20 ms now on 256 x 128 x 96 nodes; at most 64
+// registers for four blocks per SM (86 and two blocks: 0.27 ms).
+__device__ __forceinline__ double godunov_norm(const DevGrid& g, const double* __restrict__ f,
+                                               const double* __restrict__ csi, const double* __restrict__ eta,
+                                               const double* __restrict__ zet, long long l, int i, int j, int k,
+                                               bool plus) {
     const long long st[3] = {1, g.sj, g.sk};
     const double dd[3] = {g.dc, g.de, g.dz};
     const int c[3] = {i, j, k};
     const int plo[3] = {g.pb, g.pl, g.pd}, phs[3] = {g.pf, g.pr, g.pu};
     const int lo[3] = {g.ia, g.ja, g.ka}, hi[3] = {g.ib, g.jb, g.kb};
-    double mas[3], men[3];
+    double mas[3], men[3], M[9];
     const double fc = __ldg(f + l);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const long long s = st[d];
-        if (plo[d] && c[d] == lo[d]) {
-            mas[d] = dd[d] * (__ldg(f + l + s) - fc); men[d] = mas[d];
-        } else if (phs[d] && c[d] == hi[d]) {
-            men[d] = dd[d] * (fc - __ldg(f + l - s)); mas[d] = men[d];
-        } else {
-            mas[d] = dd[d] * (__ldg(f + l + s) - fc);
-            men[d] = dd[d] * (fc - __ldg(f + l - s));
-        }
+        const bool first = plo[d] && c[d] == lo[d], last = phs[d] && c[d] == hi[d];
+        double p = last ? 0.0 : __ldg(f + l + s) - fc, q = first ? 0.0 : fc - __ldg(f + l - s);
+        if (!g.unit) { p = product_ieee(dd[d], p); q = product_ieee(dd[d], q); }
+        mas[d] = last ? q : p;
+        men[d] = first ? p : q;
     }
     const double* m[3] = {csi + 3 * l, eta + 3 * l, zet + 3 * l};
-    double b[3], fw[3];
+    auto fits = [](double v) { return biased_exp(v) - 783u < 480u || mag(v) == 0u; };
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+        M[q] = __ldg(m[q / 3] + q % 3);
+        ok = ok && fits(M[q]);
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) ok = ok && fits(mas[d]) && fits(men[d]);
+    if (!ok)
+        return godunov_norm_ieee(plus, M[0], M[1], M[2], M[3], M[4], M[5], M[6], M[7], M[8], men[0], men[1], men[2],
+                                 mas[0], mas[1], mas[2]);
+    double w[3];
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
-        b[x] = __ldg(m[0] + x) * men[0] + __ldg(m[1] + x) * men[1] + __ldg(m[2] + x) * men[2];
-        fw[x] = __ldg(m[0] + x) * mas[0] + __ldg(m[1] + x) * mas[1] + __ldg(m[2] + x) * mas[2];
+        const double b = umul0(M[x], men[0]) + umul0(M[3 + x], men[1]) + umul0(M[6 + x], men[2]);
+        const double e = umul0(M[x], mas[0]) + umul0(M[3 + x], mas[1]) + umul0(M[6 + x], mas[2]);
+        const u64 p = ((d2u(b) >> 63) != 0u) != plus ? mag(b) : 0u;   // plus: b > 0, else b < 0
+        const u64 q = ((d2u(e) >> 63) != 0u) == plus ? mag(e) : 0u;   // plus: e < 0, else e > 0
+        w[x] = usqr(u2d(p > q ? p : q));
     }
-    double bp[3], bm[3], fp[3], fm[3];
-#pragma unroll
-    for (int x = 0; x < 3; ++x) {
-        double aux = b[x] / 2.0;
-        bp[x] = aux + fabs(aux); bm[x] = aux - fabs(aux);
-        aux = fw[x] / 2.0;
-        fp[x] = aux + fabs(aux); fm[x] = aux - fabs(aux);
-    }
-    *gplus = sqrt(fmax(bp[0] * bp[0], fm[0] * fm[0]) + fmax(bp[1] * bp[1], fm[1] * fm[1]) +
-                  fmax(bp[2] * bp[2], fm[2] * fm[2]));
-    *gminus = sqrt(fmax(bm[0] * bm[0], fp[0] * fp[0]) + fmax(bm[1] * bm[1], fp[1] * fp[1]) +
-                   fmax(bm[2] * bm[2], fp[2] * fp[2]));
+    return ssqrt(w[0] + w[1] + w[2]);
 }
 
 // deltaf, src/global_lsm.F90:120-133
@@ -461,7 +491,7 @@ __device__ __forceinline__ double deltaf(double v, double e) {
 }
 
 // calc_sign_ini, src/calc_sign_ini.F90:199-269 (+ deltaf(phi0) for the reinit steps)
-__global__ void sign_ini_kernel(DevGrid g, const double* __restrict__ phi0, const double* __restrict__ csi,
+__global__ void __launch_bounds__(256, 4) sign_ini_kernel(DevGrid g, const double* __restrict__ phi0, const double* __restrict__ csi,
                                 const double* __restrict__ eta, const double* __restrict__ zet, double eps,
                                 int M_Sphi0, double* __restrict__ sgn, double* __restrict__ ng,
                                 double* __restrict__ delta) {
@@ -474,10 +504,9 @@ __global__ void sign_ini_kernel(DevGrid g, const double* __restrict__ phi0, cons
         if (delta) delta[l] = 0.0;
         return;
     }
-    double gp, gm;
-    godunov_node(g, phi0, csi, eta, zet, l, i, j, k, &gp, &gm);
     const double f = phi0[l];
-    const double nrm = f > 0.0 ? gp : (f < 0.0 ? gm : 1.0);
+    const bool pos = gt0(f);
+    const double nrm = pos || lt0(f) ? godunov_norm(g, phi0, csi, eta, zet, l, i, j, k, pos) : 1.0;
     double s;
     if (M_Sphi0 == 1) {
         if (f >= eps) s = 1.0;
@@ -491,6 +520,17 @@ __global__ void sign_ini_kernel(DevGrid g, const double* __restrict__ phi0, cons
     if (delta) delta[l] = deltaf(f, eps);
 }
 
+// s (|grad d| - 1), src/calc_RH_RN.F90:185-238; s is +-1 but near the surface,
+// where the product is the factor with its sign changed
+__device__ __forceinline__ double reinit_rhs(const DevGrid& g, const double* __restrict__ d,
+                                             const double* __restrict__ csi, const double* __restrict__ eta,
+                                             const double* __restrict__ zet, long long l, int i, int j, int k,
+                                             double s) {
+    const bool pos = gt0(s);
+    const double r = (pos || lt0(s) ? godunov_norm(g, d, csi, eta, zet, l, i, j, k, pos) : 1.0) - 1.0;
+    return mag(s) == 0x3FF0000000000000ull ? (pos ? r : -r) : product_ieee(s, r);
+}
+
 // calc_RH_RN, src/calc_RH_RN.F90:185-238
 __global__ void rh_rn_kernel(DevGrid g, const double* __restrict__ d, const double* __restrict__ sgn,
                              const double* __restrict__ csi, const double* __restrict__ eta,
@@ -500,20 +540,17 @@ __global__ void rh_rn_kernel(DevGrid g, const double* __restrict__ d, const doub
     if (i >= g.ni || j >= g.nj || k >= g.nk) return;
     const long long l = gid(g, i, j, k);
     if (!non_ghost(g, i, j, k)) { rh[l] = 0.0; return; }
-    double gp, gm;
-    godunov_node(g, d, csi, eta, zet, l, i, j, k, &gp, &gm);
     const double s = sgn[l];
-    const double nrm = s > 0.0 ? gp : (s < 0.0 ? gm : 1.0);
-    rh[l] = s * (nrm - 1.0);
+    rh[l] = reinit_rhs(g, d, csi, eta, zet, l, i, j, k, s);
 }
 
-// calc_lambda_RN method 0, src/calc_lambda_RN.F90:42-63
-__device__ __forceinline__ double lambda_node(double vc, double del, double dt, double d, double p0,
+// calc_lambda_RN method 0, src/calc_lambda_RN.F90:42-63 (rdt = 1 / dt)
+__device__ __forceinline__ double lambda_node(const DevGrid& g, double del, double rdt, double d, double p0,
                                               double ng) {
-    const double Lop = del * (1.0 / dt * (d - p0));
-    const double num = vc * Lop;
-    const double den = vc * (del * del) * ng;
-    return den == 0.0 ? 0.0 : -num / den;
+    const double Lop = del * (rdt * (d - p0));
+    const double num = g.unit ? Lop : g.vc * Lop;
+    const double den = (g.unit ? del * del : g.vc * (del * del)) * ng;
+    return den == 0.0 ? 0.0 : sdiv(-num, den);
 }
 
 __global__ void lambda_rn_kernel(DevGrid g, double eps, const double* __restrict__ phi0,
@@ -524,13 +561,12 @@ __global__ void lambda_rn_kernel(DevGrid g, double eps, const double* __restrict
     if (i >= g.ni || j >= g.nj || k >= g.nk) return;
     const long long l = gid(g, i, j, k);
     if (!non_ghost(g, i, j, k)) { lam[l] = 0.0; return; }
-    const double vc = 1.0 / g.dc * (1.0 / g.de) * (1.0 / g.dz);
-    lam[l] = lambda_node(vc, deltaf(phi0[l], eps), dt, d[l], phi0[l], ng[l]);
+    lam[l] = lambda_node(g, deltaf(phi0[l], eps), 1.0 / dt, d[l], phi0[l], ng[l]);
 }
 
 // One pseudo-step of `reinitialization`, src/reinitialization.F90:55-99,
 // fused: Godunov RHS -> Euler update -> lambda -> correction.
-__global__ void reinit_step_kernel(DevGrid g, double dt, const double* __restrict__ din,
+__global__ void __launch_bounds__(256, 4) reinit_step_kernel(DevGrid g, double dt, double rdt, const double* __restrict__ din,
                                    const double* __restrict__ sgn, const double* __restrict__ ng,
                                    const double* __restrict__ delta, const double* __restrict__ phi0,
                                    const double* __restrict__ csi, const double* __restrict__ eta,
@@ -541,15 +577,11 @@ __global__ void reinit_step_kernel(DevGrid g, double dt, const double* __restric
     const long long l = gid(g, i, j, k);
     const double dc0 = din[l];
     if (!non_ghost(g, i, j, k)) { dout[l] = dc0; return; }
-    double gp, gm;
-    godunov_node(g, din, csi, eta, zet, l, i, j, k, &gp, &gm);
-    const double s = sgn[l];
-    const double nrm = s > 0.0 ? gp : (s < 0.0 ? gm : 1.0);
-    const double rh = s * (nrm - 1.0);
-    const double d1 = dc0 - dt * rh;
-    const double vc = 1.0 / g.dc * (1.0 / g.de) * (1.0 / g.dz);
+    const double d1 = dc0 - dt * reinit_rhs(g, din, csi, eta, zet, l, i, j, k, sgn[l]);
     const double del = delta[l], gn = ng[l];
-    const double lam = lambda_node(vc, del, dt, d1, phi0[l], gn);
+    // away from the surface delta is 0: lambda is 0 and the correction +0
+    if (mag(del) == 0u && finite64(gn)) { dout[l] = d2u(d1) == 1ull << 63 ? 0.0 : d1; return; }
+    const double lam = lambda_node(g, del, rdt, d1, phi0[l], gn);
     dout[l] = d1 + dt * lam * del * gn;
 }
 
@@ -677,7 +709,7 @@ void launch_reinit_step(const DevGrid& g, double dt, const double* din, const do
                         const double* delta, const double* phi0, const double* csi, const double* eta,
                         const double* zet, double* dout, cudaStream_t s) {
     ProfScope ps_("reinit_step_kernel", s);
-    reinit_step_kernel<<<LSM_BOX(g)>>>(g, dt, din, sgn, ng, delta, phi0, csi, eta, zet, dout);
+    reinit_step_kernel<<<LSM_BOX(g)>>>(g, dt, 1.0 / dt, din, sgn, ng, delta, phi0, csi, eta, zet, dout);
 }
 
 void launch_narrowband(const DevGrid& g, double thr, int isnarrow, const double* phin, int* nb, cudaStream_t s) {

@@ -49,3 +49,19 @@ def test_stage_tiles_bit_exact(ls, oracle, shape, kind):
                         oracle.calc_rh_ad_weno3(g, phi, ucn, m))
             assert same(host(ls.ad_rktvd3(G(g), P(p), dev(phi), dev(ucn), dev(aj), dm)),
                         oracle.ad_rktvd3(g, p, phi, ucn, aj, m))
+
+
+@pytest.mark.parametrize("kind", ["plain", "extreme"])
+@pytest.mark.parametrize("spacing", [(1.0, 1.0, 1.0), (0.5, 1.0, 3.0)])
+def test_godunov_bit_exact(ls, oracle, spacing, kind):
+    shape = (34, 9, 11)
+    g = O.make_grid(*shape)
+    g.dc, g.de, g.dz = spacing
+    rng = np.random.default_rng(2)
+    d = field(shape, kind, 3)
+    met = [cases.F(rng.standard_normal((3,) + shape) * (rng.random((3,) + shape) > 0.3)) for _ in range(3)]
+    sign = cases.F(rng.choice([-1.0, 1.0, 0.0, 0.37, -1e-9, 1e-310, np.nan], shape))
+    with np.errstate(all="ignore"):
+        assert same(host(ls.calc_rh_rn(G(g), dev(d), dev(sign), *map(dev, met))), oracle.calc_rh_rn(g, d, sign, *met))
+        _, ng = ls.calc_sign_ini(G(g), dev(d), *map(dev, met), 0.1)
+        assert same(host(ng), oracle.calc_sign_ini(g, d, *met, 0.1)[1])
