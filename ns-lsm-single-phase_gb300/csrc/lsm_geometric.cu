@@ -13,19 +13,20 @@
 //   - K-tetrahedron ids: an exclusive scan of popcount(cell bits) over the
 //     cells in the same order, plus the rank of the tetrahedron's bit inside
 //     its cell.
-// A pnode's tetrahedron list is then not stored: it is re-enumerated from the
-// (at most) eight cells around the node, in increasing cell index and
-// tetrahedron number, which is exactly the order GetTetrahedraList appends
-// them (src/GetTetrahedraList.F90:322-446).  The distance loops keep the
-// reference's sequential running-minimum updates per node (their rounding
-// depends on the order): one thread per pnode in k_geo_sd, one warp per
-// -1 node in k_geo_neigh (the lanes share out the distances, the chain is
-// replayed in order).
+// A pnode's tetrahedra are enumerated from the (at most) eight cells around
+// the node, in increasing cell index and tetrahedron number, which is exactly
+// the order GetTetrahedraList appends them (src/GetTetrahedraList.F90:322-446);
+// their triangles are listed per pnode in that order.  The distance loops
+// keep the results of the reference's sequential running-minimum updates per
+// node (whose rounding depends on the order): one warp per node encloses the
+// distances in FP32 and evaluates in FP64, in order, only those that the
+// final bits can depend on (k_geo_sd, k_geo_neigh).
 #include <cuda_runtime.h>
 
 #include "lsm_common.cuh"
 #include "lsm_geometric.h"
 #include "lsm_kernels.h"
+#include "lsm_soft64.cuh"
 #include "lsm_volume_dev.cuh"
 
 namespace lsm {
@@ -40,7 +41,7 @@ constexpr int kTile = 4 * kThreads;  // elements per scan tile
 // the IEEE order is the order of the bit patterns as signed integers, and
 // x < 0 holds exactly when the sign bit is set and x is not -0.  GB300's
 // FP64 pipe is its scarce resource; these are exact (no NaN reaches them).
-__device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
+__device__ __forceinline__ long long dbits(double x) { return (long long)d2u(x); }
 __device__ __forceinline__ bool nn_lt(double a, double b) { return dbits(a) < dbits(b); }   // a, b >= +0
 __device__ __forceinline__ bool nn_le(double a, double b) { return dbits(a) <= dbits(b); }  // a, b >= +0
 __device__ __forceinline__ bool neg(double x) {
@@ -62,26 +63,25 @@ __device__ __forceinline__ double norm2v(const double* a) {
         if (b != 0) {
             const double ax = __longlong_as_double(b);
             if (dbits(scale) < b) {
-                const double v = scale / ax;
+                const double v = sdiv(scale, ax);
                 r = 1.0 + r * v * v;
                 scale = ax;
             } else {
-                const double v = dbits(scale) == kOneBits ? ax : ax / scale;
+                const double v = dbits(scale) == kOneBits ? ax : sdiv(ax, scale);
                 r = r + v * v;
             }
         }
     }
-    return dbits(scale) == kOneBits ? sqrt(r) : sqrt(r) * scale;
+    const double q = ssqrt(r);
+    return dbits(scale) == kOneBits ? q : q * scale;
 }
 __device__ __forceinline__ void sub3(const double* a, const double* b, double* c) {
     c[0] = a[0] - b[0]; c[1] = a[1] - b[1]; c[2] = a[2] - b[2];
 }
+// (the reference's sum starts from 0, which changes only the sign of a zero
+// result: no use below depends on it)
 __device__ __forceinline__ double dot3g(const double* a, const double* b) {
-    double s = 0.0;
-    s = s + a[0] * b[0];
-    s = s + a[1] * b[1];
-    s = s + a[2] * b[2];
-    return s;
+    return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
 }
 __device__ __forceinline__ void cross3g(const double* a, const double* b, double* c) {
     c[0] = a[1] * b[2] - a[2] * b[1];
@@ -207,7 +207,7 @@ __device__ __forceinline__ double dist_point_line(const double* AP, const double
     if (valid) {
         double c[3];
         cross3g(AP, BP, c);
-        return norm2v(c) / nAB;
+        return sdiv(norm2v(c), nAB);
     }
     return dmin(nAP, nBP);
 }
@@ -256,8 +256,7 @@ __device__ double dist_point_triangle(const double* T, const TriGeo& g, const do
     const double v[3] = {-g.CA[0], -g.CA[1], -g.CA[2]};
     double cu[3], cw[3];
     cross3g(g.AB, PA, cu); cross3g(PA, v, cw);
-    const double alpha = dot3g(cu, g.nv) / g.nn;
-    const double beta = dot3g(cw, g.nv) / g.nn;
+    const double alpha = sdiv(dot3g(cu, g.nv), g.nn), beta = sdiv(dot3g(cw, g.nv), g.nn);
     const double gamma = 1.0 - beta - alpha;
     if (pos(alpha) && lt1(alpha) && pos(beta) && lt1(beta) && pos(gamma) && lt1(gamma)) {
         double pp[3], dd[3];
@@ -382,13 +381,12 @@ __device__ __forceinline__ void for_each_tet(const DevGrid& g, int i, int j, int
 // one K tetrahedron: its isosurface triangles (18 doubles) with their
 // triangle-only distance terms (TriGeo), area and water volume of the
 // linear reconstruction, its four pnode ids (0-based), and per triangle an
-// FP32 bounding box (rounded outwards) and FP32 vertices, used only to skip
-// distance evaluations that cannot change a running minimum
+// FP32 bounding box (rounded outwards), used only to skip distance
+// evaluations that cannot change a running minimum
 struct alignas(16) GeoTet {
     double tri[2][9];
     TriGeo tg[2];
     float box[2][6];  // lo x y z, hi x y z
-    float trf[2][9];  // the vertices rounded to FP32 (upper bounds of the distance)
     double area, wv;
     int nis;
     int v[4];
@@ -412,6 +410,47 @@ __device__ __forceinline__ bool beyond_box(const float* p, float pscale, const f
     const float dz = fmaxf(fmaxf(lo[2] - p[2], p[2] - hi[2]), 0.0f);
     const float lb = sqrtf(dx * dx + dy * dy + dz * dz);
     return lb > d + 1.0e-5f * (lb + d + pscale);
+}
+
+// One triangle in FP32, for tri_interval: vertex A, the edges AB and AC with
+// their squared inverse lengths and BC's, the gradients ga and gb of the
+// reference's alpha and beta in P - A, 1 / (least height), and a bound of the
+// inradius (-1: an edge too short for the enclosure below, whose distance is
+// bounded by the bounding box alone).
+struct alignas(16) TriF {
+    float A[3], rad, AB[3], iAB, AC[3], iAC, ga[3], iBC, gb[3], gmax;
+};
+
+__device__ void tri_f32(const double* T, const TriGeo& g, TriF& f) {
+    double len = 0.0, scale = 0.0, nga = 0.0, ngb = 0.0, ngc = 0.0;
+#pragma unroll
+    for (int c = 0; c < 9; ++c) scale = fmax(scale, fabs(T[c]));
+    len = fmin(g.nAB, fmin(g.nBC, g.nCA));
+    const double AC[3] = {-g.CA[0], -g.CA[1], -g.CA[2]};
+    double ga[3], gb[3];
+    cross3g(g.nv, g.AB, ga);
+    cross3g(AC, g.nv, gb);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        ga[c] = g.nn > 0.0 ? ga[c] / g.nn : 0.0;
+        gb[c] = g.nn > 0.0 ? gb[c] / g.nn : 0.0;
+        nga += ga[c] * ga[c];
+        ngb += gb[c] * gb[c];
+        ngc += (ga[c] + gb[c]) * (ga[c] + gb[c]);
+        f.A[c] = (float)T[c];
+        f.AB[c] = (float)g.AB[c];
+        f.AC[c] = (float)AC[c];
+        f.ga[c] = (float)ga[c];
+        f.gb[c] = (float)gb[c];
+    }
+    const double gm = sqrt(fmax(nga, fmax(ngb, ngc)));
+    f.gmax = g.nn > 0.0 && gm < 1.0e30 ? (float)gm : 3.0e38f;
+    // the inradius is at most half the least height
+    f.rad = !(len >= 1.0e-6 * (1.0 + scale)) ? -1.0f
+                                             : (gm > 0.0 ? __double2float_ru(0.500001 / gm) : __double2float_ru(len));
+    f.iAB = (float)(1.0 / (g.nAB * g.nAB));
+    f.iAC = (float)(1.0 / (g.nCA * g.nCA));
+    f.iBC = (float)(1.0 / (g.nBC * g.nBC));
 }
 
 // -------------------------------------------------------------- kernels
@@ -468,11 +507,13 @@ __device__ int block_exclusive_scan(int v, int* total) {
     return before + x - v;
 }
 
-// per-element count: mode 0 the pnode flag, mode 1 the number of K tetrahedra of the cell
+// per-element count: mode 0 the pnode flag, mode 1 the number of K tetrahedra of the cell,
+// mode 2 the -1 tag, mode 3 the number itself
 template <int MODE>
 __device__ __forceinline__ int scan_count(const void* src, long long l) {
     if (MODE == 0) return static_cast<const int*>(src)[l] ? 1 : 0;
     if (MODE == 2) return static_cast<const int*>(src)[l] < 0 ? 1 : 0;
+    if (MODE == 3) return static_cast<const int*>(src)[l];
     return __popc(static_cast<const unsigned char*>(src)[l]);
 }
 
@@ -505,8 +546,9 @@ __global__ void __launch_bounds__(kThreads) k_scan_top(int ntiles, int* __restri
 }
 
 // mode 0: ids[l] = pnode id + 1 (0: not a pnode), node_of[id] = l;
-// mode 1: tetbase[l] = first K-tetrahedron id of cell l;
-// mode 2: node_of[c] = the c-th node tagged -1
+// mode 1: tetbase[l] = first K-tetrahedron id of cell l, node_of[id] = 8 l + its number 0..5;
+// mode 2: node_of[c] = the c-th node tagged -1;
+// mode 3: out[l] = the sum of the numbers before l, out[n] = that of all
 template <int MODE>
 __global__ void __launch_bounds__(kThreads) k_scan_apply(long long n, const void* __restrict__ src,
                                                          const int* __restrict__ tile_off, int* __restrict__ out,
@@ -526,8 +568,14 @@ __global__ void __launch_bounds__(kThreads) k_scan_apply(long long n, const void
         if (MODE == 0) {
             out[base + q] = c[q] ? off + 1 : 0;
             if (c[q]) node_of[off] = base + q;
-        } else if (MODE == 1) {
+        } else if (MODE == 1 || MODE == 3) {
             out[base + q] = off;
+            if (MODE == 3 && base + q == n - 1) out[n] = off + c[q];
+            if (MODE == 1 && c[q]) {
+                int id = off;
+                for (unsigned m = static_cast<const unsigned char*>(src)[base + q]; m; m &= m - 1)
+                    node_of[id++] = 8 * (base + q) + __ffs(m) - 2;
+            }
         } else if (c[q]) {
             node_of[off] = base + q;
         }
@@ -539,50 +587,45 @@ __global__ void __launch_bounds__(kThreads) k_scan_apply(long long n, const void
 // (src/GetIsosurfaceAndDistances.F90:80-162)
 __global__ void k_geo_tets(DevGrid g, const double* __restrict__ phi, const double* __restrict__ x,
                            const double* __restrict__ y, const double* __restrict__ z,
-                           const unsigned char* __restrict__ cellbits, const int* __restrict__ tetbase,
-                           const int* __restrict__ ids, GeoTet* __restrict__ tets, unsigned* err) {
-    const long long n = (long long)g.ni * g.nj * g.nk;
-    for (long long lc = blockIdx.x * (long long)blockDim.x + threadIdx.x; lc < n;
-         lc += (long long)gridDim.x * blockDim.x) {
-        const unsigned bits = cellbits[lc];
-        if (!bits) continue;
-        int i, j, k;
-        node_ijk(g, lc, &i, &j, &k);
-        int tid = tetbase[lc];
-        for (int t = 0; t < 6; ++t) {
-            if (!(bits >> (t + 1) & 1)) continue;
-            double V[4][3], ph[4];
-            GeoTet T;
+                           int ntet, const long long* __restrict__ tet_of, const int* __restrict__ ids,
+                           GeoTet* __restrict__ tets, TriF* __restrict__ trif, unsigned* err) {
+    for (int tid = blockIdx.x * blockDim.x + threadIdx.x; tid < ntet; tid += gridDim.x * blockDim.x) {
+        const long long lc = tet_of[tid] >> 3;
+        const int t = (int)(tet_of[tid] & 7);
+        double V[4][3], ph[4];
+        GeoTet T;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int cv = c_tets[t][q];
-                const long long l = gid(g, i + c_cell_off[cv][0], j + c_cell_off[cv][1], k + c_cell_off[cv][2]);
-                V[q][0] = x[l]; V[q][1] = y[l]; V[q][2] = z[l];
-                ph[q] = phi[l];
-                T.v[q] = ids[l] - 1;
-            }
-            MT o;
-            marching_full(V, ph, o, true, err);
-            T.nis = o.ntri > 0 ? o.ntri : 0;
-            T.area = o.area;
-            T.wv = o.wv;
-            T.pad = 0;
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-#pragma unroll
-                for (int c = 0; c < 9; ++c) T.tri[q][c] = q < T.nis ? o.tri[q][c / 3][c % 3] : 0.0;
-                tri_geo(T.tri[q], T.tg[q]);
-#pragma unroll
-                for (int c = 0; c < 9; ++c) T.trf[q][c] = (float)T.tri[q][c];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const double a = T.tri[q][c], b = T.tri[q][3 + c], e = T.tri[q][6 + c];
-                    T.box[q][c] = __double2float_rd(fmin(a, fmin(b, e)));
-                    T.box[q][3 + c] = __double2float_ru(fmax(a, fmax(b, e)));
-                }
-            }
-            tets[tid++] = T;
+        for (int q = 0; q < 4; ++q) {
+            const int cv = c_tets[t][q];
+            const long long l = lc + c_cell_off[cv][0] + g.sj * c_cell_off[cv][1] + g.sk * c_cell_off[cv][2];
+            V[q][0] = x[l]; V[q][1] = y[l]; V[q][2] = z[l];
+            ph[q] = phi[l];
+            T.v[q] = ids[l] - 1;
         }
+        MT o;
+        marching_full(V, ph, o, true, err);
+        T.nis = o.ntri > 0 ? o.ntri : 0;
+        T.area = o.area;
+        T.wv = o.wv;
+        T.pad = 0;
+        // (one copy of the triangle code for both triangles)
+#pragma unroll 1
+        for (int q = 0; q < 2; ++q) {
+#pragma unroll
+            for (int c = 0; c < 9; ++c) T.tri[q][c] = q < T.nis ? o.tri[q][c / 3][c % 3] : 0.0;
+            if (q >= T.nis) continue;   // never read
+            tri_geo(T.tri[q], T.tg[q]);
+            TriF f;
+            tri_f32(T.tri[q], T.tg[q], f);
+            trif[2 * (long long)tid + q] = f;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double a = T.tri[q][c], b = T.tri[q][3 + c], e = T.tri[q][6 + c];
+                T.box[q][c] = __double2float_rd(fmin(a, fmin(b, e)));
+                T.box[q][3 + c] = __double2float_ru(fmax(a, fmax(b, e)));
+            }
+        }
+        tets[tid] = T;
     }
 }
 
@@ -602,11 +645,6 @@ __global__ void k_geo_mark(DevGrid g, int npn, const long long* __restrict__ nod
     }
 }
 
-__device__ __forceinline__ float dist3f(const float* a, const float* b) {
-    const float dx = a[0] - b[0], dy = a[1] - b[1], dz = a[2] - b[2];
-    return sqrtf(dx * dx + dy * dy + dz * dz);
-}
-
 // a point in both precisions (the FP32 copy for the culling bounds)
 struct Pt {
     double d[3];
@@ -621,45 +659,23 @@ __device__ __forceinline__ Pt make_pt(double a, double b, double c) {
     return p;
 }
 
-// a running value with its FP32 copy for the culling tests, converted
-// only when the value changes (conversions run on the FP64 pipe)
-struct Run {
-    double d;
-    float f;
-};
-__device__ __forceinline__ void set_run(Run& r, double v) {
-    if (dbits(v) != dbits(r.d)) { r.d = v; r.f = (float)v; }
-}
-
-// the triangles of tetrahedron t against point P (running minimum d); a
-// triangle whose bounding box lies beyond d is not evaluated
-__device__ __forceinline__ void tet_min(const GeoTet* __restrict__ tets, int t, const Pt& P, Run& d) {
-    const GeoTet& T = tets[t];
-    const int nis = T.nis;
-    if (nis > 0 && T.area > 0.0) {
-        for (int q = 0; q < nis; ++q) {
-            if (beyond_box(P.f, P.scale, T.box[q], T.box[q] + 3, d.f)) continue;
-            set_run(d, run_min(d.d, dist_point_triangle(T.tri[q], T.tg[q], P.d)));
-        }
-    }
-}
-
 // per pnode: the bounding box of every triangle of its K tetrahedra
-// (lo.w = 0: none of them has a triangle)
+// (lo.w = 0: none of them has a triangle) and their number
 __global__ void k_geo_prad(DevGrid g, int npn, const long long* __restrict__ node_of,
                            const unsigned char* __restrict__ cellbits, const int* __restrict__ tetbase,
-                           const GeoTet* __restrict__ tets, const double* __restrict__ x,
-                           const double* __restrict__ y, const double* __restrict__ z, float4* __restrict__ pbox) {
+                           const GeoTet* __restrict__ tets, float4* __restrict__ pbox, int* __restrict__ ntri) {
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npn; p += gridDim.x * blockDim.x) {
         int i, j, k;
         node_ijk(g, node_of[p], &i, &j, &k);
         float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
         float any = 0.0f;
+        int nt = 0;
         for_each_tet(g, i, j, k, cellbits, tetbase, [&](int t) {
             const GeoTet& T = tets[t];
             if (T.nis > 0 && T.area > 0.0)
                 for (int q = 0; q < T.nis; ++q) {
                     any = 1.0f;
+                    ++nt;
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
                         lo[c] = fminf(lo[c], T.box[q][c]);
@@ -669,6 +685,35 @@ __global__ void k_geo_prad(DevGrid g, int npn, const long long* __restrict__ nod
         });
         pbox[2 * p] = make_float4(lo[0], lo[1], lo[2], any);
         pbox[2 * p + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+        ntri[p] = nt;
+    }
+}
+
+// The triangles of every pnode in the reference's order, from the entry
+// pstart[p] on: 4 (2 tetrahedron + triangle) + min(2, ends of tetrahedra
+// between this triangle and the next).  lead[p]: min(2, tetrahedra without
+// triangles before the first one).
+__global__ void k_geo_fill(DevGrid g, int npn, const long long* __restrict__ node_of,
+                           const unsigned char* __restrict__ cellbits, const int* __restrict__ tetbase,
+                           const GeoTet* __restrict__ tets, const int* __restrict__ pstart, int* __restrict__ pent,
+                           unsigned char* __restrict__ lead) {
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npn; p += gridDim.x * blockDim.x) {
+        int i, j, k;
+        node_ijk(g, node_of[p], &i, &j, &k);
+        int at = pstart[p] - 1, cur = -1, early = 0;
+        for_each_tet(g, i, j, k, cellbits, tetbase, [&](int t) {
+            const GeoTet& T = tets[t];
+            const int nq = T.nis > 0 && T.area > 0.0 ? T.nis : 0;
+            for (int q = 0; q < nq; ++q) {
+                if (cur >= 0) pent[at] = cur;
+                ++at;
+                cur = 4 * (2 * t + q);
+            }
+            if (cur < 0) early = min(early + 1, 2);
+            else if ((cur & 3) < 2) ++cur;
+        });
+        if (cur >= 0) pent[at] = cur;
+        lead[p] = (unsigned char)early;
     }
 }
 
@@ -680,41 +725,250 @@ __device__ __forceinline__ bool pnode_beyond(int m, const Pt& P, float d, const 
     return beyond_box(P.f, P.scale, lo, hi, d);
 }
 
-// the pnodes' signed distances (src/GetIsosurfaceAndDistances.F90:166-330)
-__global__ void k_geo_sd(DevGrid g, int npn, const long long* __restrict__ node_of, const int* __restrict__ ids,
-                         const unsigned char* __restrict__ cellbits, const int* __restrict__ tetbase,
-                         const GeoTet* __restrict__ tets, const float4* __restrict__ prad,
-                         const double* __restrict__ phi, const double* __restrict__ x,
-                         const double* __restrict__ y, const double* __restrict__ z, double* __restrict__ sd_out) {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npn; p += gridDim.x * blockDim.x) {
+// ------------------------------------------------- the distance chains
+//
+// Both distance loops are chains a <- a + (c - a) where c <= a, over the
+// distances c of a node to the triangles of the pnodes in its +-4 box, in
+// the reference's order.  Two facts make most of them unnecessary:
+//   - a distance that is certainly above the running value changes nothing;
+//   - for a/2 <= c <= a the update gives exactly c (c - a is exact), whatever
+//     a was: what came before such a c is forgotten.
+// A warp encloses the distances of each pnode's triangles in FP32 (one
+// triangle per lane) and keeps, as tasks, only the triangles that can still
+// decide the final bits: a pnode that certainly falls below everything
+// before it, by less than a factor 2, drops all earlier tasks; a pnode
+// certainly above adds none; one in between adds its triangles near the
+// minimum; one that falls by a factor 2 or more adds all of its triangles.
+// The lanes then evaluate the tasks in FP64 together and the chain is
+// replayed over them in order.  The FP64 pipe (16 clocks per warp operation
+// and SM) evaluated a few hundred distances per node before, of ~150
+// operations each; now some ten.
+constexpr int kMaxTri = 48;           // triangles of a pnode: two in each of at most 24 tetrahedra
+constexpr int kTasks = 2 * kMaxTri + 32, kItems = 32;
+constexpr int kChainWarps = 4;
+enum : int { kSimple = 0, kReset = 1, kFull = 2 };
+
+struct ChainQueue {
+    double d[kTasks];
+    int ent[kTasks];                  // entries of pent
+    int item[kItems];                 // one per pnode: 4 (tasks before it) + kind
+    int aux[kItems];                  // 4 (pnode's ordinal in the box; or 1: the first task restarts dp) + lead
+};
+
+// Encloses the reference's distance of P to a triangle (dist_point_triangle).
+// E covers the FP32 rounding of the coordinates and of the operations, tau
+// that of alpha and beta.  The value is the least of the distances to the
+// edges and, inside the triangle, of the one to the reference's projection;
+// any point it can take lies in the triangle.
+__device__ __forceinline__ void tri_interval(const TriF* __restrict__ trif, const GeoTet* __restrict__ tets, int tri,
+                                             const Pt& P, float& lo, float& hi) {
+    const float4* r = reinterpret_cast<const float4*>(trif + tri);
+    const float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2), u = __ldg(r + 3), v = __ldg(r + 4);
+    const float px = P.f[0] - a.x, py = P.f[1] - a.y, pz = P.f[2] - a.z;
+    if (a.w < 0.0f) {
+        const float* box = tets[tri >> 1].box[tri & 1];
+        const float dx = fmaxf(fmaxf(box[0] - P.f[0], P.f[0] - box[3]), 0.0f);
+        const float dy = fmaxf(fmaxf(box[1] - P.f[1], P.f[1] - box[4]), 0.0f);
+        const float dz = fmaxf(fmaxf(box[2] - P.f[2], P.f[2] - box[5]), 0.0f);
+        lo = fmaxf(0.0f, 0.99997f * sqrtf(dx * dx + dy * dy + dz * dz) - 1.1e-5f * P.scale);
+        hi = 3.0e38f;
+        return;
+    }
+    auto seg = [](float x, float y, float z, float ex, float ey, float ez, float inv) {
+        const float t = fminf(fmaxf((x * ex + y * ey + z * ez) * inv, 0.0f), 1.0f);
+        const float rx = x - t * ex, ry = y - t * ey, rz = z - t * ez;
+        return rx * rx + ry * ry + rz * rz;
+    };
+    const float s2 = fminf(fminf(seg(px, py, pz, b.x, b.y, b.z, b.w), seg(px, py, pz, c.x, c.y, c.z, c.w)),
+                           seg(px - b.x, py - b.y, pz - b.z, c.x - b.x, c.y - b.y, c.z - b.z, u.w));
+    const float s = sqrtf(s2), E = 2.0e-6f * (P.scale + s) + 1.0e-12f;
+    hi = s + E;
+    lo = s - E;
+    const float al = px * u.x + py * u.y + pz * u.z, be = px * v.x + py * v.y + pz * v.z, ga = 1.0f - be - al;
+    const float tau = v.w * 1.0e-6f * (P.scale + fabsf(px) + fabsf(py) + fabsf(pz));
+    if (tau < 0.25f) {
+        const float m = fminf(al, fminf(be, ga));
+        if (m > -2.0f * tau) {
+            const float wx = px - be * b.x - ga * c.x, wy = py - be * b.y - ga * c.y, wz = pz - be * b.z - ga * c.z;
+            const float d = sqrtf(wx * wx + wy * wy + wz * wz);
+            const float e = E + 4.0f * tau * rsqrtf(fminf(b.w, c.w));
+            lo = fminf(lo, d - e);
+            if (m > 2.0f * tau) hi = fminf(hi, d + e);
+        }
+    } else {
+        lo -= a.w;   // within the inradius of an edge
+    }
+    lo = fmaxf(lo, 0.0f);
+}
+
+__device__ __forceinline__ float warp_min(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// FP32 enclosures of up to 48 triangles of a pnode: entry `lane` and `lane +
+// 32`, infinite beyond the list
+struct Encl {
+    int e0, e1;            // entries of pent
+    float lo0, hi0, lo1, hi1, lo, hi;   // and the least of each over the warp
+};
+__device__ __forceinline__ Encl enclose(const TriF* __restrict__ trif, const GeoTet* __restrict__ tets,
+                                        const int* __restrict__ pent, int s, int n, const Pt& P, int lane) {
+    Encl c;
+    c.e0 = c.e1 = 0;
+    c.lo0 = c.hi0 = c.lo1 = c.hi1 = 3.0e38f;
+    if (lane < n) {
+        c.e0 = __ldg(pent + s + lane);
+        tri_interval(trif, tets, c.e0 >> 2, P, c.lo0, c.hi0);
+    }
+    if (lane + 32 < n) {
+        c.e1 = __ldg(pent + s + 32 + lane);
+        tri_interval(trif, tets, c.e1 >> 2, P, c.lo1, c.hi1);
+    }
+    c.lo = warp_min(fminf(c.lo0, c.lo1));
+    c.hi = warp_min(fminf(c.hi0, c.hi1));
+    return c;
+}
+
+// whether a triangle bounded by its box alone can lie below v
+__device__ __forceinline__ bool box_only_near(const Encl& c, float v) {
+    return __any_sync(0xffffffffu, (c.hi0 > 1.0e38f && c.lo0 <= v) || (c.hi1 > 1.0e38f && c.lo1 <= v));
+}
+
+// appends the entries chosen by t0 / t1 in order; returns the new task count
+__device__ __forceinline__ int push_tasks(ChainQueue& Q, int nt, const Encl& c, bool t0, bool t1, int lane) {
+    const unsigned m0 = __ballot_sync(0xffffffffu, t0), m1 = __ballot_sync(0xffffffffu, t1);
+    const unsigned below = (1u << lane) - 1u;
+    if (t0) Q.ent[nt + __popc(m0 & below)] = c.e0;
+    if (t1) Q.ent[nt + __popc(m0) + __popc(m1 & below)] = c.e1;
+    return nt + __popc(m0) + __popc(m1);
+}
+
+__device__ __forceinline__ void eval_tasks(ChainQueue& Q, int nt, const GeoTet* __restrict__ tets, const Pt& P,
+                                           int lane) {
+    __syncwarp();
+    for (int q = lane; q < nt; q += 32) {
+        const int tri = Q.ent[q] >> 2;
+        const GeoTet& T = tets[tri >> 1];
+        Q.d[q] = dist_point_triangle(T.tri[tri & 1], T.tg[tri & 1], P.d);
+    }
+    __syncwarp();
+}
+
+// the +-4 box of a node, walked in k, j, i order 32 positions at a time
+struct Box9 {
+    int i0, j0, k0, ni, nj, n;
+    __device__ __forceinline__ Box9(const DevGrid& g, int i, int j, int k) {
+        i0 = max(i - 4, 0); j0 = max(j - 4, 0); k0 = max(k - 4, 0);
+        ni = min(i + 4, g.ni - 1) - i0 + 1;
+        nj = min(j + 4, g.nj - 1) - j0 + 1;
+        n = ni * nj * (min(k + 4, g.nk - 1) - k0 + 1);
+    }
+    __device__ __forceinline__ long long node(const DevGrid& g, int q) const {
+        const int r = q / ni;
+        return gid(g, i0 + q - r * ni, j0 + r % nj, k0 + r / nj);
+    }
+};
+
+// the pnodes' signed distances (src/GetIsosurfaceAndDistances.F90:166-330):
+// a running minimum dp (from 10) over the triangles of the box's pnodes and,
+// after each tetrahedron, sd <- sd + (dp - sd) where dp <= sd (from 99.9).
+// In kSimple and kReset pnodes every update is exact, so dp is the least
+// distance and sd follows it.  One more step after a kFull pnode brings sd
+// to rest; it is made when another pnode (which has at least one
+// tetrahedron) follows.
+__global__ void __launch_bounds__(32 * kChainWarps) k_geo_sd(
+        DevGrid g, int npn, const long long* __restrict__ node_of, const int* __restrict__ ids,
+        const GeoTet* __restrict__ tets, const TriF* __restrict__ trif, const int* __restrict__ pstart,
+        const int* __restrict__ pent, const unsigned char* __restrict__ lead, const float4* __restrict__ prad,
+        const double* __restrict__ phi, const double* __restrict__ x, const double* __restrict__ y,
+        const double* __restrict__ z, double* __restrict__ sd_out) {
+    __shared__ ChainQueue qs[kChainWarps];
+    ChainQueue& Q = qs[threadIdx.x >> 5];
+    const unsigned FM = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    for (int p = blockIdx.x * kChainWarps + (threadIdx.x >> 5); p < npn; p += gridDim.x * kChainWarps) {
         const long long l0 = node_of[p];
         int i, j, k;
         node_ijk(g, l0, &i, &j, &k);
         const Pt P = make_pt(x[l0], y[l0], z[l0]);
-        const double s = sgn1(phi[l0]);
-        Run dp{10.0, 10.0f};
-        double sd = 99.9;
-        auto sd_step = [&]() {
-            // sd = |sd| + exsign2 (dp - |sd|), then sign(one, phi) * sd
-            sd = copysign(mag_step(fabs(sd), dp.d), s);
-        };
-        for (int ks = max(k - 4, 0); ks <= min(k + 4, g.nk - 1); ++ks)
-            for (int js = max(j - 4, 0); js <= min(j + 4, g.nj - 1); ++js)
-                for (int is = max(i - 4, 0); is <= min(i + 4, g.ni - 1); ++is) {
-                    const int m = ids[gid(g, is, js, ks)] - 1;
-                    if (m < 0) continue;
-                    // every triangle of this pnode beyond dp: dp stays, the
-                    // signed distance update still runs once per tetrahedron
-                    if (pnode_beyond(m, P, dp.f, prad)) {
-                        for_each_tet(g, is, js, ks, cellbits, tetbase, [&](int) { sd_step(); });
-                        continue;
+        const Box9 box(g, i, j, k);
+        double dp = 10.0, sd = 99.9;          // exact state before the first queued pnode (kReset: replaced)
+        float slo = 9.9f, shi = 100.0f;       // dp and sd after the last queued one lie between
+        float dhi = 10.0f;                    // dp does not exceed
+        int nt = 0, nitem = 0, ord = 0;
+        int rest = -1;                        // ordinal of a kFull pnode (or the start) after which sd may not rest
+        auto flush = [&]() {
+            eval_tasks(Q, nt, tets, P, lane);
+            for (int it = 0; it < nitem; ++it) {
+                const int t0 = Q.item[it] >> 2, kind = Q.item[it] & 3;
+                const int t1 = it + 1 < nitem ? Q.item[it + 1] >> 2 : nt;
+                const int o = Q.aux[it] >> 2;
+                if (kind == kFull) {
+                    if (rest > -2 && o - rest > 1) sd = mag_step(sd, dp);
+                    if (Q.aux[it] & 3) sd = mag_step(sd, dp);
+                    for (int q = t0; q < t1; ++q) {
+                        const int e = Q.ent[q];
+                        const float* bx = tets[e >> 3].box[(e >> 2) & 1];
+                        if (!beyond_box(P.f, P.scale, bx, bx + 3, (float)dp)) dp = run_min(dp, Q.d[q]);
+                        for (int st = e & 3; st > 0; --st) sd = mag_step(sd, dp);
                     }
-                    for_each_tet(g, is, js, ks, cellbits, tetbase, [&](int t) {
-                        tet_min(tets, t, P, dp);
-                        sd_step();
-                    });
+                    rest = o;
+                } else {
+                    if (rest > -2) sd = mag_step(sd, dp);   // its first tetrahedron, or a pnode between
+                    rest = -2;
+                    double m = Q.d[t0];
+                    for (int q = t0 + 1; q < t1; ++q) m = dmin(m, Q.d[q]);
+                    if (kind == kReset) {
+                        dp = sd = m;
+                    } else {
+                        dp = dmin(dp, m);
+                        sd = dmin(sd, dp);
+                    }
                 }
-        sd_out[p] = sd;
+            }
+            nt = nitem = 0;
+            slo = 0.999999f * (float)fmin(dp, sd);
+            shi = 1.000001f * (float)fmax(dp, sd);
+            dhi = 1.000001f * (float)dp;
+            __syncwarp();
+        };
+        for (int q0 = 0; q0 < box.n; q0 += 32) {
+            const int q = q0 + lane;
+            const int m0 = q < box.n ? ids[box.node(g, q)] - 1 : -1;
+            const unsigned all = __ballot_sync(FM, m0 >= 0);
+            unsigned near = __ballot_sync(FM, m0 >= 0 && !pnode_beyond(m0, P, dhi, prad));
+            while (near) {
+                const int b = __ffs(near) - 1;
+                near &= near - 1;
+                const int m = __shfl_sync(FM, m0, b);
+                if (pnode_beyond(m, P, dhi, prad)) continue;
+                const int s = pstart[m], n = pstart[m + 1] - s, o = ord + __popc(all & ((1u << b) - 1u));
+                Encl c = enclose(trif, tets, pent, s, n, P, lane);
+                if (c.lo > dhi) continue;
+                if (nt > kTasks - kMaxTri || nitem == kItems) flush();
+                const bool exact = c.lo >= 0.50001f * shi && !box_only_near(c, dhi);
+                const int kind = !exact ? kFull : (c.hi < slo ? kReset : kSimple);
+                if (kind == kReset) nt = nitem = 0;
+                const float near_min = kind == kFull ? 3.0e38f : fminf(c.hi, dhi);
+                if (lane == 0) {
+                    Q.item[nitem] = 4 * nt + kind;
+                    Q.aux[nitem] = 4 * o + lead[m];
+                }
+                ++nitem;
+                nt = push_tasks(Q, nt, c, lane < n && c.lo0 <= near_min, lane + 32 < n && c.lo1 <= near_min, lane);
+                // (kFull: the roundings of dp = 10 + (c - 10) and of sd stay below 1e-12)
+                const bool below = c.hi < slo;
+                slo = 0.999999f * (below ? c.lo : fminf(slo, c.lo)) - 1.0e-12f;
+                shi = 1.000001f * fminf(shi, c.hi) + 1.0e-12f;
+                dhi = 1.000001f * fminf(dhi, c.hi) + 1.0e-12f;
+            }
+            ord += __popc(all);
+        }
+        flush();
+        if (rest > -2 && ord - 1 > rest) sd = mag_step(sd, dp);
+        if (lane == 0) sd_out[p] = copysign(sd, sgn1(phi[l0]));
     }
 }
 
@@ -853,146 +1107,122 @@ __global__ void k_geo_pnode_phi(int npn, const long long* __restrict__ node_of, 
     }
 }
 
-// NeighboursPhiCorrection on the -1 nodes (src/NeighboursPhiCorrection.F90:186-343).
-//
-// One warp per node.  The node's result is a sequential chain over the
-// pnodes of its +-4 box, in the reference's order: per pnode a running
-// minimum dp over the triangles of its K tetrahedra (reset to 10), and
-// after each tetrahedron |v| <- |v| + exsign2 (dp - |v|).  Its last bits
-// depend on that order, so the chain itself runs in order, uniformly on
-// all lanes; what the lanes share out is the FP64 work inside it, the
-// point-triangle distances.  Pnodes that can still change v (the same tests
-// as the chain: the box of all their triangles, then the triangles' own
-// boxes, against the current |v|) are queued with their tetrahedra and
-// triangles; once the queue holds a lane-full of triangles, the lanes
-// evaluate all of them, and the chain is replayed over the queued pnodes,
-// each test made again with the v of that moment.  v only decreases, so a
-// pnode skipped when queued would be skipped in the chain too; one queued
-// but skipped in the replay, or a triangle culled there by the running
-// minimum, only cost a wasted evaluation.  Every value the replay uses is
-// the one the sequential chain computes.
-constexpr int kQN = 16;    // queued pnodes
-constexpr int kQT = 160;   // queued tetrahedra
-constexpr int kQP = 96;    // queued triangles
-constexpr int kQFlush = 32;
-
-struct NeighQueue {
-    int nn, nt, np;
-    int nm[kQN];           // pnode ids
-    int nstart[kQN + 1];   // first tetrahedron slot of each queued pnode
-    int tet[kQT];          // tetrahedron ids, in order
-    int tp[kQT + 1];       // first triangle slot of each tetrahedron slot
-    int ptet[kQP];         // triangle slot -> tetrahedron id
-    unsigned char pq[kQP]; // triangle slot -> triangle 0/1 of that tetrahedron
-    double da[kQP];        // the distances
-};
-
-constexpr int kNeighWarps = 4;
-
-__global__ void __launch_bounds__(32 * kNeighWarps) k_geo_neigh(
-        DevGrid g, const int* __restrict__ ids, const unsigned char* __restrict__ cellbits,
-        const int* __restrict__ tetbase, const GeoTet* __restrict__ tets, const float4* __restrict__ prad,
-        const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
-        double* __restrict__ pc, int nsec, const long long* __restrict__ second) {
-    __shared__ NeighQueue qs[kNeighWarps];
-    NeighQueue& Q = qs[threadIdx.x >> 5];
+// NeighboursPhiCorrection on the -1 nodes (src/NeighboursPhiCorrection.F90:
+// 186-343): per pnode of the box a running minimum dp over its triangles,
+// starting at 10 again, and after each of its tetrahedra |v| <- |v| + (dp -
+// |v|) where dp <= |v|.  In kSimple and kReset pnodes every update of |v| is
+// exact, so |v| becomes the pnode's last dp where that is lower; its last
+// dp follows from the last triangle that certainly falls below the pnode's
+// earlier ones by less than a factor 2, and the later ones near it.
+__global__ void __launch_bounds__(32 * kChainWarps) k_geo_neigh(
+        DevGrid g, const int* __restrict__ ids, const GeoTet* __restrict__ tets, const TriF* __restrict__ trif,
+        const int* __restrict__ pstart, const int* __restrict__ pent, const unsigned char* __restrict__ lead,
+        const float4* __restrict__ prad, const double* __restrict__ x, const double* __restrict__ y,
+        const double* __restrict__ z, double* __restrict__ pc, int nsec, const long long* __restrict__ second) {
+    __shared__ ChainQueue qs[kChainWarps];
+    ChainQueue& Q = qs[threadIdx.x >> 5];
+    const unsigned FM = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const int nwarps = gridDim.x * kNeighWarps;
-    for (int c = blockIdx.x * kNeighWarps + (threadIdx.x >> 5); c < nsec; c += nwarps) {
-        const long long l0 = second[c];
+    for (int c0 = blockIdx.x * kChainWarps + (threadIdx.x >> 5); c0 < nsec; c0 += gridDim.x * kChainWarps) {
+        const long long l0 = second[c0];
         int i, j, k;
         node_ijk(g, l0, &i, &j, &k);
         const Pt P = make_pt(x[l0], y[l0], z[l0]);
-        double v = pc[l0];
-        float vf = (float)fabs(v);   // |v| in FP32 for the culling tests
-        int nn = 0, nt = 0, np = 0;  // uniform copies of the queue sizes
-
-        // the triangles of queued pnode slot n all beyond af (pnode box first)
-        auto all_beyond = [&](int n, float af) -> bool {
-            if (pnode_beyond(Q.nm[n], P, af, prad)) return true;
-            for (int s2 = Q.nstart[n]; s2 < Q.nstart[n + 1]; ++s2)
-                for (int p = Q.tp[s2]; p < Q.tp[s2 + 1]; ++p) {
-                    const GeoTet& T = tets[Q.ptet[p]];
-                    if (!beyond_box(P.f, P.scale, T.box[Q.pq[p]], T.box[Q.pq[p]] + 3, af)) return false;
-                }
-            return true;
+        const Box9 box(g, i, j, k);
+        const double v0 = pc[l0];
+        double av = fabs(v0);                 // exact |v| before the first queued pnode (kReset: replaced)
+        float vlo, vhi;                       // |v| after the last queued one lies between
+        int nt = 0, nitem = 0;
+        auto bounds = [&]() {
+            vlo = 0.999999f * (float)av;
+            vhi = 1.000001f * (float)av;
         };
+        bounds();
         auto flush = [&]() {
-            __syncwarp();
-            for (int p = lane; p < np; p += 32) {
-                const GeoTet& T = tets[Q.ptet[p]];
-                const int q = Q.pq[p];
-                Q.da[p] = dist_point_triangle(T.tri[q], T.tg[q], P.d);
-            }
-            __syncwarp();
-            for (int n = 0; n < nn; ++n) {
-                if (all_beyond(n, vf)) continue;
-                Run dp{10.0, 10.0f};
-                for (int s2 = Q.nstart[n]; s2 < Q.nstart[n + 1]; ++s2) {
-                    for (int p = Q.tp[s2]; p < Q.tp[s2 + 1]; ++p) {
-                        const GeoTet& T = tets[Q.ptet[p]];
-                        if (beyond_box(P.f, P.scale, T.box[Q.pq[p]], T.box[Q.pq[p]] + 3, dp.f)) continue;
-                        set_run(dp, run_min(dp.d, Q.da[p]));
+            eval_tasks(Q, nt, tets, P, lane);
+            for (int it = 0; it < nitem; ++it) {
+                const int t0 = Q.item[it] >> 2, kind = Q.item[it] & 3;
+                const int t1 = it + 1 < nitem ? Q.item[it + 1] >> 2 : nt;
+                double dp = 10.0;
+                if (kind == kFull) {
+                    for (int st = Q.aux[it] & 3; st > 0; --st) av = mag_step(av, dp);
+                    for (int q = t0; q < t1; ++q) {
+                        const int e = Q.ent[q];
+                        const float* bx = tets[e >> 3].box[(e >> 2) & 1];
+                        if (!beyond_box(P.f, P.scale, bx, bx + 3, (float)dp)) dp = run_min(dp, Q.d[q]);
+                        for (int st = e & 3; st > 0; --st) av = mag_step(av, dp);
                     }
-                    // |v| + exsign2 (dp - |v|), with the sign of v
-                    const double av = fabs(v), nv2 = mag_step(av, dp.d);
-                    if (dbits(nv2) != dbits(av)) vf = (float)nv2;
-                    v = copysign(nv2, v);
+                } else {
+                    dp = Q.aux[it] >> 2 ? Q.d[t0] : run_min(dp, Q.d[t0]);
+                    for (int q = t0 + 1; q < t1; ++q) dp = run_min(dp, Q.d[q]);
+                    av = kind == kReset ? dp : dmin(av, dp);
                 }
             }
+            nt = nitem = 0;
+            bounds();
             __syncwarp();
-            nn = nt = np = 0;
         };
-
-        for (int ks = max(k - 4, 0); ks <= min(k + 4, g.nk - 1); ++ks)
-            for (int js = max(j - 4, 0); js <= min(j + 4, g.nj - 1); ++js)
-                for (int is = max(i - 4, 0); is <= min(i + 4, g.ni - 1); ++is) {
-                    const int m = ids[gid(g, is, js, ks)] - 1;
-                    if (m < 0) continue;
-                    if (pnode_beyond(m, P, vf, prad)) continue;
-                    if (nn == kQN || nt > kQT - 24 || np > kQP - 48) flush();
-                    // queue the pnode's tetrahedra and triangles (every lane
-                    // writes the same values).  A triangle is left out when
-                    // the chain will cull it for sure: ub bounds the
-                    // running minimum from above (the reference's distance is
-                    // at most the distance to each vertex, here in FP32
-                    // with a margin, and whether an earlier triangle is
-                    // evaluated or culled the minimum stays below it), and
-                    // the cull test only gets stricter as the minimum falls.
-                    Q.nm[nn] = m;
-                    Q.nstart[nn] = nt;
-                    float ub = 10.0f;
-                    for_each_tet(g, is, js, ks, cellbits, tetbase, [&](int t) {
-                        const GeoTet& T = tets[t];
-                        const int ntri = (T.nis > 0 && T.area > 0.0) ? T.nis : 0;
-                        Q.tet[nt] = t;
-                        Q.tp[nt] = np;
-                        for (int q = 0; q < ntri; ++q) {
-                            if (!beyond_box(P.f, P.scale, T.box[q], T.box[q] + 3, ub)) {
-                                Q.ptet[np] = t;
-                                Q.pq[np] = (unsigned char)q;
-                                ++np;
-                            }
-                            float u = fminf(dist3f(P.f, T.trf[q]), fminf(dist3f(P.f, T.trf[q] + 3),
-                                                                           dist3f(P.f, T.trf[q] + 6)));
-                            u = u + 1.0e-5f * (u + P.scale) + 1.0e-30f;
-                            ub = fminf(ub, u);
+        for (int q0 = 0; q0 < box.n; q0 += 32) {
+            const int q = q0 + lane;
+            const int m0 = q < box.n ? ids[box.node(g, q)] - 1 : -1;
+            // a |v| of 10 or more follows dp = 10 after any tetrahedron
+            unsigned near = __ballot_sync(FM, m0 >= 0 && (vhi >= 9.9999f || !pnode_beyond(m0, P, vhi, prad)));
+            while (near) {
+                const int b = __ffs(near) - 1;
+                near &= near - 1;
+                const int m = __shfl_sync(FM, m0, b);
+                if (vhi < 9.9999f && pnode_beyond(m, P, vhi, prad)) continue;
+                const int s = pstart[m], n = pstart[m + 1] - s;
+                Encl c = enclose(trif, tets, pent, s, n, P, lane);
+                if (c.lo > vhi && vhi < 9.9999f) continue;
+                if (nt > kTasks - kMaxTri || nitem == kItems) flush();
+                // the steps with dp = 10 before the first triangle change no |v| below 10
+                const bool exact = c.lo >= 0.50001f * vhi && vhi < 9.9999f && !box_only_near(c, vhi);
+                const int kind = !exact ? kFull : (c.hi < vlo ? kReset : kSimple);
+                if (kind == kReset) nt = nitem = 0;
+                bool t0 = lane < n, t1 = lane + 32 < n;
+                int from = 0;
+                if (kind != kFull) {
+                    // least bounds of the earlier triangles of the pnode
+                    float ml = c.lo0, mh = c.hi0, nl = c.lo1, nh = c.hi1;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const float a = __shfl_up_sync(FM, ml, o), h = __shfl_up_sync(FM, mh, o);
+                        const float a1 = __shfl_up_sync(FM, nl, o), h1 = __shfl_up_sync(FM, nh, o);
+                        if (lane >= o) {
+                            ml = fminf(ml, a); mh = fminf(mh, h);
+                            nl = fminf(nl, a1); nh = fminf(nh, h1);
                         }
-                        ++nt;
-                    });
-                    Q.tp[nt] = np;
-                    Q.nstart[nn + 1] = nt;
-                    __syncwarp();
-                    if (all_beyond(nn, vf)) {  // not near: drop it again
-                        nt = Q.nstart[nn];
-                        np = Q.tp[nt];
-                        continue;
                     }
-                    ++nn;
-                    if (np >= kQFlush) flush();
+                    const float l31 = __shfl_sync(FM, ml, 31), h31 = __shfl_sync(FM, mh, 31);
+                    ml = __shfl_up_sync(FM, ml, 1); mh = __shfl_up_sync(FM, mh, 1);
+                    nl = __shfl_up_sync(FM, nl, 1); nh = __shfl_up_sync(FM, nh, 1);
+                    if (lane == 0) { ml = mh = nl = nh = 3.0e38f; }
+                    nl = fminf(nl, l31);
+                    nh = fminf(nh, h31);
+                    const unsigned r0 = __ballot_sync(FM, t0 && lane > 0 && c.hi0 < ml && c.lo0 >= 0.50001f * mh);
+                    const unsigned r1 = __ballot_sync(FM, t1 && c.hi1 < nl && c.lo1 >= 0.50001f * nh);
+                    from = r1 ? 63 - __clz(r1) : (r0 ? 31 - __clz(r0) : 0);
+                    t0 = t0 && (lane == from || (lane > from && c.lo0 <= mh));
+                    t1 = t1 && (lane + 32 == from || (lane + 32 > from && c.lo1 <= nh));
                 }
-        if (nn) flush();
-        if (lane == 0) pc[l0] = v;
+                if (lane == 0) {
+                    Q.item[nitem] = 4 * nt + kind;
+                    Q.aux[nitem] = (from > 0 ? 4 : 0) + lead[m];
+                }
+                ++nitem;
+                nt = push_tasks(Q, nt, c, t0, t1, lane);
+                if (vhi >= 9.9999f) {
+                    flush();   // exact again at once: rare
+                } else {
+                    // (kFull: the rounding of dp = 10 + (c - 10) stays below 1e-12)
+                    vlo = 0.999999f * (c.hi < vlo ? c.lo : fminf(vlo, c.lo)) - 1.0e-12f;
+                    vhi = 1.000001f * fminf(vhi, c.hi) + 1.0e-12f;
+                }
+            }
+        }
+        flush();
+        if (lane == 0) pc[l0] = copysign(av, v0);
     }
 }
 
@@ -1070,7 +1300,6 @@ cudaError_t geo_reinit(const DevGrid& g, const double* phi0, const double* x, co
         // 3. K-tetrahedra ids per cell
         k_scan_tiles<1><<<ntiles, kThreads, 0, s>>>(n, cellbits, tiles);
         k_scan_top<<<1, kThreads, 0, s>>>(ntiles, tiles, d_count + 1);
-        k_scan_apply<1><<<ntiles, kThreads, 0, s>>>(n, cellbits, tiles, tetbase, nullptr);
         GEO_CU(cudaGetLastError());
     }
     GEO_CU(cudaMemcpyAsync(&counts[1], d_count + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1086,15 +1315,29 @@ cudaError_t geo_reinit(const DevGrid& g, const double* phi0, const double* x, co
     if (npn == 0) return cudaSuccess;
     auto* tets = static_cast<GeoTet*>(alloc(actx, "geo_tets", sizeof(GeoTet) * (size_t)(ntet + 1), &e));
     GEO_CU(e);
+    auto* tet_of = static_cast<long long*>(alloc(actx, "geo_tet_of", 8 * (size_t)(ntet + 1), &e));
+    GEO_CU(e);
     auto* sd = static_cast<double*>(alloc(actx, "geo_sd", 8 * (size_t)npn, &e));
     GEO_CU(e);
     auto* xi = static_cast<double*>(alloc(actx, "geo_xi", 8 * (size_t)npn, &e));
     GEO_CU(e);
     auto* prad = static_cast<float4*>(alloc(actx, "geo_prad", 32 * (size_t)npn, &e));
     GEO_CU(e);
+    auto* trif = static_cast<TriF*>(alloc(actx, "geo_trif", sizeof(TriF) * 2 * (size_t)(ntet + 1), &e));
+    GEO_CU(e);
+    // a triangle is listed by the four pnodes of its tetrahedron
+    auto* pent = static_cast<int*>(alloc(actx, "geo_pent", 4 * 8 * (size_t)(ntet + 1), &e));
+    GEO_CU(e);
+    auto* ntri = static_cast<int*>(alloc(actx, "geo_ntri", 4 * (size_t)npn, &e));
+    GEO_CU(e);
+    auto* pstart = static_cast<int*>(alloc(actx, "geo_pstart", 4 * (size_t)(npn + 1), &e));
+    GEO_CU(e);
+    auto* lead = static_cast<unsigned char*>(alloc(actx, "geo_lead", (size_t)npn, &e));
+    GEO_CU(e);
     {
         ProfScope ps("k_geo_tets", s);
-        k_geo_tets<<<grid_for(n), kThreads, 0, s>>>(g, phi0, x, y, z, cellbits, tetbase, ids, tets, d_err);
+        k_scan_apply<1><<<ntiles, kThreads, 0, s>>>(n, cellbits, tiles, tetbase, tet_of);
+        k_geo_tets<<<grid_for(ntet, 64), 64, 0, s>>>(g, phi0, x, y, z, ntet, tet_of, ids, tets, trif, d_err);
         GEO_CU(cudaGetLastError());
     }
     {
@@ -1104,13 +1347,22 @@ cudaError_t geo_reinit(const DevGrid& g, const double* phi0, const double* x, co
     }
     {
         ProfScope ps("k_geo_prad", s);
-        k_geo_prad<<<grid_for(npn), kThreads, 0, s>>>(g, npn, node_of, cellbits, tetbase, tets, x, y, z, prad);
+        k_geo_prad<<<grid_for(npn), kThreads, 0, s>>>(g, npn, node_of, cellbits, tetbase, tets, prad, ntri);
+        GEO_CU(cudaGetLastError());
+    }
+    {
+        ProfScope ps("k_geo_fill", s);
+        const int pt = (npn + kTile - 1) / kTile;
+        k_scan_tiles<3><<<pt, kThreads, 0, s>>>(npn, ntri, tiles);
+        k_scan_top<<<1, kThreads, 0, s>>>(pt, tiles, d_count + 3);
+        k_scan_apply<3><<<pt, kThreads, 0, s>>>(npn, ntri, tiles, pstart, nullptr);
+        k_geo_fill<<<grid_for(npn), kThreads, 0, s>>>(g, npn, node_of, cellbits, tetbase, tets, pstart, pent, lead);
         GEO_CU(cudaGetLastError());
     }
     {
         ProfScope ps("k_geo_sd", s);
-        k_geo_sd<<<grid_for(npn), 128, 0, s>>>(g, npn, node_of, ids, cellbits, tetbase, tets, prad, phi0, x, y, z,
-                                               sd);
+        k_geo_sd<<<grid_for(npn, kChainWarps), 32 * kChainWarps, 0, s>>>(g, npn, node_of, ids, tets, trif, pstart, pent,
+                                                                        lead, prad, phi0, x, y, z, sd);
         GEO_CU(cudaGetLastError());
     }
     GEO_CU(cudaMemsetAsync(xi, 0, 8 * (size_t)npn, s));
@@ -1180,8 +1432,8 @@ cudaError_t geo_reinit(const DevGrid& g, const double* phi0, const double* x, co
     }
     {
         ProfScope ps("k_geo_neigh", s);
-        k_geo_neigh<<<grid_for(ns, kNeighWarps), 32 * kNeighWarps, 0, s>>>(g, ids, cellbits, tetbase, tets, prad, x,
-                                                                            y, z, pc, ns, second);
+        k_geo_neigh<<<grid_for(ns, kChainWarps), 32 * kChainWarps, 0, s>>>(g, ids, tets, trif, pstart, pent, lead, prad,
+                                                                           x, y, z, pc, ns, second);
         GEO_CU(cudaGetLastError());
     }
     GEO_CU(cudaStreamSynchronize(s));
