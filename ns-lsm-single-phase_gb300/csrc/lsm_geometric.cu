@@ -194,6 +194,15 @@ __device__ void marching_full(const double (&V)[4][3], const double (&ph)[4], MT
     o.wv = water_volume<true>(V, E, fi, err);
 }
 
+// norm2v and sdiv as calls: the distance code keeps to a few kB, so that the
+// warps of an SM do not wait for instructions
+__device__ __noinline__ double norm2c(double x, double y, double z) {
+    const double a[3] = {x, y, z};
+    return norm2v(a);
+}
+__device__ __forceinline__ double norm2f(const double* a) { return norm2c(a[0], a[1], a[2]); }
+__device__ __noinline__ double quot(double a, double b) { return sdiv(a, b); }
+
 // DistancePointLine, src/TetrahedronMethods.F90:1356-1399, given the
 // vectors and norms the caller already has: AP = P - A, BP = P - B,
 // AB = B - A and their norms (BA = A - B is -AB exactly)
@@ -207,7 +216,7 @@ __device__ __forceinline__ double dist_point_line(const double* AP, const double
     if (valid) {
         double c[3];
         cross3g(AP, BP, c);
-        return sdiv(norm2v(c), nAB);
+        return quot(norm2f(c), nAB);
     }
     return dmin(nAP, nBP);
 }
@@ -247,7 +256,7 @@ __device__ double dist_point_triangle(const double* T, const TriGeo& g, const do
     const double* Cv = T + 6;
     double PA[3], PB[3], PC[3];
     sub3(P, A, PA); sub3(P, B, PB); sub3(P, Cv, PC);
-    const double nA = norm2v(PA), nB = norm2v(PB), nC = norm2v(PC);
+    const double nA = norm2f(PA), nB = norm2f(PB), nC = norm2f(PC);
     double m = dmin(dmin(nA, nB), nC);
     m = dmin(m, dist_point_line(PA, PB, g.AB, nA, nB, g.nAB));
     m = dmin(m, dist_point_line(PB, PC, g.BC, nB, nC, g.nBC));
@@ -256,14 +265,14 @@ __device__ double dist_point_triangle(const double* T, const TriGeo& g, const do
     const double v[3] = {-g.CA[0], -g.CA[1], -g.CA[2]};
     double cu[3], cw[3];
     cross3g(g.AB, PA, cu); cross3g(PA, v, cw);
-    const double alpha = sdiv(dot3g(cu, g.nv), g.nn), beta = sdiv(dot3g(cw, g.nv), g.nn);
+    const double alpha = quot(dot3g(cu, g.nv), g.nn), beta = quot(dot3g(cw, g.nv), g.nn);
     const double gamma = 1.0 - beta - alpha;
     if (pos(alpha) && lt1(alpha) && pos(beta) && lt1(beta) && pos(gamma) && lt1(gamma)) {
         double pp[3], dd[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) pp[c] = alpha * A[c] + beta * B[c] + gamma * Cv[c];
         sub3(P, pp, dd);
-        m = dmin(m, norm2v(dd));
+        m = dmin(m, norm2f(dd));
     }
     return m;
 }
@@ -717,12 +726,17 @@ __global__ void k_geo_fill(DevGrid g, int npn, const long long* __restrict__ nod
     }
 }
 
-// true when pnode m's triangles all lie beyond d from P
-__device__ __forceinline__ bool pnode_beyond(int m, const Pt& P, float d, const float4* __restrict__ pbox) {
+// lower bound of the distance from P to pnode m's triangles (3e38: none)
+__device__ __forceinline__ float pnode_bound(int m, const Pt& P, const float4* __restrict__ pbox) {
     const float4 a = pbox[2 * m], b = pbox[2 * m + 1];
-    if (a.w == 0.0f) return true;
-    const float lo[3] = {a.x, a.y, a.z}, hi[3] = {b.x, b.y, b.z};
-    return beyond_box(P.f, P.scale, lo, hi, d);
+    const float dx = fmaxf(fmaxf(a.x - P.f[0], P.f[0] - b.x), 0.0f);
+    const float dy = fmaxf(fmaxf(a.y - P.f[1], P.f[1] - b.y), 0.0f);
+    const float dz = fmaxf(fmaxf(a.z - P.f[2], P.f[2] - b.z), 0.0f);
+    return a.w == 0.0f ? 3.0e38f : sqrtf(dx * dx + dy * dy + dz * dz);
+}
+// beyond_box for such a bound
+__device__ __forceinline__ bool beyond(float lb, float pscale, float d) {
+    return lb > d + 1.0e-5f * (lb + d + pscale);
 }
 
 // ------------------------------------------------- the distance chains
@@ -752,7 +766,7 @@ struct ChainQueue {
     double d[kTasks];
     int ent[kTasks];                  // entries of pent
     int item[kItems];                 // one per pnode: 4 (tasks before it) + kind
-    int aux[kItems];                  // 4 (pnode's ordinal in the box; or 1: the first task restarts dp) + lead
+    int aux[kItems];                  // 4 (k_geo_sd: pnode's ordinal in the box; k_geo_neigh: exact_min) + lead
 };
 
 // Encloses the reference's distance of P to a triangle (dist_point_triangle).
@@ -760,32 +774,32 @@ struct ChainQueue {
 // that of alpha and beta.  The value is the least of the distances to the
 // edges and, inside the triangle, of the one to the reference's projection;
 // any point it can take lies in the triangle.
-__device__ __forceinline__ void tri_interval(const TriF* __restrict__ trif, const GeoTet* __restrict__ tets, int tri,
-                                             const Pt& P, float& lo, float& hi) {
+__device__ __noinline__ float2 tri_interval(const TriF* __restrict__ trif, const GeoTet* __restrict__ tets, int tri,
+                                            float x, float y, float z, float scale) {
+    float lo, hi;
     const float4* r = reinterpret_cast<const float4*>(trif + tri);
     const float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2), u = __ldg(r + 3), v = __ldg(r + 4);
-    const float px = P.f[0] - a.x, py = P.f[1] - a.y, pz = P.f[2] - a.z;
+    const float px = x - a.x, py = y - a.y, pz = z - a.z;
     if (a.w < 0.0f) {
         const float* box = tets[tri >> 1].box[tri & 1];
-        const float dx = fmaxf(fmaxf(box[0] - P.f[0], P.f[0] - box[3]), 0.0f);
-        const float dy = fmaxf(fmaxf(box[1] - P.f[1], P.f[1] - box[4]), 0.0f);
-        const float dz = fmaxf(fmaxf(box[2] - P.f[2], P.f[2] - box[5]), 0.0f);
-        lo = fmaxf(0.0f, 0.99997f * sqrtf(dx * dx + dy * dy + dz * dz) - 1.1e-5f * P.scale);
-        hi = 3.0e38f;
-        return;
+        const float dx = fmaxf(fmaxf(box[0] - x, x - box[3]), 0.0f);
+        const float dy = fmaxf(fmaxf(box[1] - y, y - box[4]), 0.0f);
+        const float dz = fmaxf(fmaxf(box[2] - z, z - box[5]), 0.0f);
+        lo = fmaxf(0.0f, 0.99997f * sqrtf(dx * dx + dy * dy + dz * dz) - 1.1e-5f * scale);
+        return make_float2(lo, 3.0e38f);
     }
-    auto seg = [](float x, float y, float z, float ex, float ey, float ez, float inv) {
-        const float t = fminf(fmaxf((x * ex + y * ey + z * ez) * inv, 0.0f), 1.0f);
-        const float rx = x - t * ex, ry = y - t * ey, rz = z - t * ez;
+    auto seg = [](float qx, float qy, float qz, float ex, float ey, float ez, float inv) {
+        const float t = fminf(fmaxf((qx * ex + qy * ey + qz * ez) * inv, 0.0f), 1.0f);
+        const float rx = qx - t * ex, ry = qy - t * ey, rz = qz - t * ez;
         return rx * rx + ry * ry + rz * rz;
     };
     const float s2 = fminf(fminf(seg(px, py, pz, b.x, b.y, b.z, b.w), seg(px, py, pz, c.x, c.y, c.z, c.w)),
                            seg(px - b.x, py - b.y, pz - b.z, c.x - b.x, c.y - b.y, c.z - b.z, u.w));
-    const float s = sqrtf(s2), E = 2.0e-6f * (P.scale + s) + 1.0e-12f;
+    const float s = sqrtf(s2), E = 2.0e-6f * (scale + s) + 1.0e-12f;
     hi = s + E;
     lo = s - E;
     const float al = px * u.x + py * u.y + pz * u.z, be = px * v.x + py * v.y + pz * v.z, ga = 1.0f - be - al;
-    const float tau = v.w * 1.0e-6f * (P.scale + fabsf(px) + fabsf(py) + fabsf(pz));
+    const float tau = v.w * 1.0e-6f * (scale + fabsf(px) + fabsf(py) + fabsf(pz));
     if (tau < 0.25f) {
         const float m = fminf(al, fminf(be, ga));
         if (m > -2.0f * tau) {
@@ -798,7 +812,7 @@ __device__ __forceinline__ void tri_interval(const TriF* __restrict__ trif, cons
     } else {
         lo -= a.w;   // within the inradius of an edge
     }
-    lo = fmaxf(lo, 0.0f);
+    return make_float2(fmaxf(lo, 0.0f), hi);
 }
 
 __device__ __forceinline__ float warp_min(float v) {
@@ -820,11 +834,15 @@ __device__ __forceinline__ Encl enclose(const TriF* __restrict__ trif, const Geo
     c.lo0 = c.hi0 = c.lo1 = c.hi1 = 3.0e38f;
     if (lane < n) {
         c.e0 = __ldg(pent + s + lane);
-        tri_interval(trif, tets, c.e0 >> 2, P, c.lo0, c.hi0);
+        const float2 r = tri_interval(trif, tets, c.e0 >> 2, P.f[0], P.f[1], P.f[2], P.scale);
+        c.lo0 = r.x;
+        c.hi0 = r.y;
     }
     if (lane + 32 < n) {
         c.e1 = __ldg(pent + s + 32 + lane);
-        tri_interval(trif, tets, c.e1 >> 2, P, c.lo1, c.hi1);
+        const float2 r = tri_interval(trif, tets, c.e1 >> 2, P.f[0], P.f[1], P.f[2], P.scale);
+        c.lo1 = r.x;
+        c.hi1 = r.y;
     }
     c.lo = warp_min(fminf(c.lo0, c.lo1));
     c.hi = warp_min(fminf(c.hi0, c.hi1));
@@ -845,13 +863,15 @@ __device__ __forceinline__ int push_tasks(ChainQueue& Q, int nt, const Encl& c, 
     return nt + __popc(m0) + __popc(m1);
 }
 
-__device__ __forceinline__ void eval_tasks(ChainQueue& Q, int nt, const GeoTet* __restrict__ tets, const Pt& P,
-                                           int lane) {
+// (a call: one copy of the distance code for every place that flushes)
+__device__ __noinline__ void eval_tasks(ChainQueue* Q, int nt, const GeoTet* __restrict__ tets, double px, double py,
+                                        double pz) {
+    const double P[3] = {px, py, pz};
     __syncwarp();
-    for (int q = lane; q < nt; q += 32) {
-        const int tri = Q.ent[q] >> 2;
+    for (int q = threadIdx.x & 31; q < nt; q += 32) {
+        const int tri = Q->ent[q] >> 2;
         const GeoTet& T = tets[tri >> 1];
-        Q.d[q] = dist_point_triangle(T.tri[tri & 1], T.tg[tri & 1], P.d);
+        Q->d[q] = dist_point_triangle(T.tri[tri & 1], T.tg[tri & 1], P);
     }
     __syncwarp();
 }
@@ -878,7 +898,7 @@ struct Box9 {
 // distance and sd follows it.  One more step after a kFull pnode brings sd
 // to rest; it is made when another pnode (which has at least one
 // tetrahedron) follows.
-__global__ void __launch_bounds__(32 * kChainWarps) k_geo_sd(
+__global__ void __launch_bounds__(32 * kChainWarps, 8) k_geo_sd(
         DevGrid g, int npn, const long long* __restrict__ node_of, const int* __restrict__ ids,
         const GeoTet* __restrict__ tets, const TriF* __restrict__ trif, const int* __restrict__ pstart,
         const int* __restrict__ pent, const unsigned char* __restrict__ lead, const float4* __restrict__ prad,
@@ -900,7 +920,7 @@ __global__ void __launch_bounds__(32 * kChainWarps) k_geo_sd(
         int nt = 0, nitem = 0, ord = 0;
         int rest = -1;                        // ordinal of a kFull pnode (or the start) after which sd may not rest
         auto flush = [&]() {
-            eval_tasks(Q, nt, tets, P, lane);
+            eval_tasks(&Q, nt, tets, P.d[0], P.d[1], P.d[2]);
             for (int it = 0; it < nitem; ++it) {
                 const int t0 = Q.item[it] >> 2, kind = Q.item[it] & 3;
                 const int t1 = it + 1 < nitem ? Q.item[it + 1] >> 2 : nt;
@@ -938,13 +958,16 @@ __global__ void __launch_bounds__(32 * kChainWarps) k_geo_sd(
             const int q = q0 + lane;
             const int m0 = q < box.n ? ids[box.node(g, q)] - 1 : -1;
             const unsigned all = __ballot_sync(FM, m0 >= 0);
-            unsigned near = __ballot_sync(FM, m0 >= 0 && !pnode_beyond(m0, P, dhi, prad));
+            const float lb = m0 >= 0 ? pnode_bound(m0, P, prad) : 3.0e38f;
+            const bool in = !beyond(lb, P.scale, dhi);
+            const int s0 = in ? pstart[m0] : 0, n0 = in ? pstart[m0 + 1] - s0 : 0, f0 = in ? lead[m0] : 0;
+            unsigned near = __ballot_sync(FM, in);
             while (near) {
                 const int b = __ffs(near) - 1;
                 near &= near - 1;
-                const int m = __shfl_sync(FM, m0, b);
-                if (pnode_beyond(m, P, dhi, prad)) continue;
-                const int s = pstart[m], n = pstart[m + 1] - s, o = ord + __popc(all & ((1u << b) - 1u));
+                if (beyond(__shfl_sync(FM, lb, b), P.scale, dhi)) continue;
+                const int s = __shfl_sync(FM, s0, b), n = __shfl_sync(FM, n0, b), fl = __shfl_sync(FM, f0, b);
+                const int o = ord + __popc(all & ((1u << b) - 1u));
                 Encl c = enclose(trif, tets, pent, s, n, P, lane);
                 if (c.lo > dhi) continue;
                 if (nt > kTasks - kMaxTri || nitem == kItems) flush();
@@ -954,7 +977,7 @@ __global__ void __launch_bounds__(32 * kChainWarps) k_geo_sd(
                 const float near_min = kind == kFull ? 3.0e38f : fminf(c.hi, dhi);
                 if (lane == 0) {
                     Q.item[nitem] = 4 * nt + kind;
-                    Q.aux[nitem] = 4 * o + lead[m];
+                    Q.aux[nitem] = 4 * o + fl;
                 }
                 ++nitem;
                 nt = push_tasks(Q, nt, c, lane < n && c.lo0 <= near_min, lane + 32 < n && c.lo1 <= near_min, lane);
@@ -1111,10 +1134,10 @@ __global__ void k_geo_pnode_phi(int npn, const long long* __restrict__ node_of, 
 // 186-343): per pnode of the box a running minimum dp over its triangles,
 // starting at 10 again, and after each of its tetrahedra |v| <- |v| + (dp -
 // |v|) where dp <= |v|.  In kSimple and kReset pnodes every update of |v| is
-// exact, so |v| becomes the pnode's last dp where that is lower; its last
-// dp follows from the last triangle that certainly falls below the pnode's
-// earlier ones by less than a factor 2, and the later ones near it.
-__global__ void __launch_bounds__(32 * kChainWarps) k_geo_neigh(
+// exact, so |v| becomes the pnode's last dp where that is lower; that is the
+// least distance when an earlier triangle lies within a factor 2 of it, and
+// follows from the first triangle and those not above it otherwise.
+__global__ void __launch_bounds__(32 * kChainWarps, 8) k_geo_neigh(
         DevGrid g, const int* __restrict__ ids, const GeoTet* __restrict__ tets, const TriF* __restrict__ trif,
         const int* __restrict__ pstart, const int* __restrict__ pent, const unsigned char* __restrict__ lead,
         const float4* __restrict__ prad, const double* __restrict__ x, const double* __restrict__ y,
@@ -1139,7 +1162,7 @@ __global__ void __launch_bounds__(32 * kChainWarps) k_geo_neigh(
         };
         bounds();
         auto flush = [&]() {
-            eval_tasks(Q, nt, tets, P, lane);
+            eval_tasks(&Q, nt, tets, P.d[0], P.d[1], P.d[2]);
             for (int it = 0; it < nitem; ++it) {
                 const int t0 = Q.item[it] >> 2, kind = Q.item[it] & 3;
                 const int t1 = it + 1 < nitem ? Q.item[it + 1] >> 2 : nt;
@@ -1154,7 +1177,7 @@ __global__ void __launch_bounds__(32 * kChainWarps) k_geo_neigh(
                     }
                 } else {
                     dp = Q.aux[it] >> 2 ? Q.d[t0] : run_min(dp, Q.d[t0]);
-                    for (int q = t0 + 1; q < t1; ++q) dp = run_min(dp, Q.d[q]);
+                    for (int q = t0 + 1; q < t1; ++q) dp = run_min(dp, Q.d[q]);   // exact_min: the least
                     av = kind == kReset ? dp : dmin(av, dp);
                 }
             }
@@ -1166,13 +1189,15 @@ __global__ void __launch_bounds__(32 * kChainWarps) k_geo_neigh(
             const int q = q0 + lane;
             const int m0 = q < box.n ? ids[box.node(g, q)] - 1 : -1;
             // a |v| of 10 or more follows dp = 10 after any tetrahedron
-            unsigned near = __ballot_sync(FM, m0 >= 0 && (vhi >= 9.9999f || !pnode_beyond(m0, P, vhi, prad)));
+            const float lb = m0 >= 0 ? pnode_bound(m0, P, prad) : 3.0e38f;
+            const bool in = m0 >= 0 && (vhi >= 9.9999f || !beyond(lb, P.scale, vhi));
+            const int s0 = in ? pstart[m0] : 0, n0 = in ? pstart[m0 + 1] - s0 : 0, f0 = in ? lead[m0] : 0;
+            unsigned near = __ballot_sync(FM, in);
             while (near) {
                 const int b = __ffs(near) - 1;
                 near &= near - 1;
-                const int m = __shfl_sync(FM, m0, b);
-                if (vhi < 9.9999f && pnode_beyond(m, P, vhi, prad)) continue;
-                const int s = pstart[m], n = pstart[m + 1] - s;
+                if (vhi < 9.9999f && beyond(__shfl_sync(FM, lb, b), P.scale, vhi)) continue;
+                const int s = __shfl_sync(FM, s0, b), n = __shfl_sync(FM, n0, b), fl = __shfl_sync(FM, f0, b);
                 Encl c = enclose(trif, tets, pent, s, n, P, lane);
                 if (c.lo > vhi && vhi < 9.9999f) continue;
                 if (nt > kTasks - kMaxTri || nitem == kItems) flush();
@@ -1181,34 +1206,23 @@ __global__ void __launch_bounds__(32 * kChainWarps) k_geo_neigh(
                 const int kind = !exact ? kFull : (c.hi < vlo ? kReset : kSimple);
                 if (kind == kReset) nt = nitem = 0;
                 bool t0 = lane < n, t1 = lane + 32 < n;
-                int from = 0;
+                int exact_min = 0;
                 if (kind != kFull) {
-                    // least bounds of the earlier triangles of the pnode
-                    float ml = c.lo0, mh = c.hi0, nl = c.lo1, nh = c.hi1;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const float a = __shfl_up_sync(FM, ml, o), h = __shfl_up_sync(FM, mh, o);
-                        const float a1 = __shfl_up_sync(FM, nl, o), h1 = __shfl_up_sync(FM, nh, o);
-                        if (lane >= o) {
-                            ml = fminf(ml, a); mh = fminf(mh, h);
-                            nl = fminf(nl, a1); nh = fminf(nh, h1);
-                        }
-                    }
-                    const float l31 = __shfl_sync(FM, ml, 31), h31 = __shfl_sync(FM, mh, 31);
-                    ml = __shfl_up_sync(FM, ml, 1); mh = __shfl_up_sync(FM, mh, 1);
-                    nl = __shfl_up_sync(FM, nl, 1); nh = __shfl_up_sync(FM, nh, 1);
-                    if (lane == 0) { ml = mh = nl = nh = 3.0e38f; }
-                    nl = fminf(nl, l31);
-                    nh = fminf(nh, h31);
-                    const unsigned r0 = __ballot_sync(FM, t0 && lane > 0 && c.hi0 < ml && c.lo0 >= 0.50001f * mh);
-                    const unsigned r1 = __ballot_sync(FM, t1 && c.hi1 < nl && c.lo1 >= 0.50001f * nh);
-                    from = r1 ? 63 - __clz(r1) : (r0 ? 31 - __clz(r0) : 0);
-                    t0 = t0 && (lane == from || (lane > from && c.lo0 <= mh));
-                    t1 = t1 && (lane + 32 == from || (lane + 32 > from && c.lo1 <= nh));
+                    // the triangles that can be the pnode's least; an earlier
+                    // one within a factor 2 of it makes the last dp their least
+                    const bool w0 = t0 && c.lo0 <= c.hi, w1 = t1 && c.lo1 <= c.hi;
+                    const unsigned b0 = __ballot_sync(FM, w0), b1 = __ballot_sync(FM, w1);
+                    const int first = b0 ? __ffs(b0) - 1 : 31 + __ffs(b1);
+                    exact_min = __any_sync(FM, (t0 && lane < first && c.hi0 <= 1.9999f * c.lo) ||
+                                                   (t1 && lane + 32 < first && c.hi1 <= 1.9999f * c.lo));
+                    // (otherwise: the first, and what can fall below it)
+                    const float h = exact_min ? c.hi : __shfl_sync(FM, c.hi0, 0);
+                    t0 = t0 && (c.lo0 <= h || (!exact_min && lane == 0));
+                    t1 = t1 && c.lo1 <= h;
                 }
                 if (lane == 0) {
                     Q.item[nitem] = 4 * nt + kind;
-                    Q.aux[nitem] = (from > 0 ? 4 : 0) + lead[m];
+                    Q.aux[nitem] = 4 * exact_min + fl;
                 }
                 ++nitem;
                 nt = push_tasks(Q, nt, c, t0, t1, lane);
