@@ -125,7 +125,7 @@ __device__ void marching_full(const double (&V)[4][3], const double (&ph)[4], MT
         allp &= s[v] == 1; alln &= s[v] == -1; nz += s[v] == 0;
         allge &= s[v] >= 0; allle &= s[v] <= 0;
     }
-    if (allp) { o.wv = tetvol<true>(V[0], V[1], V[2], V[3]); return; }
+    if (allp) { o.wv = tetvol_ref(V[0], V[1], V[2], V[3]); return; }
     if (alln) return;
     int fi = 0;
     if (nz > 0 && (allge || allle)) {
@@ -141,7 +141,7 @@ __device__ void marching_full(const double (&V)[4][3], const double (&ph)[4], MT
                 else if (s[0] == 0 && s[3] == 0) water = s[1] == 1;
                 else water = s[0] == 1;
             }
-            o.wv = water ? tetvol<true>(V[0], V[1], V[2], V[3]) : 0.0;
+            o.wv = water ? tetvol_ref(V[0], V[1], V[2], V[3]) : 0.0;
             return;
         }
         if (nz == 3) {  // a face: one triangle
@@ -157,7 +157,7 @@ __device__ void marching_full(const double (&V)[4][3], const double (&ph)[4], MT
                     ++q;
                 }
             if (want_tri) o.area = tri_area(o.tri[0]);
-            o.wv = s[v] == 1 ? tetvol<true>(V[0], V[1], V[2], V[3]) : 0.0;
+            o.wv = s[v] == 1 ? tetvol_ref(V[0], V[1], V[2], V[3]) : 0.0;
             return;
         }
         // four zero vertices: FlagIndex stays 0
@@ -166,7 +166,7 @@ __device__ void marching_full(const double (&V)[4][3], const double (&ph)[4], MT
         for (int v = 0; v < 4; ++v)
             if (s[v] == -1) fi |= 1 << v;
     }
-    if (fi == 0) o.wv = tetvol<true>(V[0], V[1], V[2], V[3]);
+    if (fi == 0) o.wv = tetvol_ref(V[0], V[1], V[2], V[3]);
     const int ef = c_edge_flags[fi];
     if (ef == 0) return;
     double E[6][3];
@@ -191,7 +191,7 @@ __device__ void marching_full(const double (&V)[4][3], const double (&ph)[4], MT
         }
         o.area = o.area + tri_area(o.tri[t]);
     }
-    o.wv = water_volume<true>(V, E, fi, err);
+    o.wv = water_volume(V, E, fi, err);
 }
 
 // norm2v and sdiv as calls: the distance code keeps to a few kB, so that the
