@@ -70,8 +70,7 @@ ALGO_WORDS = {
     "bc_full_kernel": 2.0,
     "copy_kernel": 2.0,
     "normgrad_d_kernel": 12.0,       # phi, phizero, metrics(9); |grad phi|
-    "sussman_rk_kernel": 6.0,        # dn, dn1 (rmw), |grad|, |grad| at the iteration start, sign
-    "minmax_partial_kernel": 1.0,
+    "sussman_stage_kernel": 14.0,    # dn, d, phizero, sign, metrics(9); d
 }
 
 

@@ -320,47 +320,42 @@ int reinit_device(lsm_context* c, const lsm_grid* g, const DevGrid& dg, const ls
 
 // reinitialisation_test2 (src/reinitialisation_test2.F90:1-221, non-hybrid)
 // from phizero into dn1 (dn: scratch); *iters = pseudo-time iterations run.
-// The convergence test needs the field's maximum and minimum on the host
-// once per iteration (the reference's maxval/minval, then `exit`).
+// The convergence test (the reference's maxval/minval, then `exit`) is made
+// on the device: converged iterations leave the field alone.
 int sussman_device(lsm_context* c, const DevGrid& dg, const lsm_params* p, const double* phizero,
                    const double* csi, const double* eta, const double* zet, double* dn1, double* dn, int* iters) {
     if (p->OrderReinitialisationBoundaries < 1 || p->OrderReinitialisationBoundaries > 3)
         return set_err(c, LSM_ERR_BAD_PARAM, "OrderReinitialisationBoundaries must be 1, 2 or 3");
     cudaError_t e;
     const long long N = (long long)dg.ni * dg.nj * dg.nk;
+    const int R = p->RNitermax;
     double* sg = (double*)pool_get(c, "ss_sign", 8 * N, &e);
-    double* ng = sg ? (double*)pool_get(c, "ss_ng", 8 * N, &e) : nullptr;
-    double* ngc = ng ? (double*)pool_get(c, "ss_ngc", 8 * N, &e) : nullptr;
-    double* part = ngc ? (double*)pool_get(c, "ss_part", 16 * (size_t)lsm::minmax_partials(N) + 16, &e) : nullptr;
-    if (!part) return cuda_fail(c, e, "cudaMalloc(reinitialisation_test2)");
-    double* res = part + 2 * lsm::minmax_partials(N);
+    double* B = sg ? (double*)pool_get(c, "ss_b", 8 * N, &e) : nullptr;
+    auto* move = B ? (unsigned char*)pool_get(c, "ss_move", (size_t)N, &e) : nullptr;
+    auto* mm = move ? (unsigned long long*)pool_get(c, "ss_mm", 16 * ((size_t)R + 1), &e) : nullptr;
+    if (!mm) return cuda_fail(c, e, "cudaMalloc(reinitialisation_test2)");
     // the i-face blocks of calc_NormGrad_d take phizero at the last node of
     // the interior loop (src/calc_NormGrad_d.F90:41-56, 186-376)
     const long long stale = lsm::gid(dg, dg.ib - (dg.pf ? 1 : 0), dg.jb - (dg.pr ? 1 : 0), dg.kb - (dg.pu ? 1 : 0));
     const int order = p->OrderReinitialisationBoundaries, enobc = p->ENOBCReinitialisation ? 1 : 0;
-    const double C[3][3] = {{1.0, 0.0, 1.0}, {3.0 / 4.0, 1.0 / 4.0, 1.0 / 4.0}, {1.0 / 3.0, 2.0 / 3.0, 2.0 / 3.0}};
     lsm::launch_sign_phi0(N, phizero, p->epslsm, sg, c->stream);
     lsm::launch_copy(phizero, dn1, N, c->stream);
-    lsm::launch_normgrad_d(dg, order, enobc, dn1, phizero, stale, csi, eta, zet, ng, c->stream);
+    if (R > 0)
+        lsm::launch_sussman(dg, order, enobc, R, dn1, dn, B, move, sg, phizero, stale, csi, eta, zet, p->epslsm,
+                            p->epsReinitialisation, p->RNtimestep, mm, c->stream);
     LSM_TRY(after_launch(c));
-    int done = 0;
-    for (int it = 1; it <= p->RNitermax; ++it) {
-        double mm[2];
-        lsm::launch_minmax(N, ng, part, res, c->stream);
-        LSM_CU(c, cudaMemcpyAsync(mm, res, sizeof(mm), cudaMemcpyDeviceToHost, c->stream));
-        LSM_CU(c, cudaStreamSynchronize(c->stream));
-        if (std::fabs(mm[0] - 1.0) < p->epsReinitialisation && std::fabs(mm[1] - 1.0) < p->epsReinitialisation) break;
-        lsm::launch_copy(dn1, dn, N, c->stream);
-        lsm::launch_normgrad_d(dg, order, enobc, dn, phizero, stale, csi, eta, zet, ngc, c->stream);
-        for (int rk = 0; rk < 3; ++rk) {
-            lsm::launch_normgrad_d(dg, order, enobc, dn1, phizero, stale, csi, eta, zet, ng, c->stream);
-            lsm::launch_sussman_rk(dg, dn, dn1, ng, ngc, sg, p->epslsm, p->epsReinitialisation, p->RNtimestep,
-                                   C[rk][0], C[rk][1], C[rk][2], c->stream);
+    if (iters) {
+        // iterations run: up to the first whose extrema had converged
+        std::vector<double> v(2 * (size_t)R + 2);
+        *iters = 0;
+        if (R > 0) {
+            LSM_CU(c, cudaMemcpyAsync(v.data(), mm, 16 * (size_t)R, cudaMemcpyDeviceToHost, c->stream));
+            LSM_CU(c, cudaStreamSynchronize(c->stream));
+            while (*iters < R && !(std::fabs(v[2 * *iters] - 1.0) < p->epsReinitialisation &&
+                                   std::fabs(v[2 * *iters + 1] - 1.0) < p->epsReinitialisation))
+                ++*iters;
         }
-        LSM_TRY(after_launch(c));
-        done = it;
     }
-    if (iters) *iters = done;
     return LSM_OK;
 }
 

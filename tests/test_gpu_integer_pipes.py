@@ -65,3 +65,32 @@ def test_godunov_bit_exact(ls, oracle, spacing, kind):
         assert same(host(ls.calc_rh_rn(G(g), dev(d), dev(sign), *map(dev, met))), oracle.calc_rh_rn(g, d, sign, *met))
         _, ng = ls.calc_sign_ini(G(g), dev(d), *map(dev, met), 0.1)
         assert same(host(ng), oracle.calc_sign_ini(g, d, *met, 0.1)[1])
+
+
+@pytest.mark.parametrize("kind", ["plain", "extreme"])
+@pytest.mark.parametrize("spacing", [(1.0, 1.0, 1.0), (0.5, 1.0, 3.0)])
+def test_eno_norm_bit_exact(ls, oracle, spacing, kind):
+    shape = (35, 10, 9)
+    g = O.make_grid(*shape)
+    g.dc, g.de, g.dz = spacing
+    rng = np.random.default_rng(4)
+    d, zero = field(shape, kind, 5), field(shape, kind, 6)
+    met = [cases.F(rng.standard_normal((3,) + shape) * (rng.random((3,) + shape) > 0.3)) for _ in range(3)]
+    for order in (1, 3):
+        p = O.make_params(OrderReinitialisationBoundaries=order)
+        with np.errstate(all="ignore"):
+            assert same(host(ls.calc_normgrad_d(G(g), P(p), dev(d), dev(zero), *map(dev, met))),
+                        oracle.calc_normgrad_d(g, p, d, zero, *met))
+
+
+@pytest.mark.parametrize("tol,want", [(1e-5, 5), (0.1, 4), (10.0, 0)])
+def test_live_reinitialisation_stops_where_the_oracle_does(ls, oracle, tol, want):
+    """The device-side convergence test: all iterations, some, none (1e-13
+    normwise where CUDA's sin and cos enter, as in the other tests)."""
+    g, x, y, z, _, _ = cases.curvilinear(34, 11, 10, seed=2)
+    csi, eta, zet, _ = oracle.mg_metrics(g, x, y, z)
+    phi = cases.F(1.07 * (z - 0.45) + 0.01 * np.sin(3 * x))
+    p = O.make_params(epslsm=0.1, RNitermax=5, RNtimestep=0.04, epsReinitialisation=tol)
+    ref, it = oracle.reinitialisation_test2(g, p, phi, csi, eta, zet)
+    got, n = ls.reinitialisation_test2(G(g), P(p), *map(dev, (phi, csi, eta, zet)))
+    assert n == it == want and cases.relerr(host(got), ref) <= 1e-13
