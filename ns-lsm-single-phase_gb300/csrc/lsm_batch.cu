@@ -106,19 +106,13 @@ __device__ __forceinline__ bool flat_node(const Flat& fl, long long t, Node* nd)
     return true;
 }
 
-// Brick `blk` of adjoint map `map`: instance and first node of its tile.
+// Brick `blk` of an adjoint map: instance and first node of its tile.
 struct ABrick {
     int inst, i0, j0, k0;
 };
-__device__ __forceinline__ ABrick adj_brick(const Brick* __restrict__ bmap, int map, int blk) {
-    const int4 bk = __ldg(reinterpret_cast<const int4*>(bmap) + blk);
-    const AdjShape sh = adj_shape(map);
-    ABrick b;
-    b.inst = bk.x;
-    b.i0 = bk.y * sh.ox;
-    b.j0 = bk.z * sh.oy;
-    b.k0 = bk.w * sh.oz;
-    return b;
+__device__ __forceinline__ ABrick adj_brick(const Tiles& tl, int blk) {
+    const int4 bk = __ldg(reinterpret_cast<const int4*>(tl.b) + blk);
+    return ABrick{bk.x, bk.y, bk.z, bk.w};
 }
 
 // ------------------------------------------------------------ WENO3
@@ -214,8 +208,7 @@ __device__ __forceinline__ T stage_out(const FieldsT<T>& f, long long l, bool in
 // warp skips the recomputation when all its lanes can reuse it.
 constexpr int kStSX = 36, kStSY = 12;
 template <typename T>
-__global__ void __launch_bounds__(256) k_stage_z(const Inst* __restrict__ inst, const Brick* __restrict__ bmap,
-        int nb, FieldsT<T> f, const T* __restrict__ phin, const T* __restrict__ phi1, T* __restrict__ out, T c1, T c2,
+__global__ void __launch_bounds__(256) k_stage_z(const Inst* __restrict__ inst, Tiles tl, FieldsT<T> f, const T* __restrict__ phin, const T* __restrict__ phi1, T* __restrict__ out, T c1, T c2,
         T c3) {
     __shared__ T pl[2][kStSY][kStSX];
     const unsigned FM = 0xffffffffu;
@@ -232,13 +225,13 @@ __global__ void __launch_bounds__(256) k_stage_z(const Inst* __restrict__ inst, 
     }
     const bool has_h = t < 160;
     unsigned ph = 0;   // buffer parity, continuous over the tiles of this CTA
-    for (int blk = blockIdx.x; blk < nb; blk += gridDim.x) {
-        const ABrick ab = adj_brick(bmap, 2, blk);
+    for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {
+        const ABrick ab = adj_brick(tl, blk);
         const Inst& I = inst[ab.inst];
         const int ni = I.ni, nj = I.nj, nk = I.nk;
         const long long sk = (long long)ni * nj;
         const int i = ab.i0 + tx, j = ab.j0 + ty;
-        const int k0 = ab.k0, k1 = min(k0 + adj_shape(2).oz, nk);
+        const int k0 = ab.k0, k1 = min(k0 + tl.len, nk);
         const bool col = i < ni && j < nj;
         const int gi = ab.i0 + hx, gj = ab.j0 + hy;
         const bool hok = has_h && gi >= 0 && gi < ni && gj >= 0 && gj < nj;
@@ -381,7 +374,7 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
 // plane barrier that frees its buffer) while plane k is computed.
 constexpr int kTmaBX = 40, kTmaBY = 12, kTmaBuf = 3;
 __global__ void __launch_bounds__(256) k_stage_tma(const __grid_constant__ CUtensorMap tm, int a_in,
-        const Inst* __restrict__ inst, const Brick* __restrict__ bmap, int nb, FieldsT<float> f,
+        const Inst* __restrict__ inst, Tiles tl, FieldsT<float> f,
         const float* __restrict__ phin, const float* __restrict__ phi1, float* __restrict__ out, float c1, float c2,
         float c3, unsigned* __restrict__ err) {
     __shared__ __align__(128) float pl[kTmaBuf][kTmaBY][kTmaBX];
@@ -409,10 +402,10 @@ __global__ void __launch_bounds__(256) k_stage_tma(const __grid_constant__ CUten
         ++issued;
     };
     bool aborted = false;
-    for (int blk = blockIdx.x; blk < nb && !aborted; blk += gridDim.x) {
-        const ABrick ab = adj_brick(bmap, 2, blk);
+    for (int blk = blockIdx.x; blk < tl.n && !aborted; blk += gridDim.x) {
+        const ABrick ab = adj_brick(tl, blk);
         const int i = ab.i0 + tx, j = ab.j0 + ty;
-        const int k0 = ab.k0, k1 = min(k0 + adj_shape(2).oz, nk);
+        const int k0 = ab.k0, k1 = min(k0 + tl.len, nk);
         const bool col = i < ni && j < nj;
         const long long cb = i + (long long)ni * j;
         const bool ij_int = i > 0 && i < ni - 1 && j > 0 && j < nj - 1;
@@ -780,18 +773,17 @@ __device__ __forceinline__ T godunov_sel_v(const T (&mas)[3], const T (&men)[3],
 // dout2 (nullable) receives a second copy of d'.  d' equals reinit_node's
 // arithmetic (one_sided, godunov) bit for bit.
 template <typename T, bool SIGN, bool REC>
-__global__ void __launch_bounds__(256) k_reinit_z(const Inst* __restrict__ inst, const Brick* __restrict__ bmap,
-        int nb, FieldsT<T> f, const T* __restrict__ din, T* __restrict__ dout, T* __restrict__ dout2,
+__global__ void __launch_bounds__(256) k_reinit_z(const Inst* __restrict__ inst, Tiles tl, FieldsT<T> f, const T* __restrict__ din, T* __restrict__ dout, T* __restrict__ dout2,
         T* __restrict__ cf, long long ld, unsigned* err) {
     const unsigned FM = 0xffffffffu;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int blk = blockIdx.x; blk < nb; blk += gridDim.x) {
-        const ABrick ab = adj_brick(bmap, 2, blk);
+    for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {
+        const ABrick ab = adj_brick(tl, blk);
         const Inst& I = inst[ab.inst];
         const int ni = I.ni, nj = I.nj, nk = I.nk;
         const long long sj = ni, sk = (long long)ni * nj;
         const int i = ab.i0 + tx, j = ab.j0 + ty;
-        const int k0 = ab.k0, k1 = min(k0 + adj_shape(2).oz, nk);
+        const int k0 = ab.k0, k1 = min(k0 + tl.len, nk);
         const bool col = i < ni && j < nj;
         const long long cb = I.off + i + sj * j;
         const bool xm = i > 0, xp = i < ni - 1, ym = j > 0, yp = j < nj - 1;
@@ -874,17 +866,16 @@ __global__ void __launch_bounds__(256) k_reinit_z(const Inst* __restrict__ inst,
 // (the tile's edge lanes load the one outside), the y neighbours are
 // loaded (L1/L2).
 template <typename T>
-__global__ void __launch_bounds__(256) k_adj_reinit_c(const Inst* __restrict__ inst, const Brick* __restrict__ bmap,
-        int nb, const T* __restrict__ cf, long long ld, const T* __restrict__ lam, T* __restrict__ lam_out) {
+__global__ void __launch_bounds__(256) k_adj_reinit_c(const Inst* __restrict__ inst, Tiles tl, const T* __restrict__ cf, long long ld, const T* __restrict__ lam, T* __restrict__ lam_out) {
     const unsigned FM = 0xffffffffu;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int blk = blockIdx.x; blk < nb; blk += gridDim.x) {
-        const ABrick ab = adj_brick(bmap, 2, blk);
+    for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {
+        const ABrick ab = adj_brick(tl, blk);
         const Inst& I = inst[ab.inst];
         const int ni = I.ni, nj = I.nj, nk = I.nk;
         const long long sj = ni, sk = (long long)ni * nj;
         const int i = ab.i0 + tx, j = ab.j0 + ty;
-        const int k0 = ab.k0, k1 = min(k0 + adj_shape(2).oz, nk);
+        const int k0 = ab.k0, k1 = min(k0 + tl.len, nk);
         const bool col = i < ni && j < nj;
         const long long cb = I.off + i + sj * j;
         const bool xm = i > 0, xp = i < ni - 1, ym = j > 0, yp = j < nj - 1;
@@ -1322,18 +1313,18 @@ __device__ __forceinline__ long long warp_sum_nn(long long v) {
     return (long long)(s0 + (s1 << 22) + (s2 << 44));
 }
 
-// Bulk water volumes of the cells and the interface-cell list (SUMS: also
-// add the bulk cells' fixed-point volumes to acc[4 inst + 2]), on the tiles
-// of adjoint map 2: thread (lane, row) owns the cell column (i0 + lane, j0 +
+// Bulk water volumes of the cells (added to acc[4 inst + 2]) and the
+// interface-cell list, on the tiles of adjoint map 2 (FULL: tiles of the
+// longest march, a constant that saves 4 registers and with them a block per
+// SM: 111 against 125 us on 512 x 256 x 256 nodes): thread (lane, row) owns the cell column (i0 + lane, j0 +
 // row) and marches the tile's planes in k.  A cell's eight vertices are the
 // 2 x 2 quads of planes k and k + 1; a quad is the thread's own node and
 // the one at j + 1 (loaded), with the i + 1 pair from the next lane by a
 // shuffle (the tile's last lane loads it).  Each plane is loaded once, a
 // plane ahead of its use; a quad is reduced to two flags (all water, all
 // air) and a cell is water / air when both of its quads are.
-template <typename T, bool SUMS>
-__global__ void __launch_bounds__(256) k_vol_scan_z(const Inst* __restrict__ inst, const Brick* __restrict__ bmap,
-        int nb, FieldsT<T> f, const T* __restrict__ phi, unsigned long long* __restrict__ acc,
+template <typename T, bool FULL>
+__global__ void __launch_bounds__(256) k_vol_scan_z(const Inst* __restrict__ inst, Tiles tl, FieldsT<T> f, const T* __restrict__ phi, unsigned long long* __restrict__ acc,
         unsigned* __restrict__ list, unsigned* __restrict__ count) {
     const T eps = T(kEpsSims);
     const unsigned FM = 0xffffffffu;
@@ -1345,9 +1336,9 @@ __global__ void __launch_bounds__(256) k_vol_scan_z(const Inst* __restrict__ ins
         if (tx == 0 && v != 0) atomicAdd(acc + 4 * (long long)cur + 2, (unsigned long long)v);
         Bq = 0;
     };
-    for (int blk = blockIdx.x; blk < nb; blk += gridDim.x) {
-        const ABrick ab = adj_brick(bmap, 2, blk);
-        if (SUMS && ab.inst != cur) {
+    for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {
+        const ABrick ab = adj_brick(tl, blk);
+        if (ab.inst != cur) {
             if (cur >= 0) flush();
             cur = ab.inst;
         }
@@ -1356,7 +1347,7 @@ __global__ void __launch_bounds__(256) k_vol_scan_z(const Inst* __restrict__ ins
         const long long sj = ni, sk = (long long)ni * nj;
         const int i = ab.i0 + tx, j = ab.j0 + ty;
         // cells k0 .. kc1 - 1 (a cell's top plane k + 1 stays inside the grid)
-        const int k0 = ab.k0, kc1 = min(k0 + adj_shape(2).oz, nk - 1);
+        const int k0 = ab.k0, kc1 = min(k0 + (FULL ? adj_shape(2).oz : tl.len), nk - 1);
         const bool cell = i < ni - 1 && j < nj - 1;
         const bool own = i < ni && j < nj - 1, edge = tx == 31 && i + 1 < ni && j < nj - 1;
         const long long cb = I.off + i + sj * j;
@@ -1388,7 +1379,7 @@ __global__ void __launch_bounds__(256) k_vol_scan_z(const Inst* __restrict__ ins
             Quad q0;
             ld(k0, q0);
             ld(k0 + 1, qn);
-            if (SUMS && cell) cv = __ldg(f.cellfix + cb + sk * k0);
+            if (cell) cv = __ldg(f.cellfix + cb + sk * k0);
             flags(q0, qw0, qa0);
         }
         for (int k = k0; k < kc1; ++k) {
@@ -1396,12 +1387,12 @@ __global__ void __launch_bounds__(256) k_vol_scan_z(const Inst* __restrict__ ins
             long long cvn = 0;
             if (k + 1 < kc1) {
                 ld(k + 2, qq);
-                if (SUMS && cell) cvn = __ldg(f.cellfix + cb + sk * (k + 1));
+                if (cell) cvn = __ldg(f.cellfix + cb + sk * (k + 1));
             }
             bool qw1, qa1;
             flags(qn, qw1, qa1);
             const bool allw = qw0 && qw1, alla = qa0 && qa1;
-            if (SUMS && cell && allw) Bq += cv;
+            if (cell && allw) Bq += cv;
             const bool mix = cell && !allw && !alla;
             const unsigned m = __ballot_sync(FM, mix);
             if (m) {
@@ -1416,7 +1407,7 @@ __global__ void __launch_bounds__(256) k_vol_scan_z(const Inst* __restrict__ ins
             cv = cvn;
         }
     }
-    if (SUMS && cur >= 0) flush();
+    if (cur >= 0) flush();
 }
 
 // the eight vertex values and the coordinates relative to vertex 0 of the
@@ -1587,14 +1578,13 @@ __global__ void __launch_bounds__(128) k_mass_weights(Flat fl, FieldsT<T> f, con
 // FP64.  FP32 lam is first summed in FP32 over runs of 8 planes (the FP64
 // pipe would otherwise take a conversion and an add per node).
 template <typename T>
-__global__ void __launch_bounds__(256) k_tile_sum(const Inst* __restrict__ inst, const Brick* __restrict__ bmap,
-                                                   int nb, const T* __restrict__ lam, double* __restrict__ part) {
+__global__ void __launch_bounds__(256) k_tile_sum(const Inst* __restrict__ inst, Tiles tl, const T* __restrict__ lam, double* __restrict__ part) {
     __shared__ double red[8];
     const int t = threadIdx.x, tx = t & 31, ty = t >> 5;
-    for (int blk = blockIdx.x; blk < nb; blk += gridDim.x) {
-        const ABrick ab = adj_brick(bmap, 2, blk);
+    for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {
+        const ABrick ab = adj_brick(tl, blk);
         const Inst& I = inst[ab.inst];
-        const int i = ab.i0 + tx, j = ab.j0 + ty, k1 = min(ab.k0 + adj_shape(2).oz, I.nk);
+        const int i = ab.i0 + tx, j = ab.j0 + ty, k1 = min(ab.k0 + tl.len, I.nk);
         double sacc = 0.0;
         if (i < I.ni && j < I.nj) {
             const long long sk = (long long)I.ni * I.nj;
@@ -1625,12 +1615,12 @@ __global__ void __launch_bounds__(256) k_tile_sum(const Inst* __restrict__ inst,
 }
 
 // part 3: one block per instance sums its tiles' partials in a fixed order
-__global__ void __launch_bounds__(256) k_inst_sum(const Inst* __restrict__ inst, const double* __restrict__ part,
+__global__ void __launch_bounds__(256) k_inst_sum(const Inst* __restrict__ inst, int len, const double* __restrict__ part,
                                                   double* __restrict__ out) {
     __shared__ double red[8];
     const Inst& I = inst[blockIdx.x];
     const int t0 = I.am[2][0];
-    const int nt = I.am[2][1] * I.am[2][2] * ((I.nk + adj_shape(2).oz - 1) / adj_shape(2).oz);
+    const int nt = I.am[2][1] * I.am[2][2] * ((I.nk + len - 1) / len);
     double s = 0.0;
     for (int u = threadIdx.x; u < nt; u += blockDim.x) s += part[t0 + u];
 #pragma unroll
@@ -1829,12 +1819,11 @@ __device__ __forceinline__ T stage_node_grad(const T (&s)[5], T w, T lp, bool lo
 // Writes lam_in = c2 lamP0 - c3 acc_x (+ lamPhin + c1 lamP0 when last),
 // updates lamPhin and lamW_x.
 template <typename T>
-__global__ void __launch_bounds__(256) k_adj_stage_x(const Inst* __restrict__ inst, const Brick* __restrict__ bmap,
-        int nb, FieldsT<T> f, const T* __restrict__ in, const T* __restrict__ lamP0, T* __restrict__ lam_in,
+__global__ void __launch_bounds__(256) k_adj_stage_x(const Inst* __restrict__ inst, Tiles tl, FieldsT<T> f, const T* __restrict__ in, const T* __restrict__ lamP0, T* __restrict__ lam_in,
         T* __restrict__ lamPhin, T* __restrict__ lamW0, T c1, T c2, T c3, int last) {
     const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
-    for (int blk = blockIdx.x; blk < nb; blk += gridDim.x) {
-        const ABrick ab = adj_brick(bmap, 0, blk);
+    for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {
+        const ABrick ab = adj_brick(tl, blk);
         const Inst& I = inst[ab.inst];
         const int ni = I.ni, nj = I.nj, nk = I.nk;
         const int j = ab.j0 + row, k = ab.k0;
@@ -1913,18 +1902,18 @@ __global__ void __launch_bounds__(256) k_adj_stage_x(const Inst* __restrict__ in
     }
 }
 
-// Stage adjoint, y (AX = 1, adjoint map 1) or z (AX = 2, map 2) part: each
-// thread marches one line along AX over adj_shape(map) outputs, keeping
+// Stage adjoint, y (AX = 1, adjoint map 1) or z (AX = 2, map 4) part: each
+// thread marches one line along AX over Tiles::len outputs (FULL: the
+// longest, a constant; registers for five blocks per SM in the z part, 283
+// against 290 us on 512 x 256 x 256 nodes), keeping
 // windows of five G, lamP0 and D values in registers; lam_in -= c3 acc,
 // lamW_AX -= c3 lamP0 D.
-template <typename T, int AX>
-__global__ void __launch_bounds__(256) k_adj_stage_m(const Inst* __restrict__ inst, const Brick* __restrict__ bmap,
-        int nb, FieldsT<T> f, const T* __restrict__ in, const T* __restrict__ lamP0, T* __restrict__ lam_in,
+template <typename T, int AX, bool FULL>
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : (AX == 2 ? 5 : 4)) k_adj_stage_m(const Inst* __restrict__ inst, Tiles tl, FieldsT<T> f, const T* __restrict__ in, const T* __restrict__ lamP0, T* __restrict__ lam_in,
         T* __restrict__ lamW, T c3) {
-    constexpr int MAP = AX;
     const int tx = threadIdx.x & 31, tq = threadIdx.x >> 5;
-    for (int blk = blockIdx.x; blk < nb; blk += gridDim.x) {
-        const ABrick ab = adj_brick(bmap, MAP, blk);
+    for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {
+        const ABrick ab = adj_brick(tl, blk);
         const Inst& I = inst[ab.inst];
         const int ni = I.ni, nj = I.nj, nk = I.nk;
         const long long sj = ni, sk = (long long)ni * nj;
@@ -1933,7 +1922,7 @@ __global__ void __launch_bounds__(256) k_adj_stage_m(const Inst* __restrict__ in
         const int c2 = AX == 1 ? ab.k0 + tq : ab.j0 + tq;
         const int n2 = AX == 1 ? nk : nj, nm = AX == 1 ? nj : nk;
         const int m0 = AX == 1 ? ab.j0 : ab.k0;
-        const int m1 = min(m0 + (AX == 1 ? adj_shape(1).oy : adj_shape(2).oz), nm);
+        const int m1 = min(m0 + (FULL ? (AX == 1 ? adj_shape(1).oy : adj_shape(4).oz) : tl.len), nm);
         const bool col = i < ni && c2 < n2;
         const bool line = col && i >= 1 && i <= ni - 2 && c2 >= 1 && c2 <= n2 - 2;
         const long long st = AX == 1 ? sj : sk;
@@ -2050,20 +2039,20 @@ __device__ __forceinline__ void coef_eval(const CoefIn<T>& c, T dtau, const bool
 // later, after every thread has passed the barrier between).
 template <typename T>
 __global__ void __launch_bounds__(32 * kReinRY, sizeof(T) == 4 ? 2 : 1) k_adj_reinit(const Inst* __restrict__ inst,
-        const Brick* __restrict__ bmap, int nb, FieldsT<T> f, const T* __restrict__ d, const T* __restrict__ lam,
+        Tiles tl, FieldsT<T> f, const T* __restrict__ d, const T* __restrict__ lam,
         T* __restrict__ lam_out) {
     constexpr int RY = kReinRY;
     __shared__ T sD[2][RY + 2][32];   // row ty + 1 holds row ty (rows 0, RY + 1: padding)
     __shared__ T sA1[2][RY][32], sB1[2][RY][32];
     const unsigned FM = 0xffffffffu;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int blk = blockIdx.x; blk < nb; blk += gridDim.x) {
-        const ABrick ab = adj_brick(bmap, 3, blk);
+    for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {
+        const ABrick ab = adj_brick(tl, blk);
         const Inst& I = inst[ab.inst];
         const int ni = I.ni, nj = I.nj, nk = I.nk;
         const long long sj = ni, sk = (long long)ni * nj;
         const int i = ab.i0 - 1 + tx, j = ab.j0 - 1 + ty;
-        const int k0 = ab.k0, k1 = min(k0 + adj_shape(3).oz, nk);
+        const int k0 = ab.k0, k1 = min(k0 + tl.len, nk);
         const bool node = i >= 0 && i < ni && j >= 0 && j < nj;
         const bool out = node && tx >= 1 && tx <= 30 && ty >= 1 && ty <= RY - 2;
         const T dtau = ipar<T>(I.dtau, I.dtau64);
@@ -2229,16 +2218,16 @@ void contra(int shape, int grid, const Inst* inst, const Brick* bi, int nb, Fiel
     dispatch<RunContra, T>(shape, grid, inst, bi, nb, f, s);
 }
 template <typename T>
-void stage(int grid, const Inst* inst, const Brick* bmap2, int nb, FieldsT<T> f, const T* phin, const T* phi1, T* out,
+void stage(int grid, const Inst* inst, Tiles tl, FieldsT<T> f, const T* phin, const T* phi1, T* out,
            double c1, double c2, double c3, cudaStream_t s) {
     ProfScope ps_("k_stage_z", s);
-    k_stage_z<T><<<grid, 256, 0, s>>>(inst, bmap2, nb, f, phin, phi1, out, T(c1), T(c2), T(c3));
+    k_stage_z<T><<<grid, 256, 0, s>>>(inst, tl, f, phin, phi1, out, T(c1), T(c2), T(c3));
 }
-void stage_tma(int grid, const CUtensorMap* tm, int a_in, const Inst* inst, const Brick* bmap2, int nb,
+void stage_tma(int grid, const CUtensorMap* tm, int a_in, const Inst* inst, Tiles tl,
                FieldsT<float> f, const float* phin, const float* phi1, float* out, double c1, double c2, double c3,
                unsigned* err, cudaStream_t s) {
     ProfScope ps_("k_stage_tma", s);
-    k_stage_tma<<<grid, 256, 0, s>>>(*tm, a_in, inst, bmap2, nb, f, phin, phi1, out, (float)c1, (float)c2, (float)c3,
+    k_stage_tma<<<grid, 256, 0, s>>>(*tm, a_in, inst, tl, f, phin, phi1, out, (float)c1, (float)c2, (float)c3,
                                      err);
 }
 int stage_tma_blocks_per_sm() {
@@ -2280,27 +2269,27 @@ void sign_reinit(int shape, int grid, const Inst* inst, const Brick* bi, int nb,
     dispatch<RunSignReinit, T>(shape, grid, inst, bi, nb, f, phi0, dout, err, s);
 }
 template <typename T>
-void reinit_z(int kind, int grid, const Inst* inst, const Brick* bmap2, int nb, FieldsT<T> f, const T* din, T* dout,
+void reinit_z(int kind, int grid, const Inst* inst, Tiles tl, FieldsT<T> f, const T* din, T* dout,
               T* dout2, T* cf, long long ld, unsigned* err, cudaStream_t s) {
     switch (kind) {
     case 0: {
         ProfScope ps_("k_reinit_z", s);
-        k_reinit_z<T, false, false><<<grid, 256, 0, s>>>(inst, bmap2, nb, f, din, dout, dout2, cf, ld, err);
+        k_reinit_z<T, false, false><<<grid, 256, 0, s>>>(inst, tl, f, din, dout, dout2, cf, ld, err);
         break;
     }
     case 1: {
         ProfScope ps_("k_reinit_rec_z", s);
-        k_reinit_z<T, false, true><<<grid, 256, 0, s>>>(inst, bmap2, nb, f, din, dout, dout2, cf, ld, err);
+        k_reinit_z<T, false, true><<<grid, 256, 0, s>>>(inst, tl, f, din, dout, dout2, cf, ld, err);
         break;
     }
     case 2: {
         ProfScope ps_("k_sign_reinit_z", s);
-        k_reinit_z<T, true, false><<<grid, 256, 0, s>>>(inst, bmap2, nb, f, din, dout, dout2, cf, ld, err);
+        k_reinit_z<T, true, false><<<grid, 256, 0, s>>>(inst, tl, f, din, dout, dout2, cf, ld, err);
         break;
     }
     default: {
         ProfScope ps_("k_sign_reinit_rec_z", s);
-        k_reinit_z<T, true, true><<<grid, 256, 0, s>>>(inst, bmap2, nb, f, din, dout, dout2, cf, ld, err);
+        k_reinit_z<T, true, true><<<grid, 256, 0, s>>>(inst, tl, f, din, dout, dout2, cf, ld, err);
         break;
     }
     }
@@ -2312,10 +2301,10 @@ int reinit_z_blocks_per_sm() {
     return n;
 }
 template <typename T>
-void adj_reinit_c(int grid, const Inst* inst, const Brick* bmap2, int nb, const T* cf, long long ld, const T* lam,
+void adj_reinit_c(int grid, const Inst* inst, Tiles tl, const T* cf, long long ld, const T* lam,
                   T* lam_out, cudaStream_t s) {
     ProfScope ps_("k_adj_reinit_c", s);
-    k_adj_reinit_c<T><<<grid, 256, 0, s>>>(inst, bmap2, nb, cf, ld, lam, lam_out);
+    k_adj_reinit_c<T><<<grid, 256, 0, s>>>(inst, tl, cf, ld, lam, lam_out);
 }
 template <typename T>
 int adj_reinit_c_blocks_per_sm() {
@@ -2331,12 +2320,13 @@ void bc_reinit(const Inst* inst, int ninst, long long nface, FieldsT<T> f, BC bc
 }
 inline unsigned list_blocks() { return 152 * 8; }
 template <typename T>
-void volume(int grid2, const Inst* inst, const Brick* bmap2, int nb2, const Flat& fl, FieldsT<T> f, const T* phi,
+void volume(int grid2, const Inst* inst, Tiles tl, const Flat& fl, FieldsT<T> f, const T* phi,
             unsigned long long* acc, bool slope, unsigned* list, unsigned* count, cudaStream_t s) {
     cudaMemsetAsync(count, 0, sizeof(unsigned), s);
     {
         ProfScope ps_("k_vol_scan_z", s);
-        k_vol_scan_z<T, true><<<grid2, 256, 0, s>>>(inst, bmap2, nb2, f, phi, acc, list, count);
+        if (tl.len == adj_shape(2).oz) k_vol_scan_z<T, true><<<grid2, 256, 0, s>>>(inst, tl, f, phi, acc, list, count);
+        else k_vol_scan_z<T, false><<<grid2, 256, 0, s>>>(inst, tl, f, phi, acc, list, count);
     }
     if (slope) {
         ProfScope ps_("k_vol_iface_slope", s);
@@ -2357,7 +2347,7 @@ void mass_shift(const Flat& fl, const Mass* mass, const T* src, T* dst, cudaStre
     k_mass_shift<T><<<(unsigned)std::min<long long>((fl.n + 255) / 256, 152 * 16), 256, 0, s>>>(fl, mass, src, dst);
 }
 template <typename T>
-void mass_adjoint(const Inst* inst, const Brick* bmap2, int nb2, const Flat& fl, FieldsT<T> f, const T* phi_pre,
+void mass_adjoint(const Inst* inst, Tiles tl, const Flat& fl, FieldsT<T> f, const T* phi_pre,
                   const Mass* mass, T* lam, unsigned long long* wfix, double* part, double* ssum, const unsigned* list,
                   const unsigned* count, cudaStream_t s) {
     {
@@ -2366,11 +2356,11 @@ void mass_adjoint(const Inst* inst, const Brick* bmap2, int nb2, const Flat& fl,
     }
     {
         ProfScope ps_("k_tile_sum", s);
-        k_tile_sum<T><<<std::min(nb2, 152 * 8), 256, 0, s>>>(inst, bmap2, nb2, lam, part);
+        k_tile_sum<T><<<std::min(tl.n, 152 * 8), 256, 0, s>>>(inst, tl, lam, part);
     }
     {
         ProfScope ps_("k_inst_sum", s);
-        k_inst_sum<<<fl.ninst, 256, 0, s>>>(inst, part, ssum);
+        k_inst_sum<<<fl.ninst, 256, 0, s>>>(inst, tl.len, part, ssum);
     }
     ProfScope ps_("k_mass_apply", s);
     k_mass_apply<T><<<list_blocks(), 128, 0, s>>>(fl, mass, ssum, list, count, lam, wfix);
@@ -2414,35 +2404,41 @@ void adj_face(const Flat& fl, int face, long long nplane, int nface, BC bc, int 
                                                               T(c2), lam);
 }
 template <typename T>
-void adj_stage(const int* grid, const Inst* inst, const Brick* const* bmap, const int* nb, FieldsT<T> f, const T* in,
+void adj_stage(const int* grid, const Inst* inst, const Tiles* tl, FieldsT<T> f, const T* in,
                const T* lamP0, T* lam_in, T* lamPhin, T* lamW0, T* lamW1, T* lamW2, double c1, double c2, double c3,
                bool last, cudaStream_t s) {
     {
         ProfScope ps_("k_adj_stage_x", s);
-        k_adj_stage_x<T><<<grid[0], 256, 0, s>>>(inst, bmap[0], nb[0], f, in, lamP0, lam_in, lamPhin, lamW0, T(c1),
+        k_adj_stage_x<T><<<grid[0], 256, 0, s>>>(inst, tl[0], f, in, lamP0, lam_in, lamPhin, lamW0, T(c1),
                                                  T(c2), T(c3), last ? 1 : 0);
     }
     {
         ProfScope ps_("k_adj_stage_y", s);
-        k_adj_stage_m<T, 1><<<grid[1], 256, 0, s>>>(inst, bmap[1], nb[1], f, in, lamP0, lam_in, lamW1, T(c3));
+        if (tl[1].len == adj_shape(1).oy)
+            k_adj_stage_m<T, 1, true><<<grid[1], 256, 0, s>>>(inst, tl[1], f, in, lamP0, lam_in, lamW1, T(c3));
+        else
+            k_adj_stage_m<T, 1, false><<<grid[1], 256, 0, s>>>(inst, tl[1], f, in, lamP0, lam_in, lamW1, T(c3));
     }
     ProfScope ps_("k_adj_stage_z", s);
-    k_adj_stage_m<T, 2><<<grid[2], 256, 0, s>>>(inst, bmap[2], nb[2], f, in, lamP0, lam_in, lamW2, T(c3));
+    if (tl[4].len == adj_shape(4).oz)
+        k_adj_stage_m<T, 2, true><<<grid[4], 256, 0, s>>>(inst, tl[4], f, in, lamP0, lam_in, lamW2, T(c3));
+    else
+        k_adj_stage_m<T, 2, false><<<grid[4], 256, 0, s>>>(inst, tl[4], f, in, lamP0, lam_in, lamW2, T(c3));
 }
 template <typename T>
-void adj_reinit(int grid, const Inst* inst, const Brick* bmap, int nb, FieldsT<T> f, const T* d, const T* lam,
+void adj_reinit(int grid, const Inst* inst, Tiles tl, FieldsT<T> f, const T* d, const T* lam,
                 T* lam_out, cudaStream_t s) {
     ProfScope ps_("k_adj_reinit", s);
-    k_adj_reinit<T><<<grid, 32 * kReinRY, 0, s>>>(inst, bmap, nb, f, d, lam, lam_out);
+    k_adj_reinit<T><<<grid, 32 * kReinRY, 0, s>>>(inst, tl, f, d, lam, lam_out);
 }
 template <typename T>
 int adj_blocks_per_sm(int map) {
     int n = 0;
     switch (map) {
     case 0: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_stage_x<T>, 256, 0); break;
-    case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_stage_m<T, 1>, 256, 0); break;
-    case 2: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_stage_m<T, 2>, 256, 0); break;
-    default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_reinit<T>, 32 * kReinRY, 0); break;
+    case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_stage_m<T, 1, true>, 256, 0); break;
+    case 3: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_reinit<T>, 32 * kReinRY, 0); break;
+    default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_stage_m<T, 2, true>, 256, 0); break;
     }
     return n;
 }
@@ -2456,7 +2452,7 @@ void adj_contra(const Flat& fl, FieldsT<T> f, const T* w0, const T* w1, const T*
 #define LSM_BATCH_INSTANTIATE(T)                                                                                      \
     template void contra<T>(int, int, const Inst*, const Brick*, int, FieldsT<T>, cudaStream_t);                       \
     template int stage_blocks_per_sm<T>();                                                                      \
-    template void stage<T>(int, const Inst*, const Brick*, int, FieldsT<T>, const T*, const T*, T*, double,            \
+    template void stage<T>(int, const Inst*, Tiles, FieldsT<T>, const T*, const T*, T*, double,            \
                            double, double, cudaStream_t);                                                                     \
     template void bc_stage<T>(const Inst*, int, long long, BC, const T*, const T*, T*, double, double, cudaStream_t);   \
     template void bc_full<T>(int, int, const Inst*, const Brick*, int, BC, const T*, T*, unsigned*, cudaStream_t);      \
@@ -2466,24 +2462,24 @@ void adj_contra(const Flat& fl, FieldsT<T> f, const T* w0, const T* w1, const T*
                             cudaStream_t);                                                                            \
     template void sign_reinit<T>(int, int, const Inst*, const Brick*, int, FieldsT<T>, const T*, T*, unsigned*,      \
                                  cudaStream_t);                                                                   \
-    template void reinit_z<T>(int, int, const Inst*, const Brick*, int, FieldsT<T>, const T*, T*, T*, T*, long long, \
+    template void reinit_z<T>(int, int, const Inst*, Tiles, FieldsT<T>, const T*, T*, T*, T*, long long, \
                               unsigned*, cudaStream_t);                                                         \
     template int reinit_z_blocks_per_sm<T>();                                                                   \
-    template void adj_reinit_c<T>(int, const Inst*, const Brick*, int, const T*, long long, const T*, T*,           \
+    template void adj_reinit_c<T>(int, const Inst*, Tiles, const T*, long long, const T*, T*,           \
                                   cudaStream_t);                                                                \
     template int adj_reinit_c_blocks_per_sm<T>();                                                               \
-    template void volume<T>(int, const Inst*, const Brick*, int, const Flat&, FieldsT<T>, const T*,                \
+    template void volume<T>(int, const Inst*, Tiles, const Flat&, FieldsT<T>, const T*,                \
                             unsigned long long*, bool, unsigned*, unsigned*, cudaStream_t);                          \
     template int vol_scan_blocks_per_sm<T>();                                                                   \
     template void mass_shift<T>(const Flat&, const Mass*, const T*, T*, cudaStream_t);                                 \
-    template void mass_adjoint<T>(const Inst*, const Brick*, int, const Flat&, FieldsT<T>, const T*, const Mass*,  \
+    template void mass_adjoint<T>(const Inst*, Tiles, const Flat&, FieldsT<T>, const T*, const Mass*,  \
                                   T*, unsigned long long*, double*, double*, const unsigned*, const unsigned*,          \
                                   cudaStream_t);                                                                     \
     template void adj_face<T>(const Flat&, int, long long, int, BC, int, const T*, const T*, const T*, double, double, \
                               T*, cudaStream_t);                                                                     \
-    template void adj_stage<T>(const int*, const Inst*, const Brick* const*, const int*, FieldsT<T>, const T*,      \
+    template void adj_stage<T>(const int*, const Inst*, const Tiles*, FieldsT<T>, const T*,      \
                                const T*, T*, T*, T*, T*, T*, double, double, double, bool, cudaStream_t);      \
-    template void adj_reinit<T>(int, const Inst*, const Brick*, int, FieldsT<T>, const T*, const T*, T*,            \
+    template void adj_reinit<T>(int, const Inst*, Tiles, FieldsT<T>, const T*, const T*, T*,            \
                                 cudaStream_t);                                                                \
     template int adj_blocks_per_sm<T>(int);                                                                     \
     template void adj_contra<T>(const Flat&, FieldsT<T>, const T*, const T*, const T*, T*, T*, T*, cudaStream_t);

@@ -16,6 +16,8 @@
 namespace lsm {
 namespace batch {
 
+constexpr int kMaps = 5;   // tile maps (adj_shape)
+
 struct Inst {
     long long off;     // first node of the instance in the packed arrays
     int ni, nj, nk;
@@ -24,11 +26,11 @@ struct Inst {
     float dt;          // advection time step (multiplied into W)
     float dtau;        // reinitialisation pseudo time step
     float eps;         // smoothing half-width epslsm
-    float pad;
+    int pad;
     long long face0;   // first boundary-face node of the instance (forward bc kernels)
     long long fpre[3]; // first node of the instance's i-, j-, k-face planes (adjoint face kernels)
     double dt64, dtau64, eps64;  // the same three parameters for the FP64 kernels
-    int am[4][3];                // adjoint brick maps (adj_shape): first brick, bricks per row, per plane
+    int am[kMaps][3];            // adjoint brick maps (adj_shape): first brick, bricks per row, per plane
 };
 
 // Packed fields of one batch (device pointers), scalar type T.
@@ -81,9 +83,17 @@ struct BC {
     float BigPhi;
 };
 
-// One brick of a brick table: its instance and brick coordinates.
+// One brick of a brick table: its instance and brick coordinates; in the
+// tables of the adjoint maps, the first node of the tile per axis.
 struct __align__(16) Brick {
     int inst, bx, by, bz;
+};
+
+// The tiles of an adjoint map (adj_shape): their table and the nodes that one
+// spans along its march.
+struct Tiles {
+    const Brick* b;
+    int n, len;
 };
 
 // A flat walk of the packed nodes (one thread per node, the instance found
@@ -109,7 +119,7 @@ void contra(int shape, int grid, const Inst* inst, const Brick* bricks, int nbri
 // adjoint map 2 (z march, shared-memory planes); grid from
 // stage_blocks_per_sm
 template <typename T>
-void stage(int grid, const Inst* inst, const Brick* bmap2, int nb, FieldsT<T> f, const T* phin, const T* phi1,
+void stage(int grid, const Inst* inst, Tiles tl, FieldsT<T> f, const T* phin, const T* phi1,
            T* out, double c1, double c2, double c3, cudaStream_t s);
 template <typename T>
 int stage_blocks_per_sm();
@@ -117,7 +127,7 @@ int stage_blocks_per_sm();
 // shared memory by TMA copies: a batch of one instance with ni a multiple
 // of 4; phi1 is array a_in of the 4-D tensor map tm (ni, nj, nk, arrays);
 // err gets kErrTimeout if a copy's completion never arrived
-void stage_tma(int grid, const CUtensorMap* tm, int a_in, const Inst* inst, const Brick* bmap2, int nb,
+void stage_tma(int grid, const CUtensorMap* tm, int a_in, const Inst* inst, Tiles tl,
                FieldsT<float> f, const float* phin, const float* phi1, float* out, double c1, double c2, double c3,
                unsigned* err, cudaStream_t s);
 int stage_tma_blocks_per_sm();
@@ -151,7 +161,7 @@ void bc_reinit(const Inst* inst, int ninst, long long nface, FieldsT<T> f, BC bc
 // pseudo-step, 3 the same recorded; dout2 (nullable) gets a second copy of
 // the output
 template <typename T>
-void reinit_z(int kind, int grid, const Inst* inst, const Brick* bmap2, int nb, FieldsT<T> f, const T* din, T* dout,
+void reinit_z(int kind, int grid, const Inst* inst, Tiles tl, FieldsT<T> f, const T* din, T* dout,
               T* dout2, T* cf, long long ld, unsigned* err, cudaStream_t s);
 template <typename T>
 int reinit_z_blocks_per_sm();
@@ -164,7 +174,7 @@ int reinit_z_blocks_per_sm();
 // none) it also forms each instance's mass correction into mass[inst] and,
 // when mrec is not null, mrec[inst]
 template <typename T>
-void volume(int grid2, const Inst* inst, const Brick* bmap2, int nb2, const Flat& fl, FieldsT<T> f, const T* phi,
+void volume(int grid2, const Inst* inst, Tiles tl, const Flat& fl, FieldsT<T> f, const T* phi,
             unsigned long long* acc, bool slope, unsigned* list, unsigned* count, cudaStream_t s);
 template <typename T>
 int vol_scan_blocks_per_sm();
@@ -192,17 +202,19 @@ int max_blocks_per_sm(int shape, int kernel);
 // Tile maps besides the forward brick table (output nodes per tile ox x oy
 // x oz, adj_shape): 0 stage adjoint x part (8 whole rows, one warp marching
 // each), 1 stage adjoint y march, 2 the k marches over 32 x 8 columns (RK
-// stage, pseudo-steps, stage adjoint z part, reverse pseudo-step from
-// stored coefficients), 3 reverse pseudo-step recomputing its coefficients
-// (overlapped 32 x kReinRY tile marching in k).
+// stage, pseudo-steps, volume scan, reverse pseudo-step from stored
+// coefficients), 3 reverse pseudo-step recomputing its coefficients
+// (overlapped 32 x kReinRY tile marching in k), 4 stage adjoint z march.
 // The face and velocity adjoints walk the packed nodes with one thread per
 // node (instance found by binary search over the node offsets `offs`).
+// The extents along the march (y in map 1, z in maps 2 to 4) are the
+// longest; a batch with few tiles takes shorter ones (Tiles::len).
 struct AdjShape { int ox, oy, oz; };
 constexpr int kReinRY = 12;
 // (map 0: ox = 0 means a brick spans whole rows)
 __host__ __device__ constexpr AdjShape adj_shape(int map) {
     return map == 0 ? AdjShape{0, 8, 1}
-                    : map == 1 ? AdjShape{32, 32, 8} : map == 2 ? AdjShape{32, 8, 32} : AdjShape{30, kReinRY - 2, 32};
+                    : map == 1 ? AdjShape{32, 32, 8} : map == 3 ? AdjShape{30, kReinRY - 2, 32} : AdjShape{32, 8, 32};
 }
 // Reverse of one bcond_lsm face (face = 0..5: i1, im, j1, jm, k1, km) on the
 // adjoint field lam, in place.  The forward values that decide the BigPhi
@@ -221,19 +233,19 @@ void adj_face(const Flat& fl, int face, long long nface_nodes, int nface, BC bc,
 // (+ lamPhin + c1 lamP0 when last, which also clears lamPhin), otherwise
 // accumulates lamPhin += c1 lamP0; and lamW_m -= c3 lamP0 D_m.
 template <typename T>
-void adj_stage(const int* grid, const Inst* inst, const Brick* const* bmap, const int* nb, FieldsT<T> f, const T* in,
+void adj_stage(const int* grid, const Inst* inst, const Tiles* tl, FieldsT<T> f, const T* in,
                const T* lamP0, T* lam_in, T* lamPhin, T* lamW0, T* lamW1, T* lamW2, double c1, double c2, double c3,
                bool last, cudaStream_t s);
 // Reverse of one reinitialisation pseudo-step d' = d - dtau s (G(d) - 1)
 // from its input d: lam_out = (dd'/dd)^T lam (adjoint map 3).
 template <typename T>
-void adj_reinit(int grid, const Inst* inst, const Brick* bmap, int nb, FieldsT<T> f, const T* d, const T* lam,
+void adj_reinit(int grid, const Inst* inst, Tiles tl, FieldsT<T> f, const T* d, const T* lam,
                 T* lam_out, cudaStream_t s);
 // Reverse of one recorded pseudo-step from the coefficients reinit_rec
 // stored: a 7-point stencil on lam, on the tiles of adjoint map 2 (grid
 // from adj_reinit_c_blocks_per_sm)
 template <typename T>
-void adj_reinit_c(int grid, const Inst* inst, const Brick* bmap2, int nb, const T* cf, long long ld, const T* lam,
+void adj_reinit_c(int grid, const Inst* inst, Tiles tl, const T* cf, long long ld, const T* lam,
                   T* lam_out, cudaStream_t s);
 template <typename T>
 int adj_reinit_c_blocks_per_sm();
@@ -250,7 +262,7 @@ void mass_shift(const Flat& fl, const Mass* mass, const T* src, T* dst, cudaStre
 // (one per instance) are scratch; (list, count) are the interface cells of
 // phi_pre as the forward step's volume pass listed them
 template <typename T>
-void mass_adjoint(const Inst* inst, const Brick* bmap2, int nb2, const Flat& fl, FieldsT<T> f, const T* phi_pre,
+void mass_adjoint(const Inst* inst, Tiles tl, const Flat& fl, FieldsT<T> f, const T* phi_pre,
                   const Mass* mass, T* lam, unsigned long long* wfix, double* part, double* ssum, const unsigned* list,
                   const unsigned* count, cudaStream_t s);
 // lam_u_c += sum_m M[m][c] dt lamW_m  (the W = dt M u chain rule)

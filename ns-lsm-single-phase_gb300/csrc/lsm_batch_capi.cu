@@ -66,8 +66,9 @@ struct lsm_batch {
     long long* d_offs = nullptr;
     lsm::batch::Brick* d_brick = nullptr;
     int nbricks = 0;
-    lsm::batch::Brick* d_amap[4] = {};  // brick tables of the adjoint stencil kernels (lsm::batch::adj_shape)
-    int namap[4] = {0, 0, 0, 0}, agrid[4] = {1, 1, 1, 1};
+    lsm::batch::Brick* d_amap[lsm::batch::kMaps] = {};  // brick tables of the adjoint stencil kernels (lsm::batch::adj_shape)
+    int namap[lsm::batch::kMaps] = {}, agrid[lsm::batch::kMaps] = {};
+    int len[lsm::batch::kMaps] = {};         // march lengths of the maps' tiles
     int sgrid = 1, acgrid = 1, rzgrid = 1;   // CTAs of the map-2 kernels: stage, k_adj_reinit_c, reinit_z
     int vgrid = 1;                           // CTAs of the map-2 volume scan
     bool reinit_march = true;   // plain pseudo-steps march in k (reinit_z) rather than walk the brick table
@@ -283,18 +284,50 @@ int store_out(lsm_batch* b, double* dst, long long n, int stride, int c0, int nc
     return LSM_OK;
 }
 
+lsm::batch::Tiles tiles(const lsm_batch* b, int m) { return {b->d_amap[m], b->namap[m], b->len[m]}; }
+
+// March lengths of the adjoint maps: the longest of 32, 16, 8, 4 that gives
+// the GPU enough tiles (six per SM, three for the stage adjoint and the
+// recomputing reverse pseudo-step), since a march reuses what it has loaded
+// and evaluated; the stage adjoint evaluates four planes more than it
+// writes, so its marches keep to 8 and more.  Measured, against 32 always:
+// 128^3 (256 tiles of 32) k_stage_z 54 -> 32 us, k_reinit_rec_z 41 -> 35 us;
+// two FP64 grids of about 40^3 k_stage_z 260 -> 65 us, k_adj_reinit 375 ->
+// 70 us, k_adj_stage_y 234 -> 88 us (106 us at 4); 512 x 256 x 256 (4096
+// tiles of 32) loses 6 % at 8.
+void march_lengths(const lsm_batch* b, int (&len)[lsm::batch::kMaps]) {
+    const int sms = 152;
+    for (int m = 0; m < lsm::batch::kMaps; ++m) {
+        const auto a = lsm::batch::adj_shape(m);
+        len[m] = m == 1 ? a.oy : a.oz;
+        if (m == 0) continue;
+        const int least = m == 1 || m == 4 ? 8 : 4;
+        const long long want = (m == 2 ? 6 : 3) * sms;
+        for (; len[m] > least; len[m] /= 2) {
+            const int oy = m == 1 ? len[m] : a.oy, oz = m == 1 ? a.oz : len[m];
+            long long tiles = 0;
+            for (const auto& I : b->inst)
+                tiles += (long long)((I.ni + a.ox - 1) / a.ox) * ((I.nj + oy - 1) / oy) * ((I.nk + oz - 1) / oz);
+            if (tiles >= want) break;
+        }
+    }
+}
+
 int build_bricks(lsm_batch* b, int shape) {
     if (b->prec) shape = 0;     // FP64 kernels exist for tile shape 0 only
     const auto sh = lsm::batch::kShapes[shape];
     std::vector<Inst> hi(b->ninst);
     using lsm::batch::Brick;
-    std::vector<Brick> brick, amap[4];
-    // bricks in x-fastest order, each with its instance and coordinates
-    auto add = [](std::vector<Brick>& v, int q, int bx, int by, int bz) {
+    std::vector<Brick> brick, amap[lsm::batch::kMaps];
+    // bricks in x-fastest order, each with its instance and coordinates (times
+    // the extents sx, sy, sz)
+    auto add = [](std::vector<Brick>& v, int q, int bx, int by, int bz, int sx, int sy, int sz) {
         for (int z = 0; z < bz; ++z)
             for (int y = 0; y < by; ++y)
-                for (int x = 0; x < bx; ++x) v.push_back(Brick{q, x, y, z});
+                for (int x = 0; x < bx; ++x) v.push_back(Brick{q, x * sx, y * sy, z * sz});
     };
+    int(&len)[lsm::batch::kMaps] = b->len;
+    march_lengths(b, len);
     long long face = 0, pre[3] = {0, 0, 0};
     for (int q = 0; q < b->ninst; ++q) {
         const auto& I = b->inst[q];
@@ -310,26 +343,27 @@ int build_bricks(lsm_batch* b, int shape) {
         d.dt = (float)I.dt;
         d.dtau = (float)I.dtau;
         d.eps = (float)I.eps;
-        d.pad = 0.f;
+        d.pad = 0;
         d.dt64 = I.dt;
         d.dtau64 = I.dtau;
         d.eps64 = I.eps;
         d.face0 = face;
         face += 2LL * ((long long)I.nj * I.nk + (long long)I.ni * I.nk + (long long)I.ni * I.nj);
         for (int a = 0; a < 3; ++a) d.fpre[a] = pre[a];
-        for (int m = 0; m < 4; ++m) {
-            const auto a = lsm::batch::adj_shape(m);
+        for (int m = 0; m < lsm::batch::kMaps; ++m) {
+            auto a = lsm::batch::adj_shape(m);
+            (m == 1 ? a.oy : a.oz) = len[m];
             const int bx = a.ox > 0 ? (I.ni + a.ox - 1) / a.ox : 1;
             const int by = (I.nj + a.oy - 1) / a.oy, bz = (I.nk + a.oz - 1) / a.oz;
             d.am[m][0] = (int)amap[m].size();
             d.am[m][1] = bx;
             d.am[m][2] = by;
-            add(amap[m], q, bx, by, bz);
+            add(amap[m], q, bx, by, bz, a.ox, a.oy, a.oz);
         }
         pre[0] += (long long)I.nj * I.nk;
         pre[1] += (long long)I.ni * I.nk;
         pre[2] += (long long)I.ni * I.nj;
-        add(brick, q, d.nbx, d.nby, nbz);
+        add(brick, q, d.nbx, d.nby, nbz, 1, 1, 1);
     }
     b->nface = face;
     for (int a = 0; a < 3; ++a) b->nplane[a] = pre[a];
@@ -339,7 +373,7 @@ int build_bricks(lsm_batch* b, int shape) {
         cudaFree(b->d_brick);
         b->d_brick = nullptr;
     }
-    for (int m = 0; m < 4; ++m) {
+    for (int m = 0; m < lsm::batch::kMaps; ++m) {
         if (b->d_amap[m]) {
             cudaFree(b->d_amap[m]);
             b->d_amap[m] = nullptr;
@@ -360,7 +394,7 @@ int build_bricks(lsm_batch* b, int shape) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
     const int per = std::max(1, lsm::batch::max_blocks_per_sm(shape, 0));
     b->grid = std::max(1, std::min(b->nbricks, sms * per));
-    for (int m = 0; m < 4; ++m) {
+    for (int m = 0; m < lsm::batch::kMaps; ++m) {
         const int pa = std::max(1, b->prec ? lsm::batch::adj_blocks_per_sm<double>(m)
                                            : lsm::batch::adj_blocks_per_sm<float>(m));
         b->agrid[m] = std::max(1, std::min(b->namap[m], sms * pa));
@@ -450,13 +484,13 @@ void enqueue_stage(lsm_batch* b, FieldsT<T> f, const T* phin, const T* in, T* ou
                 }
             }
             if (map && a < (1LL << 31)) {
-                B::stage_tma(b->tgrid, map, (int)a, b->d_inst, b->d_amap[2], b->namap[2], f, phin, in, out, kC[s][0],
+                B::stage_tma(b->tgrid, map, (int)a, b->d_inst, tiles(b, 2), f, phin, in, out, kC[s][0],
                              kC[s][1], kC[s][2], b->d_err, b->stream);
                 return;
             }
         }
     }
-    B::stage<T>(b->sgrid, b->d_inst, b->d_amap[2], b->namap[2], f, phin, in, out, kC[s][0], kC[s][1], kC[s][2],
+    B::stage<T>(b->sgrid, b->d_inst, tiles(b, 2), f, phin, in, out, kC[s][0], kC[s][1], kC[s][2],
                 b->stream);
 }
 
@@ -481,7 +515,7 @@ void enqueue_step_io(lsm_batch* b, const T* phin, T* phi_out, const Rec<T>* rec,
     if (rec && !coef) f.sgn = rec->sgn;
     const Flat fl{b->d_inst, b->d_offs, b->ninst, b->N};
     if (vol && !mc) {
-        B::volume<T>(b->vgrid, b->d_inst, b->d_amap[2], b->namap[2], fl, f, phin, b->d_vacc, false, b->d_ilist,
+        B::volume<T>(b->vgrid, b->d_inst, tiles(b, 2), fl, f, phin, b->d_vacc, false, b->d_ilist,
                      b->d_icount, b->stream);
         B::volume_final(b->ninst, b->d_vacc, b->d_vols, nullptr, nullptr, nullptr, b->stream);
     }
@@ -513,7 +547,7 @@ void enqueue_step_io(lsm_batch* b, const T* phin, T* phi_out, const Rec<T>* rec,
             unsigned* err = (last && !rec) || (o2 && check) ? b->d_err : nullptr;
             T* cf = coef ? rec->C + 6LL * it * (long long)b->ld : nullptr;
             if (march)
-                B::reinit_z<T>((it == 0 ? 2 : 0) + (coef ? 1 : 0), b->rzgrid, b->d_inst, b->d_amap[2], b->namap[2], f,
+                B::reinit_z<T>((it == 0 ? 2 : 0) + (coef ? 1 : 0), b->rzgrid, b->d_inst, tiles(b, 2), f,
                                cur, o, o2, cf, (long long)b->ld, err, b->stream);
             else if (it == 0)
                 B::sign_reinit<T>(sh, gr, b->d_inst, b->d_brick, nb, f, cur, o, err, b->stream);
@@ -536,7 +570,7 @@ void enqueue_step_io(lsm_batch* b, const T* phin, T* phi_out, const Rec<T>* rec,
         // and phi_out = result + C
         // a recorded step keeps the interface cells of its result for the
         // reverse of the correction
-        B::volume<T>(b->vgrid, b->d_inst, b->d_amap[2], b->namap[2], fl, f, res, b->d_vacc, true,
+        B::volume<T>(b->vgrid, b->d_inst, tiles(b, 2), fl, f, res, b->d_vacc, true,
                      rec ? rec->list : b->d_ilist, rec ? rec->count : b->d_icount, b->stream);
         B::volume_final(b->ninst, b->d_vacc, b->d_vols, b->d_target, b->d_mass, mrec, b->stream);
         if (phi_out) B::mass_shift<T>(fl, b->d_mass, res, phi_out, b->stream);
@@ -601,9 +635,9 @@ int autotune(lsm_batch* b) {
     }
     // the marching pseudo-steps do not depend on the brick shape
     const int st = timed(&dummy, &zm, [&]() {}, [&]() {
-        B::reinit_z<float>(2, b->rzgrid, b->d_inst, b->d_amap[2], b->namap[2], f, f.phi, f.d[0], nullptr, nullptr, 0,
+        B::reinit_z<float>(2, b->rzgrid, b->d_inst, tiles(b, 2), f, f.phi, f.d[0], nullptr, nullptr, 0,
                            nullptr, b->stream);
-        B::reinit_z<float>(0, b->rzgrid, b->d_inst, b->d_amap[2], b->namap[2], f, f.d[0], f.d[1], nullptr, nullptr, 0,
+        B::reinit_z<float>(0, b->rzgrid, b->d_inst, tiles(b, 2), f, f.d[0], f.d[1], nullptr, nullptr, 0,
                            nullptr, b->stream);
     });
     if (st != LSM_OK) return done(st);
@@ -622,11 +656,11 @@ int autotune(lsm_batch* b) {
         const int st2 = timed(
             &ms_plain, &ms_tma,
             [&]() {
-                B::stage<float>(b->sgrid, b->d_inst, b->d_amap[2], b->namap[2], f, f.phi, f.phi, f.stage[0], 1.0, 0.0,
+                B::stage<float>(b->sgrid, b->d_inst, tiles(b, 2), f, f.phi, f.phi, f.stage[0], 1.0, 0.0,
                                 1.0, b->stream);
             },
             [&]() {
-                B::stage_tma(b->tgrid, &b->tm_field, 0, b->d_inst, b->d_amap[2], b->namap[2], f, f.phi, f.phi,
+                B::stage_tma(b->tgrid, &b->tm_field, 0, b->d_inst, tiles(b, 2), f, f.phi, f.phi,
                              f.stage[0], 1.0, 0.0, 1.0, b->d_err, b->stream);
             });
         if (st2 != LSM_OK) return done(st2);
@@ -848,7 +882,7 @@ void adj_step(lsm_batch* b, AdjView<T>& v, const Rec<T>& r, const T* phin, const
     const int R = b->cfg.RNitermax;
     // reverse of the mass correction phi^{n+1} = P + C(P), in place on lam
     if (b->cfg.mass_correction)
-        B::mass_adjoint<T>(b->d_inst, b->d_amap[2], b->namap[2], fl, f, r.P, m, v.lam, b->wfix, b->d_tpart,
+        B::mass_adjoint<T>(b->d_inst, tiles(b, 2), fl, f, r.P, m, v.lam, b->wfix, b->d_tpart,
                            b->d_ssum, r.list, r.count, b->stream);
     auto faces = [&](int kind, const T* pn, const T* in, const T* out, double c1, double c2) {
         for (int ax = 2; ax >= 0; --ax) {
@@ -864,22 +898,24 @@ void adj_step(lsm_batch* b, AdjView<T>& v, const Rec<T>& r, const T* phin, const
         faces(1, nullptr, nullptr, rec_d(b, r, R - 1), 0.0, 0.0);
         for (int k = R - 1; k >= 0; --k) {
             if (r.C) {
-                B::adj_reinit_c<T>(b->acgrid, b->d_inst, b->d_amap[2], b->namap[2], r.C + 6LL * k * (long long)b->ld,
+                B::adj_reinit_c<T>(b->acgrid, b->d_inst, tiles(b, 2), r.C + 6LL * k * (long long)b->ld,
                                    (long long)b->ld, v.lam, v.lam2, b->stream);
             } else {
                 const T* dk = k == 0 ? r.A[2] : rec_d(b, r, k - 1);
-                B::adj_reinit<T>(b->agrid[3], b->d_inst, b->d_amap[3], b->namap[3], f, dk, v.lam, v.lam2, b->stream);
+                B::adj_reinit<T>(b->agrid[3], b->d_inst, tiles(b, 3), f, dk, v.lam, v.lam2, b->stream);
             }
             std::swap(v.lam, v.lam2);
         }
     } else {
         faces(1, nullptr, nullptr, r.A[2], 0.0, 0.0);
     }
+    B::Tiles all[B::kMaps];
+    for (int m = 0; m < B::kMaps; ++m) all[m] = tiles(b, m);
     // stages 3, 2, 1: inputs A2, A1, phi^n; outputs A3, A2, A1
     const T* ins[3] = {phin, r.A[0], r.A[1]};
     for (int s = 2; s >= 0; --s) {
         faces(0, phin, ins[s], r.A[s], kC[s][0], kC[s][1]);
-        B::adj_stage<T>(b->agrid, b->d_inst, b->d_amap, b->namap, f, ins[s], v.lam, v.lam2, v.lamPhin, v.lamW[0],
+        B::adj_stage<T>(b->agrid, b->d_inst, all, f, ins[s], v.lam, v.lam2, v.lamPhin, v.lamW[0],
                         v.lamW[1], v.lamW[2], kC[s][0], kC[s][1], kC[s][2], s == 0, b->stream);
         std::swap(v.lam, v.lam2);
     }
@@ -1083,7 +1119,7 @@ int lsm_batch_destroy(lsm_batch_handle b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     for (void* p : {b->field_arena, (void*)b->xyz, (void*)b->staging, (void*)b->d_inst, (void*)b->d_offs,
                     (void*)b->d_brick, (void*)b->d_amap[0], (void*)b->d_amap[1], (void*)b->d_amap[2],
-                    (void*)b->d_amap[3], (void*)b->d_vacc, (void*)b->d_vols, (void*)b->d_err, b->adj,
+                    (void*)b->d_amap[3], (void*)b->d_amap[4], (void*)b->d_vacc, (void*)b->d_vols, (void*)b->d_err, b->adj,
                     (void*)b->d_target, (void*)b->d_mass, (void*)b->wfix, (void*)b->d_tpart, (void*)b->d_ssum,
                     (void*)b->d_ilist, (void*)b->d_icount, (void*)b->f64x, (void*)b->d_p64, (void*)b->cellrel})
         if (p) cudaFree(p);
@@ -1290,10 +1326,10 @@ int lsm_batch_water_volume(lsm_batch_handle b, double* volumes) {
     namespace B = lsm::batch;
     const Flat fl{b->d_inst, b->d_offs, b->ninst, b->N};
     if (b->prec)
-        B::volume<double>(b->vgrid, b->d_inst, b->d_amap[2], b->namap[2], fl, b->f64, b->f64.phi, b->d_vacc, false,
+        B::volume<double>(b->vgrid, b->d_inst, tiles(b, 2), fl, b->f64, b->f64.phi, b->d_vacc, false,
                           b->d_ilist, b->d_icount, b->stream);
     else
-        B::volume<float>(b->vgrid, b->d_inst, b->d_amap[2], b->namap[2], fl, b->f32, b->f32.phi, b->d_vacc, false,
+        B::volume<float>(b->vgrid, b->d_inst, tiles(b, 2), fl, b->f32, b->f32.phi, b->d_vacc, false,
                          b->d_ilist, b->d_icount, b->stream);
     B::volume_final(b->ninst, b->d_vacc, b->d_vols, nullptr, nullptr, nullptr, b->stream);
     BCU(b, cudaGetLastError());
