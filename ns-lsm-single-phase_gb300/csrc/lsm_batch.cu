@@ -176,6 +176,40 @@ __global__ void k_w64(long long off, long long n, double dt, const double* const
 
 // ------------------------------------------------------------ RK stage
 
+// (double)f and (float)d on the integer pipes (a conversion takes the FP64
+// pipe as long as a product): exact / rounded to nearest even for 0 and
+// normal values whose result is 0 or normal; `ok` is cleared otherwise
+__device__ __forceinline__ double widen(float f, bool& ok) {
+    const unsigned u = __float_as_uint(f), m = u & 0x7FFFFFFFu;
+    ok = ok && (m - 0x00800000u < 0x7F000000u || m == 0u);
+    return __hiloint2double((int)((u & 0x80000000u) | (m ? (m >> 3) + 0x38000000u : 0u)), (int)(u << 29));
+}
+__device__ __forceinline__ float narrow(double d, bool& ok) {
+    const unsigned h = (unsigned)__double2hiint(d), l = (unsigned)__double2loint(d), m = h & 0x7FFFFFFFu;
+    const unsigned q = ((m - 0x38000000u) << 3) | (l >> 29), r = l << 3;   // truncated, rest
+    ok = ok && m - 0x38100000u < 0x0FD00000u;
+    return __uint_as_float((h & 0x80000000u) | (q + ((r > 0x80000000u || (r == 0x80000000u && (q & 1u))) ? 1u : 0u)));
+}
+__device__ __noinline__ float stage_band_any(double W0, double W1, double W2, float D0, float D1, float D2, float c1,
+                                             float c2, float c3, float pn, float w2) {
+    const double r = W0 * (double)D0 + W1 * (double)D1 + W2 * (double)D2;
+    return (float)((double)c1 * (double)pn + (double)c2 * (double)w2 - (double)c3 * r);
+}
+// The stage in FP64 over the FP32 differences: six operations of the FP64
+// pipe instead of fifteen.  A call, so that only the warps with such a node
+// pay for it (inlined, its operations were predicated, and predicated-off
+// operations occupy the FP64 pipe of every warp: 56 % of k_stage_z's time on
+// 64 grids of 32..96 nodes an axis).
+__device__ __noinline__ float stage_band(double W0, double W1, double W2, float D0, float D1, float D2, float c1,
+                                         float c2, float c3, float pn, float w2) {
+    bool ok = true;
+    const double d0 = widen(D0, ok), d1 = widen(D1, ok), d2 = widen(D2, ok);
+    const double p = widen(pn, ok), w = widen(w2, ok), a = widen(c1, ok), b = widen(c2, ok), c = widen(c3, ok);
+    const double r = W0 * d0 + W1 * d1 + W2 * d2;
+    const float v = narrow(a * p + b * w - c * r, ok);
+    return ok ? v : stage_band_any(W0, W1, W2, D0, D1, D2, c1, c2, c3, pn, w2);
+}
+
 // The stage output c1 phi^n + c2 phi1 - c3 R at node l.  FP32 batches that
 // keep the FP64 contravariant velocity combine the nodes within kBand64 eps
 // of the interface in FP64: R = sum_m W64_m D_m over the FP32 differences D.
@@ -183,11 +217,9 @@ template <typename T>
 __device__ __forceinline__ T stage_out(const FieldsT<T>& f, long long l, bool interior, T c1, T c2, T c3, T pn, T w2,
                                        T R, T D0, T D1, T D2, T eps) {
     if constexpr (sizeof(T) == 4) {
-        if (interior && f.W64[0] && fabsf(w2) < kBand64 * eps) {
-            const double r = __ldg(f.W64[0] + l) * (double)D0 + __ldg(f.W64[1] + l) * (double)D1 +
-                             __ldg(f.W64[2] + l) * (double)D2;
-            return (T)((double)c1 * (double)pn + (double)c2 * (double)w2 - (double)c3 * r);
-        }
+        if (interior && f.W64[0] && fabsf(w2) < kBand64 * eps)
+            return stage_band(__ldg(f.W64[0] + l), __ldg(f.W64[1] + l), __ldg(f.W64[2] + l), D0, D1, D2, c1, c2, c3, pn,
+                              w2);
     }
     return c1 * pn + c2 * w2 - c3 * R;
 }
