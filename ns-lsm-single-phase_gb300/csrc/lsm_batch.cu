@@ -546,30 +546,58 @@ __device__ __forceinline__ bool face_on(const BC& bc, int face) {
     return t == 0 || t == 1 || (t == 2 && face == 1);
 }
 
-template <typename T, class P0>
-__device__ T bval_i(const BC& bc, const P0& p0, int ni, int i, int j, int k) {
-    if (i == 0 && face_on(bc, 0)) return bc_rule<T>(bc.type[0], p0(1, j, k), p0(2, j, k), bc.BigPhi);
-    if (i == ni - 1 && face_on(bc, 1)) return bc_rule<T>(bc.type[1], p0(i - 1, j, k), p0(i - 2, j, k), bc.BigPhi);
-    return p0(i, j, k);
-}
-template <typename T, class P0>
-__device__ T bval_j(const BC& bc, const P0& p0, int ni, int nj, int i, int j, int k) {
-    if (j == 0 && face_on(bc, 2))
-        return bc_rule<T>(bc.type[2], bval_i<T>(bc, p0, ni, i, 1, k), bval_i<T>(bc, p0, ni, i, 2, k), bc.BigPhi);
-    if (j == nj - 1 && face_on(bc, 3))
-        return bc_rule<T>(bc.type[3], bval_i<T>(bc, p0, ni, i, j - 1, k), bval_i<T>(bc, p0, ni, i, j - 2, k),
-                          bc.BigPhi);
-    return bval_i<T>(bc, p0, ni, i, j, k);
-}
-template <typename T, class P0>
-__device__ T bval_k(const BC& bc, const P0& p0, int ni, int nj, int nk, int i, int j, int k) {
-    if (k == 0 && face_on(bc, 4))
-        return bc_rule<T>(bc.type[4], bval_j<T>(bc, p0, ni, nj, i, j, 1), bval_j<T>(bc, p0, ni, nj, i, j, 2),
-                          bc.BigPhi);
-    if (k == nk - 1 && face_on(bc, 5))
-        return bc_rule<T>(bc.type[5], bval_j<T>(bc, p0, ni, nj, i, j, k - 1), bval_j<T>(bc, p0, ni, nj, i, j, k - 2),
-                          bc.BigPhi);
-    return bval_j<T>(bc, p0, ni, nj, i, j, k);
+// Value of node (i, j, k) after the first `axes` axes' faces of bcond_lsm
+// (i, then j, then k), from the pre-BC field p0: per axis whose face rule
+// applies, the rule on the two nodes inward, eight nodes for a corner and two
+// for a node of one face.  ONE: one evaluation of p0 in a loop for a field
+// that is costly to evaluate (the last pseudo-step: k_bc_reinit 101 us on 64
+// grids of 32..96 with all nested calls inlined, 40 us so); otherwise the
+// nodes' loads go out together, those not needed predicated off (k_bc_stage
+// 32.7 us, 29.0 us).
+template <typename T, bool ONE, class P0>
+__device__ __forceinline__ T bc_value(const BC& bc, const P0& p0, int ni, int nj, int nk, int i, int j, int k,
+                                      int axes = 3) {
+    auto dir = [&](int c, int n, int face) { return c == 0 && face_on(bc, face) ? 1 : (c == n - 1 && face_on(bc, face + 1) ? -1 : 0); };
+    const int di = axes > 0 ? dir(i, ni, 0) : 0, dj = axes > 1 ? dir(j, nj, 2) : 0, dk = axes > 2 ? dir(k, nk, 4) : 0;
+    const int ti = bc.type[di < 0 ? 1 : 0], tj = bc.type[dj < 0 ? 3 : 2], tk = bc.type[dk < 0 ? 5 : 4];
+    if constexpr (ONE) {
+        if ((di != 0) + (dj != 0) + (dk != 0) == 1) {   // one face: both values in flight at once
+            const T v1 = p0(i + di, j + dj, k + dk), v2 = p0(i + 2 * di, j + 2 * dj, k + 2 * dk);
+            return bc_rule<T>(di ? ti : dj ? tj : tk, v1, v2, bc.BigPhi);
+        }
+        T vk = T(0);
+#pragma unroll 1
+        for (int a = 0; a < (dk ? 2 : 1); ++a) {
+            T vj = T(0);
+#pragma unroll 1
+            for (int b = 0; b < (dj ? 2 : 1); ++b) {
+                T vi = T(0);
+#pragma unroll 1
+                for (int c = 0; c < (di ? 2 : 1); ++c) {
+                    const T v = p0(di ? i + di * (c + 1) : i, dj ? j + dj * (b + 1) : j, dk ? k + dk * (a + 1) : k);
+                    vi = c == 0 ? v : bc_rule<T>(ti, vi, v, bc.BigPhi);
+                }
+                vj = b == 0 ? vi : bc_rule<T>(tj, vj, vi, bc.BigPhi);
+            }
+            vk = a == 0 ? vj : bc_rule<T>(tk, vk, vj, bc.BigPhi);
+        }
+        return vk;
+    } else {
+        T v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int c = q & 1, b = (q >> 1) & 1, a = q >> 2;
+            v[q] = T(0);
+            if ((!c || di) && (!b || dj) && (!a || dk)) v[q] = p0(i + di * (c + 1), j + dj * (b + 1), k + dk * (a + 1));
+        }
+#pragma unroll
+        for (int q = 0; q < 8; q += 2)
+            if (di) v[q] = bc_rule<T>(ti, v[q], v[q + 1], bc.BigPhi);
+#pragma unroll
+        for (int q = 0; q < 8; q += 4)
+            if (dj) v[q] = bc_rule<T>(tj, v[q], v[q + 2], bc.BigPhi);
+        return dk ? bc_rule<T>(tk, v[0], v[4], bc.BigPhi) : v[0];
+    }
 }
 
 template <typename T>
@@ -600,14 +628,15 @@ __device__ __forceinline__ int face_instance(const Inst* __restrict__ inst, int 
     return lo;
 }
 
-__device__ __forceinline__ bool face_coords(const Inst& I, long long r, int* pi, int* pj, int* pk) {
-    const long long nI = (long long)I.nj * I.nk, nJ = (long long)I.ni * I.nk, nK = (long long)I.ni * I.nj;
-    if (r < 2 * nI) { *pi = r < nI ? 0 : I.ni - 1; r %= nI; *pj = (int)(r % I.nj); *pk = (int)(r / I.nj); return true; }
+__device__ __forceinline__ bool face_coords(const Inst& I, unsigned r, int* pi, int* pj, int* pk) {
+    // an instance's face nodes number below 2^32, as its nodes do
+    const unsigned ni = I.ni, nj = I.nj, nk = I.nk, nI = nj * nk, nJ = ni * nk, nK = ni * nj;
+    if (r < 2 * nI) { *pi = r < nI ? 0 : I.ni - 1; r = r < nI ? r : r - nI; *pj = (int)(r % nj); *pk = (int)(r / nj); return true; }
     r -= 2 * nI;
-    if (r < 2 * nJ) { *pj = r < nJ ? 0 : I.nj - 1; r %= nJ; *pi = (int)(r % I.ni); *pk = (int)(r / I.ni); return true; }
+    if (r < 2 * nJ) { *pj = r < nJ ? 0 : I.nj - 1; r = r < nJ ? r : r - nJ; *pi = (int)(r % ni); *pk = (int)(r / ni); return true; }
     r -= 2 * nJ;
     if (r >= 2 * nK) return false;
-    *pk = r < nK ? 0 : I.nk - 1; r %= nK; *pi = (int)(r % I.ni); *pj = (int)(r / I.ni);
+    *pk = r < nK ? 0 : I.nk - 1; r = r < nK ? r : r - nK; *pi = (int)(r % ni); *pj = (int)(r / ni);
     return true;
 }
 
@@ -618,9 +647,9 @@ __global__ void k_bc_stage(const Inst* __restrict__ inst, int ninst, long long n
     if (t >= nface) return;
     const Inst& I = inst[face_instance(inst, ninst, t)];
     int i, j, k;
-    if (!face_coords(I, t - I.face0, &i, &j, &k)) return;
+    if (!face_coords(I, (unsigned)(t - I.face0), &i, &j, &k)) return;
     P0Stage<T> p0{phin, phi1, out, I.off, I.ni, (long long)I.ni * I.nj, I.ni, I.nj, I.nk, c1, c2};
-    out[I.off + i + p0.sj * j + p0.sk * k] = bval_k<T>(bc, p0, I.ni, I.nj, I.nk, i, j, k);
+    out[I.off + i + p0.sj * j + p0.sk * k] = bc_value<T, false>(bc, p0, I.ni, I.nj, I.nk, i, j, k);
 }
 
 // bcond_lsm on the faces of dst from the pre-BC field src (interior nodes
@@ -632,10 +661,10 @@ __global__ void k_bc_faces(const Inst* __restrict__ inst, int ninst, long long n
     if (t >= nface) return;
     const Inst& I = inst[face_instance(inst, ninst, t)];
     int i, j, k;
-    if (!face_coords(I, t - I.face0, &i, &j, &k)) return;
+    if (!face_coords(I, (unsigned)(t - I.face0), &i, &j, &k)) return;
     const long long sj = I.ni, sk = (long long)I.ni * I.nj;
     P0Src<T> p0{src, I.off, sj, sk};
-    const T v = bval_k<T>(bc, p0, I.ni, I.nj, I.nk, i, j, k);
+    const T v = bc_value<T, false>(bc, p0, I.ni, I.nj, I.nk, i, j, k);
     dst[I.off + i + sj * j + sk * k] = v;
     if (err && !vfinite(v)) atomicOr(err, (unsigned)kErrNonFinite);
 }
@@ -654,7 +683,7 @@ __global__ void __launch_bounds__(TX * TY * TZ) k_bc_full(const Inst* __restrict
         T v;
         if (bnd) {
             P0Src<T> p0{src, I.off, sj, sk};
-            v = bval_k<T>(bc, p0, I.ni, I.nj, I.nk, b.i, b.j, b.k);
+            v = bc_value<T, false>(bc, p0, I.ni, I.nj, I.nk, b.i, b.j, b.k);
         } else {
             v = src[l];
         }
@@ -991,9 +1020,9 @@ __global__ void k_bc_reinit(const Inst* __restrict__ inst, int ninst, long long 
     if (t >= nface) return;
     const Inst& I = inst[face_instance(inst, ninst, t)];
     int i, j, k;
-    if (!face_coords(I, t - I.face0, &i, &j, &k)) return;
+    if (!face_coords(I, (unsigned)(t - I.face0), &i, &j, &k)) return;
     P0Reinit<T> p0{f, din, dout, &I};
-    dout[I.off + i + (long long)I.ni * (j + (long long)I.nj * k)] = bval_k<T>(bc, p0, I.ni, I.nj, I.nk, i, j, k);
+    dout[I.off + i + (long long)I.ni * (j + (long long)I.nj * k)] = bc_value<T, true>(bc, p0, I.ni, I.nj, I.nk, i, j, k);
 }
 
 // ------------------------------------------------------------ volume
@@ -1747,13 +1776,6 @@ __global__ void k_cell_rel(long long off, int ni, int nj, int nk, const double* 
 // face rule's weights (the BigPhi switch evaluated on the forward value of
 // n2 at that point of the face sequence).  Distinct nodes of one plane have
 // distinct targets, so the kernel needs no atomics.
-template <typename T, class P0>
-__device__ __forceinline__ T prev_value(const BC& bc, const P0& p0, int face, int ni, int nj, int i, int j, int k) {
-    if (face < 2) return p0(i, j, k);
-    if (face < 4) return bval_i<T>(bc, p0, ni, i, j, k);
-    return bval_j<T>(bc, p0, ni, nj, i, j, k);
-}
-
 template <typename T>
 __global__ void k_adj_face(Flat fl, int face0, long long nplane, int nface, BC bc, int kind,
                            const T* __restrict__ phin, const T* __restrict__ in, const T* __restrict__ out, T c1, T c2,
@@ -1774,11 +1796,11 @@ __global__ void k_adj_face(Flat fl, int face0, long long nplane, int nface, BC b
         if (fl.inst[mid].fpre[ax] <= t) lo = mid; else hi = mid - 1;
     }
     const Inst& I = fl.inst[lo];
-    const long long r = t - I.fpre[ax];
+    const unsigned r = (unsigned)(t - I.fpre[ax]), ni = I.ni, nj = I.nj;
     int i, j, k;
-    if (ax == 0) { i = (face == 0) ? 0 : I.ni - 1; j = (int)(r % I.nj); k = (int)(r / I.nj); }
-    else if (ax == 1) { j = (face == 2) ? 0 : I.nj - 1; i = (int)(r % I.ni); k = (int)(r / I.ni); }
-    else { k = (face == 4) ? 0 : I.nk - 1; i = (int)(r % I.ni); j = (int)(r / I.ni); }
+    if (ax == 0) { i = (face == 0) ? 0 : I.ni - 1; j = (int)(r % nj); k = (int)(r / nj); }
+    else if (ax == 1) { j = (face == 2) ? 0 : I.nj - 1; i = (int)(r % ni); k = (int)(r / ni); }
+    else { k = (face == 4) ? 0 : I.nk - 1; i = (int)(r % ni); j = (int)(r / ni); }
     const int dir = (face & 1) ? -1 : 1;     // inward direction
     const long long sj = I.ni, sk = (long long)I.ni * I.nj;
     const long long st = ax == 0 ? 1 : (ax == 1 ? sj : sk);
@@ -1793,10 +1815,10 @@ __global__ void k_adj_face(Flat fl, int face0, long long nplane, int nface, BC b
         T v2;
         if (kind == 0) {
             P0Stage<T> p0{phin, in, out, I.off, sj, sk, I.ni, I.nj, I.nk, c1, c2};
-            v2 = prev_value<T>(bc, p0, face, I.ni, I.nj, i2, j2, k2);
+            v2 = bc_value<T, false>(bc, p0, I.ni, I.nj, I.nk, i2, j2, k2, ax);
         } else {
             P0Src<T> p0{out, I.off, sj, sk};
-            v2 = prev_value<T>(bc, p0, face, I.ni, I.nj, i2, j2, k2);
+            v2 = bc_value<T, false>(bc, p0, I.ni, I.nj, I.nk, i2, j2, k2, ax);
         }
         if (fabs(v2) >= T(bc.BigPhi)) { a = T(1); c = T(0); }
         else { a = T(4.0 / 3.0); c = T(-1.0 / 3.0); }
@@ -1941,7 +1963,7 @@ __global__ void __launch_bounds__(256) k_adj_stage_x(const Inst* __restrict__ in
 // windows of five G, lamP0 and D values in registers; lam_in -= c3 acc,
 // lamW_AX -= c3 lamP0 D.
 template <typename T, int AX, bool FULL>
-__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : (AX == 2 ? 5 : 4)) k_adj_stage_m(const Inst* __restrict__ inst, Tiles tl, FieldsT<T> f, const T* __restrict__ in, const T* __restrict__ lamP0, T* __restrict__ lam_in,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 && AX == 2 ? 5 : 0) k_adj_stage_m(const Inst* __restrict__ inst, Tiles tl, FieldsT<T> f, const T* __restrict__ in, const T* __restrict__ lamP0, T* __restrict__ lam_in,
         T* __restrict__ lamW, T c3) {
     const int tx = threadIdx.x & 31, tq = threadIdx.x >> 5;
     for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {

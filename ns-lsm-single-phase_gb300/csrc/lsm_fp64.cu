@@ -280,57 +280,66 @@ void launch_weno(const DevGrid& g, const StageArgs& a, cudaStream_t s) {
 // bcond_lsm, src/bcond_lsm.F90:2-287.  The six faces are applied in the
 // order i1, im, j1, jm, k1, km, each reading the two nodes inward of it as
 // left by the faces before it.  A boundary node's final value is therefore a
-// fixed function of the pre-BC field ("P0"): val_k(val_j(val_i(P0))).  Each
-// thread evaluates that chain for one boundary node reading P0 only, so the
-// kernel never reads a node that another thread writes.
-struct BCRule {
-    __device__ static double ext(double n1, double n2, double BigPhi) {
-        const double a2 = 4.0 / 3.0, b2 = -1.0 / 3.0, a1 = 1.0, b1 = 0.0;
-        const double exsign = (1.0 + copysign(1.0, fabs(n2) - BigPhi)) / 2.0;
-        const double itpa = a2 + exsign * (a1 - a2);
-        const double itpb = b2 + exsign * (b1 - b2);
-        return itpa * n1 + itpb * n2;
-    }
-    __device__ static double apply(int type, int face, double n1, double n2, double BigPhi) {
-        if (type == 0) return n1;
-        if (type == 1) return ext(n1, n2, BigPhi);
-        (void)face;
-        return 2.0 * n1 - 1.0 * n2;  // type 2, only on the im face
-    }
-};
-
-__device__ __forceinline__ bool face_applies(const DevBC& bc, int face, int phys) {
-    const int t = bc.type[face];
-    return phys && (t == 0 || t == 1 || (t == 2 && face == 1));
+// fixed function of the pre-BC field ("P0"): per axis whose face rule applies
+// to the node, the rule on its values at the two nodes inward along that
+// axis, i innermost, then j, then k.  Each thread evaluates that chain for
+// one boundary node reading P0 only, so the kernel never reads a node that
+// another thread writes.  A node of one face reads two values; the loops
+// keep the edge's four and the corner's eight out of its way (written out as
+// nested calls, a warp walked all 27 evaluations: 22 us on the smallest
+// grids, launch and timer included; 8 us so).
+//
+// One rule: itpa n1 + itpb n2 with itpa = 4/3 + ex (1 - 4/3), itpb = -1/3 +
+// ex (0 + 1/3), ex = 1 where |n2| >= BigPhi: 1 and 0 exactly, else 4/3 and
+// -1/3.
+__device__ __forceinline__ double bc_rule(const DevBC& bc, int face, double n1, double n2) {
+    const int type = bc.type[face];
+    if (type == 0) return n1;
+    const u64 big = d2u(bc.BigPhi) >> 63 ? 0u : d2u(bc.BigPhi);
+    const bool first = mag(n2) >= big;
+    const double a = type == 2 ? 2.0 : (first ? 1.0 : 4.0 / 3.0);   // type 2: 2 n1 - n2, only on the im face
+    const double b = type == 2 ? -1.0 : (first ? 0.0 : -1.0 / 3.0);
+    return a * n1 + b * n2;
 }
 
-template <class P0>
-__device__ double val_i(const DevGrid& g, const DevBC& bc, const P0& p0, int i, int j, int k) {
-    if (i == g.ia && face_applies(bc, 0, g.pb))
-        return BCRule::apply(bc.type[0], 0, p0(i + 1, j, k), p0(i + 2, j, k), bc.BigPhi);
-    if (i == g.ib && face_applies(bc, 1, g.pf))
-        return BCRule::apply(bc.type[1], 1, p0(i - 1, j, k), p0(i - 2, j, k), bc.BigPhi);
-    return p0(i, j, k);
+// direction inward and face of the rule that applies at coordinate c (0: none)
+__device__ __forceinline__ int bc_dir(const DevBC& bc, int c, int lo, int hi, int plo, int phs, int face, int* f) {
+    auto on = [&](int q) { return bc.type[q] == 0 || bc.type[q] == 1 || (bc.type[q] == 2 && q == 1); };
+    if (plo && c == lo && on(face)) { *f = face; return 1; }
+    if (phs && c == hi && on(face + 1)) { *f = face + 1; return -1; }
+    *f = face;
+    return 0;
 }
+
 template <class P0>
-__device__ double val_j(const DevGrid& g, const DevBC& bc, const P0& p0, int i, int j, int k) {
-    if (j == g.ja && face_applies(bc, 2, g.pl))
-        return BCRule::apply(bc.type[2], 2, val_i(g, bc, p0, i, j + 1, k), val_i(g, bc, p0, i, j + 2, k),
-                             bc.BigPhi);
-    if (j == g.jb && face_applies(bc, 3, g.pr))
-        return BCRule::apply(bc.type[3], 3, val_i(g, bc, p0, i, j - 1, k), val_i(g, bc, p0, i, j - 2, k),
-                             bc.BigPhi);
-    return val_i(g, bc, p0, i, j, k);
-}
-template <class P0>
-__device__ double val_k(const DevGrid& g, const DevBC& bc, const P0& p0, int i, int j, int k) {
-    if (k == g.ka && face_applies(bc, 4, g.pd))
-        return BCRule::apply(bc.type[4], 4, val_j(g, bc, p0, i, j, k + 1), val_j(g, bc, p0, i, j, k + 2),
-                             bc.BigPhi);
-    if (k == g.kb && face_applies(bc, 5, g.pu))
-        return BCRule::apply(bc.type[5], 5, val_j(g, bc, p0, i, j, k - 1), val_j(g, bc, p0, i, j, k - 2),
-                             bc.BigPhi);
-    return val_j(g, bc, p0, i, j, k);
+__device__ __forceinline__ double bc_value(const DevGrid& g, const DevBC& bc, const P0& p0, int i, int j, int k) {
+    int fi, fj, fk;
+    const int di = bc_dir(bc, i, g.ia, g.ib, g.pb, g.pf, 0, &fi), dj = bc_dir(bc, j, g.ja, g.jb, g.pl, g.pr, 2, &fj),
+              dk = bc_dir(bc, k, g.ka, g.kb, g.pd, g.pu, 4, &fk);
+    if ((di != 0) + (dj != 0) + (dk != 0) == 1) {   // one face: both values in flight at once
+        const double n1 = p0(i + di, j + dj, k + dk), n2 = p0(i + 2 * di, j + 2 * dj, k + 2 * dk);
+        return bc_rule(bc, di ? fi : dj ? fj : fk, n1, n2);
+    }
+    double vk = 0.0;
+#pragma unroll 1
+    for (int a = 0; a < (dk ? 2 : 1); ++a) {
+        double vj = 0.0;
+#pragma unroll 1
+        for (int b = 0; b < (dj ? 2 : 1); ++b) {
+            double vi = 0.0;
+#pragma unroll 1
+            for (int c = 0; c < (di ? 2 : 1); ++c) {
+                const double v = p0(di ? i + di * (c + 1) : i, dj ? j + dj * (b + 1) : j, dk ? k + dk * (a + 1) : k);
+                if (c == 0) vi = v;
+                else vi = bc_rule(bc, fi, vi, v);
+            }
+            if (b == 0) vj = vi;
+            else vj = bc_rule(bc, fj, vj, vi);
+        }
+        if (a == 0) vk = vj;
+        else vk = bc_rule(bc, fk, vk, vj);
+    }
+    return vk;
 }
 
 __device__ __forceinline__ bool on_phys_face(const DevGrid& g, int i, int j, int k) {
@@ -364,20 +373,29 @@ struct P0Field {
 
 // Boundary nodes of the six face planes (edge nodes appear twice and are
 // written twice with the same value).
-__device__ __forceinline__ bool face_node(const DevGrid& g, long long t, int* pi, int* pj, int* pk) {
-    const long long Ni = g.ib - g.ia + 1, Nj = g.jb - g.ja + 1, Nk = g.kb - g.ka + 1;
-    const long long nI = Nj * Nk, nJ = Ni * Nk, nK = Ni * Nj;
-    const long long off[6] = {0, nI, 2 * nI, 2 * nI + nJ, 2 * nI + 2 * nJ, 2 * nI + 2 * nJ + nK};
-    int f = 5;
-    for (int q = 1; q < 6; ++q)
-        if (t < off[q]) { f = q - 1; break; }
-    if (t >= off[5] + nK) return false;
-    const long long r = t - off[f];
-    const int phys[6] = {g.pb, g.pf, g.pl, g.pr, g.pd, g.pu};
-    if (!phys[f]) return false;
-    if (f < 2) { *pi = f == 0 ? g.ia : g.ib; *pj = g.ja + (int)(r % Nj); *pk = g.ka + (int)(r / Nj); }
-    else if (f < 4) { *pj = f == 2 ? g.ja : g.jb; *pi = g.ia + (int)(r % Ni); *pk = g.ka + (int)(r / Ni); }
-    else { *pk = f == 4 ? g.ka : g.kb; *pi = g.ia + (int)(r % Ni); *pj = g.ja + (int)(r / Ni); }
+__device__ __forceinline__ bool face_node(const DevGrid& g, unsigned t, int* pi, int* pj, int* pk) {
+    const unsigned Ni = g.ib - g.ia + 1, Nj = g.jb - g.ja + 1, Nk = g.kb - g.ka + 1;
+    const unsigned nI = Nj * Nk, nJ = Ni * Nk, nK = Ni * Nj;   // below 2^32 in all, as the nodes are
+    if (t < 2 * nI) {
+        const bool up = t >= nI;
+        if (!(up ? g.pf : g.pb)) return false;
+        const unsigned r = up ? t - nI : t;
+        *pi = up ? g.ib : g.ia; *pj = g.ja + (int)(r % Nj); *pk = g.ka + (int)(r / Nj);
+        return true;
+    }
+    t -= 2 * nI;
+    if (t < 2 * nJ) {
+        const bool up = t >= nJ;
+        if (!(up ? g.pr : g.pl)) return false;
+        const unsigned r = up ? t - nJ : t;
+        *pj = up ? g.jb : g.ja; *pi = g.ia + (int)(r % Ni); *pk = g.ka + (int)(r / Ni);
+        return true;
+    }
+    t -= 2 * nJ;
+    const bool up = t >= nK;
+    if (t >= 2 * nK || !(up ? g.pu : g.pd)) return false;
+    const unsigned r = up ? t - nK : t;
+    *pk = up ? g.kb : g.ka; *pi = g.ia + (int)(r % Ni); *pj = g.ja + (int)(r / Ni);
     return true;
 }
 
@@ -385,8 +403,8 @@ __global__ void bc_rk_kernel(DevGrid g, DevBC bc, P0Stage p0, double* __restrict
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= nface) return;
     int i, j, k;
-    if (!face_node(g, t, &i, &j, &k)) return;
-    dst[gid(g, i, j, k)] = val_k(g, bc, p0, i, j, k);
+    if (!face_node(g, (unsigned)t, &i, &j, &k)) return;
+    dst[gid(g, i, j, k)] = bc_value(g, bc, p0, i, j, k);
 }
 
 // dst = bcond_lsm(src) over the full array (ghosts copied); flags non-finite output.
@@ -399,12 +417,12 @@ __global__ void bc_full_kernel(DevGrid g, DevBC bc, const double* __restrict__ s
     double v;
     if (non_ghost(g, i, j, k) && on_phys_face(g, i, j, k)) {
         P0Field p0{g, src};
-        v = val_k(g, bc, p0, i, j, k);
+        v = bc_value(g, bc, p0, i, j, k);
     } else {
         v = src[l];
     }
     dst[l] = v;
-    if (errflag && !isfinite(v)) atomicOr(errflag, (unsigned)kErrNonFinite);
+    if (errflag && !finite64(v)) atomicOr(errflag, (unsigned)kErrNonFinite);
 }
 
 // ------------------------------------------------------------ R1 / R2 ----
@@ -677,7 +695,7 @@ void launch_bc_rk(const DevGrid& g, const DevBC& bc, int orderAD, const double* 
     const long long nface = 2 * (Nj * Nk + Ni * Nk + Ni * Nj);
     P0Stage p0{g, orderAD, phin, phi1, ucn, aj, dst, mask, c1, c2, c3, dt};
     ProfScope ps_("bc_rk_kernel", s);
-    bc_rk_kernel<<<(unsigned)((nface + 255) / 256), 256, 0, s>>>(g, bc, p0, dst, nface);
+    bc_rk_kernel<<<(unsigned)((nface + 127) / 128), 128, 0, s>>>(g, bc, p0, dst, nface);
 }
 
 void launch_bc_full(const DevGrid& g, const DevBC& bc, const double* src, double* dst, unsigned* errflag,
