@@ -317,6 +317,7 @@ BATCH = dict(n_inst=64, lo=32, hi=96, seed=0, reinit_iters=5, cfl=0.5)
 BATCH_ALGO_BYTES = {
     "k_stage_z": 17.0 / 3.0 * 4,   # phi_prev, phi^n (stages 2-3), W(3); phi
     "k_reinit_z": 12.0 * 4,      # d, s, metrics(9); d
+    "k_reinit_pair": 12.0 * 4,   # the same for two pseudo-steps
     "k_sign_reinit_z": 12.0 * 4, # phi0, metrics(9); s, d
     "k_reinit": 12.0 * 4,        # brick-table pseudo-step: d, s, metrics(9); d
     "k_sign_reinit": 12.0 * 4,   # brick-table first pseudo-step: phi0, metrics(9); s, d
@@ -552,6 +553,7 @@ FWDADJ_BYTES = {
     "k_contra": 15 * 4,            # u(3), metrics(9); W(3)
     "k_stage_z": 17.0 / 3.0 * 4,     # phi_prev, phi^n (stages 2-3), W(3); stage output
     "k_reinit_z": 12 * 4,          # d, s, metrics(9); d
+    "k_reinit_pair": 12 * 4,       # the same for two pseudo-steps
     "k_sign_reinit_z": 12 * 4,     # phi0, metrics(9); s, d
     "k_reinit_rec_z": 18 * 4,      # d, s, metrics(9); d, adjoint coefficients(6)
     "k_sign_reinit_rec_z": 18 * 4, # phi0, metrics(9); s, d, adjoint coefficients(6)

@@ -72,7 +72,8 @@ typedef struct lsm_batch_config {
     int use_graph;      /* 1: capture the per-step launches in a CUDA graph */
     int autotune;       /* 1: time the candidates on this batch and keep the fastest */
     int shape;          /* when autotune == 0: 0..4 tile shape (pseudo-steps on the brick
-                           table), 5 tile shape 0 with the pseudo-steps marching in k */
+                           table), 5 tile shape 0 with the pseudo-steps marching in k,
+                           FP32 ones two at a time */
     int precision;      /* 0: FP32 stencils, 1: FP64 stencils (tile shape 0, no autotune) */
     int adjoint_mode;   /* 0: recorded pseudo-steps store their adjoint coefficients (6 arrays
                            each; the reverse sweep is a stencil), 1: the reverse sweep

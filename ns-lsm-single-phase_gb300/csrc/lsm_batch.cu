@@ -693,44 +693,64 @@ __global__ void __launch_bounds__(TX * TY * TZ) k_bc_full(const Inst* __restrict
 }
 
 // ------------------------------------------------------------ Godunov |grad|
-// One-sided differences (calc_RH_RN.F90:36-170) along one axis: mas
-// (forward) and men (backward); on a physical face both take the one
-// available difference.
+// max(a, b) with a NaN a dropped (b is not one)
+template <typename T> __device__ __forceinline__ T pmax(T a, T b) { return a > b ? a : b; }
+template <> __device__ __forceinline__ float pmax<float>(float a, float b) { return fmaxf(a, b); }
+
+// One-sided differences (calc_RH_RN.F90:36-170) along one axis times the
+// branch sign sg (+-1: the product with it is exact): mas (forward) and men
+// (backward); on a physical face both take the one available difference.
 template <typename T>
-__device__ __forceinline__ void one_sided(const T* __restrict__ d, long long l, long long s, int c, int n, T* mas,
-                                          T* men) {
-    const T x = __ldg(d + l);
-    const T a = c < n - 1 ? __ldg(d + l + s) - x : T(0);
-    const T b = c > 0 ? x - __ldg(d + l - s) : T(0);
+__device__ __forceinline__ void one_sided(const T* __restrict__ d, long long l, long long s, int c, int n, T sg, T sx,
+                                          T* mas, T* men) {
+    // both loads unconditional (the node itself past a face): none waits for a branch
+    const T a = vfma(sg, __ldg(d + (c < n - 1 ? l + s : l)), -sx), b = vfma(-sg, __ldg(d + (c > 0 ? l - s : l)), sx);
     *mas = c < n - 1 ? a : b;
     *men = c > 0 ? b : a;
 }
 
-template <typename T>
-__device__ __forceinline__ void godunov_diffs(const T* __restrict__ d, const Inst& I, long long l, int i, int j, int k,
-                                              T (&mas)[3], T (&men)[3]) {
-    one_sided(d, l, 1, i, I.ni, &mas[0], &men[0]);
-    one_sided(d, l, (long long)I.ni, j, I.nj, &mas[1], &men[1]);
-    one_sided(d, l, (long long)I.ni * I.nj, k, I.nk, &mas[2], &men[2]);
-}
-
-// Godunov norm (calc_RH_RN.F90:190-236) chosen by the sign s
-template <typename T>
-__device__ __forceinline__ T godunov(const FieldsT<T>& f, const T* __restrict__ d, const Inst& I, long long l, int i,
-                                     int j, int k, T s) {
-    T mas[3], men[3];
-    godunov_diffs(d, I, l, i, j, k, mas, men);
+// Godunov norm squared (calc_RH_RN.F90:190-236) from those differences.
+// With P the positive part of the backward and -Q that of the negated forward
+// product, max(P^2, Q^2) is the square of the larger.  SEL: the selections
+// too, per axis the P taken (e) or the Q taken (g).
+template <bool SEL, typename T>
+__device__ __forceinline__ T godunov_sel_v(const T (&mas)[3], const T (&men)[3], const T (&M)[9], T (&e)[3],
+                                           T (&g)[3]) {
     T acc = T(0);
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
-        const T m0 = __ldg(f.m[x] + l), m1 = __ldg(f.m[3 + x] + l), m2 = __ldg(f.m[6 + x] + l);
-        const T bb = m0 * men[0] + m1 * men[1] + m2 * men[2];
-        const T ff = m0 * mas[0] + m1 * mas[1] + m2 * mas[2];
-        const T P = s > T(0) ? vmax(bb, T(0)) : vmin(bb, T(0));
-        const T Q = s > T(0) ? vmin(ff, T(0)) : vmax(ff, T(0));
-        acc += vmax(P * P, Q * Q);
+        const T bb = vfma(M[6 + x], men[2], vfma(M[3 + x], men[1], M[x] * men[0]));
+        const T ff = vfma(M[6 + x], mas[2], vfma(M[3 + x], mas[1], M[x] * mas[0]));
+        // max(P^2, Q^2) is the square of the larger of P and -Q
+        const T p = pmax(bb, T(0)), v = pmax(-ff, p);
+        acc = vfma(v, v, acc);
+        if (SEL) {
+            const bool takeP = p * p >= v * v;
+            e[x] = takeP ? p : T(0);
+            g[x] = takeP ? T(0) : -v;
+        }
     }
-    return vsqrt(acc);
+    return acc;
+}
+
+// Godunov norm chosen by the sign s
+template <typename T>
+__device__ __forceinline__ T godunov(const FieldsT<T>& f, const T* __restrict__ d, const Inst& I, long long l, int i,
+                                     int j, int k, T x, T s) {
+    T mas[3], men[3], M[9], e[3], g[3];
+#pragma unroll
+    for (int c = 0; c < 9; ++c) M[c] = __ldg(f.m[c] + l);
+    const T sg = s > T(0) ? T(1) : T(-1), sx = sg * x;
+    one_sided(d, l, 1, i, I.ni, sg, sx, &mas[0], &men[0]);
+    one_sided(d, l, (long long)I.ni, j, I.nj, sg, sx, &mas[1], &men[1]);
+    one_sided(d, l, (long long)I.ni * I.nj, k, I.nk, sg, sx, &mas[2], &men[2]);
+    return vsqrt(godunov_sel_v<false>(mas, men, M, e, g));
+}
+
+// the pseudo-step's value from the norm G (every kernel's, bit for bit)
+template <typename T>
+__device__ __forceinline__ T reinit_value(T d, T s, T dtau, T G) {
+    return s == T(0) ? d : vfma(-(dtau * s), G - T(1), d);
 }
 
 // calc_sign_ini (Kang sign) with the frozen band folded in: s = 0 where
@@ -751,8 +771,8 @@ __device__ __forceinline__ T reinit_node(const FieldsT<T>& f, const T* __restric
     // every load is issued before the frozen-node test (one memory round trip)
     const T s = __ldg(f.sgn + l);
     const T d = __ldg(din + l);
-    const T g = godunov(f, din, I, l, i, j, k, s);
-    return s == T(0) ? d : d - ipar<T>(I.dtau, I.dtau64) * s * (g - T(1));
+    const T g = godunov(f, din, I, l, i, j, k, d, s);
+    return reinit_value(d, s, ipar<T>(I.dtau, I.dtau64), g);
 }
 
 template <typename T, int TX, int TY, int TZ>
@@ -785,10 +805,10 @@ __global__ void __launch_bounds__(TX * TY * TZ) k_sign_reinit(const Inst* __rest
         const Inst& I = inst[b.inst];
         const long long l = I.off + b.i + (long long)I.ni * (b.j + (long long)I.nj * b.k);
         const T p = __ldg(phi0 + l);
-        const T g = godunov(f, phi0, I, l, b.i, b.j, b.k, p > T(0) ? T(1) : T(-1));
+        const T g = godunov(f, phi0, I, l, b.i, b.j, b.k, p, p);
         const T s = sign_of(p, g, ipar<T>(I.eps, I.eps64));
         f.sgn[l] = s;
-        const T r = s == T(0) ? p : p - ipar<T>(I.dtau, I.dtau64) * s * (g - T(1));
+        const T r = reinit_value(p, s, ipar<T>(I.dtau, I.dtau64), g);
         dout[l] = r;
         if (err && !vfinite(r)) atomicOr(err, (unsigned)kErrNonFinite);
     }
@@ -803,25 +823,6 @@ __global__ void __launch_bounds__(TX * TY * TZ) k_sign_reinit(const Inst* __rest
 // serves both sides), and the pseudo-step's adjoint is
 //   lam_out(j) = lam(j) - sum_m [lam(j) (A'_m - B'_m)(j)
 //                - lam(j+e_m) A'_m(j+e_m) + lam(j-e_m) B'_m(j-e_m)].
-// acc is accumulated exactly as in godunov() (bit-identical pseudo-step).
-template <typename T>
-__device__ __forceinline__ T godunov_sel_v(const T (&mas)[3], const T (&men)[3], const T (&M)[9], T sel, T (&e)[3],
-                                           T (&g)[3]) {
-    const T sg = sel > T(0) ? T(1) : T(-1);
-    T acc = T(0);
-#pragma unroll
-    for (int x = 0; x < 3; ++x) {
-        const T bb = sg * (M[x] * men[0] + M[3 + x] * men[1] + M[6 + x] * men[2]);
-        const T ff = sg * (M[x] * mas[0] + M[3 + x] * mas[1] + M[6 + x] * mas[2]);
-        const T p = vmax(bb, T(0)), q = vmin(ff, T(0));
-        const bool takeP = p * p >= q * q;
-        acc += takeP ? p * p : q * q;
-        e[x] = takeP ? p : T(0);
-        g[x] = takeP ? T(0) : q;
-    }
-    return acc;
-}
-
 // One reinitialisation pseudo-step on the tiles of adjoint map 2 (32 x 8
 // columns marching 32 planes in k): each node loads d (and s) and its
 // metrics once, a plane ahead; the z neighbours of d stay in a register
@@ -880,23 +881,23 @@ __global__ void __launch_bounds__(256) k_reinit_z(const Inst* __restrict__ inst,
                 const T dxm = tx == 0 ? pc.dxe : xl, dxp = tx == 31 ? pc.dxe : xr;
                 const T nbm[3] = {dxm, pc.dym, dm}, nbp[3] = {dxp, pc.dyp, dp};
                 const bool lo[3] = {!xm, !ym, k == 0}, hi[3] = {!xp, !yp, k == nk - 1};
+                const T sg = (SIGN ? dc : pc.s) > T(0) ? T(1) : T(-1), sc = sg * dc;
                 T mas[3], men[3];
 #pragma unroll
                 for (int m = 0; m < 3; ++m) {
-                    const T a = hi[m] ? T(0) : nbp[m] - dc;
-                    const T b = lo[m] ? T(0) : dc - nbm[m];
+                    const T a = vfma(sg, nbp[m], -sc), b = vfma(-sg, nbm[m], sc);
                     mas[m] = hi[m] ? b : a;
                     men[m] = lo[m] ? a : b;
                 }
                 T e[3], g[3];
                 const long long l = cb + sk * k;
-                const T acc = godunov_sel_v(mas, men, pc.M, SIGN ? (dc > T(0) ? T(1) : T(-1)) : pc.s, e, g);
+                const T acc = godunov_sel_v<REC>(mas, men, pc.M, e, g);
                 T s = pc.s;
                 if (SIGN) {
                     s = sign_of(dc, vsqrt(acc), eps);
                     f.sgn[l] = s;
                 }
-                const T r = s == T(0) ? dc : dc - dtau * s * (vsqrt(acc) - T(1));
+                const T r = reinit_value(dc, s, dtau, vsqrt(acc));
                 dout[l] = r;
                 if (dout2) dout2[l] = r;
                 if (REC) {
@@ -916,6 +917,132 @@ __global__ void __launch_bounds__(256) k_reinit_z(const Inst* __restrict__ inst,
             dp = dn;
             pc = pn;
         }
+    }
+}
+
+// Two pseudo-steps of the FP32 batch in one pass over the metrics.  A
+// pseudo-step is bound by its bytes, twelve words per node, and by the issue
+// of its instructions; nine of the words are the metrics, which two steps
+// share, and the field between the steps stays on the chip.  Measured on 64
+// grids of 32..96: 2 x 170 us -> 242 us (512 threads; 266 with 384).  (With the adjoint coefficients, whose
+// twelve words per node and pair are written all the same, the pair was
+// slower than two recorded steps: 884 against 790 us on 512 x 256 x 256.)
+//
+// A tile is rw x rh columns of one instance plus, where it does not span the
+// instance, a rim of one column, in row-major order over the threads (Inst's
+// rw, rh: whole rows where the instance is narrow, so that few lanes idle).
+// The block marches in k.  Iteration k evaluates the first step on plane k at
+// every thread, from d in a register window in z and in shared memory in x
+// and y (the values just outside the rim come there by one more load of some
+// threads), and the second step on plane k - 1 inside the rim, from the first
+// step's planes k - 2 .. k.  One barrier per plane: the shared planes rotate
+// over three buffers, in step with the three planes' registers, and each is
+// written again only after a barrier that follows its last read.  A node's
+// loads go out one plane ahead, on 32-bit byte offsets from the arrays'
+// bases (the batch is below 2^30 nodes).  The arithmetic is k_reinit_z's.
+struct PairPlane {
+    float s, M[9], o;   // sign, metrics, the thread's value outside the rim
+};
+constexpr int kPairSmem = 3 * (kPairThreads + 2);   // (ew + 2) (eh + 2) for ew eh <= kPairThreads
+__device__ __forceinline__ float ldo(const float* p, unsigned o) {
+    return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + o));
+}
+__device__ __forceinline__ void sto(float* p, unsigned o, float v) {
+    *reinterpret_cast<float*>(reinterpret_cast<char*>(p) + o) = v;
+}
+__global__ void __launch_bounds__(kPairThreads, 2) k_reinit_pair(const Inst* __restrict__ inst, Tiles tl,
+        FieldsT<float> f, const float* __restrict__ din, float* __restrict__ dout, float* __restrict__ dout2,
+        unsigned* err) {
+    __shared__ float sd[3][kPairSmem], se[3][kPairSmem];
+    const int t = threadIdx.x;
+    for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {
+        const ABrick ab = adj_brick(tl, blk);
+        const Inst& I = inst[ab.inst];
+        const int ni = I.ni, nj = I.nj, nk = I.nk;
+        const int ox = I.rw < ni ? 1 : 0, oy = I.rh < nj ? 1 : 0;
+        const int ew = I.rw + 2 * ox, eh = I.rh + 2 * oy, pitch = ew + 2;
+        const int y = t / ew, x = t - y * ew;
+        const int i = ab.i0 + x - ox, j = ab.j0 + y - oy;
+        const bool col = y < eh && i >= 0 && i < ni && j >= 0 && j < nj;
+        const bool core = col && x >= ox && x < I.rw + ox && y >= oy && y < I.rh + oy;
+        const int k0 = ab.k0, k1 = min(k0 + tl.len, nk);
+        const unsigned sk = 4u * (unsigned)ni * (unsigned)nj;
+        const unsigned base = 4u * (unsigned)I.off;
+        const unsigned cb = base + 4u * (unsigned)(i + ni * j);
+        const bool xm = i == 0, xp = i == ni - 1, ym = j == 0, yp = j == nj - 1;
+        // slot in the shared planes, and the value outside the rim that this
+        // thread brings there: rows -1 and eh, then columns -1 and ew
+        const int me = min(y + 1, eh) * pitch + x + 1;
+        int hx = -1, hy = -1;
+        if (t < 2 * ew) { hx = t < ew ? t : t - ew; hy = t < ew ? -1 : eh; }
+        else if (t < 2 * (ew + eh)) { const int r = t - 2 * ew; hy = r < eh ? r : r - eh; hx = r < eh ? -1 : ew; }
+        const int hi_ = ab.i0 + hx - ox, hj = ab.j0 + hy - oy;
+        const bool hok = t < 2 * (ew + eh) && hi_ >= 0 && hi_ < ni && hj >= 0 && hj < nj;
+        const int hs = (hy + 1) * pitch + hx + 1;
+        const unsigned hb = base + 4u * (unsigned)(hi_ + ni * hj);
+        const float dtau = I.dtau;
+        auto ldd = [&](int k) { return col && k >= 0 && k < nk ? ldo(din, cb + sk * (unsigned)k) : 0.f; };
+        auto ld_plane = [&](int k, PairPlane& p) {
+            if (k >= nk) return;
+            if (hok) p.o = ldo(din, hb + sk * (unsigned)k);
+            if (!col) return;
+            const unsigned l = cb + sk * (unsigned)k;
+            p.s = ldo(f.sgn, l);
+#pragma unroll
+            for (int c = 0; c < 9; ++c) p.M[c] = ldo(f.m[c], l);
+        };
+        // one pseudo-step at a node of plane k from its neighbours' values
+        auto step = [&](float dc, const float* P, float zl, float zr, int k, const PairPlane& p) {
+            const float nbm[3] = {P[me - 1], P[me - pitch], zl}, nbp[3] = {P[me + 1], P[me + pitch], zr};
+            const bool lo[3] = {xm, ym, k == 0}, hi[3] = {xp, yp, k == nk - 1};
+            const float sg = p.s > 0.f ? 1.f : -1.f, sc = sg * dc;
+            float mas[3], men[3], e[3], g[3];
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                const float a = fmaf(sg, nbp[m], -sc), b = fmaf(-sg, nbm[m], sc);
+                mas[m] = hi[m] ? b : a;
+                men[m] = lo[m] ? a : b;
+            }
+            return reinit_value(dc, p.s, dtau, vsqrt(godunov_sel_v<false>(mas, men, p.M, e, g)));
+        };
+        const int ks = max(k0 - 1, 0);
+        float dm = ldd(ks - 1), dc = ldd(ks), dp = ldd(ks + 1);
+        float em = 0.f, ec = 0.f;   // the first step's values at planes k - 2, k - 1
+        PairPlane p0, p1, p2;
+        ld_plane(ks, p1);
+        auto plane = [&](int k, PairPlane& pm, PairPlane& pc, PairPlane& pn, float* D, float* E, const float* Em) {
+            const float dn = ldd(k + 2);
+            if (k < k1) ld_plane(k + 1, pn);
+            if (y < eh) D[me] = dc;
+            if (hok) D[hs] = pc.o;
+            __syncthreads();
+            float e1 = 0.f;
+            if (col && k < nk) e1 = step(dc, D, dm, dp, k, pc);
+            if (core && k > k0) {
+                const float r = step(ec, Em, em, e1, k - 1, pm);
+                const unsigned l = cb + sk * (unsigned)(k - 1);
+                sto(dout, l, r);
+                if (dout2) sto(dout2, l, r);
+                if (err && !vfinite(r)) atomicOr(err, (unsigned)kErrNonFinite);
+            }
+            if (y < eh) E[me] = e1;
+            em = ec;
+            ec = e1;
+            dm = dc;
+            dc = dp;
+            dp = dn;
+        };
+        // planes ks .. k1 (k1 = nk: the second step alone), three at a time so
+        // that registers and buffers keep their places
+        for (int k = ks;;) {
+            plane(k, p0, p1, p2, sd[1], se[1], se[0]);
+            if (++k > k1) break;
+            plane(k, p1, p2, p0, sd[2], se[2], se[1]);
+            if (++k > k1) break;
+            plane(k, p2, p0, p1, sd[0], se[0], se[2]);
+            if (++k > k1) break;
+        }
+        __syncthreads();   // the next tile writes the buffers that this one's last plane reads
     }
 }
 
@@ -2347,6 +2474,16 @@ void reinit_z(int kind, int grid, const Inst* inst, Tiles tl, FieldsT<T> f, cons
         break;
     }
     }
+}
+void reinit_pair(int grid, const Inst* inst, Tiles tl, FieldsT<float> f, const float* din, float* dout, float* dout2,
+                 unsigned* err, cudaStream_t s) {
+    ProfScope ps_("k_reinit_pair", s);
+    k_reinit_pair<<<grid, kPairThreads, 0, s>>>(inst, tl, f, din, dout, dout2, err);
+}
+int reinit_pair_blocks_per_sm() {
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_reinit_pair, kPairThreads, 0);
+    return n;
 }
 template <typename T>
 int reinit_z_blocks_per_sm() {

@@ -30,6 +30,7 @@ struct Inst {
     long long face0;   // first boundary-face node of the instance (forward bc kernels)
     long long fpre[3]; // first node of the instance's i-, j-, k-face planes (adjoint face kernels)
     double dt64, dtau64, eps64;  // the same three parameters for the FP64 kernels
+    int rw, rh;                  // columns of a tile of reinit_pair, without its rim
     int am[kMaps][3];            // adjoint brick maps (adj_shape): first brick, bricks per row, per plane
 };
 
@@ -165,6 +166,13 @@ void reinit_z(int kind, int grid, const Inst* inst, Tiles tl, FieldsT<T> f, cons
               T* dout2, T* cf, long long ld, unsigned* err, cudaStream_t s);
 template <typename T>
 int reinit_z_blocks_per_sm();
+// Two plain pseudo-steps in one pass (FP32, fewer than 2^30 nodes), on tiles
+// of Inst's rw x rh columns (their table holds each tile's first node); dout
+// must not be din; dout2 (nullable) gets a second copy of the output
+constexpr int kPairThreads = 512;
+void reinit_pair(int grid, const Inst* inst, Tiles tl, FieldsT<float> f, const float* din, float* dout, float* dout2,
+                 unsigned* err, cudaStream_t s);
+int reinit_pair_blocks_per_sm();
 // water volume of every instance: the cells' 64-bit fixed-point sums (K, S,
 // bulk and, with `slope`, dK/dC) are added to acc[4 * inst + c] (zero on
 // entry) by a streaming pass over the tiles of map 2 (grid2 CTAs) that also

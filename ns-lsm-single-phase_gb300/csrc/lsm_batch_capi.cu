@@ -71,6 +71,9 @@ struct lsm_batch {
     int len[lsm::batch::kMaps] = {};         // march lengths of the maps' tiles
     int sgrid = 1, acgrid = 1, rzgrid = 1;   // CTAs of the map-2 kernels: stage, k_adj_reinit_c, reinit_z
     int vgrid = 1;                           // CTAs of the map-2 volume scan
+    lsm::batch::Brick* d_pmap = nullptr;   // tiles of reinit_pair, their number, planes of one, CTAs
+    int npmap = 0, plen = 0, pgrid = 1;
+    bool reinit_pair = true;    // FP32 pseudo-steps two at a time (reinit_pair) where two are left
     bool reinit_march = true;   // plain pseudo-steps march in k (reinit_z) rather than walk the brick table
     unsigned long long* d_vacc = nullptr;   // volume accumulators, 4 per instance
     unsigned* d_ilist = nullptr;            // interface cells of a volume pass (N entries) and their count
@@ -313,12 +316,53 @@ void march_lengths(const lsm_batch* b, int (&len)[lsm::batch::kMaps]) {
     }
 }
 
+// reinit_pair's offsets are 32-bit bytes from the arrays' bases
+bool pairs_on(const lsm_batch* b) { return b->reinit_pair && !b->prec && b->N < (1LL << 30); }
+
+// Columns of a reinit_pair tile on an instance: whole rows, or parts of a row
+// of whole 32-byte sectors with a rim, as many rows as the threads hold; the
+// shape with the fewest tiles, the wider one of two.
+void pair_tile(int ni, int nj, int* rw, int* rh) {
+    long long best = -1;
+    for (int p = 1; p <= std::max(1, (ni + 7) / 8); ++p) {
+        const int w = p == 1 ? ni : ((ni + p - 1) / p + 7) / 8 * 8;
+        if (p > 1 && w >= ni) continue;
+        const int rows = lsm::batch::kPairThreads / (w < ni ? w + 2 : w);
+        if (rows < 3 && rows < nj) continue;
+        const int py = rows >= nj ? 1 : (nj + rows - 3) / (rows - 2);
+        const long long n = (long long)((ni + w - 1) / w) * py;
+        if (best >= 0 && n >= best) continue;
+        best = n;
+        *rw = w;
+        *rh = (nj + py - 1) / py;
+    }
+}
+
+// Planes of a reinit_pair tile: a march of n planes reads and evaluates two
+// more and starts with a wait of about one, so the fewest rounds of the
+// CTAs times n + 3.
+int pair_length(const lsm_batch* b, const std::vector<Inst>& inst, int slots) {
+    int best = 4;
+    double cost = 0.0;
+    for (int n = 4; n <= 64; ++n) {
+        long long tiles = 0;
+        for (const Inst& I : inst)
+            tiles += (long long)((I.ni + I.rw - 1) / I.rw) * ((I.nj + I.rh - 1) / I.rh) * ((I.nk + n - 1) / n);
+        const double c = (double)((tiles + slots - 1) / slots) * (n + 3);
+        if (n == 4 || c < cost) {
+            cost = c;
+            best = n;
+        }
+    }
+    return best;
+}
+
 int build_bricks(lsm_batch* b, int shape) {
     if (b->prec) shape = 0;     // FP64 kernels exist for tile shape 0 only
     const auto sh = lsm::batch::kShapes[shape];
     std::vector<Inst> hi(b->ninst);
     using lsm::batch::Brick;
-    std::vector<Brick> brick, amap[lsm::batch::kMaps];
+    std::vector<Brick> brick, amap[lsm::batch::kMaps], pmap;
     // bricks in x-fastest order, each with its instance and coordinates (times
     // the extents sx, sy, sz)
     auto add = [](std::vector<Brick>& v, int q, int bx, int by, int bz, int sx, int sy, int sz) {
@@ -344,6 +388,7 @@ int build_bricks(lsm_batch* b, int shape) {
         d.dtau = (float)I.dtau;
         d.eps = (float)I.eps;
         d.pad = 0;
+        pair_tile(I.ni, I.nj, &d.rw, &d.rh);
         d.dt64 = I.dt;
         d.dtau64 = I.dtau;
         d.eps64 = I.eps;
@@ -365,6 +410,17 @@ int build_bricks(lsm_batch* b, int shape) {
         pre[2] += (long long)I.ni * I.nj;
         add(brick, q, d.nbx, d.nby, nbz, 1, 1, 1);
     }
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
+    const int pslots = sms * std::max(1, lsm::batch::reinit_pair_blocks_per_sm());
+    b->plen = pair_length(b, hi, pslots);
+    for (int q = 0; q < b->ninst; ++q) {
+        const Inst& d = hi[q];
+        add(pmap, q, (d.ni + d.rw - 1) / d.rw, (d.nj + d.rh - 1) / d.rh, (d.nk + b->plen - 1) / b->plen, d.rw, d.rh,
+            b->plen);
+    }
+    b->npmap = (int)pmap.size();
+    b->pgrid = std::max(1, std::min(b->npmap, pslots));
     b->nface = face;
     for (int a = 0; a < 3; ++a) b->nplane[a] = pre[a];
     b->nbricks = (int)brick.size();
@@ -383,6 +439,12 @@ int build_bricks(lsm_batch* b, int shape) {
         BCU(b, cudaMemcpyAsync(b->d_amap[m], amap[m].data(), sizeof(Brick) * amap[m].size(), cudaMemcpyHostToDevice,
                                b->stream));
     }
+    if (b->d_pmap) {
+        cudaFree(b->d_pmap);
+        b->d_pmap = nullptr;
+    }
+    BCU(b, cudaMalloc(&b->d_pmap, sizeof(Brick) * pmap.size()));
+    BCU(b, cudaMemcpyAsync(b->d_pmap, pmap.data(), sizeof(Brick) * pmap.size(), cudaMemcpyHostToDevice, b->stream));
     BCU(b, cudaMalloc(&b->d_brick, sizeof(Brick) * brick.size()));
     BCU(b, cudaMemcpyAsync(b->d_brick, brick.data(), sizeof(Brick) * brick.size(), cudaMemcpyHostToDevice, b->stream));
     BCU(b, cudaMemcpyAsync(b->d_inst, hi.data(), sizeof(Inst) * hi.size(), cudaMemcpyHostToDevice, b->stream));
@@ -390,8 +452,6 @@ int build_bricks(lsm_batch* b, int shape) {
         BCU(b, cudaMalloc(&b->d_vacc, sizeof(unsigned long long) * 4 * (size_t)b->ninst));
         BCU(b, cudaMemsetAsync(b->d_vacc, 0, sizeof(unsigned long long) * 4 * (size_t)b->ninst, b->stream));
     }
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
     const int per = std::max(1, lsm::batch::max_blocks_per_sm(shape, 0));
     b->grid = std::max(1, std::min(b->nbricks, sms * per));
     for (int m = 0; m < lsm::batch::kMaps; ++m) {
@@ -532,33 +592,40 @@ void enqueue_step_io(lsm_batch* b, const T* phin, T* phi_out, const Rec<T>* rec,
         // reinitialization (src/reinitialization.F90:55-104); the last
         // pseudo-step writes phi and gets the final bcond_lsm
         // (src/levelsetmethod.F90:318-321)
-        // the sign field and the first pseudo-step in one pass, then one
-        // launch per pseudo-step
+        // the sign field and the first pseudo-step in one pass, the others two
+        // per pass where the batch runs pairs and two are left
         const T* cur = S[2];
         bool twice = false;
-        for (int it = 0; it < R; ++it) {
-            const bool last = it == R - 1;
-            T* o = coef ? (last ? rec->D : f.d[it & 1]) : rec ? rec_d(b, *rec, it) : (last ? res : f.d[it & 1]);
-            const bool march = coef || b->reinit_march;
-            // a recorded step's last pseudo-step also writes phi^{n+1} (its
-            // faces are then redone from the raw output)
-            T* o2 = rec && last && res && march ? res : nullptr;
+        int tog = 0;
+        for (int it = 0, n = 1; it < R; it += n) {
+            n = pairs_on(b) && !rec && it > 0 && it + 1 < R ? 2 : 1;
+            const bool last = it + n == R, march = coef || b->reinit_march || n == 2;
+            T* const next = f.d[tog];
+            tog ^= 1;
+            T* o = coef ? (last ? rec->D : next) : rec ? rec_d(b, *rec, it) : (last && n == 1 ? res : next);
+            // a last pass that keeps its raw output, or is a pair, writes
+            // phi^{n+1} too (its faces are then redone from the raw output)
+            T* o2 = last && (rec || n == 2) && res && march ? res : nullptr;
             twice = twice || o2 != nullptr;
             unsigned* err = (last && !rec) || (o2 && check) ? b->d_err : nullptr;
             T* cf = coef ? rec->C + 6LL * it * (long long)b->ld : nullptr;
-            if (march)
+            if (n == 2) {
+                if constexpr (sizeof(T) == 4)
+                    B::reinit_pair(b->pgrid, b->d_inst, {b->d_pmap, b->npmap, b->plen}, f, cur, o, o2, err, b->stream);
+            } else if (march)
                 B::reinit_z<T>((it == 0 ? 2 : 0) + (coef ? 1 : 0), b->rzgrid, b->d_inst, tiles(b, 2), f,
                                cur, o, o2, cf, (long long)b->ld, err, b->stream);
             else if (it == 0)
                 B::sign_reinit<T>(sh, gr, b->d_inst, b->d_brick, nb, f, cur, o, err, b->stream);
             else
                 B::reinit<T>(sh, gr, b->d_inst, b->d_brick, nb, f, cur, o, err, b->stream);
-            if (last && !rec) B::bc_reinit<T>(b->d_inst, b->ninst, b->nface, f, bc, cur, res, b->stream);
+            if (last && !rec && n == 1)
+                B::bc_reinit<T>(b->d_inst, b->ninst, b->nface, f, bc, cur, res, b->stream);
             cur = o;
         }
         // recorded steps keep the raw last pseudo-step and write phi^{n+1} apart
-        if (rec && res && twice)
-            B::bc_faces<T>(b->d_inst, b->ninst, b->nface, bc, cur, res, check ? b->d_err : nullptr, b->stream);
+        if (res && twice)
+            B::bc_faces<T>(b->d_inst, b->ninst, b->nface, bc, cur, res, !rec || check ? b->d_err : nullptr, b->stream);
         else if (rec && res)
             B::bc_full<T>(sh, gr, b->d_inst, b->d_brick, nb, bc, cur, res, check ? b->d_err : nullptr, b->stream);
     } else if (res) {
@@ -593,10 +660,13 @@ int refresh_w(lsm_batch* b) {
     return LSM_OK;
 }
 
-// Chooses the tile shape of the brick-table kernels and whether the plain
-// pseudo-steps march in k (reinit_z) or walk the brick table: times, on
-// the batch itself, the brick pseudo-steps for every shape and the marching
-// pseudo-steps once (the per-step kernels that depend on the choice).
+// Chooses the tile shape of the brick-table kernels, whether the plain
+// pseudo-steps march in k (reinit_z) or walk the brick table, and whether
+// they run in pairs: times, on the batch itself, the brick pseudo-steps for
+// every shape, and the marching pseudo-steps and the pair once (the per-step
+// kernels that depend on the choice, all with the same results).  On 64 grids
+// of 32..96 a pair takes 242 us and two brick steps 346 us; on three grids of
+// 12..24, where launches and one march's latency count, 8.1 and 8.5 us.
 int autotune(lsm_batch* b) {
     namespace B = lsm::batch;
     cudaEvent_t ev[3];
@@ -620,7 +690,7 @@ int autotune(lsm_batch* b) {
         cudaEventElapsedTime(ms_b, ev[1], ev[2]);
         return LSM_OK;
     };
-    float br[B::kNumShapes], zm = 0.f, dummy = 0.f;
+    float br[B::kNumShapes], zm = 0.f, pair = 0.f, dummy = 0.f;
     for (int s = 0; s < B::kNumShapes; ++s) {
         const int bs = build_bricks(b, s);
         if (bs != LSM_OK) return done(bs);
@@ -633,18 +703,26 @@ int autotune(lsm_batch* b) {
             });
         if (st != LSM_OK) return done(st);
     }
-    // the marching pseudo-steps do not depend on the brick shape
-    const int st = timed(&dummy, &zm, [&]() {}, [&]() {
-        B::reinit_z<float>(2, b->rzgrid, b->d_inst, tiles(b, 2), f, f.phi, f.d[0], nullptr, nullptr, 0,
-                           nullptr, b->stream);
-        B::reinit_z<float>(0, b->rzgrid, b->d_inst, tiles(b, 2), f, f.d[0], f.d[1], nullptr, nullptr, 0,
-                           nullptr, b->stream);
-    });
+    // the marching pseudo-steps and the pairs do not depend on the brick shape
+    const int st = timed(
+        &pair, &zm,
+        [&]() {
+            if (!pairs_on(b)) return;
+            B::reinit_pair(b->pgrid, b->d_inst, {b->d_pmap, b->npmap, b->plen}, f, f.phi, f.d[0], nullptr, nullptr,
+                           b->stream);
+        },
+        [&]() {
+            B::reinit_z<float>(2, b->rzgrid, b->d_inst, tiles(b, 2), f, f.phi, f.d[0], nullptr, nullptr, 0, nullptr,
+                               b->stream);
+            B::reinit_z<float>(0, b->rzgrid, b->d_inst, tiles(b, 2), f, f.d[0], f.d[1], nullptr, nullptr, 0, nullptr,
+                               b->stream);
+        });
     if (st != LSM_OK) return done(st);
     int best_b = 0;
     for (int s = 1; s < B::kNumShapes; ++s)
         if (br[s] < br[best_b]) best_b = s;
     b->reinit_march = zm < br[best_b];
+    b->reinit_pair = pairs_on(b) && pair < std::min(zm, br[best_b]);
     const int bs = build_bricks(b, best_b);
     if (bs != LSM_OK) return done(bs);
     // the RK stage: plane tiles staged by TMA copies or by the threads,
@@ -689,10 +767,10 @@ int prepare(lsm_batch* b) {
             BTRY(autotune(b));
         } else {
             // shape 0..4: that tile shape, pseudo-steps on the brick table;
-            // 5: tile shape 0, pseudo-steps marching in k
+            // 5: tile shape 0, pseudo-steps marching in k and in pairs
             const int sh = std::min(std::max(b->cfg.shape, 0), 5);
             BTRY(build_bricks(b, sh == 5 ? 0 : sh));
-            b->reinit_march = sh == 5;
+            b->reinit_march = b->reinit_pair = sh == 5;
             b->tma_stage = b->tma_eligible;
         }
         const int ov = stage_override();
@@ -1118,7 +1196,7 @@ int lsm_batch_destroy(lsm_batch_handle b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->exec) cudaGraphExecDestroy(b->exec);
     for (void* p : {b->field_arena, (void*)b->xyz, (void*)b->staging, (void*)b->d_inst, (void*)b->d_offs,
-                    (void*)b->d_brick, (void*)b->d_amap[0], (void*)b->d_amap[1], (void*)b->d_amap[2],
+                    (void*)b->d_brick, (void*)b->d_pmap, (void*)b->d_amap[0], (void*)b->d_amap[1], (void*)b->d_amap[2],
                     (void*)b->d_amap[3], (void*)b->d_amap[4], (void*)b->d_vacc, (void*)b->d_vols, (void*)b->d_err, b->adj,
                     (void*)b->d_target, (void*)b->d_mass, (void*)b->wfix, (void*)b->d_tpart, (void*)b->d_ssum,
                     (void*)b->d_ilist, (void*)b->d_icount, (void*)b->f64x, (void*)b->d_p64, (void*)b->cellrel})
@@ -1371,11 +1449,11 @@ int lsm_batch_stage_kernel(lsm_batch_handle b) { return b ? (b->tma_stage ? 1 : 
 int lsm_batch_launches_per_step(lsm_batch_handle b) {
     if (!b) return 0;
     // volume 3 (scan, interface cells, final), three stages x (stencil +
-    // faces) 6, then RNitermax pseudo-steps (the first with the sign field)
-    // + final faces, or one full bcond pass; the mass correction's shift 1
+    // faces) 6, then RNitermax pseudo-steps (the first with the sign field,
+    // then two per pass where the batch runs pairs) + final faces, or one full bcond pass; the mass correction's shift 1
     // (W is formed outside the step, once per change of its inputs)
-    const int R = b->cfg.RNitermax;
-    return 3 + 6 + (R > 0 ? R + 1 : 1) + (b->cfg.mass_correction ? 1 : 0);
+    const int R = b->cfg.RNitermax, passes = pairs_on(b) ? R / 2 + 1 : R;
+    return 3 + 6 + (R > 0 ? passes + 1 : 1) + (b->cfg.mass_correction ? 1 : 0);
 }
 
 const char* lsm_batch_last_error(lsm_batch_handle b) { return b ? b->err.c_str() : ""; }
