@@ -315,7 +315,7 @@ BATCH = dict(n_inst=64, lo=32, hi=96, seed=0, reinit_iters=5, cfl=0.5)
 
 # algorithmic HBM bytes per node for one launch of the batched FP32 kernels
 BATCH_ALGO_BYTES = {
-    "k_stage_z": 17.0 / 3.0 * 4,   # phi_prev, phi^n (stages 2-3), W(3); phi
+    "k_stage": 17.0 / 3.0 * 4,   # phi_prev, phi^n (stages 2-3), W(3); phi
     "k_reinit_z": 12.0 * 4,      # d, s, metrics(9); d
     "k_reinit_pair": 12.0 * 4,   # the same for two pseudo-steps
     "k_sign_reinit_z": 12.0 * 4, # phi0, metrics(9); s, d
@@ -551,7 +551,7 @@ FWDADJ_WORKLOAD = ("large_free_surface %dx%dx%d curvilinear, CFL 0.4, %d RK3 ste
 # (each distinct array read once and written once; halos not counted)
 FWDADJ_BYTES = {
     "k_contra": 15 * 4,            # u(3), metrics(9); W(3)
-    "k_stage_z": 17.0 / 3.0 * 4,     # phi_prev, phi^n (stages 2-3), W(3); stage output
+    "k_stage": 17.0 / 3.0 * 4,     # phi_prev, phi^n (stages 2-3), W(3); stage output
     "k_reinit_z": 12 * 4,          # d, s, metrics(9); d
     "k_reinit_pair": 12 * 4,       # the same for two pseudo-steps
     "k_sign_reinit_z": 12 * 4,     # phi0, metrics(9); s, d

@@ -43,6 +43,7 @@
 #include "lsm_batch.cuh"
 #include "lsm_common.cuh"
 #include "lsm_kernels.h"
+#include "lsm_soft64.cuh"
 #include "lsm_volume_dev.cuh"
 
 namespace lsm {
@@ -52,8 +53,15 @@ namespace {
 // ------------------------------------------------------------ scalar helpers
 template <typename T> __device__ __forceinline__ T vmax(T a, T b) { return a > b ? a : b; }
 template <typename T> __device__ __forceinline__ T vmin(T a, T b) { return a < b ? a : b; }
-template <typename T> __device__ __forceinline__ T vdiv(T a, T b) { return a / b; }
-template <> __device__ __forceinline__ float vdiv<float>(float a, float b) { return __fdividef(a, b); }
+// 1 / (a sum of smoothness weights, at least 3e-12): FP32 by the hardware's
+// approximation without the general quotient's care for subnormal divisors,
+// FP64 on the integer pipes
+template <typename T> __device__ __forceinline__ T wrcp(T b) { return sdiv(1.0, b); }
+template <> __device__ __forceinline__ float wrcp<float>(float b) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    return r;
+}
 template <typename T> __device__ __forceinline__ T vfma(T a, T b, T c) { return fma(a, b, c); }
 template <> __device__ __forceinline__ float vfma<float>(float a, float b, float c) { return fmaf(a, b, c); }
 template <typename T> __device__ __forceinline__ T vsqrt(T a) { return sqrt(a); }
@@ -67,6 +75,15 @@ template <typename T> __device__ __forceinline__ bool vfinite(T a) { return isfi
 template <typename T> __device__ __forceinline__ T ipar(float f, double d);
 template <> __device__ __forceinline__ float ipar<float>(float f, double) { return f; }
 template <> __device__ __forceinline__ double ipar<double>(float, double d) { return d; }
+
+// element at a byte offset from an array's base (of 32 bits: one instruction,
+// the base in a uniform register)
+template <typename T, typename O> __device__ __forceinline__ T ldo(const T* p, O o) {
+    return __ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + o));
+}
+template <typename T, typename O> __device__ __forceinline__ void sto(T* p, O o, T v) {
+    *reinterpret_cast<T*>(reinterpret_cast<char*>(p) + o) = v;
+}
 
 // ------------------------------------------------------------ node walks
 struct Node {
@@ -119,14 +136,17 @@ __device__ __forceinline__ ABrick adj_brick(const Tiles& tl, int blk) {
 // GetWENO3Reconstruction (src/AdvectionMethods.F90:195-245) on an oriented
 // stencil (fL, fC, fR): weights 2/3, 1/3 over (beta + 1e-6)^2, rearranged to
 // one division: w0 = 2 t1^2 / (2 t1^2 + t0^2), Phi = u1 + w0 (u0 - u1).
+// Every operation's rounding is fixed here: all forms of a stage agree.
+template <typename T>
+__device__ __forceinline__ T rec3_value(T fL, T fC, T g, T w0) {
+    return vfma(w0, g, vfma(T(1.5), fC, T(-0.5) * fL));
+}
 template <typename T>
 __device__ __forceinline__ T rec3(T fL, T fC, T fR) {
-    const T b0 = (fC - fR) * (fC - fR), b1 = (fL - fC) * (fL - fC);
-    const T t0 = b0 + T(1.0e-6), t1 = b1 + T(1.0e-6);
-    const T a0 = T(2) * t1 * t1, a1 = t0 * t0;
-    const T w0 = vdiv(a0, a0 + a1);
-    const T u1 = T(1.5) * fC - T(0.5) * fL;
-    return vfma(w0, T(0.5) * (fL + fR) - fC, u1);
+    const T eL = fL - fC, eR = fC - fR;
+    const T t0 = vfma(eR, eR, T(1.0e-6)), t1 = vfma(eL, eL, T(1.0e-6));
+    const T a0 = (t1 + t1) * t1;
+    return rec3_value(fL, fC, vfma(T(0.5), fL + fR, -fC), a0 * wrcp(vfma(t0, t0, a0)));
 }
 
 // Phi_{+1/2} - Phi_{-1/2} along one axis for the node with stencil
@@ -141,6 +161,21 @@ __device__ __forceinline__ T weno_diff(T m2, T m1, T c, T p1, T p2, T w, bool lo
     const T fp = rec3(P ? m1 : p2, P ? c : p1, P ? p1 : c);
     const T fm = rec3(M ? m2 : p1, M ? m1 : c, M ? c : m1);
     return fp - fm;
+}
+
+// sgn(w) (Phi_{+1/2} - Phi_{-1/2}), weno_diff's bits: q0, q1, q3 are the
+// neighbours two and one against the wind and one along it.  The faces share
+// a difference and its smoothness.  `edge`: the first (wind up) or last (wind
+// down) interior node, whose upwind face takes the stencil (q3, c, q1) instead
+// of (q0, q1, c).
+template <typename T>
+__device__ __forceinline__ T weno_wind(T q0, T q1, T c, T q3, bool edge) {
+    const T fL = edge ? q3 : q0, fC = edge ? c : q1, fR = edge ? q1 : c;
+    const T e0 = fL - fC, e1 = q1 - c, e2 = c - q3;   // (fC - fR)^2 is e1^2
+    const T t0 = vfma(e0, e0, T(1.0e-6)), t1 = vfma(e1, e1, T(1.0e-6)), t2 = vfma(e2, e2, T(1.0e-6));
+    const T au = (t0 + t0) * t0, ad = (t1 + t1) * t1;
+    const T wu = au * wrcp(vfma(t1, t1, au)), wd = ad * wrcp(vfma(t2, t2, ad));
+    return rec3_value(q1, c, vfma(T(0.5), q1 + q3, -c), wd) - rec3_value(fL, fC, vfma(T(0.5), fL + fR, -fC), wu);
 }
 
 // ------------------------------------------------------------ contra
@@ -198,7 +233,7 @@ __device__ __noinline__ float stage_band_any(double W0, double W1, double W2, fl
 // The stage in FP64 over the FP32 differences: six operations of the FP64
 // pipe instead of fifteen.  A call, so that only the warps with such a node
 // pay for it (inlined, its operations were predicated, and predicated-off
-// operations occupy the FP64 pipe of every warp: 56 % of k_stage_z's time on
+// operations occupy the FP64 pipe of every warp: 56 % of the stage's time on
 // 64 grids of 32..96 nodes an axis).
 __device__ __noinline__ float stage_band(double W0, double W1, double W2, float D0, float D1, float D2, float c1,
                                          float c2, float c3, float pn, float w2) {
@@ -224,129 +259,98 @@ __device__ __forceinline__ T stage_out(const FieldsT<T>& f, long long l, bool in
     return c1 * pn + c2 * w2 - c3 * R;
 }
 
-// RK stage on the tiles of adjoint map 2 (32 x 8 columns marching 32 planes
-// in k).  Each plane of phi1 is staged in shared memory with a two-node
-// halo in x and y (double-buffered, one barrier per plane: the x and y
-// stencils read it there); the z stencil is a five-plane register window.
-// Loads per node: phi1 once (plus the halo share), phi^n and W.  Interior
-// nodes: out = c1 phi^n + c2 phi1 - c3 sum_m W_m (Phi+ - Phi-)_m
-// (calc_RH_AD_WENO3 x aj dt, the x term first); other nodes get R = 0 and
-// their faces from bcond_lsm afterwards.  Halo slots: threads 0..127 hold the y-halo rows
-// -2, -1, 8, 9 of the tile, threads 128..159 the x-halo columns -2, -1, 32,
-// 33 (the cross stencil needs no corners).
-// The z face k-1/2 of a node is the z face k+1/2 of the node below it with
-// the same stencil whenever their upwind choices agree (M at k equals P at
-// k - 1): that reconstruction is carried from the previous plane, and a
-// warp skips the recomputation when all its lanes can reuse it.
-constexpr int kStSX = 36, kStSY = 12;
-template <typename T>
-__global__ void __launch_bounds__(256) k_stage_z(const Inst* __restrict__ inst, Tiles tl, FieldsT<T> f, const T* __restrict__ phin, const T* __restrict__ phi1, T* __restrict__ out, T c1, T c2,
-        T c3) {
-    __shared__ T pl[2][kStSY][kStSX];
-    const unsigned FM = 0xffffffffu;
-    const int t = threadIdx.x, tx = t & 31, ty = t >> 5;
-    int hx = 0, hy = 0;
-    if (t < 128) {
-        const int r = t >> 5;
-        hy = r < 2 ? r - 2 : r + 6;
-        hx = tx;
-    } else if (t < 160) {
-        const int u = t - 128, c = u & 3;
-        hy = u >> 2;
-        hx = c < 2 ? c - 2 : c + 30;
-    }
-    const bool has_h = t < 160;
-    unsigned ph = 0;   // buffer parity, continuous over the tiles of this CTA
+// RK stage: interior nodes out = c1 phi^n + c2 phi1 - c3 sum_m W_m (Phi+ -
+// Phi-)_m (calc_RH_AD_WENO3 x aj dt, the x term first), other nodes with a sum
+// of 0; their faces come from bcond_lsm afterwards.  On flat tiles: sw x sh
+// columns of one instance (Inst; whole rows or parts of them), in row-major
+// order over the threads, so that few lanes idle where the instance's width is
+// no multiple of 32; each thread marches in k with the z stencil in a register
+// window.
+// What bounds it is the issue of its instructions, and the warps that wait
+// where some hold interface nodes (stage_band).  So a face's operations are
+// few (weno_wind), neighbours are loaded by the wind's side, the x and y ones
+// plainly: the window has brought their lines to L1 three planes before, and
+// no warp waits for another at a barrier.  Offsets are bytes of type O, 32 bits
+// where an array has fewer than 2^32 (one instruction per access), and two
+// planes per turn of the loop keep a plane's registers in their places.
+// Measured against tiles of 32 x 8 staged in shared memory: 64 grids of 32..96
+// 242 -> 150 us, 512 x 256 x 256 301 -> 238 us, 128^3 31 -> 18 us, two FP64
+// grids of 40^3 60 -> 25 us; six blocks per SM (five: 165 us on the 64 grids,
+// seven: 158 us).
+template <typename T, typename O>
+__global__ void __launch_bounds__(kStageThreads, sizeof(T) == 4 ? kStageBlocks : 2) k_stage(const Inst* __restrict__ inst,
+        Tiles tl, FieldsT<T> f, const T* __restrict__ phin, const T* __restrict__ phi1, T* __restrict__ out, T c1, T c2, T c3) {
+    struct Pl {
+        T W0, W1, W2, pn;
+    };
+    const int t = threadIdx.x;
     for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {
         const ABrick ab = adj_brick(tl, blk);
         const Inst& I = inst[ab.inst];
         const int ni = I.ni, nj = I.nj, nk = I.nk;
-        const long long sk = (long long)ni * nj;
-        const int i = ab.i0 + tx, j = ab.j0 + ty;
+        const int y = t / I.sw, x = t - y * I.sw;
+        const int i = ab.i0 + x, j = ab.j0 + y;
+        const bool col = y < I.sh && i < ni && j < nj;
         const int k0 = ab.k0, k1 = min(k0 + tl.len, nk);
-        const bool col = i < ni && j < nj;
-        const int gi = ab.i0 + hx, gj = ab.j0 + hy;
-        const bool hok = has_h && gi >= 0 && gi < ni && gj >= 0 && gj < nj;
-        const long long cb = I.off + i + (long long)ni * j;
-        const long long hb = I.off + gi + (long long)ni * gj;
-        const bool ij_int = i > 0 && i < ni - 1 && j > 0 && j < nj - 1;
-        auto own = [&](int k) { return col && k >= 0 && k < nk ? __ldg(phi1 + cb + sk * k) : T(0); };
-        T w0 = own(k0 - 2), w1 = own(k0 - 1), w2 = own(k0), w3 = own(k0 + 1), w4 = own(k0 + 2);
-        T hv = hok ? __ldg(phi1 + hb + sk * k0) : T(0);
-        T W0 = T(0), W1 = T(0), W2 = T(0), pn = T(0);
+        constexpr O E = sizeof(T);
+        const O sj = E * (O)ni, sk = sj * (O)nj;
+        O l = E * (O)I.off + sk * (O)k0 + E * (O)i + sj * (O)j;   // plane k
+        const bool ij_int = col && i > 0 && i < ni - 1 && j > 0 && j < nj - 1;
+        const bool ilo = i == 1, ihi = i == ni - 2, jlo = j == 1, jhi = j == nj - 2;
+        const T eps = ipar<T>(I.eps, I.eps64);
+        T w0 = T(0), w1 = T(0), w2 = T(0), w3 = T(0), w4 = T(0);
+        Pl a, b;
+        auto ld = [&](Pl& p, O l) {
+            p.W0 = ldo(f.W[0], l);
+            p.W1 = ldo(f.W[1], l);
+            p.W2 = ldo(f.W[2], l);
+            p.pn = ldo(phin, l);
+        };
         if (col) {
-            const long long l = cb + sk * k0;
-            W0 = __ldg(f.W[0] + l);
-            W1 = __ldg(f.W[1] + l);
-            W2 = __ldg(f.W[2] + l);
-            pn = __ldg(phin + l);
+            if (k0 > 1) w0 = ldo(phi1, l - 2 * sk);
+            if (k0 > 0) w1 = ldo(phi1, l - sk);
+            w2 = ldo(phi1, l);
+            if (k0 + 1 < nk) w3 = ldo(phi1, l + sk);
+            if (k0 + 2 < nk) w4 = ldo(phi1, l + 2 * sk);
+            ld(a, l);
         }
-        // the z face k - 1/2 carried from the previous plane (Pz: its stencil choice)
-        T fpz = T(0);
-        bool Pz = false, have = false;
-        for (int k = k0; k < k1; ++k) {
-            // loads of plane k + 1 (window plane k + 3) go out first
-            const bool nx = k + 1 < k1;
-            const T w5 = nx ? own(k + 3) : T(0);
-            T hvn = T(0), W0n = T(0), W1n = T(0), W2n = T(0), pnn = T(0);
-            if (hok && nx) hvn = __ldg(phi1 + hb + sk * (k + 1));
-            if (col && nx) {
-                const long long l = cb + sk * (k + 1);
-                W0n = __ldg(f.W[0] + l);
-                W1n = __ldg(f.W[1] + l);
-                W2n = __ldg(f.W[2] + l);
-                pnn = __ldg(phin + l);
+        auto plane = [&](int k, const Pl& c, Pl& n) {
+            T w5 = T(0);
+            if (col && k + 1 < k1) {
+                if (k + 3 < nk) w5 = ldo(phi1, l + 3 * sk);
+                ld(n, l + sk);
             }
-            T (*P)[kStSX] = pl[ph & 1u];
-            ++ph;
-            P[ty + 2][tx + 2] = w2;
-            if (has_h) P[hy + 2][hx + 2] = hv;
-            __syncthreads();
-            const bool interior = col && ij_int && k > 0 && k < nk - 1;
-            // z stencil choices (weno_diff's P and M)
-            const bool upz = W2 > T(0);
-            const bool Pk = upz || k == nk - 2, Mk = upz && k != 1;
-            const bool reuse = !interior || (have && Mk == Pz);
-            const bool all_reuse = __all_sync(FM, reuse);
-            if (col) {
-                T R = T(0);
-                T D0 = T(0), D1 = T(0), D2 = T(0);
-                if (interior) {
-                    const int x = tx + 2, y = ty + 2;
-                    // the outer stencil values are read unconditionally: every
-                    // slot of the cross is written each plane (zero outside the
-                    // grid), and weno_diff leaves m2 unused at the first
-                    // interior node and p2 at the last
-                    D0 = weno_diff(P[y][x - 2], P[y][x - 1], w2, P[y][x + 1], P[y][x + 2], W0, i == 1, i == ni - 2);
-                    D1 = weno_diff(P[y - 2][x], P[y - 1][x], w2, P[y + 1][x], P[y + 2][x], W1, j == 1, j == nj - 2);
-                    const T p2 = w4;
-                    const T fp = rec3(Pk ? w1 : p2, Pk ? w2 : w3, Pk ? w3 : w2);
-                    T fm = fpz;
-                    if (!all_reuse) {
-                        const T g = rec3(Mk ? w0 : w3, Mk ? w1 : w2, Mk ? w2 : w1);
-                        if (!reuse) fm = g;
-                    }
-                    D2 = fp - fm;
-                    R = W0 * D0;
-                    R = vfma(W1, D1, R);
-                    R = vfma(W2, D2, R);
-                    fpz = fp;
-                    Pz = Pk;
-                }
-                out[cb + sk * k] = stage_out(f, cb + sk * k, interior, c1, c2, c3, pn, w2, R, D0, D1, D2,
-                                             ipar<T>(I.eps, I.eps64));
+            const bool interior = ij_int && k > 0 && k < nk - 1;
+            T R = T(0), D0 = T(0), D1 = T(0), D2 = T(0);
+            if (interior) {
+                // in the array for every interior node; q0 is not used at an edge
+                const bool ux = c.W0 > T(0), uy = c.W1 > T(0), uz = c.W2 > T(0);
+                const O ox = ux ? E : O(0) - E, oy = uy ? sj : O(0) - sj;
+                const T x0 = ldo(phi1, l - 2 * ox), x1 = ldo(phi1, l - ox), x3 = ldo(phi1, l + ox);
+                const T y0 = ldo(phi1, l - 2 * oy), y1 = ldo(phi1, l - oy), y3 = ldo(phi1, l + oy);
+                D2 = weno_wind(uz ? w0 : w4, uz ? w1 : w3, w2, uz ? w3 : w1, uz ? k == 1 : k == nk - 2);
+                D0 = weno_wind(x0, x1, w2, x3, ux ? ilo : ihi);
+                D1 = weno_wind(y0, y1, w2, y3, uy ? jlo : jhi);
+                R = fabs(c.W0) * D0;
+                R = vfma(fabs(c.W1), D1, R);
+                R = vfma(fabs(c.W2), D2, R);
+                if (!ux) D0 = -D0;
+                if (!uy) D1 = -D1;
+                if (!uz) D2 = -D2;
             }
-            have = interior;
+            if (col) sto(out, l, stage_out(f, (long long)(l / E), interior, c1, c2, c3, c.pn, w2, R, D0, D1, D2, eps));
             w0 = w1;
             w1 = w2;
             w2 = w3;
             w3 = w4;
             w4 = w5;
-            hv = hvn;
-            W0 = W0n;
-            W1 = W1n;
-            W2 = W2n;
-            pn = pnn;
+            l += sk;
+        };
+        for (int k = k0;;) {
+            plane(k, a, b);
+            if (++k >= k1) break;
+            plane(k, b, a);
+            if (++k >= k1) break;
         }
     }
 }
@@ -395,9 +399,12 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
         : "memory");
 }
 
-// RK stage (FP32) with the plane tiles staged by TMA: the same arithmetic,
-// tiles and z window as k_stage_z, for a batch of one instance whose rows
-// are whole 16-byte units (ni a multiple of 4).  The stage input phi1 is
+// RK stage (FP32) with the plane tiles staged by TMA: the same arithmetic (the
+// same bits as k_stage), on the tiles of adjoint map 2 (32 x 8 columns) with
+// the z stencil in a register window, for a batch of one instance whose rows
+// are whole 16-byte units (ni a multiple of 4).  The z face k - 1/2 is
+// carried from the plane below where the upwind choices agree, and a warp
+// skips its evaluation where all lanes' do.  The stage input phi1 is
 // array `a_in` of the 4-D tensor map `tm` ((ni, nj, nk, arrays), the
 // arena's arrays ld apart).  Per plane one thread issues the copy of a 40 x
 // 12 box starting at (i0 - 4, j0 - 2): x rounded down to a 16-byte boundary,
@@ -697,6 +704,12 @@ __global__ void __launch_bounds__(TX * TY * TZ) k_bc_full(const Inst* __restrict
 template <typename T> __device__ __forceinline__ T pmax(T a, T b) { return a > b ? a : b; }
 template <> __device__ __forceinline__ float pmax<float>(float a, float b) { return fmaxf(a, b); }
 
+// acc + v^2, the square rounded by itself in FP32
+template <typename T> __device__ __forceinline__ T add_square(T acc, T v) { return fma(v, v, acc); }
+template <> __device__ __forceinline__ float add_square<float>(float acc, float v) {
+    return __fadd_rn(acc, __fmul_rn(v, v));
+}
+
 // One-sided differences (calc_RH_RN.F90:36-170) along one axis times the
 // branch sign sg (+-1: the product with it is exact): mas (forward) and men
 // (backward); on a physical face both take the one available difference.
@@ -719,11 +732,11 @@ __device__ __forceinline__ T godunov_sel_v(const T (&mas)[3], const T (&men)[3],
     T acc = T(0);
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
-        const T bb = vfma(M[6 + x], men[2], vfma(M[3 + x], men[1], M[x] * men[0]));
-        const T ff = vfma(M[6 + x], mas[2], vfma(M[3 + x], mas[1], M[x] * mas[0]));
+        const T bb = vfma(M[6 + x], men[2], vfma(M[x], men[0], M[3 + x] * men[1]));
+        const T ff = vfma(M[6 + x], mas[2], vfma(M[x], mas[0], M[3 + x] * mas[1]));
         // max(P^2, Q^2) is the square of the larger of P and -Q
         const T p = pmax(bb, T(0)), v = pmax(-ff, p);
-        acc = vfma(v, v, acc);
+        acc = add_square(acc, v);
         if (SEL) {
             const bool takeP = p * p >= v * v;
             e[x] = takeP ? p : T(0);
@@ -924,7 +937,7 @@ __global__ void __launch_bounds__(256) k_reinit_z(const Inst* __restrict__ inst,
 // pseudo-step is bound by its bytes, twelve words per node, and by the issue
 // of its instructions; nine of the words are the metrics, which two steps
 // share, and the field between the steps stays on the chip.  Measured on 64
-// grids of 32..96: 2 x 170 us -> 242 us (512 threads; 266 with 384).  (With the adjoint coefficients, whose
+// grids of 32..96: 2 x 170 us -> 246 us (512 threads; 268 with 384).  (With the adjoint coefficients, whose
 // twelve words per node and pair are written all the same, the pair was
 // slower than two recorded steps: 884 against 790 us on 512 x 256 x 256.)
 //
@@ -938,18 +951,13 @@ __global__ void __launch_bounds__(256) k_reinit_z(const Inst* __restrict__ inst,
 // step's planes k - 2 .. k.  One barrier per plane: the shared planes rotate
 // over three buffers, in step with the three planes' registers, and each is
 // written again only after a barrier that follows its last read.  A node's
-// loads go out one plane ahead, on 32-bit byte offsets from the arrays'
-// bases (the batch is below 2^30 nodes).  The arithmetic is k_reinit_z's.
+// loads go out one plane ahead, on byte offsets of type O as in k_stage.  The
+// arithmetic is k_reinit_z's.
 struct PairPlane {
     float s, M[9], o;   // sign, metrics, the thread's value outside the rim
 };
 constexpr int kPairSmem = 3 * (kPairThreads + 2);   // (ew + 2) (eh + 2) for ew eh <= kPairThreads
-__device__ __forceinline__ float ldo(const float* p, unsigned o) {
-    return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + o));
-}
-__device__ __forceinline__ void sto(float* p, unsigned o, float v) {
-    *reinterpret_cast<float*>(reinterpret_cast<char*>(p) + o) = v;
-}
+template <typename O>
 __global__ void __launch_bounds__(kPairThreads, 2) k_reinit_pair(const Inst* __restrict__ inst, Tiles tl,
         FieldsT<float> f, const float* __restrict__ din, float* __restrict__ dout, float* __restrict__ dout2,
         unsigned* err) {
@@ -966,9 +974,9 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_reinit_pair(const Inst* __r
         const bool col = y < eh && i >= 0 && i < ni && j >= 0 && j < nj;
         const bool core = col && x >= ox && x < I.rw + ox && y >= oy && y < I.rh + oy;
         const int k0 = ab.k0, k1 = min(k0 + tl.len, nk);
-        const unsigned sk = 4u * (unsigned)ni * (unsigned)nj;
-        const unsigned base = 4u * (unsigned)I.off;
-        const unsigned cb = base + 4u * (unsigned)(i + ni * j);
+        const O sk = O(4) * (O)ni * (O)nj;
+        const O base = O(4) * (O)I.off;
+        const O cb = base + O(4) * (O)i + O(4) * (O)ni * (O)j;
         const bool xm = i == 0, xp = i == ni - 1, ym = j == 0, yp = j == nj - 1;
         // slot in the shared planes, and the value outside the rim that this
         // thread brings there: rows -1 and eh, then columns -1 and ew
@@ -979,14 +987,14 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_reinit_pair(const Inst* __r
         const int hi_ = ab.i0 + hx - ox, hj = ab.j0 + hy - oy;
         const bool hok = t < 2 * (ew + eh) && hi_ >= 0 && hi_ < ni && hj >= 0 && hj < nj;
         const int hs = (hy + 1) * pitch + hx + 1;
-        const unsigned hb = base + 4u * (unsigned)(hi_ + ni * hj);
+        const O hb = base + O(4) * (O)hi_ + O(4) * (O)ni * (O)hj;
         const float dtau = I.dtau;
-        auto ldd = [&](int k) { return col && k >= 0 && k < nk ? ldo(din, cb + sk * (unsigned)k) : 0.f; };
+        auto ldd = [&](int k) { return col && k >= 0 && k < nk ? ldo(din, cb + sk * (O)k) : 0.f; };
         auto ld_plane = [&](int k, PairPlane& p) {
             if (k >= nk) return;
-            if (hok) p.o = ldo(din, hb + sk * (unsigned)k);
+            if (hok) p.o = ldo(din, hb + sk * (O)k);
             if (!col) return;
-            const unsigned l = cb + sk * (unsigned)k;
+            const O l = cb + sk * (O)k;
             p.s = ldo(f.sgn, l);
 #pragma unroll
             for (int c = 0; c < 9; ++c) p.M[c] = ldo(f.m[c], l);
@@ -1020,10 +1028,10 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_reinit_pair(const Inst* __r
             if (col && k < nk) e1 = step(dc, D, dm, dp, k, pc);
             if (core && k > k0) {
                 const float r = step(ec, Em, em, e1, k - 1, pm);
-                const unsigned l = cb + sk * (unsigned)(k - 1);
+                const O l = cb + sk * (O)(k - 1);
                 sto(dout, l, r);
                 if (dout2) sto(dout2, l, r);
-                if (err && !vfinite(r)) atomicOr(err, (unsigned)kErrNonFinite);
+                if (err && !vfinite(r)) atomicOr(err, (O)kErrNonFinite);
             }
             if (y < eh) E[me] = e1;
             em = ec;
@@ -1955,21 +1963,20 @@ __global__ void k_adj_face(Flat fl, int face0, long long nplane, int nface, BC b
     lam[l] = T(0);
 }
 
-// value and gradient of rec3 (one reciprocal)
+// value and gradient of rec3 (one reciprocal r)
 template <typename T>
 __device__ __forceinline__ T rec3_vg(T fL, T fC, T fR, T* dL, T* dC, T* dR) {
-    const T eL = fL - fC, eR = fC - fR;
-    const T t0 = eR * eR + T(1.0e-6), t1 = eL * eL + T(1.0e-6);
-    const T a0 = T(2) * t1 * t1, a1 = t0 * t0;
-    const T r = vdiv(T(1), a0 + a1);
-    const T w0 = a0 * r;
-    const T g = T(0.5) * (fL + fR) - fC;
-    // d w0 / d t1 = 4 t1 a1 r^2, d w0 / d t0 = -2 t0 a0 r^2
-    const T q1 = T(4) * t1 * a1 * r * r * g, q0 = T(-2) * t0 * a0 * r * r * g;
-    *dL = T(-0.5) + T(0.5) * w0 + q1 * (T(2) * eL);
-    *dC = T(1.5) - w0 - q1 * (T(2) * eL) + q0 * (T(2) * eR);
-    *dR = T(0.5) * w0 - q0 * (T(2) * eR);
-    return vfma(w0, g, T(1.5) * fC - T(0.5) * fL);
+    const T eL = fL - fC, eR = fC - fR, h = eL - eR;
+    const T t0 = vfma(eR, eR, T(1.0e-6)), t1 = vfma(eL, eL, T(1.0e-6));
+    const T q = t1 * t1, a1 = t0 * t0;
+    const T r = wrcp(vfma(T(2), q, a1));
+    const T v = q * r, z = T(4) * r * h;
+    // h dv / d eL = 4 t1 a1 r^2 h eL, h dv / d eR = -4 t0 t1^2 r^2 h eR
+    const T xL = t1 * a1 * r * z * eL, xR = -(t0 * q * r) * z * eR;
+    *dL = v - T(0.5) + xL;
+    *dC = T(1.5) - T(2) * v - xL + xR;
+    *dR = v - xR;
+    return vfma(v, h, vfma(T(-0.5), eL, fC));
 }
 
 // D = Phi+ - Phi- of a node (stencil s, orientation frozen by w) and the
@@ -2399,10 +2406,20 @@ void contra(int shape, int grid, const Inst* inst, const Brick* bi, int nb, Fiel
     dispatch<RunContra, T>(shape, grid, inst, bi, nb, f, s);
 }
 template <typename T>
-void stage(int grid, const Inst* inst, Tiles tl, FieldsT<T> f, const T* phin, const T* phi1, T* out,
+void stage(int grid, const Inst* inst, Tiles tl, bool wide, FieldsT<T> f, const T* phin, const T* phi1, T* out,
            double c1, double c2, double c3, cudaStream_t s) {
-    ProfScope ps_("k_stage_z", s);
-    k_stage_z<T><<<grid, 256, 0, s>>>(inst, tl, f, phin, phi1, out, T(c1), T(c2), T(c3));
+    ProfScope ps_("k_stage", s);
+    auto go = [&](auto kernel) {
+        kernel<<<grid, kStageThreads, 0, s>>>(inst, tl, f, phin, phi1, out, T(c1), T(c2), T(c3));
+    };
+    if (wide) go(k_stage<T, unsigned long long>);
+    else go(k_stage<T, unsigned>);
+}
+template <typename T>
+int stage_blocks_per_sm() {
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_stage<T, unsigned>, kStageThreads, 0);
+    return n;
 }
 void stage_tma(int grid, const CUtensorMap* tm, int a_in, const Inst* inst, Tiles tl,
                FieldsT<float> f, const float* phin, const float* phi1, float* out, double c1, double c2, double c3,
@@ -2414,12 +2431,6 @@ void stage_tma(int grid, const CUtensorMap* tm, int a_in, const Inst* inst, Tile
 int stage_tma_blocks_per_sm() {
     int n = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_stage_tma, 256, 0);
-    return n;
-}
-template <typename T>
-int stage_blocks_per_sm() {
-    int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_stage_z<T>, 256, 0);
     return n;
 }
 template <typename T>
@@ -2475,14 +2486,16 @@ void reinit_z(int kind, int grid, const Inst* inst, Tiles tl, FieldsT<T> f, cons
     }
     }
 }
-void reinit_pair(int grid, const Inst* inst, Tiles tl, FieldsT<float> f, const float* din, float* dout, float* dout2,
-                 unsigned* err, cudaStream_t s) {
+void reinit_pair(int grid, const Inst* inst, Tiles tl, bool wide, FieldsT<float> f, const float* din, float* dout,
+                 float* dout2, unsigned* err, cudaStream_t s) {
     ProfScope ps_("k_reinit_pair", s);
-    k_reinit_pair<<<grid, kPairThreads, 0, s>>>(inst, tl, f, din, dout, dout2, err);
+    auto go = [&](auto kernel) { kernel<<<grid, kPairThreads, 0, s>>>(inst, tl, f, din, dout, dout2, err); };
+    if (wide) go(k_reinit_pair<unsigned long long>);
+    else go(k_reinit_pair<unsigned>);
 }
 int reinit_pair_blocks_per_sm() {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_reinit_pair, kPairThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_reinit_pair<unsigned>, kPairThreads, 0);
     return n;
 }
 template <typename T>
@@ -2643,8 +2656,8 @@ void adj_contra(const Flat& fl, FieldsT<T> f, const T* w0, const T* w1, const T*
 #define LSM_BATCH_INSTANTIATE(T)                                                                                      \
     template void contra<T>(int, int, const Inst*, const Brick*, int, FieldsT<T>, cudaStream_t);                       \
     template int stage_blocks_per_sm<T>();                                                                      \
-    template void stage<T>(int, const Inst*, Tiles, FieldsT<T>, const T*, const T*, T*, double,            \
-                           double, double, cudaStream_t);                                                                     \
+    template void stage<T>(int, const Inst*, Tiles, bool, FieldsT<T>, const T*, const T*, T*, double, double, double,  \
+                           cudaStream_t);                                                                         \
     template void bc_stage<T>(const Inst*, int, long long, BC, const T*, const T*, T*, double, double, cudaStream_t);   \
     template void bc_full<T>(int, int, const Inst*, const Brick*, int, BC, const T*, T*, unsigned*, cudaStream_t);      \
     template void bc_faces<T>(const Inst*, int, long long, BC, const T*, T*, unsigned*, cudaStream_t);                 \

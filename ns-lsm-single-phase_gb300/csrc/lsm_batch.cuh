@@ -31,6 +31,7 @@ struct Inst {
     long long fpre[3]; // first node of the instance's i-, j-, k-face planes (adjoint face kernels)
     double dt64, dtau64, eps64;  // the same three parameters for the FP64 kernels
     int rw, rh;                  // columns of a tile of reinit_pair, without its rim
+    int sw, sh;                  // columns of a tile of stage
     int am[kMaps][3];            // adjoint brick maps (adj_shape): first brick, bricks per row, per plane
 };
 
@@ -116,12 +117,13 @@ constexpr Shape kShapes[kNumShapes] = {{32, 4, 2}, {32, 8, 1}, {64, 4, 1}, {32, 
 template <typename T>
 void contra(int shape, int grid, const Inst* inst, const Brick* bricks, int nbricks, FieldsT<T> f,
             cudaStream_t s);
-// RK stage out = c1 phin + c2 phi1 - c3 dt aj RH(phi1) on the tiles of
-// adjoint map 2 (z march, shared-memory planes); grid from
-// stage_blocks_per_sm
+// RK stage out = c1 phin + c2 phi1 - c3 dt aj RH(phi1) on flat tiles of Inst's
+// sw x sh columns (their table holds each tile's first node; grid from
+// stage_blocks_per_sm); wide: arrays of 2^32 bytes and more
+constexpr int kStageThreads = 256, kStageBlocks = 6;
 template <typename T>
-void stage(int grid, const Inst* inst, Tiles tl, FieldsT<T> f, const T* phin, const T* phi1,
-           T* out, double c1, double c2, double c3, cudaStream_t s);
+void stage(int grid, const Inst* inst, Tiles tl, bool wide, FieldsT<T> f, const T* phin, const T* phi1, T* out,
+           double c1, double c2, double c3, cudaStream_t s);
 template <typename T>
 int stage_blocks_per_sm();
 // The same stage (FP32) with each plane's tile + two-node halo staged in
@@ -166,12 +168,12 @@ void reinit_z(int kind, int grid, const Inst* inst, Tiles tl, FieldsT<T> f, cons
               T* dout2, T* cf, long long ld, unsigned* err, cudaStream_t s);
 template <typename T>
 int reinit_z_blocks_per_sm();
-// Two plain pseudo-steps in one pass (FP32, fewer than 2^30 nodes), on tiles
-// of Inst's rw x rh columns (their table holds each tile's first node); dout
-// must not be din; dout2 (nullable) gets a second copy of the output
+// Two plain pseudo-steps in one pass (FP32), on flat tiles of Inst's rw x rh
+// columns and a rim; wide as for stage; dout must not be din; dout2 (nullable)
+// gets a second copy of the output
 constexpr int kPairThreads = 512;
-void reinit_pair(int grid, const Inst* inst, Tiles tl, FieldsT<float> f, const float* din, float* dout, float* dout2,
-                 unsigned* err, cudaStream_t s);
+void reinit_pair(int grid, const Inst* inst, Tiles tl, bool wide, FieldsT<float> f, const float* din, float* dout,
+                 float* dout2, unsigned* err, cudaStream_t s);
 int reinit_pair_blocks_per_sm();
 // water volume of every instance: the cells' 64-bit fixed-point sums (K, S,
 // bulk and, with `slope`, dK/dC) are added to acc[4 * inst + c] (zero on

@@ -14,6 +14,7 @@
 #include <string>
 #include <initializer_list>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "lsm_batch.cuh"
@@ -69,10 +70,14 @@ struct lsm_batch {
     lsm::batch::Brick* d_amap[lsm::batch::kMaps] = {};  // brick tables of the adjoint stencil kernels (lsm::batch::adj_shape)
     int namap[lsm::batch::kMaps] = {}, agrid[lsm::batch::kMaps] = {};
     int len[lsm::batch::kMaps] = {};         // march lengths of the maps' tiles
-    int sgrid = 1, acgrid = 1, rzgrid = 1;   // CTAs of the map-2 kernels: stage, k_adj_reinit_c, reinit_z
+    int acgrid = 1, rzgrid = 1;   // CTAs of the map-2 kernels k_adj_reinit_c and reinit_z
     int vgrid = 1;                           // CTAs of the map-2 volume scan
-    lsm::batch::Brick* d_pmap = nullptr;   // tiles of reinit_pair, their number, planes of one, CTAs
-    int npmap = 0, plen = 0, pgrid = 1;
+    // flat tiles of reinit_pair and of stage: their table, number, planes of one, CTAs
+    struct FlatMap {
+        lsm::batch::Brick* d = nullptr;
+        int n = 0, len = 0, grid = 1;
+        lsm::batch::Tiles tiles() const { return {d, n, len}; }
+    } pmap, smap;
     bool reinit_pair = true;    // FP32 pseudo-steps two at a time (reinit_pair) where two are left
     bool reinit_march = true;   // plain pseudo-steps march in k (reinit_z) rather than walk the brick table
     unsigned long long* d_vacc = nullptr;   // volume accumulators, 4 per instance
@@ -294,9 +299,8 @@ lsm::batch::Tiles tiles(const lsm_batch* b, int m) { return {b->d_amap[m], b->na
 // recomputing reverse pseudo-step), since a march reuses what it has loaded
 // and evaluated; the stage adjoint evaluates four planes more than it
 // writes, so its marches keep to 8 and more.  Measured, against 32 always:
-// 128^3 (256 tiles of 32) k_stage_z 54 -> 32 us, k_reinit_rec_z 41 -> 35 us;
-// two FP64 grids of about 40^3 k_stage_z 260 -> 65 us, k_adj_reinit 375 ->
-// 70 us, k_adj_stage_y 234 -> 88 us (106 us at 4); 512 x 256 x 256 (4096
+// 128^3 (256 tiles of 32) k_reinit_rec_z 41 -> 35 us; two FP64 grids of about
+// 40^3 k_adj_reinit 375 -> 70 us, k_adj_stage_y 234 -> 88 us (106 us at 4); 512 x 256 x 256 (4096
 // tiles of 32) loses 6 % at 8.
 void march_lengths(const lsm_batch* b, int (&len)[lsm::batch::kMaps]) {
     const int sms = 152;
@@ -316,20 +320,28 @@ void march_lengths(const lsm_batch* b, int (&len)[lsm::batch::kMaps]) {
     }
 }
 
-// reinit_pair's offsets are 32-bit bytes from the arrays' bases
-bool pairs_on(const lsm_batch* b) { return b->reinit_pair && !b->prec && b->N < (1LL << 30); }
+// The kernels on flat tiles take byte offsets from the arrays' bases, of 32
+// bits where they suffice (LSM_BATCH_WIDE=1: of 64 all the same, for tests)
+bool wide(const lsm_batch* b) {
+    static const bool forced = std::getenv("LSM_BATCH_WIDE") != nullptr;
+    return forced || b->N >= (1LL << 32) / (b->prec ? 8 : 4);
+}
+bool pairs_on(const lsm_batch* b) { return b->reinit_pair && !b->prec; }
 
-// Columns of a reinit_pair tile on an instance: whole rows, or parts of a row
-// of whole 32-byte sectors with a rim, as many rows as the threads hold; the
-// shape with the fewest tiles, the wider one of two.
-void pair_tile(int ni, int nj, int* rw, int* rh) {
+// Columns of a flat tile on an instance: whole rows, or parts of a row of
+// whole 32-byte sectors, as many rows as the threads hold with the tile's rim
+// (columns that are evaluated twice; only where the tile ends inside the
+// instance); the shape with the fewest tiles, the widest of those (squarer
+// ones with less read around them: 152 against 145 us for the RK stage of 64
+// grids of 32..96, 246 against 238 us on 512 x 256 x 256).
+void flat_tile(int ni, int nj, int threads, int rim, int* rw, int* rh) {
     long long best = -1;
     for (int p = 1; p <= std::max(1, (ni + 7) / 8); ++p) {
         const int w = p == 1 ? ni : ((ni + p - 1) / p + 7) / 8 * 8;
         if (p > 1 && w >= ni) continue;
-        const int rows = lsm::batch::kPairThreads / (w < ni ? w + 2 : w);
-        if (rows < 3 && rows < nj) continue;
-        const int py = rows >= nj ? 1 : (nj + rows - 3) / (rows - 2);
+        const int rows = threads / (w < ni ? w + 2 * rim : w);
+        if (rows < 1 || (rows <= 2 * rim && rows < nj)) continue;
+        const int py = rows >= nj ? 1 : (nj + rows - 2 * rim - 1) / (rows - 2 * rim);
         const long long n = (long long)((ni + w - 1) / w) * py;
         if (best >= 0 && n >= best) continue;
         best = n;
@@ -338,23 +350,41 @@ void pair_tile(int ni, int nj, int* rw, int* rh) {
     }
 }
 
-// Planes of a reinit_pair tile: a march of n planes reads and evaluates two
-// more and starts with a wait of about one, so the fewest rounds of the
-// CTAs times n + 3.
-int pair_length(const lsm_batch* b, const std::vector<Inst>& inst, int slots) {
-    int best = 4;
+// Table of the flat tiles (columns from `tile`) on at most `slots` CTAs at a
+// time.  A march of n planes costs about three more (its first loads, the
+// planes that it reads or evaluates beyond its own), so n is the length with
+// the fewest rounds of the CTAs times n + 3.
+template <class Tile>
+int flat_map(lsm_batch* b, const std::vector<Inst>& inst, int slots, lsm_batch::FlatMap& m, Tile tile) {
+    using lsm::batch::Brick;
     double cost = 0.0;
     for (int n = 4; n <= 64; ++n) {
         long long tiles = 0;
-        for (const Inst& I : inst)
-            tiles += (long long)((I.ni + I.rw - 1) / I.rw) * ((I.nj + I.rh - 1) / I.rh) * ((I.nk + n - 1) / n);
+        for (const Inst& I : inst) {
+            const auto [w, h] = tile(I);
+            tiles += (long long)((I.ni + w - 1) / w) * ((I.nj + h - 1) / h) * ((I.nk + n - 1) / n);
+        }
         const double c = (double)((tiles + slots - 1) / slots) * (n + 3);
         if (n == 4 || c < cost) {
             cost = c;
-            best = n;
+            m.len = n;
         }
     }
-    return best;
+    std::vector<Brick> v;
+    for (int q = 0; q < (int)inst.size(); ++q) {
+        const Inst& I = inst[q];
+        const auto [w, h] = tile(I);
+        for (int z = 0; z < I.nk; z += m.len)
+            for (int y = 0; y < I.nj; y += h)
+                for (int x = 0; x < I.ni; x += w) v.push_back(Brick{q, x, y, z});
+    }
+    m.n = (int)v.size();
+    m.grid = std::max(1, std::min(m.n, slots));
+    cudaFree(m.d);
+    m.d = nullptr;
+    BCU(b, cudaMalloc(&m.d, sizeof(Brick) * v.size()));
+    BCU(b, cudaMemcpy(m.d, v.data(), sizeof(Brick) * v.size(), cudaMemcpyHostToDevice));
+    return LSM_OK;
 }
 
 int build_bricks(lsm_batch* b, int shape) {
@@ -362,7 +392,7 @@ int build_bricks(lsm_batch* b, int shape) {
     const auto sh = lsm::batch::kShapes[shape];
     std::vector<Inst> hi(b->ninst);
     using lsm::batch::Brick;
-    std::vector<Brick> brick, amap[lsm::batch::kMaps], pmap;
+    std::vector<Brick> brick, amap[lsm::batch::kMaps];
     // bricks in x-fastest order, each with its instance and coordinates (times
     // the extents sx, sy, sz)
     auto add = [](std::vector<Brick>& v, int q, int bx, int by, int bz, int sx, int sy, int sz) {
@@ -388,7 +418,8 @@ int build_bricks(lsm_batch* b, int shape) {
         d.dtau = (float)I.dtau;
         d.eps = (float)I.eps;
         d.pad = 0;
-        pair_tile(I.ni, I.nj, &d.rw, &d.rh);
+        flat_tile(I.ni, I.nj, lsm::batch::kPairThreads, 1, &d.rw, &d.rh);
+        flat_tile(I.ni, I.nj, lsm::batch::kStageThreads, 0, &d.sw, &d.sh);
         d.dt64 = I.dt;
         d.dtau64 = I.dtau;
         d.eps64 = I.eps;
@@ -412,15 +443,6 @@ int build_bricks(lsm_batch* b, int shape) {
     }
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-    const int pslots = sms * std::max(1, lsm::batch::reinit_pair_blocks_per_sm());
-    b->plen = pair_length(b, hi, pslots);
-    for (int q = 0; q < b->ninst; ++q) {
-        const Inst& d = hi[q];
-        add(pmap, q, (d.ni + d.rw - 1) / d.rw, (d.nj + d.rh - 1) / d.rh, (d.nk + b->plen - 1) / b->plen, d.rw, d.rh,
-            b->plen);
-    }
-    b->npmap = (int)pmap.size();
-    b->pgrid = std::max(1, std::min(b->npmap, pslots));
     b->nface = face;
     for (int a = 0; a < 3; ++a) b->nplane[a] = pre[a];
     b->nbricks = (int)brick.size();
@@ -439,12 +461,12 @@ int build_bricks(lsm_batch* b, int shape) {
         BCU(b, cudaMemcpyAsync(b->d_amap[m], amap[m].data(), sizeof(Brick) * amap[m].size(), cudaMemcpyHostToDevice,
                                b->stream));
     }
-    if (b->d_pmap) {
-        cudaFree(b->d_pmap);
-        b->d_pmap = nullptr;
-    }
-    BCU(b, cudaMalloc(&b->d_pmap, sizeof(Brick) * pmap.size()));
-    BCU(b, cudaMemcpyAsync(b->d_pmap, pmap.data(), sizeof(Brick) * pmap.size(), cudaMemcpyHostToDevice, b->stream));
+    BTRY(flat_map(b, hi, sms * std::max(1, lsm::batch::reinit_pair_blocks_per_sm()), b->pmap,
+                  [](const Inst& I) { return std::pair<int, int>(I.rw, I.rh); }));
+    BTRY(flat_map(b, hi,
+                  sms * std::max(1, b->prec ? lsm::batch::stage_blocks_per_sm<double>()
+                                            : lsm::batch::stage_blocks_per_sm<float>()),
+                  b->smap, [](const Inst& I) { return std::pair<int, int>(I.sw, I.sh); }));
     BCU(b, cudaMalloc(&b->d_brick, sizeof(Brick) * brick.size()));
     BCU(b, cudaMemcpyAsync(b->d_brick, brick.data(), sizeof(Brick) * brick.size(), cudaMemcpyHostToDevice, b->stream));
     BCU(b, cudaMemcpyAsync(b->d_inst, hi.data(), sizeof(Inst) * hi.size(), cudaMemcpyHostToDevice, b->stream));
@@ -459,9 +481,6 @@ int build_bricks(lsm_batch* b, int shape) {
                                            : lsm::batch::adj_blocks_per_sm<float>(m));
         b->agrid[m] = std::max(1, std::min(b->namap[m], sms * pa));
     }
-    const int ps = std::max(1, b->prec ? lsm::batch::stage_blocks_per_sm<double>()
-                                       : lsm::batch::stage_blocks_per_sm<float>());
-    b->sgrid = std::max(1, std::min(b->namap[2], sms * ps));
     const int pac = std::max(1, b->prec ? lsm::batch::adj_reinit_c_blocks_per_sm<double>()
                                         : lsm::batch::adj_reinit_c_blocks_per_sm<float>());
     b->acgrid = std::max(1, std::min(b->namap[2], sms * pac));
@@ -550,7 +569,7 @@ void enqueue_stage(lsm_batch* b, FieldsT<T> f, const T* phin, const T* in, T* ou
             }
         }
     }
-    B::stage<T>(b->sgrid, b->d_inst, tiles(b, 2), f, phin, in, out, kC[s][0], kC[s][1], kC[s][2],
+    B::stage<T>(b->smap.grid, b->d_inst, b->smap.tiles(), wide(b), f, phin, in, out, kC[s][0], kC[s][1], kC[s][2],
                 b->stream);
 }
 
@@ -611,7 +630,7 @@ void enqueue_step_io(lsm_batch* b, const T* phin, T* phi_out, const Rec<T>* rec,
             T* cf = coef ? rec->C + 6LL * it * (long long)b->ld : nullptr;
             if (n == 2) {
                 if constexpr (sizeof(T) == 4)
-                    B::reinit_pair(b->pgrid, b->d_inst, {b->d_pmap, b->npmap, b->plen}, f, cur, o, o2, err, b->stream);
+                    B::reinit_pair(b->pmap.grid, b->d_inst, b->pmap.tiles(), wide(b), f, cur, o, o2, err, b->stream);
             } else if (march)
                 B::reinit_z<T>((it == 0 ? 2 : 0) + (coef ? 1 : 0), b->rzgrid, b->d_inst, tiles(b, 2), f,
                                cur, o, o2, cf, (long long)b->ld, err, b->stream);
@@ -665,7 +684,7 @@ int refresh_w(lsm_batch* b) {
 // they run in pairs: times, on the batch itself, the brick pseudo-steps for
 // every shape, and the marching pseudo-steps and the pair once (the per-step
 // kernels that depend on the choice, all with the same results).  On 64 grids
-// of 32..96 a pair takes 242 us and two brick steps 346 us; on three grids of
+// of 32..96 a pair takes 246 us and two brick steps 346 us; on three grids of
 // 12..24, where launches and one march's latency count, 8.1 and 8.5 us.
 int autotune(lsm_batch* b) {
     namespace B = lsm::batch;
@@ -707,8 +726,7 @@ int autotune(lsm_batch* b) {
     const int st = timed(
         &pair, &zm,
         [&]() {
-            if (!pairs_on(b)) return;
-            B::reinit_pair(b->pgrid, b->d_inst, {b->d_pmap, b->npmap, b->plen}, f, f.phi, f.d[0], nullptr, nullptr,
+            B::reinit_pair(b->pmap.grid, b->d_inst, b->pmap.tiles(), wide(b), f, f.phi, f.d[0], nullptr, nullptr,
                            b->stream);
         },
         [&]() {
@@ -722,7 +740,7 @@ int autotune(lsm_batch* b) {
     for (int s = 1; s < B::kNumShapes; ++s)
         if (br[s] < br[best_b]) best_b = s;
     b->reinit_march = zm < br[best_b];
-    b->reinit_pair = pairs_on(b) && pair < std::min(zm, br[best_b]);
+    b->reinit_pair = pair < std::min(zm, br[best_b]);
     const int bs = build_bricks(b, best_b);
     if (bs != LSM_OK) return done(bs);
     // the RK stage: plane tiles staged by TMA copies or by the threads,
@@ -734,8 +752,8 @@ int autotune(lsm_batch* b) {
         const int st2 = timed(
             &ms_plain, &ms_tma,
             [&]() {
-                B::stage<float>(b->sgrid, b->d_inst, tiles(b, 2), f, f.phi, f.phi, f.stage[0], 1.0, 0.0,
-                                1.0, b->stream);
+                B::stage<float>(b->smap.grid, b->d_inst, b->smap.tiles(), wide(b), f, f.phi, f.phi, f.stage[0], 1.0,
+                                0.0, 1.0, b->stream);
             },
             [&]() {
                 B::stage_tma(b->tgrid, &b->tm_field, 0, b->d_inst, tiles(b, 2), f, f.phi, f.phi,
@@ -1196,7 +1214,7 @@ int lsm_batch_destroy(lsm_batch_handle b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->exec) cudaGraphExecDestroy(b->exec);
     for (void* p : {b->field_arena, (void*)b->xyz, (void*)b->staging, (void*)b->d_inst, (void*)b->d_offs,
-                    (void*)b->d_brick, (void*)b->d_pmap, (void*)b->d_amap[0], (void*)b->d_amap[1], (void*)b->d_amap[2],
+                    (void*)b->d_brick, (void*)b->pmap.d, (void*)b->smap.d, (void*)b->d_amap[0], (void*)b->d_amap[1], (void*)b->d_amap[2],
                     (void*)b->d_amap[3], (void*)b->d_amap[4], (void*)b->d_vacc, (void*)b->d_vols, (void*)b->d_err, b->adj,
                     (void*)b->d_target, (void*)b->d_mass, (void*)b->wfix, (void*)b->d_tpart, (void*)b->d_ssum,
                     (void*)b->d_ilist, (void*)b->d_icount, (void*)b->f64x, (void*)b->d_p64, (void*)b->cellrel})
