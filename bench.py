@@ -560,9 +560,8 @@ FWDADJ_BYTES = {
     "k_adj_reinit_c": 8 * 4,       # lam, coefficients(6); lam_out
     "k_vol_scan_z": 4 + 8,         # phi (FP32) + fixed-point cell volume; interface cells listed
     "k_bc_full": 2 * 4,            # phi in, phi out
-    "k_adj_stage_x": 8 * 4,        # in, W_x, lamP0, lamPhin (rmw), lamW_x (rmw); lam_in
+    "k_adj_stage_xz": 11 * 4,      # in, W_x, W_z, lamP0, lamPhin (rmw), lamW_x (rmw), lamW_z (rmw); lam_in
     "k_adj_stage_y": 7 * 4,        # in, W_y, lamP0, lam_in (rmw), lamW_y (rmw)
-    "k_adj_stage_z": 7 * 4,        # in, W_z, lamP0, lam_in (rmw), lamW_z (rmw)
     "k_adj_reinit": 13 * 4,        # d, s, metrics(9), lam; lam_out
     "k_adj_contra": 18 * 4,        # lamW(3), metrics(9), lam_u(3, rmw)
     "k_cvt_in": 8 + 4,

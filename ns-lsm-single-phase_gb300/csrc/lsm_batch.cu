@@ -81,6 +81,10 @@ template <> __device__ __forceinline__ double ipar<double>(float, double d) { re
 template <typename T, typename O> __device__ __forceinline__ T ldo(const T* p, O o) {
     return __ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + o));
 }
+// the same from an array that the kernel writes
+template <typename T, typename O> __device__ __forceinline__ T ldv(const T* p, O o) {
+    return *reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + o);
+}
 template <typename T, typename O> __device__ __forceinline__ void sto(T* p, O o, T v) {
     *reinterpret_cast<T*>(reinterpret_cast<char*>(p) + o) = v;
 }
@@ -400,7 +404,7 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
 }
 
 // RK stage (FP32) with the plane tiles staged by TMA: the same arithmetic (the
-// same bits as k_stage), on the tiles of adjoint map 2 (32 x 8 columns) with
+// same bits as k_stage), on the tiles of adjoint map 1 (32 x 8 columns) with
 // the z stencil in a register window, for a batch of one instance whose rows
 // are whole 16-byte units (ni a multiple of 4).  The z face k - 1/2 is
 // carried from the plane below where the upwind choices agree, and a warp
@@ -836,7 +840,7 @@ __global__ void __launch_bounds__(TX * TY * TZ) k_sign_reinit(const Inst* __rest
 // serves both sides), and the pseudo-step's adjoint is
 //   lam_out(j) = lam(j) - sum_m [lam(j) (A'_m - B'_m)(j)
 //                - lam(j+e_m) A'_m(j+e_m) + lam(j-e_m) B'_m(j-e_m)].
-// One reinitialisation pseudo-step on the tiles of adjoint map 2 (32 x 8
+// One reinitialisation pseudo-step on the tiles of adjoint map 1 (32 x 8
 // columns marching 32 planes in k): each node loads d (and s) and its
 // metrics once, a plane ahead; the z neighbours of d stay in a register
 // window, the x neighbours come by warp shuffles (the tile's edge lanes load
@@ -1055,81 +1059,75 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_reinit_pair(const Inst* __r
 }
 
 // Reverse of one recorded pseudo-step from its stored coefficients (cf:
-// A'_0..2, B'_0..2, ld apart), on the tiles of adjoint map 2 (32 x 8
-// columns marching 32 planes in k).  Each node loads its own lam and six
-// coefficients once (one plane ahead); the z neighbours (lam, A'_2 above,
-// B'_2 below) stay in registers, the x neighbours come by warp shuffles
-// (the tile's edge lanes load the one outside), the y neighbours are
-// loaded (L1/L2).
-template <typename T>
-__global__ void __launch_bounds__(256) k_adj_reinit_c(const Inst* __restrict__ inst, Tiles tl, const T* __restrict__ cf, long long ld, const T* __restrict__ lam, T* __restrict__ lam_out) {
-    const unsigned FM = 0xffffffffu;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+// A'_0..2, B'_0..2, ld apart), on flat tiles marching in k.  Bound
+// by its bytes: eight words per node.  A node's own lam and coefficients come
+// one plane ahead, what the plane below takes of it (lam, A'_2) two, its share
+// of the plane above is carried; the x and y neighbours are plain loads that
+// mostly hit L1.  512 x 256 x 256: 213 us (32 x 8 tiles, own values shuffled,
+// the plane above awaited) -> 204 us, 128^3 18 -> 15 us; five blocks per SM
+// (six: 215 us, eight: 228 us: too many planes at once for L2).
+template <typename T, typename O>
+__global__ void __launch_bounds__(kStageThreads, sizeof(T) == 4 ? 5 : 3) k_adj_reinit_c(const Inst* __restrict__ inst,
+        Tiles tl, const T* __restrict__ cf, long long ld, const T* __restrict__ lam, T* __restrict__ lam_out) {
+    struct Pl {
+        T A0, A1, B0, B1, B2;
+    };
+    const int t = threadIdx.x;
     for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {
         const ABrick ab = adj_brick(tl, blk);
         const Inst& I = inst[ab.inst];
         const int ni = I.ni, nj = I.nj, nk = I.nk;
-        const long long sj = ni, sk = (long long)ni * nj;
-        const int i = ab.i0 + tx, j = ab.j0 + ty;
+        const int y = t / I.sw, x = t - y * I.sw;
+        const int i = ab.i0 + x, j = ab.j0 + y;
+        if (y >= I.sh || i >= ni || j >= nj) continue;
         const int k0 = ab.k0, k1 = min(k0 + tl.len, nk);
-        const bool col = i < ni && j < nj;
-        const long long cb = I.off + i + sj * j;
         const bool xm = i > 0, xp = i < ni - 1, ym = j > 0, yp = j < nj - 1;
-        const bool exm = col && xm && tx == 0, exp_ = col && xp && tx == 31;
-        // own values of a plane: lam, A'_0..2, B'_0..2; the x-edge lanes' outside
-        // neighbour (lam, and A'_0 above / B'_0 below); the y neighbours
-        struct Plane {
-            T L, A[3], B[3], Le, Ce, Lym, Bym, Lyp, Ayp;
+        constexpr O E = sizeof(T);
+        const O sj = E * (O)ni, sk = sj * (O)nj;
+        O l = E * (O)I.off + E * (O)i + sj * (O)j + sk * (O)k0;   // plane k
+        auto ld_own = [&](O l, Pl& p) {
+            p.A0 = ldo(cf, l);
+            p.A1 = ldo(cf + ld, l);
+            p.B0 = ldo(cf + 3 * ld, l);
+            p.B1 = ldo(cf + 4 * ld, l);
+            p.B2 = ldo(cf + 5 * ld, l);
         };
-        auto ld_plane = [&](int k, Plane& p) {
-            p.L = p.Le = p.Ce = p.Lym = p.Bym = p.Lyp = p.Ayp = T(0);
-#pragma unroll
-            for (int m = 0; m < 3; ++m) p.A[m] = p.B[m] = T(0);
-            if (!col || k < 0 || k >= nk) return;
-            const long long l = cb + sk * k;
-            p.L = __ldg(lam + l);
-#pragma unroll
-            for (int m = 0; m < 3; ++m) {
-                p.A[m] = __ldg(cf + m * ld + l);
-                p.B[m] = __ldg(cf + (3 + m) * ld + l);
+        Pl a, b;
+        ld_own(l, a);
+        T L = ldo(lam, l), A2 = ldo(cf + 2 * ld, l), Ln = T(0), An = T(0);
+        if (k0 + 1 < nk) {
+            Ln = ldo(lam, l + sk);
+            An = ldo(cf + 2 * ld, l + sk);
+        }
+        T zb = k0 > 0 ? ldo(lam, l - sk) * ldo(cf + 5 * ld, l - sk) : T(0);   // lam B'_2 of the plane below
+        auto plane = [&](int k, const Pl& c, Pl& n) {
+            T Lnn = T(0), Ann = T(0);
+            if (k + 1 < k1) {
+                ld_own(l + sk, n);
+                if (k + 2 < nk) {
+                    Lnn = ldo(lam, l + 2 * sk);
+                    Ann = ldo(cf + 2 * ld, l + 2 * sk);
+                }
             }
-            if (exm) {
-                p.Le = __ldg(lam + l - 1);
-                p.Ce = __ldg(cf + 3 * ld + l - 1);
-            }
-            if (exp_) {
-                p.Le = __ldg(lam + l + 1);
-                p.Ce = __ldg(cf + l + 1);
-            }
-            if (ym) {
-                p.Lym = __ldg(lam + l - sj);
-                p.Bym = __ldg(cf + 4 * ld + l - sj);
-            }
-            if (yp) {
-                p.Lyp = __ldg(lam + l + sj);
-                p.Ayp = __ldg(cf + ld + l + sj);
-            }
+            T t0 = L * (c.A0 - c.B0), t1 = L * (c.A1 - c.B1);
+            if (xp) t0 -= ldo(lam, l + E) * ldo(cf, l + E);
+            if (xm) t0 += ldo(lam, l - E) * ldo(cf + 3 * ld, l - E);
+            if (yp) t1 -= ldo(lam, l + sj) * ldo(cf + ld, l + sj);
+            if (ym) t1 += ldo(lam, l - sj) * ldo(cf + 4 * ld, l - sj);
+            const T t2 = L * (A2 - c.B2) - Ln * An + zb;
+            sto(lam_out, l, L - t0 - t1 - t2);
+            zb = L * c.B2;
+            L = Ln;
+            A2 = An;
+            Ln = Lnn;
+            An = Ann;
+            l += sk;
         };
-        Plane pm, pc, pn;          // planes k-1, k, k+1
-        ld_plane(k0 - 1, pm);
-        ld_plane(k0, pc);
-        for (int k = k0; k < k1; ++k) {
-            ld_plane(k + 1, pn);
-            // x neighbours: lam and A'_0 of i+1, lam and B'_0 of i-1
-            const T Lxp = __shfl_down_sync(FM, pc.L, 1), Axp = __shfl_down_sync(FM, pc.A[0], 1);
-            const T Lxm = __shfl_up_sync(FM, pc.L, 1), Bxm = __shfl_up_sync(FM, pc.B[0], 1);
-            if (col) {
-                const T L = pc.L;
-                const T lxp = xp ? (tx == 31 ? pc.Le : Lxp) : T(0), axp = xp ? (tx == 31 ? pc.Ce : Axp) : T(0);
-                const T lxm = xm ? (tx == 0 ? pc.Le : Lxm) : T(0), bxm = xm ? (tx == 0 ? pc.Ce : Bxm) : T(0);
-                const bool zm = k > 0, zp = k < nk - 1;
-                const T t0 = L * pc.A[0] - L * pc.B[0] - lxp * axp + lxm * bxm;
-                const T t1 = L * pc.A[1] - L * pc.B[1] - pc.Lyp * pc.Ayp + pc.Lym * pc.Bym;
-                const T t2 = L * pc.A[2] - L * pc.B[2] - (zp ? pn.L * pn.A[2] : T(0)) + (zm ? pm.L * pm.B[2] : T(0));
-                lam_out[cb + sk * k] = L - t0 - t1 - t2;
-            }
-            pm = pc;
-            pc = pn;
+        for (int k = k0;;) {
+            plane(k, a, b);
+            if (++k >= k1) break;
+            plane(k, b, a);
+            if (++k >= k1) break;
         }
     }
 }
@@ -1484,7 +1482,7 @@ __device__ void cell_mass_weights(const P (&ph8)[8], const P (&C)[8][3], P Cs, P
 }
 
 // The volume pass runs in two kernels.  k_vol_scan_z streams every cell of
-// every instance (a k march over the tiles of adjoint map 2): cells whose
+// every instance (a k march over the tiles of adjoint map 1): cells whose
 // eight vertices are water (phi > eps_sims, in the phi type) add their
 // precomputed FP64 hexahedron volume in 64-bit fixed point; interface cells
 // (any other mix) are appended to a list, each warp reserving its slots with
@@ -1510,7 +1508,7 @@ __device__ __forceinline__ long long warp_sum_nn(long long v) {
 }
 
 // Bulk water volumes of the cells (added to acc[4 inst + 2]) and the
-// interface-cell list, on the tiles of adjoint map 2 (FULL: tiles of the
+// interface-cell list, on the tiles of adjoint map 1 (FULL: tiles of the
 // longest march, a constant that saves 4 registers and with them a block per
 // SM: 111 against 125 us on 512 x 256 x 256 nodes): thread (lane, row) owns the cell column (i0 + lane, j0 +
 // row) and marches the tile's planes in k.  A cell's eight vertices are the
@@ -1543,7 +1541,7 @@ __global__ void __launch_bounds__(256) k_vol_scan_z(const Inst* __restrict__ ins
         const long long sj = ni, sk = (long long)ni * nj;
         const int i = ab.i0 + tx, j = ab.j0 + ty;
         // cells k0 .. kc1 - 1 (a cell's top plane k + 1 stays inside the grid)
-        const int k0 = ab.k0, kc1 = min(k0 + (FULL ? adj_shape(2).oz : tl.len), nk - 1);
+        const int k0 = ab.k0, kc1 = min(k0 + (FULL ? adj_shape(1).oz : tl.len), nk - 1);
         const bool cell = i < ni - 1 && j < nj - 1;
         const bool own = i < ni && j < nj - 1, edge = tx == 31 && i + 1 < ni && j < nj - 1;
         const long long cb = I.off + i + sj * j;
@@ -1768,7 +1766,7 @@ __global__ void __launch_bounds__(128) k_mass_weights(Flat fl, FieldsT<T> f, con
     }
 }
 
-// Adjoint of the shift, part 2: per tile of adjoint map 2 (32 x 8 columns
+// Adjoint of the shift, part 2: per tile of adjoint map 1 (32 x 8 columns
 // x 32 planes, inside one instance) the sum of lam over the tile, in a
 // fixed order (each thread its column, then a fixed tree), accumulated in
 // FP64.  FP32 lam is first summed in FP32 over runs of 8 planes (the FP64
@@ -1815,8 +1813,8 @@ __global__ void __launch_bounds__(256) k_inst_sum(const Inst* __restrict__ inst,
                                                   double* __restrict__ out) {
     __shared__ double red[8];
     const Inst& I = inst[blockIdx.x];
-    const int t0 = I.am[2][0];
-    const int nt = I.am[2][1] * I.am[2][2] * ((I.nk + len - 1) / len);
+    const int t0 = I.am[1][0];
+    const int nt = I.am[1][1] * I.am[1][2] * ((I.nk + len - 1) / len);
     double s = 0.0;
     for (int u = threadIdx.x; u < nt; u += blockDim.x) s += part[t0 + u];
 #pragma unroll
@@ -1963,12 +1961,11 @@ __global__ void k_adj_face(Flat fl, int face0, long long nplane, int nface, BC b
     lam[l] = T(0);
 }
 
-// value and gradient of rec3 (one reciprocal r)
+// value of rec3 on a stencil with differences eL, eR and smoothness t1, t0, and
+// its gradient (one reciprocal r)
 template <typename T>
-__device__ __forceinline__ T rec3_vg(T fL, T fC, T fR, T* dL, T* dC, T* dR) {
-    const T eL = fL - fC, eR = fC - fR, h = eL - eR;
-    const T t0 = vfma(eR, eR, T(1.0e-6)), t1 = vfma(eL, eL, T(1.0e-6));
-    const T q = t1 * t1, a1 = t0 * t0;
+__device__ __forceinline__ T rec3_vg(T fC, T eL, T eR, T t1, T t0, T* dL, T* dC, T* dR) {
+    const T h = eL - eR, q = t1 * t1, a1 = t0 * t0;
     const T r = wrcp(vfma(T(2), q, a1));
     const T v = q * r, z = T(4) * r * h;
     // h dv / d eL = 4 t1 a1 r^2 h eL, h dv / d eR = -4 t0 t1^2 r^2 h eR
@@ -1979,188 +1976,242 @@ __device__ __forceinline__ T rec3_vg(T fL, T fC, T fR, T* dL, T* dC, T* dR) {
     return vfma(v, h, vfma(T(-0.5), eL, fC));
 }
 
-// D = Phi+ - Phi- of a node (stencil s, orientation frozen by w) and the
-// gradient G = lp w dD/ds of lp w D, branch-free
+// D = Phi+ - Phi- of a node and the gradient G = lp w dD/ds of lp w D over its
+// stencil s = -2 .. 2, the orientation frozen by w; the neighbours and `edge`
+// as for weno_wind
 template <typename T>
-__device__ __forceinline__ T stage_node_grad(const T (&s)[5], T w, T lp, bool lo, bool hi, T (&G)[5]) {
+__device__ __forceinline__ T stage_node_grad(T q0, T q1, T c, T q3, bool edge, T w, T lp, T (&G)[5]) {
+    const T fL = edge ? q3 : q0, fC = edge ? c : q1;
+    const T e0 = fL - fC, e1 = q1 - c, e2 = c - q3;
+    const T t0 = vfma(e0, e0, T(1.0e-6)), t1 = vfma(e1, e1, T(1.0e-6)), t2 = vfma(e2, e2, T(1.0e-6));
+    T dL, dC, dR, uL, uC, uR;
+    const T vd = rec3_vg(c, e1, e2, t1, t2, &dL, &dC, &dR);
+    const T vu = rec3_vg(fC, e0, edge ? -e1 : e1, t0, t1, &uL, &uC, &uR);
     const bool up = w > T(0);
-    const bool P = up || hi, M = up && !lo;
-    T a, b, c, a2, b2, c2;
-    const T vp = rec3_vg(P ? s[1] : s[4], P ? s[2] : s[3], P ? s[3] : s[2], &a, &b, &c);
-    const T vm = rec3_vg(M ? s[0] : s[3], M ? s[1] : s[2], M ? s[2] : s[1], &a2, &b2, &c2);
-    const T k = lp * w;
-    G[0] = -k * (M ? a2 : T(0));
-    G[1] = k * ((P ? a : T(0)) - (M ? b2 : c2));
-    G[2] = k * ((P ? b : c) - (M ? c2 : b2));
-    G[3] = k * ((P ? c : b) - (M ? T(0) : a2));
-    G[4] = k * (P ? T(0) : a);
-    return vp - vm;
+    const T k = lp * fabs(w), D = vd - vu;
+    const T g0 = edge ? T(0) : -k * uL, g1 = k * (dL - (edge ? uR : uC)), g3 = k * (dR - (edge ? uL : T(0)));
+    G[0] = up ? g0 : T(0);
+    G[1] = up ? g1 : g3;
+    G[2] = k * (dC - (edge ? uC : uR));
+    G[3] = up ? g3 : g1;
+    G[4] = up ? T(0) : g0;
+    return up ? D : -D;
+}
+// the same from the stencil
+template <typename T>
+__device__ __forceinline__ T stage_node_grad(T m2, T m1, T c, T p1, T p2, bool lo, bool hi, T w, T lp, T (&G)[5]) {
+    const bool up = w > T(0);
+    return stage_node_grad(up ? m2 : p2, up ? m1 : p1, c, up ? p1 : m1, up ? lo : hi, w, lp, G);
 }
 
-// Stage adjoint, x part (adjoint map 0: bricks of 8 whole rows of one
-// plane, one warp per row) plus the pointwise terms.  The warp marches its
-// row in aligned chunks of 32 nodes: it evaluates G_x of chunk c + 1, then
-// writes chunk c, gathering the five contributions of each node by warp
-// shuffles from chunks c - 1, c, c + 1 held in registers.  Each warp starts
-// at its own chunk (rows hashed over the row length) and wraps around, so
-// that the warps of the GPU do not all stream the same columns at once.
-// Writes lam_in = c2 lamP0 - c3 acc_x (+ lamPhin + c1 lamP0 when last),
-// updates lamPhin and lamW_x.
-template <typename T>
-__global__ void __launch_bounds__(256) k_adj_stage_x(const Inst* __restrict__ inst, Tiles tl, FieldsT<T> f, const T* __restrict__ in, const T* __restrict__ lamP0, T* __restrict__ lam_in,
-        T* __restrict__ lamPhin, T* __restrict__ lamW0, T c1, T c2, T c3, int last) {
-    const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+// Stage adjoint, x and z parts and the pointwise terms, on flat tiles (Inst's
+// xw x xh columns and, where they are not whole rows, a rim of two nodes in x;
+// row-major over the threads) marching in k.  At plane q a thread evaluates
+// G_z of its node, which it adds to the sums of the nodes q - 2 .. q + 2 in
+// registers, and G_x, whose outer components its neighbours take from shared
+// memory (one barrier per plane, two buffers; a node next to a row's end has
+// no component across it).  Plane q - 2 is then complete: lam_in = c2 lamP0 -
+// c3 (acc_x + acc_z) (+ lamPhin + c1 lamP0 when last), lamPhin, lamW_x and
+// lamW_z.  Eleven words per node are read or written (fifteen in a pass each,
+// x by warps along their rows); issue-bound then and now.  Measured on 512 x
+// 256 x 256 nodes: 265 + 243 -> 474 us, 128^3 25 + 23 -> 30 us, two FP64 grids
+// of 40^3 48 + 70 -> 57 us; 128 threads, so that a barrier holds up few warps,
+// eight blocks per SM (256 threads: 454, 31 and 65 us; three quarters of the
+// warps 502 us).
+template <typename T, typename O>
+__global__ void __launch_bounds__(kAdjThreads, sizeof(T) == 4 ? 8 : 4) k_adj_stage_xz(const Inst* __restrict__ inst,
+        Tiles tl, FieldsT<T> f, const T* __restrict__ in, const T* __restrict__ lamP0, T* __restrict__ lam_in,
+        T* __restrict__ lamPhin, T* __restrict__ lamW0, T* __restrict__ lamW2, T c1, T c2, T c3, int last) {
+    __shared__ T gx[2][4][kAdjThreads + 4];   // components 4, 3, 1, 0 of the block's nodes, two zeros around
+    struct Pl {
+        T s, lp, W0, W2, phin, w0, w2;   // in of plane q + 2; plane q; the old values of plane q - 2
+    };
+    const int t = threadIdx.x;
+    if (t < 32) {
+        const int r = t & 3;
+        gx[t >> 4][(t >> 2) & 3][r < 2 ? r : kAdjThreads + r] = T(0);
+    }
     for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {
         const ABrick ab = adj_brick(tl, blk);
         const Inst& I = inst[ab.inst];
         const int ni = I.ni, nj = I.nj, nk = I.nk;
-        const int j = ab.j0 + row, k = ab.k0;
-        if (j >= nj) continue;   // whole warp
-        const bool jk_int = j >= 1 && j <= nj - 2 && k >= 1 && k <= nk - 2;
-        const long long rowbase = I.off + (long long)ni * (j + (long long)nj * k);
-        const int nc = (ni + 31) >> 5;
-        // G_x of chunk c (zero outside the row and at non-interior nodes)
-        auto eval = [&](int c, T (&G)[5], T& D, T& lp) {
-#pragma unroll
-            for (int p = 0; p < 5; ++p) G[p] = T(0);
-            D = lp = T(0);
-            const int ii = (c << 5) + lane;
-            if (c >= 0 && c < nc && ii < ni) {
-                const long long l = rowbase + ii;
-                lp = __ldg(lamP0 + l);
-                if (jk_int && ii >= 1 && ii <= ni - 2) {
-                    const T sv[5] = {ii >= 2 ? __ldg(in + l - 2) : T(0), __ldg(in + l - 1), __ldg(in + l),
-                                     __ldg(in + l + 1), ii <= ni - 3 ? __ldg(in + l + 2) : T(0)};
-                    D = stage_node_grad(sv, __ldg(f.W[0] + l), lp, ii == 1, ii == ni - 2, G);
-                }
+        const int rim = I.xw < ni ? 2 : 0, ew = I.xw + 2 * rim;
+        const int y = t / ew, x = t - y * ew;
+        const int i = ab.i0 + x - rim, j = ab.j0 + y;
+        const bool col = y < I.xh && i >= 0 && i < ni && j < nj;
+        const bool core = col && x >= rim && x < I.xw + rim;
+        const bool ij_int = col && i > 0 && i < ni - 1 && j > 0 && j < nj - 1;
+        const bool ilo = i == 1, ihi = i == ni - 2;
+        const int k0 = ab.k0, k1 = min(k0 + tl.len, nk);
+        constexpr O E = sizeof(T);
+        const O sk = E * (O)ni * (O)nj;
+        O l = E * (O)I.off + E * (O)i + E * (O)ni * (O)j + sk * (O)(k0 - 2);   // plane q
+        T s0 = T(0), s1 = T(0), s2 = T(0), s3 = T(0);
+        T A0 = T(0), A1 = T(0), A2 = T(0), A3 = T(0);   // z sums of planes q - 2 .. q + 1
+        T ax1 = T(0), ax2 = T(0), d1 = T(0), d2 = T(0), z1 = T(0), z2 = T(0), p1 = T(0), p2 = T(0);
+        // what plane q needs, one plane ahead
+        auto ld = [&](int q, O l, Pl& p) {
+            p.s = p.lp = T(0);
+            if (!col) return;
+            if (q + 2 < nk && q + 2 <= k1 + 3) p.s = ldo(in, l + 2 * sk);
+            if (q >= 0 && q < nk && q < k1 + 2) {
+                p.lp = ldo(lamP0, l);
+                p.W0 = ldo(f.W[0], l);
+                p.W2 = ldo(f.W[2], l);
+            }
+            if (core && q - 2 >= k0 && q - 2 < k1) {
+                p.phin = ldv(lamPhin, l - 2 * sk);
+                p.w0 = ldv(lamW0, l - 2 * sk);
+                p.w2 = ldv(lamW2, l - 2 * sk);
             }
         };
-        // march chunks a .. b-1 (outputs), with chunk a-1 primed
-        auto segment = [&](int a, int b) {
-            T Gp[5], Gc[5], Gn[5], Dc, Dn, lpc, lpn;
-            eval(a - 1, Gc, Dc, lpc);
-#pragma unroll
-            for (int p = 0; p < 5; ++p) Gp[p] = T(0);
-            for (int c = a; c <= b; ++c) {
-                // read-modify-write values of the output chunk c - 1 first, so
-                // that their loads are in flight together with chunk c's
-                const int io = ((c - 1) << 5) + lane;
-                const bool wo = c > a && io < ni;
-                const long long lo = rowbase + io;
-                T phin_old = T(0), w_old = T(0);
-                if (wo) {
-                    phin_old = lamPhin[lo];
-                    w_old = lamW0[lo];
+        if (col) {
+            if (k0 >= 4) s0 = ldo(in, l - 2 * sk);
+            if (k0 >= 3) s1 = ldo(in, l - sk);
+            if (k0 >= 2) s2 = ldo(in, l);
+            if (k0 >= 1) s3 = ldo(in, l + sk);
+        }
+        Pl a, b;
+        ld(k0 - 2, l, a);
+        auto plane = [&](int q, const Pl& c, Pl& n, T (*g)[kAdjThreads + 4]) {
+            ld(q + 1, l + sk, n);
+            const T s4 = c.s;
+            const bool zin = q > 0 && q < nk - 1;
+            T Gz[5] = {T(0), T(0), T(0), T(0), T(0)}, dz = T(0), dx = T(0), ax = T(0);
+            if (zin && core && ij_int)
+                dz = stage_node_grad(s0, s1, s2, s3, s4, q == 1, q == nk - 2, c.W2, c.lp, Gz);
+            if (q >= k0 && q < k1) {
+                T Gx[5] = {T(0), T(0), T(0), T(0), T(0)};
+                if (zin && ij_int) {
+                    const bool up = c.W0 > T(0);
+                    const O o = up ? E : O(0) - E;   // in the array for every interior node
+                    dx = stage_node_grad(ldo(in, l - 2 * o), ldo(in, l - o), s2, ldo(in, l + o), up ? ilo : ihi, c.W0,
+                                         c.lp, Gx);
                 }
-                eval(c, Gn, Dn, lpn);
-                if (c > a) {
-                    // node lane + o of chunk c - 1 contributes component 2 - o;
-                    // across the chunk edges it lies in chunk c - 2 (Gp) or c (Gn)
-                    const unsigned FM = 0xffffffffu;
-                    const T m2c = __shfl_sync(FM, Gc[4], (lane - 2) & 31), m2p = __shfl_sync(FM, Gp[4], (lane - 2) & 31);
-                    const T m1c = __shfl_sync(FM, Gc[3], (lane - 1) & 31), m1p = __shfl_sync(FM, Gp[3], (lane - 1) & 31);
-                    const T p1c = __shfl_sync(FM, Gc[1], (lane + 1) & 31), p1n = __shfl_sync(FM, Gn[1], (lane + 1) & 31);
-                    const T p2c = __shfl_sync(FM, Gc[0], (lane + 2) & 31), p2n = __shfl_sync(FM, Gn[0], (lane + 2) & 31);
-                    const T acc = (lane >= 2 ? m2c : m2p) + (lane >= 1 ? m1c : m1p) + Gc[2] +
-                                  (lane <= 30 ? p1c : p1n) + (lane <= 29 ? p2c : p2n);
-                    if (wo) {
-                        lamW0[lo] = w_old - c3 * lpc * Dc;
-                        T r = c2 * lpc - c3 * acc;
-                        if (last) {
-                            r += phin_old + c1 * lpc;
-                            lamPhin[lo] = T(0);
-                        } else {
-                            lamPhin[lo] = phin_old + c1 * lpc;
-                        }
-                        lam_in[lo] = r;
-                    }
-                }
-#pragma unroll
-                for (int p = 0; p < 5; ++p) {
-                    Gp[p] = Gc[p];
-                    Gc[p] = Gn[p];
-                }
-                Dc = Dn;
-                lpc = lpn;
+                g[0][t + 2] = Gx[4];
+                g[1][t + 2] = Gx[3];
+                g[2][t + 2] = Gx[1];
+                g[3][t + 2] = Gx[0];
+                __syncthreads();
+                ax = g[0][t] + g[1][t + 1] + Gx[2] + g[2][t + 3] + g[3][t + 4];
             }
+            const T acc = A0 + Gz[0];
+            if (core && q - 2 >= k0) {
+                const O lo = l - 2 * sk;
+                sto(lamW0, lo, c.w0 - c3 * p2 * d2);
+                sto(lamW2, lo, c.w2 - c3 * p2 * z2);
+                T r = c2 * p2 - c3 * (ax2 + acc);
+                if (last) r += c.phin + c1 * p2;
+                sto(lamPhin, lo, last ? T(0) : c.phin + c1 * p2);
+                sto(lam_in, lo, r);
+            }
+            A0 = A1 + Gz[1];
+            A1 = A2 + Gz[2];
+            A2 = A3 + Gz[3];
+            A3 = Gz[4];
+            ax2 = ax1;
+            ax1 = ax;
+            d2 = d1;
+            d1 = dx;
+            z2 = z1;
+            z1 = dz;
+            p2 = p1;
+            p1 = c.lp;
+            s0 = s1;
+            s1 = s2;
+            s2 = s3;
+            s3 = s4;
+            l += sk;
         };
-        const int s0 = (int)(((unsigned)(j + 7 * k) * 2654435761u >> 16) % (unsigned)nc);
-        segment(s0, nc);
-        if (s0 > 0) segment(0, s0);
+        for (int q = k0 - 2;;) {
+            plane(q, a, b, gx[0]);
+            if (++q >= k1 + 2) break;
+            plane(q, b, a, gx[1]);
+            if (++q >= k1 + 2) break;
+        }
+        __syncthreads();   // the next tile writes the buffers that this one's last plane reads
     }
 }
 
-// Stage adjoint, y (AX = 1, adjoint map 1) or z (AX = 2, map 4) part: each
-// thread marches one line along AX over Tiles::len outputs (FULL: the
-// longest, a constant; registers for five blocks per SM in the z part, 283
-// against 290 us on 512 x 256 x 256 nodes), keeping
-// windows of five G, lamP0 and D values in registers; lam_in -= c3 acc,
-// lamW_AX -= c3 lamP0 D.
-template <typename T, int AX, bool FULL>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 && AX == 2 ? 5 : 0) k_adj_stage_m(const Inst* __restrict__ inst, Tiles tl, FieldsT<T> f, const T* __restrict__ in, const T* __restrict__ lamP0, T* __restrict__ lam_in,
-        T* __restrict__ lamW, T c3) {
-    const int tx = threadIdx.x & 31, tq = threadIdx.x >> 5;
+// Stage adjoint, y part: flat tiles of Inst's yw x yh columns in (i, k),
+// marching in j as the z part does in k; lam_in -= c3 acc, lamW_y -= c3 lamP0 D.
+// 512 x 256 x 256: 242 -> 202 us, 128^3 22 -> 18 us, two FP64 grids of 40^3 70
+// -> 41 us.
+template <typename T, typename O>
+__global__ void __launch_bounds__(kAdjThreads, sizeof(T) == 4 ? 12 : 4) k_adj_stage_y(const Inst* __restrict__ inst,
+        Tiles tl, FieldsT<T> f, const T* __restrict__ in, const T* __restrict__ lamP0, T* __restrict__ lam_in,
+        T* __restrict__ lamW1, T c3) {
+    struct Pl {
+        T s, lp, W, lin, w;   // in of row q + 2; row q; the old values of row q - 2
+    };
+    const int t = threadIdx.x;
     for (int blk = blockIdx.x; blk < tl.n; blk += gridDim.x) {
         const ABrick ab = adj_brick(tl, blk);
         const Inst& I = inst[ab.inst];
         const int ni = I.ni, nj = I.nj, nk = I.nk;
-        const long long sj = ni, sk = (long long)ni * nj;
-        const int i = ab.i0 + tx;
-        // the other coordinate (k for AX = 1, j for AX = 2) and the march range
-        const int c2 = AX == 1 ? ab.k0 + tq : ab.j0 + tq;
-        const int n2 = AX == 1 ? nk : nj, nm = AX == 1 ? nj : nk;
-        const int m0 = AX == 1 ? ab.j0 : ab.k0;
-        const int m1 = min(m0 + (FULL ? (AX == 1 ? adj_shape(1).oy : adj_shape(4).oz) : tl.len), nm);
-        const bool col = i < ni && c2 < n2;
-        const bool line = col && i >= 1 && i <= ni - 2 && c2 >= 1 && c2 <= n2 - 2;
-        const long long st = AX == 1 ? sj : sk;
-        const long long base = I.off + i + (AX == 1 ? sk * c2 : sj * c2);
-        // windows over march positions q-4 .. q (index 0..4)
-        T g[5][5], lpw[5], dw[5];
-#pragma unroll
-        for (int a = 0; a < 5; ++a) {
-            lpw[a] = dw[a] = T(0);
-#pragma unroll
-            for (int p = 0; p < 5; ++p) g[a][p] = T(0);
+        const int y = t / I.yw, x = t - y * I.yw;
+        const int i = ab.i0 + x, k = ab.k0 + y;
+        const bool col = y < I.yh && i < ni && k < nk;
+        const bool line = col && i > 0 && i < ni - 1 && k > 0 && k < nk - 1;
+        const int m0 = ab.j0, m1 = min(m0 + tl.len, nj);
+        constexpr O E = sizeof(T);
+        const O st = E * (O)ni;
+        O l = E * (O)I.off + E * (O)i + st * (O)nj * (O)k + st * (O)(m0 - 2);   // row q
+        T s0 = T(0), s1 = T(0), s2 = T(0), s3 = T(0);
+        T A0 = T(0), A1 = T(0), A2 = T(0), A3 = T(0);
+        T z1 = T(0), z2 = T(0), p1 = T(0), p2 = T(0);
+        auto ld = [&](int q, O l, Pl& p) {
+            p.s = p.lp = T(0);
+            if (!col) return;
+            if (q + 2 < nj && q + 2 <= m1 + 3) p.s = ldo(in, l + 2 * st);
+            if (q >= 0 && q < nj && q < m1 + 2) {
+                p.lp = ldo(lamP0, l);
+                p.W = ldo(f.W[1], l);
+            }
+            if (q - 2 >= m0 && q - 2 < m1) {
+                p.lin = ldv(lam_in, l - 2 * st);
+                p.w = ldv(lamW1, l - 2 * st);
+            }
+        };
+        if (col) {
+            if (m0 >= 4) s0 = ldo(in, l - 2 * st);
+            if (m0 >= 3) s1 = ldo(in, l - st);
+            if (m0 >= 2) s2 = ldo(in, l);
+            if (m0 >= 1) s3 = ldo(in, l + st);
         }
-        for (int q = m0 - 2; q < m1 + 2; ++q) {
-            const int jo = q - 2;   // output position: window index 2 after the shift
-            const bool wo = col && jo >= m0 && jo < m1;
-            const long long lo = base + st * jo;
-            T lin_old = T(0), w_old = T(0);
-            if (wo) {
-                lin_old = lam_in[lo];
-                w_old = lamW[lo];
+        Pl a, b;
+        ld(m0 - 2, l, a);
+        auto row = [&](int q, const Pl& c, Pl& n) {
+            ld(q + 1, l + st, n);
+            const T s4 = c.s;
+            T G[5] = {T(0), T(0), T(0), T(0), T(0)}, D = T(0);
+            if (line && q > 0 && q < nj - 1)
+                D = stage_node_grad(s0, s1, s2, s3, s4, q == 1, q == nj - 2, c.W, c.lp, G);
+            const T acc = A0 + G[0];
+            if (col && q - 2 >= m0) {
+                const O lo = l - 2 * st;
+                sto(lam_in, lo, c.lin - c3 * acc);
+                sto(lamW1, lo, c.w - c3 * p2 * z2);
             }
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                lpw[a] = lpw[a + 1];
-                dw[a] = dw[a + 1];
-#pragma unroll
-                for (int p = 0; p < 5; ++p) g[a][p] = g[a + 1][p];
-            }
-            T G[5] = {T(0), T(0), T(0), T(0), T(0)};
-            T D = T(0), lp = T(0);
-            if (col && q >= 0 && q < nm) {
-                const long long l = base + st * q;
-                lp = __ldg(lamP0 + l);
-                if (line && q >= 1 && q <= nm - 2) {
-                    const T sv[5] = {q >= 2 ? __ldg(in + l - 2 * st) : T(0), __ldg(in + l - st), __ldg(in + l),
-                                     __ldg(in + l + st), q <= nm - 3 ? __ldg(in + l + 2 * st) : T(0)};
-                    D = stage_node_grad(sv, __ldg(f.W[AX] + l), lp, q == 1, q == nm - 2, G);
-                }
-            }
-            lpw[4] = lp;
-            dw[4] = D;
-#pragma unroll
-            for (int p = 0; p < 5; ++p) g[4][p] = G[p];
-            if (wo) {
-                T acc = T(0);
-#pragma unroll
-                for (int o = -2; o <= 2; ++o) acc += g[2 + o][2 - o];
-                lam_in[lo] = lin_old - c3 * acc;
-                lamW[lo] = w_old - c3 * lpw[2] * dw[2];
-            }
+            A0 = A1 + G[1];
+            A1 = A2 + G[2];
+            A2 = A3 + G[3];
+            A3 = G[4];
+            z2 = z1;
+            z1 = D;
+            p2 = p1;
+            p1 = c.lp;
+            s0 = s1;
+            s1 = s2;
+            s2 = s3;
+            s3 = s4;
+            l += st;
+        };
+        for (int q = m0 - 2;;) {
+            row(q, a, b);
+            if (++q >= m1 + 2) break;
+            row(q, b, a);
+            if (++q >= m1 + 2) break;
         }
     }
 }
@@ -2213,7 +2264,7 @@ __device__ __forceinline__ void coef_eval(const CoefIn<T>& c, T dtau, const bool
 
 // Reverse of one reinitialisation pseudo-step d' = d - dtau s (G(d) - 1):
 //   lam_out(j) = lam(j) - sum_m [A_m(j) - B_m(j) - A_m(j+e_m) + B_m(j-e_m)]
-// (adjoint map 3).  A block of 32 x kReinRY threads covers nodes i0-1 ..
+// (adjoint map 0).  A block of 32 x kReinRY threads covers nodes i0-1 ..
 // i0+30, j0-1 .. j0+kReinRY-2 and writes the inner 30 x (kReinRY-2); it
 // marches in k.  Iteration k evaluates the coefficients of plane k and
 // writes plane k-1.  Each node loads its own d, s, lam and metrics only:
@@ -2505,15 +2556,17 @@ int reinit_z_blocks_per_sm() {
     return n;
 }
 template <typename T>
-void adj_reinit_c(int grid, const Inst* inst, Tiles tl, const T* cf, long long ld, const T* lam,
-                  T* lam_out, cudaStream_t s) {
+void adj_reinit_c(int grid, const Inst* inst, Tiles tl, bool wide, const T* cf, long long ld, const T* lam, T* lam_out,
+                  cudaStream_t s) {
     ProfScope ps_("k_adj_reinit_c", s);
-    k_adj_reinit_c<T><<<grid, 256, 0, s>>>(inst, tl, cf, ld, lam, lam_out);
+    auto go = [&](auto kernel) { kernel<<<grid, kStageThreads, 0, s>>>(inst, tl, cf, ld, lam, lam_out); };
+    if (wide) go(k_adj_reinit_c<T, unsigned long long>);
+    else go(k_adj_reinit_c<T, unsigned>);
 }
 template <typename T>
 int adj_reinit_c_blocks_per_sm() {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_reinit_c<T>, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_reinit_c<T, unsigned>, kStageThreads, 0);
     return n;
 }
 template <typename T>
@@ -2529,7 +2582,7 @@ void volume(int grid2, const Inst* inst, Tiles tl, const Flat& fl, FieldsT<T> f,
     cudaMemsetAsync(count, 0, sizeof(unsigned), s);
     {
         ProfScope ps_("k_vol_scan_z", s);
-        if (tl.len == adj_shape(2).oz) k_vol_scan_z<T, true><<<grid2, 256, 0, s>>>(inst, tl, f, phi, acc, list, count);
+        if (tl.len == adj_shape(1).oz) k_vol_scan_z<T, true><<<grid2, 256, 0, s>>>(inst, tl, f, phi, acc, list, count);
         else k_vol_scan_z<T, false><<<grid2, 256, 0, s>>>(inst, tl, f, phi, acc, list, count);
     }
     if (slope) {
@@ -2608,26 +2661,31 @@ void adj_face(const Flat& fl, int face, long long nplane, int nface, BC bc, int 
                                                               T(c2), lam);
 }
 template <typename T>
-void adj_stage(const int* grid, const Inst* inst, const Tiles* tl, FieldsT<T> f, const T* in,
+void adj_stage(const int (&grid)[2], const Inst* inst, const Tiles (&tl)[2], bool wide, FieldsT<T> f, const T* in,
                const T* lamP0, T* lam_in, T* lamPhin, T* lamW0, T* lamW1, T* lamW2, double c1, double c2, double c3,
                bool last, cudaStream_t s) {
     {
-        ProfScope ps_("k_adj_stage_x", s);
-        k_adj_stage_x<T><<<grid[0], 256, 0, s>>>(inst, tl[0], f, in, lamP0, lam_in, lamPhin, lamW0, T(c1),
-                                                 T(c2), T(c3), last ? 1 : 0);
+        ProfScope ps_("k_adj_stage_xz", s);
+        auto go = [&](auto kernel) {
+            kernel<<<grid[0], kAdjThreads, 0, s>>>(inst, tl[0], f, in, lamP0, lam_in, lamPhin, lamW0, lamW2, T(c1),
+                                                   T(c2), T(c3), last ? 1 : 0);
+        };
+        if (wide) go(k_adj_stage_xz<T, unsigned long long>);
+        else go(k_adj_stage_xz<T, unsigned>);
     }
-    {
-        ProfScope ps_("k_adj_stage_y", s);
-        if (tl[1].len == adj_shape(1).oy)
-            k_adj_stage_m<T, 1, true><<<grid[1], 256, 0, s>>>(inst, tl[1], f, in, lamP0, lam_in, lamW1, T(c3));
-        else
-            k_adj_stage_m<T, 1, false><<<grid[1], 256, 0, s>>>(inst, tl[1], f, in, lamP0, lam_in, lamW1, T(c3));
-    }
-    ProfScope ps_("k_adj_stage_z", s);
-    if (tl[4].len == adj_shape(4).oz)
-        k_adj_stage_m<T, 2, true><<<grid[4], 256, 0, s>>>(inst, tl[4], f, in, lamP0, lam_in, lamW2, T(c3));
-    else
-        k_adj_stage_m<T, 2, false><<<grid[4], 256, 0, s>>>(inst, tl[4], f, in, lamP0, lam_in, lamW2, T(c3));
+    ProfScope ps_("k_adj_stage_y", s);
+    auto go = [&](auto kernel) {
+        kernel<<<grid[1], kAdjThreads, 0, s>>>(inst, tl[1], f, in, lamP0, lam_in, lamW1, T(c3));
+    };
+    if (wide) go(k_adj_stage_y<T, unsigned long long>);
+    else go(k_adj_stage_y<T, unsigned>);
+}
+template <typename T>
+int adj_stage_blocks_per_sm(int part) {
+    int n = 0;
+    if (part == 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_stage_xz<T, unsigned>, kAdjThreads, 0);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_stage_y<T, unsigned>, kAdjThreads, 0);
+    return n;
 }
 template <typename T>
 void adj_reinit(int grid, const Inst* inst, Tiles tl, FieldsT<T> f, const T* d, const T* lam,
@@ -2636,14 +2694,9 @@ void adj_reinit(int grid, const Inst* inst, Tiles tl, FieldsT<T> f, const T* d, 
     k_adj_reinit<T><<<grid, 32 * kReinRY, 0, s>>>(inst, tl, f, d, lam, lam_out);
 }
 template <typename T>
-int adj_blocks_per_sm(int map) {
+int adj_reinit_blocks_per_sm() {
     int n = 0;
-    switch (map) {
-    case 0: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_stage_x<T>, 256, 0); break;
-    case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_stage_m<T, 1, true>, 256, 0); break;
-    case 3: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_reinit<T>, 32 * kReinRY, 0); break;
-    default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_stage_m<T, 2, true>, 256, 0); break;
-    }
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adj_reinit<T>, 32 * kReinRY, 0);
     return n;
 }
 template <typename T>
@@ -2669,7 +2722,7 @@ void adj_contra(const Flat& fl, FieldsT<T> f, const T* w0, const T* w1, const T*
     template void reinit_z<T>(int, int, const Inst*, Tiles, FieldsT<T>, const T*, T*, T*, T*, long long, \
                               unsigned*, cudaStream_t);                                                         \
     template int reinit_z_blocks_per_sm<T>();                                                                   \
-    template void adj_reinit_c<T>(int, const Inst*, Tiles, const T*, long long, const T*, T*,           \
+    template void adj_reinit_c<T>(int, const Inst*, Tiles, bool, const T*, long long, const T*, T*,           \
                                   cudaStream_t);                                                                \
     template int adj_reinit_c_blocks_per_sm<T>();                                                               \
     template void volume<T>(int, const Inst*, Tiles, const Flat&, FieldsT<T>, const T*,                \
@@ -2681,11 +2734,12 @@ void adj_contra(const Flat& fl, FieldsT<T> f, const T* w0, const T* w1, const T*
                                   cudaStream_t);                                                                     \
     template void adj_face<T>(const Flat&, int, long long, int, BC, int, const T*, const T*, const T*, double, double, \
                               T*, cudaStream_t);                                                                     \
-    template void adj_stage<T>(const int*, const Inst*, const Tiles*, FieldsT<T>, const T*,      \
-                               const T*, T*, T*, T*, T*, T*, double, double, double, bool, cudaStream_t);      \
+    template void adj_stage<T>(const int (&)[2], const Inst*, const Tiles (&)[2], bool, FieldsT<T>, const T*,          \
+                               const T*, T*, T*, T*, T*, T*, double, double, double, bool, cudaStream_t);          \
+    template int adj_stage_blocks_per_sm<T>(int);                                                                  \
     template void adj_reinit<T>(int, const Inst*, Tiles, FieldsT<T>, const T*, const T*, T*,            \
                                 cudaStream_t);                                                                \
-    template int adj_blocks_per_sm<T>(int);                                                                     \
+    template int adj_reinit_blocks_per_sm<T>();                                                                     \
     template void adj_contra<T>(const Flat&, FieldsT<T>, const T*, const T*, const T*, T*, T*, T*, cudaStream_t);
 
 LSM_BATCH_INSTANTIATE(float)

@@ -16,7 +16,7 @@
 namespace lsm {
 namespace batch {
 
-constexpr int kMaps = 5;   // tile maps (adj_shape)
+constexpr int kMaps = 2;   // tile maps (adj_shape)
 
 struct Inst {
     long long off;     // first node of the instance in the packed arrays
@@ -31,7 +31,8 @@ struct Inst {
     long long fpre[3]; // first node of the instance's i-, j-, k-face planes (adjoint face kernels)
     double dt64, dtau64, eps64;  // the same three parameters for the FP64 kernels
     int rw, rh;                  // columns of a tile of reinit_pair, without its rim
-    int sw, sh;                  // columns of a tile of stage
+    int sw, sh;                  // columns of a tile of stage and of adj_reinit_c
+    int xw, xh, yw, yh;          // columns of a tile of the stage adjoint's parts: (i, j) without its rim, (i, k)
     int am[kMaps][3];            // adjoint brick maps (adj_shape): first brick, bricks per row, per plane
 };
 
@@ -157,7 +158,7 @@ void sign_reinit(int shape, int grid, const Inst* inst, const Brick* bricks, int
 template <typename T>
 void bc_reinit(const Inst* inst, int ninst, long long nface, FieldsT<T> f, BC bc, const T* din, T* dout,
                cudaStream_t s);
-// One reinitialisation pseudo-step on the tiles of adjoint map 2 (z march;
+// One reinitialisation pseudo-step on the tiles of adjoint map 1 (z march;
 // grid from reinit_z_blocks_per_sm): kind 0 plain, 1 recorded (the
 // pseudo-step's adjoint coefficients A'_0..2, B'_0..2 also written to cf,
 // arrays ld apart), 2 the sign field of phi0 (din) fused with the first
@@ -177,7 +178,7 @@ void reinit_pair(int grid, const Inst* inst, Tiles tl, bool wide, FieldsT<float>
 int reinit_pair_blocks_per_sm();
 // water volume of every instance: the cells' 64-bit fixed-point sums (K, S,
 // bulk and, with `slope`, dK/dC) are added to acc[4 * inst + c] (zero on
-// entry) by a streaming pass over the tiles of map 2 (grid2 CTAs) that also
+// entry) by a streaming pass over the tiles of map 1 (grid2 CTAs) that also
 // lists the interface cells (list: at least one entry per cell of the batch;
 // count: one word, reset here) and a pass over that list; volume_final writes vols[4 * inst + 0..3] = (K, S,
 // bulk, total) and clears acc; with `mass` (target volumes `target`, NaN =
@@ -209,22 +210,18 @@ void cell_rel(long long off, int ni, int nj, int nk, const double* x, const doub
 int max_blocks_per_sm(int shape, int kernel);
 
 // ------------------------------------------------------------ adjoint
-// Tile maps besides the forward brick table (output nodes per tile ox x oy
-// x oz, adj_shape): 0 stage adjoint x part (8 whole rows, one warp marching
-// each), 1 stage adjoint y march, 2 the k marches over 32 x 8 columns (RK
-// stage, pseudo-steps, volume scan, reverse pseudo-step from stored
-// coefficients), 3 reverse pseudo-step recomputing its coefficients
-// (overlapped 32 x kReinRY tile marching in k), 4 stage adjoint z march.
-// The face and velocity adjoints walk the packed nodes with one thread per
-// node (instance found by binary search over the node offsets `offs`).
-// The extents along the march (y in map 1, z in maps 2 to 4) are the
-// longest; a batch with few tiles takes shorter ones (Tiles::len).
+// Tile maps besides the forward brick table and the flat tiles (output nodes
+// per tile ox x oy x oz, adj_shape): 0 reverse pseudo-step recomputing its
+// coefficients (overlapped 32 x kReinRY tile marching in k), 1 the k marches
+// over 32 x 8 columns (pseudo-steps, volume scan, TMA stage, reverse
+// pseudo-step from stored coefficients).  The face and velocity adjoints walk
+// the packed nodes with one thread per node (instance found by binary search
+// over the node offsets `offs`).  The extent along the march is the longest;
+// a batch with few tiles takes shorter ones (Tiles::len).
 struct AdjShape { int ox, oy, oz; };
 constexpr int kReinRY = 12;
-// (map 0: ox = 0 means a brick spans whole rows)
 __host__ __device__ constexpr AdjShape adj_shape(int map) {
-    return map == 0 ? AdjShape{0, 8, 1}
-                    : map == 1 ? AdjShape{32, 32, 8} : map == 3 ? AdjShape{30, kReinRY - 2, 32} : AdjShape{32, 8, 32};
+    return map == 0 ? AdjShape{30, kReinRY - 2, 32} : AdjShape{32, 8, 32};
 }
 // Reverse of one bcond_lsm face (face = 0..5: i1, im, j1, jm, k1, km) on the
 // adjoint field lam, in place.  The forward values that decide the BigPhi
@@ -237,38 +234,41 @@ __host__ __device__ constexpr AdjShape adj_shape(int map) {
 template <typename T>
 void adj_face(const Flat& fl, int face, long long nface_nodes, int nface, BC bc, int kind, const T* phin,
               const T* in, const T* out, double c1, double c2, T* lam, cudaStream_t s);
-// Reverse of one RK stage in three passes (x on adjoint map 0 by warp
-// shuffles, y and z marches on maps 1 and 2).  lamP0: adjoint of the
-// stage's pre-BC field; writes lam_in = c2 lamP0 - c3 (dR/din)^T lamP0
-// (+ lamPhin + c1 lamP0 when last, which also clears lamPhin), otherwise
-// accumulates lamPhin += c1 lamP0; and lamW_m -= c3 lamP0 D_m.
+// Reverse of one RK stage in two passes on flat tiles: x and z parts (Inst's
+// xw x xh columns and a rim, k march: tl[0]), y part (yw x yh columns in (i,
+// k), j march: tl[1]); wide as for stage.  lamP0: adjoint of the stage's
+// pre-BC field; writes lam_in = c2 lamP0 - c3 (dR/din)^T lamP0 (+ lamPhin + c1
+// lamP0 when last, which also clears lamPhin), otherwise accumulates lamPhin
+// += c1 lamP0; and lamW_m -= c3 lamP0 D_m.
+constexpr int kAdjThreads = 128;
 template <typename T>
-void adj_stage(const int* grid, const Inst* inst, const Tiles* tl, FieldsT<T> f, const T* in,
+void adj_stage(const int (&grid)[2], const Inst* inst, const Tiles (&tl)[2], bool wide, FieldsT<T> f, const T* in,
                const T* lamP0, T* lam_in, T* lamPhin, T* lamW0, T* lamW1, T* lamW2, double c1, double c2, double c3,
                bool last, cudaStream_t s);
+template <typename T>
+int adj_stage_blocks_per_sm(int part);
 // Reverse of one reinitialisation pseudo-step d' = d - dtau s (G(d) - 1)
-// from its input d: lam_out = (dd'/dd)^T lam (adjoint map 3).
+// from its input d: lam_out = (dd'/dd)^T lam (adjoint map 0).
 template <typename T>
 void adj_reinit(int grid, const Inst* inst, Tiles tl, FieldsT<T> f, const T* d, const T* lam,
                 T* lam_out, cudaStream_t s);
-// Reverse of one recorded pseudo-step from the coefficients reinit_rec
-// stored: a 7-point stencil on lam, on the tiles of adjoint map 2 (grid
-// from adj_reinit_c_blocks_per_sm)
+// Reverse of one recorded pseudo-step from the coefficients that it stored: a
+// 7-point stencil on lam, on flat tiles of Inst's sw x sh columns; wide as for
+// stage
 template <typename T>
-void adj_reinit_c(int grid, const Inst* inst, Tiles tl, const T* cf, long long ld, const T* lam,
-                  T* lam_out, cudaStream_t s);
+void adj_reinit_c(int grid, const Inst* inst, Tiles tl, bool wide, const T* cf, long long ld, const T* lam, T* lam_out,
+                  cudaStream_t s);
 template <typename T>
 int adj_reinit_c_blocks_per_sm();
-// resident blocks per SM of the kernel of adjoint map `map`
 template <typename T>
-int adj_blocks_per_sm(int map);
+int adj_reinit_blocks_per_sm();
 // Mass correction: dst = src + mass[inst].C on every node (dst may alias src)
 template <typename T>
 void mass_shift(const Flat& fl, const Mass* mass, const T* src, T* dst, cudaStream_t s);
 // Reverse of the shift phi' = phi + C(phi) in place on lam (the adjoint of
 // phi'): lam -= (sum(lam) / A) (dK/dphi + C d(dK/dC)/dphi), evaluated on
 // the step's pre-correction field phi_pre; wfix (N 64-bit words, zero on
-// entry and on exit), part (one double per tile of adjoint map 2) and ssum
+// entry and on exit), part (one double per tile of adjoint map 1) and ssum
 // (one per instance) are scratch; (list, count) are the interface cells of
 // phi_pre as the forward step's volume pass listed them
 template <typename T>

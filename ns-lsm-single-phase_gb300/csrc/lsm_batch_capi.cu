@@ -68,16 +68,16 @@ struct lsm_batch {
     lsm::batch::Brick* d_brick = nullptr;
     int nbricks = 0;
     lsm::batch::Brick* d_amap[lsm::batch::kMaps] = {};  // brick tables of the adjoint stencil kernels (lsm::batch::adj_shape)
-    int namap[lsm::batch::kMaps] = {}, agrid[lsm::batch::kMaps] = {};
+    int namap[lsm::batch::kMaps] = {}, argrid = 1;   // argrid: CTAs of k_adj_reinit
     int len[lsm::batch::kMaps] = {};         // march lengths of the maps' tiles
-    int acgrid = 1, rzgrid = 1;   // CTAs of the map-2 kernels k_adj_reinit_c and reinit_z
-    int vgrid = 1;                           // CTAs of the map-2 volume scan
-    // flat tiles of reinit_pair and of stage: their table, number, planes of one, CTAs
+    int rzgrid = 1;   // CTAs of reinit_z
+    int vgrid = 1;                           // CTAs of the map-1 volume scan
+    // flat tiles of reinit_pair, stage, adj_reinit_c and adj_stage: their table, number, planes of one, CTAs
     struct FlatMap {
         lsm::batch::Brick* d = nullptr;
         int n = 0, len = 0, grid = 1;
         lsm::batch::Tiles tiles() const { return {d, n, len}; }
-    } pmap, smap;
+    } pmap, smap, cmap, jmap[2];
     bool reinit_pair = true;    // FP32 pseudo-steps two at a time (reinit_pair) where two are left
     bool reinit_march = true;   // plain pseudo-steps march in k (reinit_z) rather than walk the brick table
     unsigned long long* d_vacc = nullptr;   // volume accumulators, 4 per instance
@@ -295,26 +295,21 @@ int store_out(lsm_batch* b, double* dst, long long n, int stride, int c0, int nc
 lsm::batch::Tiles tiles(const lsm_batch* b, int m) { return {b->d_amap[m], b->namap[m], b->len[m]}; }
 
 // March lengths of the adjoint maps: the longest of 32, 16, 8, 4 that gives
-// the GPU enough tiles (six per SM, three for the stage adjoint and the
-// recomputing reverse pseudo-step), since a march reuses what it has loaded
-// and evaluated; the stage adjoint evaluates four planes more than it
-// writes, so its marches keep to 8 and more.  Measured, against 32 always:
-// 128^3 (256 tiles of 32) k_reinit_rec_z 41 -> 35 us; two FP64 grids of about
-// 40^3 k_adj_reinit 375 -> 70 us, k_adj_stage_y 234 -> 88 us (106 us at 4); 512 x 256 x 256 (4096
-// tiles of 32) loses 6 % at 8.
+// the GPU enough tiles (six per SM, three for the recomputing reverse
+// pseudo-step), since a march reuses what it has loaded and evaluated.
+// Measured, against 32 always: 128^3 (256 tiles of 32) k_reinit_rec_z 41 -> 35
+// us; two FP64 grids of about 40^3 k_adj_reinit 375 -> 70 us; 512 x 256 x 256
+// (4096 tiles of 32) loses 6 % at 8.
 void march_lengths(const lsm_batch* b, int (&len)[lsm::batch::kMaps]) {
     const int sms = 152;
     for (int m = 0; m < lsm::batch::kMaps; ++m) {
         const auto a = lsm::batch::adj_shape(m);
-        len[m] = m == 1 ? a.oy : a.oz;
-        if (m == 0) continue;
-        const int least = m == 1 || m == 4 ? 8 : 4;
-        const long long want = (m == 2 ? 6 : 3) * sms;
-        for (; len[m] > least; len[m] /= 2) {
-            const int oy = m == 1 ? len[m] : a.oy, oz = m == 1 ? a.oz : len[m];
+        const long long want = (m == 1 ? 6 : 3) * sms;
+        for (len[m] = a.oz; len[m] > 4; len[m] /= 2) {
             long long tiles = 0;
             for (const auto& I : b->inst)
-                tiles += (long long)((I.ni + a.ox - 1) / a.ox) * ((I.nj + oy - 1) / oy) * ((I.nk + oz - 1) / oz);
+                tiles += (long long)((I.ni + a.ox - 1) / a.ox) * ((I.nj + a.oy - 1) / a.oy) *
+                         ((I.nk + len[m] - 1) / len[m]);
             if (tiles >= want) break;
         }
     }
@@ -334,14 +329,14 @@ bool pairs_on(const lsm_batch* b) { return b->reinit_pair && !b->prec; }
 // instance); the shape with the fewest tiles, the widest of those (squarer
 // ones with less read around them: 152 against 145 us for the RK stage of 64
 // grids of 32..96, 246 against 238 us on 512 x 256 x 256).
-void flat_tile(int ni, int nj, int threads, int rim, int* rw, int* rh) {
+void flat_tile(int ni, int nj, int threads, int rimx, int rimy, int* rw, int* rh) {
     long long best = -1;
     for (int p = 1; p <= std::max(1, (ni + 7) / 8); ++p) {
         const int w = p == 1 ? ni : ((ni + p - 1) / p + 7) / 8 * 8;
         if (p > 1 && w >= ni) continue;
-        const int rows = threads / (w < ni ? w + 2 * rim : w);
-        if (rows < 1 || (rows <= 2 * rim && rows < nj)) continue;
-        const int py = rows >= nj ? 1 : (nj + rows - 2 * rim - 1) / (rows - 2 * rim);
+        const int rows = threads / (w < ni ? w + 2 * rimx : w);
+        if (rows < 1 || (rows <= 2 * rimy && rows < nj)) continue;
+        const int py = rows >= nj ? 1 : (nj + rows - 2 * rimy - 1) / (rows - 2 * rimy);
         const long long n = (long long)((ni + w - 1) / w) * py;
         if (best >= 0 && n >= best) continue;
         best = n;
@@ -350,21 +345,24 @@ void flat_tile(int ni, int nj, int threads, int rim, int* rw, int* rh) {
     }
 }
 
-// Table of the flat tiles (columns from `tile`) on at most `slots` CTAs at a
-// time.  A march of n planes costs about three more (its first loads, the
+// Table of the flat tiles (columns from `tile`: w x h of an instance's (i, j),
+// or of its (i, k) for a march in j) on at most `slots` CTAs at a time.  A
+// march of n planes costs about `more` of them besides (its first loads, the
 // planes that it reads or evaluates beyond its own), so n is the length with
-// the fewest rounds of the CTAs times n + 3.
+// the fewest rounds of the CTAs times n + more.
 template <class Tile>
-int flat_map(lsm_batch* b, const std::vector<Inst>& inst, int slots, lsm_batch::FlatMap& m, Tile tile) {
+int flat_map(lsm_batch* b, const std::vector<Inst>& inst, int slots, int more, bool in_j, lsm_batch::FlatMap& m,
+             Tile tile) {
     using lsm::batch::Brick;
     double cost = 0.0;
     for (int n = 4; n <= 64; ++n) {
         long long tiles = 0;
         for (const Inst& I : inst) {
             const auto [w, h] = tile(I);
-            tiles += (long long)((I.ni + w - 1) / w) * ((I.nj + h - 1) / h) * ((I.nk + n - 1) / n);
+            const int hn = in_j ? I.nk : I.nj, mn = in_j ? I.nj : I.nk;
+            tiles += (long long)((I.ni + w - 1) / w) * ((hn + h - 1) / h) * ((mn + n - 1) / n);
         }
-        const double c = (double)((tiles + slots - 1) / slots) * (n + 3);
+        const double c = (double)((tiles + slots - 1) / slots) * (n + more);
         if (n == 4 || c < cost) {
             cost = c;
             m.len = n;
@@ -374,8 +372,9 @@ int flat_map(lsm_batch* b, const std::vector<Inst>& inst, int slots, lsm_batch::
     for (int q = 0; q < (int)inst.size(); ++q) {
         const Inst& I = inst[q];
         const auto [w, h] = tile(I);
-        for (int z = 0; z < I.nk; z += m.len)
-            for (int y = 0; y < I.nj; y += h)
+        const int sy = in_j ? m.len : h, sz = in_j ? h : m.len;
+        for (int z = 0; z < I.nk; z += sz)
+            for (int y = 0; y < I.nj; y += sy)
                 for (int x = 0; x < I.ni; x += w) v.push_back(Brick{q, x, y, z});
     }
     m.n = (int)v.size();
@@ -418,8 +417,10 @@ int build_bricks(lsm_batch* b, int shape) {
         d.dtau = (float)I.dtau;
         d.eps = (float)I.eps;
         d.pad = 0;
-        flat_tile(I.ni, I.nj, lsm::batch::kPairThreads, 1, &d.rw, &d.rh);
-        flat_tile(I.ni, I.nj, lsm::batch::kStageThreads, 0, &d.sw, &d.sh);
+        flat_tile(I.ni, I.nj, lsm::batch::kPairThreads, 1, 1, &d.rw, &d.rh);
+        flat_tile(I.ni, I.nj, lsm::batch::kStageThreads, 0, 0, &d.sw, &d.sh);
+        flat_tile(I.ni, I.nj, lsm::batch::kAdjThreads, 2, 0, &d.xw, &d.xh);
+        flat_tile(I.ni, I.nk, lsm::batch::kAdjThreads, 0, 0, &d.yw, &d.yh);
         d.dt64 = I.dt;
         d.dtau64 = I.dtau;
         d.eps64 = I.eps;
@@ -428,8 +429,8 @@ int build_bricks(lsm_batch* b, int shape) {
         for (int a = 0; a < 3; ++a) d.fpre[a] = pre[a];
         for (int m = 0; m < lsm::batch::kMaps; ++m) {
             auto a = lsm::batch::adj_shape(m);
-            (m == 1 ? a.oy : a.oz) = len[m];
-            const int bx = a.ox > 0 ? (I.ni + a.ox - 1) / a.ox : 1;
+            a.oz = len[m];
+            const int bx = (I.ni + a.ox - 1) / a.ox;
             const int by = (I.nj + a.oy - 1) / a.oy, bz = (I.nk + a.oz - 1) / a.oz;
             d.am[m][0] = (int)amap[m].size();
             d.am[m][1] = bx;
@@ -461,12 +462,20 @@ int build_bricks(lsm_batch* b, int shape) {
         BCU(b, cudaMemcpyAsync(b->d_amap[m], amap[m].data(), sizeof(Brick) * amap[m].size(), cudaMemcpyHostToDevice,
                                b->stream));
     }
-    BTRY(flat_map(b, hi, sms * std::max(1, lsm::batch::reinit_pair_blocks_per_sm()), b->pmap,
-                  [](const Inst& I) { return std::pair<int, int>(I.rw, I.rh); }));
-    BTRY(flat_map(b, hi,
-                  sms * std::max(1, b->prec ? lsm::batch::stage_blocks_per_sm<double>()
-                                            : lsm::batch::stage_blocks_per_sm<float>()),
-                  b->smap, [](const Inst& I) { return std::pair<int, int>(I.sw, I.sh); }));
+    namespace B = lsm::batch;
+    auto slots = [&](int per) { return sms * std::max(1, per); };
+    using WH = std::pair<int, int>;
+    BTRY(flat_map(b, hi, slots(B::reinit_pair_blocks_per_sm()), 3, false, b->pmap,
+                  [](const Inst& I) { return WH(I.rw, I.rh); }));
+    BTRY(flat_map(b, hi, slots(b->prec ? B::stage_blocks_per_sm<double>() : B::stage_blocks_per_sm<float>()), 3, false,
+                  b->smap, [](const Inst& I) { return WH(I.sw, I.sh); }));
+    BTRY(flat_map(b, hi, slots(b->prec ? B::adj_reinit_c_blocks_per_sm<double>() : B::adj_reinit_c_blocks_per_sm<float>()),
+                  3, false, b->cmap, [](const Inst& I) { return WH(I.sw, I.sh); }));
+    for (int part = 0; part < 2; ++part) {
+        const int per = b->prec ? B::adj_stage_blocks_per_sm<double>(part) : B::adj_stage_blocks_per_sm<float>(part);
+        BTRY(flat_map(b, hi, slots(per), 5, part == 1, b->jmap[part],
+                      [part](const Inst& I) { return part == 0 ? WH(I.xw, I.xh) : WH(I.yw, I.yh); }));
+    }
     BCU(b, cudaMalloc(&b->d_brick, sizeof(Brick) * brick.size()));
     BCU(b, cudaMemcpyAsync(b->d_brick, brick.data(), sizeof(Brick) * brick.size(), cudaMemcpyHostToDevice, b->stream));
     BCU(b, cudaMemcpyAsync(b->d_inst, hi.data(), sizeof(Inst) * hi.size(), cudaMemcpyHostToDevice, b->stream));
@@ -476,22 +485,17 @@ int build_bricks(lsm_batch* b, int shape) {
     }
     const int per = std::max(1, lsm::batch::max_blocks_per_sm(shape, 0));
     b->grid = std::max(1, std::min(b->nbricks, sms * per));
-    for (int m = 0; m < lsm::batch::kMaps; ++m) {
-        const int pa = std::max(1, b->prec ? lsm::batch::adj_blocks_per_sm<double>(m)
-                                           : lsm::batch::adj_blocks_per_sm<float>(m));
-        b->agrid[m] = std::max(1, std::min(b->namap[m], sms * pa));
-    }
-    const int pac = std::max(1, b->prec ? lsm::batch::adj_reinit_c_blocks_per_sm<double>()
-                                        : lsm::batch::adj_reinit_c_blocks_per_sm<float>());
-    b->acgrid = std::max(1, std::min(b->namap[2], sms * pac));
+    const int par = std::max(1, b->prec ? lsm::batch::adj_reinit_blocks_per_sm<double>()
+                                        : lsm::batch::adj_reinit_blocks_per_sm<float>());
+    b->argrid = std::max(1, std::min(b->namap[0], sms * par));
     const int prz = std::max(1, b->prec ? lsm::batch::reinit_z_blocks_per_sm<double>()
                                         : lsm::batch::reinit_z_blocks_per_sm<float>());
-    b->rzgrid = std::max(1, std::min(b->namap[2], sms * prz));
+    b->rzgrid = std::max(1, std::min(b->namap[1], sms * prz));
     const int pv = std::max(1, b->prec ? lsm::batch::vol_scan_blocks_per_sm<double>()
                                        : lsm::batch::vol_scan_blocks_per_sm<float>());
-    b->vgrid = std::max(1, std::min(b->namap[2], sms * pv));
+    b->vgrid = std::max(1, std::min(b->namap[1], sms * pv));
     if (b->tma_eligible)
-        b->tgrid = std::max(1, std::min(b->namap[2], sms * std::max(1, lsm::batch::stage_tma_blocks_per_sm())));
+        b->tgrid = std::max(1, std::min(b->namap[1], sms * std::max(1, lsm::batch::stage_tma_blocks_per_sm())));
     b->shape = shape;
     BCU(b, cudaStreamSynchronize(b->stream));
     return LSM_OK;
@@ -563,7 +567,7 @@ void enqueue_stage(lsm_batch* b, FieldsT<T> f, const T* phin, const T* in, T* ou
                 }
             }
             if (map && a < (1LL << 31)) {
-                B::stage_tma(b->tgrid, map, (int)a, b->d_inst, tiles(b, 2), f, phin, in, out, kC[s][0],
+                B::stage_tma(b->tgrid, map, (int)a, b->d_inst, tiles(b, 1), f, phin, in, out, kC[s][0],
                              kC[s][1], kC[s][2], b->d_err, b->stream);
                 return;
             }
@@ -594,7 +598,7 @@ void enqueue_step_io(lsm_batch* b, const T* phin, T* phi_out, const Rec<T>* rec,
     if (rec && !coef) f.sgn = rec->sgn;
     const Flat fl{b->d_inst, b->d_offs, b->ninst, b->N};
     if (vol && !mc) {
-        B::volume<T>(b->vgrid, b->d_inst, tiles(b, 2), fl, f, phin, b->d_vacc, false, b->d_ilist,
+        B::volume<T>(b->vgrid, b->d_inst, tiles(b, 1), fl, f, phin, b->d_vacc, false, b->d_ilist,
                      b->d_icount, b->stream);
         B::volume_final(b->ninst, b->d_vacc, b->d_vols, nullptr, nullptr, nullptr, b->stream);
     }
@@ -632,7 +636,7 @@ void enqueue_step_io(lsm_batch* b, const T* phin, T* phi_out, const Rec<T>* rec,
                 if constexpr (sizeof(T) == 4)
                     B::reinit_pair(b->pmap.grid, b->d_inst, b->pmap.tiles(), wide(b), f, cur, o, o2, err, b->stream);
             } else if (march)
-                B::reinit_z<T>((it == 0 ? 2 : 0) + (coef ? 1 : 0), b->rzgrid, b->d_inst, tiles(b, 2), f,
+                B::reinit_z<T>((it == 0 ? 2 : 0) + (coef ? 1 : 0), b->rzgrid, b->d_inst, tiles(b, 1), f,
                                cur, o, o2, cf, (long long)b->ld, err, b->stream);
             else if (it == 0)
                 B::sign_reinit<T>(sh, gr, b->d_inst, b->d_brick, nb, f, cur, o, err, b->stream);
@@ -656,7 +660,7 @@ void enqueue_step_io(lsm_batch* b, const T* phin, T* phi_out, const Rec<T>* rec,
         // and phi_out = result + C
         // a recorded step keeps the interface cells of its result for the
         // reverse of the correction
-        B::volume<T>(b->vgrid, b->d_inst, tiles(b, 2), fl, f, res, b->d_vacc, true,
+        B::volume<T>(b->vgrid, b->d_inst, tiles(b, 1), fl, f, res, b->d_vacc, true,
                      rec ? rec->list : b->d_ilist, rec ? rec->count : b->d_icount, b->stream);
         B::volume_final(b->ninst, b->d_vacc, b->d_vols, b->d_target, b->d_mass, mrec, b->stream);
         if (phi_out) B::mass_shift<T>(fl, b->d_mass, res, phi_out, b->stream);
@@ -730,9 +734,9 @@ int autotune(lsm_batch* b) {
                            b->stream);
         },
         [&]() {
-            B::reinit_z<float>(2, b->rzgrid, b->d_inst, tiles(b, 2), f, f.phi, f.d[0], nullptr, nullptr, 0, nullptr,
+            B::reinit_z<float>(2, b->rzgrid, b->d_inst, tiles(b, 1), f, f.phi, f.d[0], nullptr, nullptr, 0, nullptr,
                                b->stream);
-            B::reinit_z<float>(0, b->rzgrid, b->d_inst, tiles(b, 2), f, f.d[0], f.d[1], nullptr, nullptr, 0, nullptr,
+            B::reinit_z<float>(0, b->rzgrid, b->d_inst, tiles(b, 1), f, f.d[0], f.d[1], nullptr, nullptr, 0, nullptr,
                                b->stream);
         });
     if (st != LSM_OK) return done(st);
@@ -756,7 +760,7 @@ int autotune(lsm_batch* b) {
                                 0.0, 1.0, b->stream);
             },
             [&]() {
-                B::stage_tma(b->tgrid, &b->tm_field, 0, b->d_inst, tiles(b, 2), f, f.phi, f.phi,
+                B::stage_tma(b->tgrid, &b->tm_field, 0, b->d_inst, tiles(b, 1), f, f.phi, f.phi,
                              f.stage[0], 1.0, 0.0, 1.0, b->d_err, b->stream);
             });
         if (st2 != LSM_OK) return done(st2);
@@ -924,7 +928,7 @@ int forward_record_t(lsm_batch* b, int nsteps, int ck) {
         // and every reverse step leaves them at zero)
         BCU(b, cudaMalloc(&b->wfix, sizeof(unsigned long long) * (size_t)b->N));
         BCU(b, cudaMemsetAsync(b->wfix, 0, sizeof(unsigned long long) * (size_t)b->N, b->stream));
-        BCU(b, cudaMalloc(&b->d_tpart, sizeof(double) * (size_t)std::max(1, b->namap[2])));
+        BCU(b, cudaMalloc(&b->d_tpart, sizeof(double) * (size_t)std::max(1, b->namap[1])));
         BCU(b, cudaMalloc(&b->d_ssum, sizeof(double) * (size_t)b->ninst));
     }
     b->rec_steps = nsteps;
@@ -978,7 +982,7 @@ void adj_step(lsm_batch* b, AdjView<T>& v, const Rec<T>& r, const T* phin, const
     const int R = b->cfg.RNitermax;
     // reverse of the mass correction phi^{n+1} = P + C(P), in place on lam
     if (b->cfg.mass_correction)
-        B::mass_adjoint<T>(b->d_inst, tiles(b, 2), fl, f, r.P, m, v.lam, b->wfix, b->d_tpart,
+        B::mass_adjoint<T>(b->d_inst, tiles(b, 1), fl, f, r.P, m, v.lam, b->wfix, b->d_tpart,
                            b->d_ssum, r.list, r.count, b->stream);
     auto faces = [&](int kind, const T* pn, const T* in, const T* out, double c1, double c2) {
         for (int ax = 2; ax >= 0; --ax) {
@@ -994,25 +998,25 @@ void adj_step(lsm_batch* b, AdjView<T>& v, const Rec<T>& r, const T* phin, const
         faces(1, nullptr, nullptr, rec_d(b, r, R - 1), 0.0, 0.0);
         for (int k = R - 1; k >= 0; --k) {
             if (r.C) {
-                B::adj_reinit_c<T>(b->acgrid, b->d_inst, tiles(b, 2), r.C + 6LL * k * (long long)b->ld,
+                B::adj_reinit_c<T>(b->cmap.grid, b->d_inst, b->cmap.tiles(), wide(b), r.C + 6LL * k * (long long)b->ld,
                                    (long long)b->ld, v.lam, v.lam2, b->stream);
             } else {
                 const T* dk = k == 0 ? r.A[2] : rec_d(b, r, k - 1);
-                B::adj_reinit<T>(b->agrid[3], b->d_inst, tiles(b, 3), f, dk, v.lam, v.lam2, b->stream);
+                B::adj_reinit<T>(b->argrid, b->d_inst, tiles(b, 0), f, dk, v.lam, v.lam2, b->stream);
             }
             std::swap(v.lam, v.lam2);
         }
     } else {
         faces(1, nullptr, nullptr, r.A[2], 0.0, 0.0);
     }
-    B::Tiles all[B::kMaps];
-    for (int m = 0; m < B::kMaps; ++m) all[m] = tiles(b, m);
+    const B::Tiles tl[2] = {b->jmap[0].tiles(), b->jmap[1].tiles()};
+    const int grid[2] = {b->jmap[0].grid, b->jmap[1].grid};
     // stages 3, 2, 1: inputs A2, A1, phi^n; outputs A3, A2, A1
     const T* ins[3] = {phin, r.A[0], r.A[1]};
     for (int s = 2; s >= 0; --s) {
         faces(0, phin, ins[s], r.A[s], kC[s][0], kC[s][1]);
-        B::adj_stage<T>(b->agrid, b->d_inst, all, f, ins[s], v.lam, v.lam2, v.lamPhin, v.lamW[0],
-                        v.lamW[1], v.lamW[2], kC[s][0], kC[s][1], kC[s][2], s == 0, b->stream);
+        B::adj_stage<T>(grid, b->d_inst, tl, wide(b), f, ins[s], v.lam, v.lam2, v.lamPhin, v.lamW[0], v.lamW[1],
+                        v.lamW[2], kC[s][0], kC[s][1], kC[s][2], s == 0, b->stream);
         std::swap(v.lam, v.lam2);
     }
 }
@@ -1214,8 +1218,8 @@ int lsm_batch_destroy(lsm_batch_handle b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->exec) cudaGraphExecDestroy(b->exec);
     for (void* p : {b->field_arena, (void*)b->xyz, (void*)b->staging, (void*)b->d_inst, (void*)b->d_offs,
-                    (void*)b->d_brick, (void*)b->pmap.d, (void*)b->smap.d, (void*)b->d_amap[0], (void*)b->d_amap[1], (void*)b->d_amap[2],
-                    (void*)b->d_amap[3], (void*)b->d_amap[4], (void*)b->d_vacc, (void*)b->d_vols, (void*)b->d_err, b->adj,
+                    (void*)b->d_brick, (void*)b->pmap.d, (void*)b->smap.d, (void*)b->cmap.d, (void*)b->jmap[0].d,
+                    (void*)b->jmap[1].d, (void*)b->d_amap[0], (void*)b->d_amap[1], (void*)b->d_vacc, (void*)b->d_vols, (void*)b->d_err, b->adj,
                     (void*)b->d_target, (void*)b->d_mass, (void*)b->wfix, (void*)b->d_tpart, (void*)b->d_ssum,
                     (void*)b->d_ilist, (void*)b->d_icount, (void*)b->f64x, (void*)b->d_p64, (void*)b->cellrel})
         if (p) cudaFree(p);
@@ -1422,10 +1426,10 @@ int lsm_batch_water_volume(lsm_batch_handle b, double* volumes) {
     namespace B = lsm::batch;
     const Flat fl{b->d_inst, b->d_offs, b->ninst, b->N};
     if (b->prec)
-        B::volume<double>(b->vgrid, b->d_inst, tiles(b, 2), fl, b->f64, b->f64.phi, b->d_vacc, false,
+        B::volume<double>(b->vgrid, b->d_inst, tiles(b, 1), fl, b->f64, b->f64.phi, b->d_vacc, false,
                           b->d_ilist, b->d_icount, b->stream);
     else
-        B::volume<float>(b->vgrid, b->d_inst, tiles(b, 2), fl, b->f32, b->f32.phi, b->d_vacc, false,
+        B::volume<float>(b->vgrid, b->d_inst, tiles(b, 1), fl, b->f32, b->f32.phi, b->d_vacc, false,
                          b->d_ilist, b->d_icount, b->stream);
     B::volume_final(b->ninst, b->d_vacc, b->d_vols, nullptr, nullptr, nullptr, b->stream);
     BCU(b, cudaGetLastError());
