@@ -1653,8 +1653,10 @@ __device__ __forceinline__ int node_instance(const Flat& fl, long long t) {
 }
 
 // K and S volumes (and with SLOPE dK/dC) of the listed interface cells into
-// acc[4 inst + 0, 1, 3]: lanes of a warp that all hold one instance add a
-// warp sum, otherwise each lane adds its own
+// acc[4 inst + 0, 1, 3].  The list holds short runs of an instance's cells, so
+// a warp sums per instance: an atomic per lane on a few addresses clogged the
+// memory pipe (64 grids of 32..96, 570 000 cells: 157 -> 46 us, with enough
+// blocks to even out the warps: 61 us with eight per SM).
 template <typename T, bool SLOPE>
 __global__ void __launch_bounds__(128) k_vol_iface(Flat fl, FieldsT<T> f, const T* __restrict__ phi,
                                                    const unsigned* __restrict__ list, const unsigned* __restrict__ count,
@@ -1680,18 +1682,17 @@ __global__ void __launch_bounds__(128) k_vol_iface(Flat fl, FieldsT<T> f, const 
             Sq = __double2ll_rn(S * kVolScale);
             if (SLOPE) Aq = __double2ll_rn(A * kVolScale);
         }
-        const int q0 = __shfl_sync(FM, q, 0);
-        if (__all_sync(FM, q == q0)) {
-            const long long v[3] = {warp_sum_nn(Kq), warp_sum_nn(Sq), SLOPE ? warp_sum_nn(Aq) : 0};
-            if (lane == 0 && q0 >= 0) {
-                if (v[0]) atomicAdd(acc + 4 * (long long)q0, (unsigned long long)v[0]);
-                if (v[1]) atomicAdd(acc + 4 * (long long)q0 + 1, (unsigned long long)v[1]);
-                if (v[2]) atomicAdd(acc + 4 * (long long)q0 + 3, (unsigned long long)v[2]);
+        // one sum and one atomic per instance that the warp holds
+        for (unsigned left = __ballot_sync(FM, valid); left;) {
+            const int ql = __shfl_sync(FM, q, __ffs(left) - 1);
+            const bool in = q == ql;
+            left &= ~__ballot_sync(FM, in);
+            const long long v[3] = {warp_sum_nn(in ? Kq : 0), warp_sum_nn(in ? Sq : 0), SLOPE ? warp_sum_nn(in ? Aq : 0) : 0};
+            if (lane == 0) {
+                if (v[0]) atomicAdd(acc + 4 * (long long)ql, (unsigned long long)v[0]);
+                if (v[1]) atomicAdd(acc + 4 * (long long)ql + 1, (unsigned long long)v[1]);
+                if (v[2]) atomicAdd(acc + 4 * (long long)ql + 3, (unsigned long long)v[2]);
             }
-        } else if (valid) {
-            if (Kq) atomicAdd(acc + 4 * (long long)q, (unsigned long long)Kq);
-            if (Sq) atomicAdd(acc + 4 * (long long)q + 1, (unsigned long long)Sq);
-            if (SLOPE && Aq) atomicAdd(acc + 4 * (long long)q + 3, (unsigned long long)Aq);
         }
     }
 }
@@ -2575,7 +2576,7 @@ void bc_reinit(const Inst* inst, int ninst, long long nface, FieldsT<T> f, BC bc
     ProfScope ps_("k_bc_reinit", s);
     k_bc_reinit<T><<<flat_blocks(nface), 256, 0, s>>>(inst, ninst, nface, bc, f, din, dout);
 }
-inline unsigned list_blocks() { return 152 * 8; }
+inline unsigned list_blocks() { return 152 * 32; }
 template <typename T>
 void volume(int grid2, const Inst* inst, Tiles tl, const Flat& fl, FieldsT<T> f, const T* phi,
             unsigned long long* acc, bool slope, unsigned* list, unsigned* count, cudaStream_t s) {
