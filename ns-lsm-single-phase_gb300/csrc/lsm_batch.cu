@@ -6,16 +6,18 @@
 // (grid = SMs x resident CTAs) walking a table of tiles, each tile inside
 // one instance:
 //  - brick tables (TX x TY x TZ nodes, one thread per node; the autotuned
-//    forward shape): contra, volume, boundary passes, and the brick
-//    variants of the pseudo-step;
-//  - adjoint-map tiles (adj_shape): the stencil passes that march in k
-//    over 32 x 8 columns (RK stage, pseudo-steps, the reverse pseudo-step
-//    from stored coefficients), march rows / lines (stage adjoint) or an
-//    overlapped 32 x kReinRY tile (reverse pseudo-step recomputing its
-//    coefficients).
+//    forward shape): contra, boundary passes, and the brick variants of the
+//    pseudo-step;
+//  - flat tiles (columns of an instance in row-major order over the threads,
+//    marching in k or j): RK stage, pseudo-steps in pairs, stage adjoint, the
+//    reverse pseudo-step from stored coefficients;
+//  - adjoint-map tiles (adj_shape): k marches over 32 x 8 columns (single
+//    pseudo-steps, volume scan, TMA stage) or an overlapped 32 x kReinRY tile
+//    (reverse pseudo-step recomputing its coefficients).
 // Per-node algorithmic traffic (FP32 words): contra 15 (u 3, metrics 9;
 // W 3), RK stage 5/6/6 (phi_prev, phi^n, W 3; phi), pseudo-step 12 (d, s,
-// metrics 9; d) or 18 recorded (+ six adjoint coefficients), volume 3 (phi
+// metrics 9; d; a pair 12 for both) or 18 recorded (+ six adjoint
+// coefficients), volume 3 (phi
 // + 64-bit fixed-point cell volume).
 //
 // Arithmetic: the reference's formulas rearranged for the GPU (one division

@@ -135,15 +135,6 @@ LSM_HD double half_of(double x) {
     if (e - 2u < 0x7FDu) return u2d(d2u(x) - kOne52);
     return 0.5 * x;
 }
-// 0.5 a + 0.5 b with each product and the sum rounded: halving is exact, so
-// the sum is formed first and halved in its exponent
-LSM_HD double half_sum(double a, double b) {
-    const double x = a + b;
-    const u32 e = biased_exp(x);
-    if (e - 128u < 0x7FFu - 128u) return u2d(d2u(x) - kOne52);
-    return 0.5 * a + 0.5 * b;   // tiny (a product may round) or not finite
-}
-
 LSM_HD u64 sig53(u64 u) { return (u & kFrac) | kOne52; }
 
 // Rounds hi 2^64 + lo (51 or 52 fraction bits in hi, the rest in lo) to 53
