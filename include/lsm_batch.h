@@ -165,7 +165,7 @@ int lsm_batch_shape(lsm_batch_handle h, int* index, int* tx, int* ty, int* tz);
 /* RK stage kernel in use after the first step: 1 plane tiles staged by TMA
    copies (FP32 batches of one instance with ni a multiple of 4, when the
    autotuner finds it faster; the environment variable LSM_BATCH_STAGE=tma
-   or =smem forces the choice), 0 staged by the threads, -1 no handle. */
+   or =smem forces the choice), 0 plain loads, -1 no handle. */
 int lsm_batch_stage_kernel(lsm_batch_handle h);
 /* Total nodes of the batch and kernels launched per physical step. */
 long long lsm_batch_nodes(lsm_batch_handle h);
