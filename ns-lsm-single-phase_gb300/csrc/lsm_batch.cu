@@ -66,9 +66,10 @@ template <> __device__ __forceinline__ float wrcp<float>(float b) {
 }
 template <typename T> __device__ __forceinline__ T vfma(T a, T b, T c) { return fma(a, b, c); }
 template <> __device__ __forceinline__ float vfma<float>(float a, float b, float c) { return fmaf(a, b, c); }
-template <typename T> __device__ __forceinline__ T vsqrt(T a) { return sqrt(a); }
+// (FP64 on the integer pipes: the same bits)
+template <typename T> __device__ __forceinline__ T vsqrt(T a) { return ssqrt(a); }
 template <> __device__ __forceinline__ float vsqrt<float>(float a) { return sqrtf(a); }
-template <typename T> __device__ __forceinline__ T vrsqrt(T a) { return T(1) / sqrt(a); }
+template <typename T> __device__ __forceinline__ T vrsqrt(T a) { return sdiv(1.0, ssqrt(a)); }
 template <> __device__ __forceinline__ float vrsqrt<float>(float a) { return rsqrtf(a); }
 template <typename T> __device__ __forceinline__ T vsin(T a) { return sin(a); }
 template <> __device__ __forceinline__ float vsin<float>(float a) { return sinf(a); }
