@@ -707,8 +707,13 @@ __global__ void __launch_bounds__(TX * TY * TZ) k_bc_full(const Inst* __restrict
 }
 
 // ------------------------------------------------------------ Godunov |grad|
-// max(a, b) with a NaN a dropped (b is not one)
-template <typename T> __device__ __forceinline__ T pmax(T a, T b) { return a > b ? a : b; }
+// max(a, b) for b >= 0, a NaN a dropped; FP64 on the bit patterns (ordered as
+// signed integers against a b >= 0: a comparison takes the FP64 pipe as long as
+// an addition)
+template <typename T> __device__ __forceinline__ T pmax(T a, T b) {
+    const i64 u = (i64)d2u(a);
+    return u > (i64)d2u(b) && u <= (i64)0x7FF0000000000000ll ? a : b;
+}
 template <> __device__ __forceinline__ float pmax<float>(float a, float b) { return fmaxf(a, b); }
 
 // acc + v^2, the square rounded by itself in FP32
@@ -2237,25 +2242,16 @@ struct CoefIn {
 template <typename T>
 __device__ __forceinline__ void coef_eval(const CoefIn<T>& c, T dtau, const bool (&lo)[3], const bool (&hi)[3],
                                           T (&A)[3], T (&B)[3]) {
-    const T sg = c.s > T(0) ? T(1) : T(-1);
+    const T sg = c.s > T(0) ? T(1) : T(-1), sc = sg * c.d[0];
     T mas[3], men[3];
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-        const T fwd = c.d[2 + 2 * m] - c.d[0], bwd = c.d[0] - c.d[1 + 2 * m];
-        mas[m] = sg * (hi[m] ? bwd : fwd);
-        men[m] = sg * (lo[m] ? fwd : bwd);
+        const T fwd = vfma(sg, c.d[2 + 2 * m], -sc), bwd = vfma(-sg, c.d[1 + 2 * m], sc);
+        mas[m] = hi[m] ? bwd : fwd;
+        men[m] = lo[m] ? fwd : bwd;
     }
-    T e[3], g[3], acc = T(0);
-#pragma unroll
-    for (int x = 0; x < 3; ++x) {
-        const T bb = c.M[x] * men[0] + c.M[3 + x] * men[1] + c.M[6 + x] * men[2];   // sigma bb
-        const T ff = c.M[x] * mas[0] + c.M[3 + x] * mas[1] + c.M[6 + x] * mas[2];   // sigma ff
-        const T p = vmax(bb, T(0)), q = vmin(ff, T(0));
-        const bool takeP = p * p >= q * q;
-        acc += takeP ? p * p : q * q;
-        e[x] = takeP ? p : T(0);
-        g[x] = takeP ? T(0) : q;
-    }
+    T e[3], g[3];
+    const T acc = godunov_sel_v<true>(mas, men, c.M, e, g);
     const T wgt = (c.s != T(0) && acc > T(0)) ? dtau * fabs(c.s) * c.lam * vrsqrt(acc) : T(0);
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
