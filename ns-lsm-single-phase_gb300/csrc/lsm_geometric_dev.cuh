@@ -750,10 +750,20 @@ struct ChainQueue {
 };
 
 // Encloses the reference's distance of P to a triangle (dist_point_triangle).
-// E covers the FP32 rounding of the coordinates and of the operations, tau
-// that of alpha and beta.  The value is the least of the distances to the
-// edges and, inside the triangle, of the one to the reference's projection;
-// any point it can take lies in the triangle.
+// The value is the least of the distances to the edges and, inside the
+// triangle, of the one to the reference's projection; any point it can take
+// lies in the triangle.  E covers the FP32 roundings of an edge's distance,
+// tau those of alpha and beta.  With u = 2^-24, p = P - A (n1 its sum of
+// magnitudes) and l the longer of AB and AC:
+//   P and A rounded, and their difference: 3.5 u scale + 2 u n1;
+//   the foot on an edge (a dot product, the inverse length) and the vector to
+//   it, for a vector q to the edge's start: 11 u |q|, |q| <= n1 + l;
+//   AB and AC rounded, BC's direction and its inverse length from their
+//   difference: 22 u l;
+//   the square root of the sum of squares: 3 u s
+// -- each below its share of E (2e-6 = 33 u).  n1 and l count where the point
+// is near the origin of the coordinates and near the surface: scale and s are
+// then small beside the triangle.
 __device__ __noinline__ float2 tri_interval(const TriF* __restrict__ trif, const GeoTet* __restrict__ tets, int tri,
                                             float x, float y, float z, float scale) {
     float lo, hi;
@@ -775,17 +785,18 @@ __device__ __noinline__ float2 tri_interval(const TriF* __restrict__ trif, const
     };
     const float s2 = fminf(fminf(seg(px, py, pz, b.x, b.y, b.z, b.w), seg(px, py, pz, c.x, c.y, c.z, c.w)),
                            seg(px - b.x, py - b.y, pz - b.z, c.x - b.x, c.y - b.y, c.z - b.z, u.w));
-    const float s = sqrtf(s2), E = 2.0e-6f * (scale + s) + 1.0e-12f;
+    const float n1 = fabsf(px) + fabsf(py) + fabsf(pz), l = rsqrtf(fminf(b.w, c.w));
+    const float s = sqrtf(s2), E = 2.0e-6f * (scale + n1 + 2.0f * l + s) + 1.0e-12f;
     hi = s + E;
     lo = s - E;
     const float al = px * u.x + py * u.y + pz * u.z, be = px * v.x + py * v.y + pz * v.z, ga = 1.0f - be - al;
-    const float tau = v.w * 1.0e-6f * (scale + fabsf(px) + fabsf(py) + fabsf(pz));
+    const float tau = v.w * 1.0e-6f * (scale + n1);
     if (tau < 0.25f) {
         const float m = fminf(al, fminf(be, ga));
         if (m > -2.0f * tau) {
             const float wx = px - be * b.x - ga * c.x, wy = py - be * b.y - ga * c.y, wz = pz - be * b.z - ga * c.z;
             const float d = sqrtf(wx * wx + wy * wy + wz * wz);
-            const float e = E + 4.0f * tau * rsqrtf(fminf(b.w, c.w));
+            const float e = E + 4.0f * tau * l;
             lo = fminf(lo, d - e);
             if (m > 2.0f * tau) hi = fminf(hi, d + e);
         }

@@ -1,0 +1,97 @@
+"""The distance chains of the geometric reinitialisation on the CPU: the
+kernels' own device code (csrc/lsm_geometric_dev.cuh) on a warp of host fibers
+against the sequential loops, bit for bit, and its FP32 enclosures against the
+FP64 distances that they have to hold.  The surfaces pass close to a node at
+the coordinate origin (corner or middle of the grid), where the point's
+coordinates and its distance are small while the triangles are a cell wide, on
+cells of aspect 1 to 100, smooth and rough."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "ns-lsm-single-phase_gb300", "csrc")
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    gxx = shutil.which("g++")
+    if not gxx:
+        pytest.skip("needs g++")
+    out = str(tmp_path_factory.mktemp("geo") / "libgeo.so")
+    r = subprocess.run([gxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-ffp-contract=off", "-I",
+                        os.path.join(HERE, "simt"), "-I", CSRC, os.path.join(HERE, "geo_chain_harness.cpp"), "-o", out],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    d = C.CDLL(out)
+    d.geo_enclosures.restype = C.c_long
+    return d
+
+
+def ptr(a):
+    return C.c_void_p(a.ctypes.data)
+
+
+def chains(lib, x, y, z, phi, pc, at, reach):
+    """(nodes, signed distances and |v| that differ, largest difference)"""
+    x, y, z, phi, pc = (np.asfortranarray(a, dtype=np.float64) for a in (x, y, z, phi, pc))
+    n = np.zeros(4)
+    lib.geo_chains(*phi.shape, ptr(phi), ptr(x), ptr(y), ptr(z), ptr(pc), *at, reach, ptr(n))
+    return n
+
+
+def grid(n, at, h, shift=(0.0, 0.0, 0.0)):
+    """Coordinates of n^3 nodes, spacing h per axis, (0, 0, 0) + shift at node `at`."""
+    return np.meshgrid(*((np.arange(n) - at) * h[c] + shift[c] for c in range(3)), indexing="ij")
+
+
+def rough(rng, n, at, h, off, amp):
+    """A surface `off` cells from node `at`, noisy by `amp` cells."""
+    X, Y, Z = np.meshgrid(*(np.arange(n) - float(at),) * 3, indexing="ij")
+    s = rng.standard_normal(2) * 0.6
+    f = (Z + s[0] * X + s[1] * Y - off) * min(h)
+    return f + amp * min(h) * rng.standard_normal((n,) * 3) * (np.abs(X) + np.abs(Y) + np.abs(Z) > 0)
+
+
+@pytest.mark.parametrize("place", ["corner", "middle"])
+@pytest.mark.parametrize("aspect", [1, 10, 100])
+def test_surfaces_near_an_origin_node(lib, place, aspect):
+    n, at = (9, 0) if place == "corner" else (11, 5)
+    total = np.zeros(4)
+    for off in (0.3, 0.03, 0.003):
+        for amp in (0.0, 0.3, 2.0):
+            for s in range(4):
+                rng = np.random.default_rng([s, aspect, int(off * 1000), int(amp * 10)])
+                h = np.array([1.0, 1.0, 1.0 / aspect]) * rng.choice([0.02, 1.0])
+                pc = rng.standard_normal((n,) * 3) * rng.choice([20.0, 0.1, 9.9])
+                total += chains(lib, *grid(n, at, h), rough(rng, n, at, h, off, amp), pc, (at,) * 3, 1)
+    assert total[0] > 200
+    assert (total[1:3] == 0).all(), total
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_enclosures_hold_the_distance(lib, seed):
+    """Random triangles of all shapes and points at all distances and offsets
+    from the origin; the point at or near a vertex, an edge, the plane."""
+    rng = np.random.default_rng(seed)
+    n = 400000
+    size = 10.0 ** rng.uniform(-3, 3, (n, 1, 1))
+    T = rng.standard_normal((n, 3, 3)) * size * 10.0 ** rng.uniform(-3, 0, (n, 1, 3))
+    k = rng.integers(0, 4, n)
+    T[k == 1, 2] = T[k == 1, 1] + 1e-3 * (T[k == 1, 2] - T[k == 1, 1])            # short edges
+    T[k == 2, 2] = T[k == 2, 0] + 0.6 * (T[k == 2, 1] - T[k == 2, 0]) + 1e-3 * T[k == 2, 2]   # slivers
+    w = rng.dirichlet((0.5, 0.5, 0.5), n)[:, :, None]
+    d = rng.standard_normal((n, 3)) * size[:, 0] * 10.0 ** rng.uniform(-7, 1, (n, 1))
+    on = np.where(rng.random((n, 1)) < 0.5, (T * w).sum(1), T[np.arange(n), rng.integers(0, 3, n)])
+    P = on + d
+    m = rng.integers(0, 3, n)
+    o = np.where((m == 0)[:, None], P, 0.0)                                       # the point at the origin
+    o = np.where((m == 1)[:, None], P + rng.standard_normal((n, 3)) * size[:, 0] * 10.0 ** rng.uniform(-7, 3, (n, 1)), o)
+    T, P = np.ascontiguousarray(T - o[:, None]), np.ascontiguousarray(P - o)
+    width = np.zeros(1)
+    missed = lib.geo_enclosures(n, ptr(T), ptr(P), ptr(width))
+    assert missed == 0, missed
