@@ -14,6 +14,7 @@ import numpy as np
 import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
+SEEDS = (693240, 218490, 327034, 345658, 4699, 5467, 17083, 125244, 126044, 141148, 253, 701, 1021, 2110, 42718, 52254)
 CSRC = os.path.join(os.path.dirname(HERE), "ns-lsm-single-phase_gb300", "csrc")
 
 
@@ -71,6 +72,23 @@ def test_surfaces_near_an_origin_node(lib, place, aspect):
                 total += chains(lib, *grid(n, at, h), rough(rng, n, at, h, off, amp), pc, (at,) * 3, 1)
     assert total[0] > 200
     assert (total[1:3] == 0).all(), total
+
+
+def deciding(seed):
+    rng = np.random.default_rng([seed, 5])
+    n, at = ((5, 0), (9, 4))[seed & 1]
+    off, amp = (0.03, 0.01, 0.003, 0.001)[(seed >> 1) & 3], (0.01, 0.1, 0.3, 1.0)[(seed >> 3) & 3]
+    h = np.array([1.0, 1.0, 1.0 / (1, 10)[(seed >> 5) & 1]])
+    return n, at, grid(n, at, h), rough(rng, n, at, h, off, amp)
+
+
+@pytest.mark.parametrize("seed", SEEDS)
+def test_surfaces_that_decide_by_an_enclosure(lib, seed):
+    """Rough surfaces within 0.03 cells of a node at the origin: the last bits of
+    its distance depend on triangles that an enclosure without the triangle's size loses."""
+    n, at, xyz, phi = deciding(seed)
+    c = chains(lib, *xyz, phi, np.full((n,) * 3, -9.9), (at,) * 3, 0)
+    assert c[0] == 1 and (c[1:3] == 0).all(), c
 
 
 @pytest.mark.parametrize("seed", range(4))

@@ -9,12 +9,20 @@ import pytest
 
 import cases
 import oracle as O
-from test_geometric_chain_cpu import grid, rough
+from test_geometric_chain_cpu import SEEDS, deciding, grid, rough
 from test_gpu_geometric import seed
 from test_gpu_parity import G, P, dev, host
 
 pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
+
+
+def check(ls, oracle, g, p, phi, x, y, z):
+    pc = seed(phi)
+    ref, rids, _ = oracle.geometric_reinitialisation(g, p, phi, x, y, z, 0.0, pc)
+    out, ids, _ = ls.geometric_reinitialisation(G(g), P(p), *map(dev, (phi, x, y, z)), 0.0, dev(pc))
+    assert np.array_equal(host(ids), rids)
+    assert np.array_equal(host(out), ref)
 
 
 @pytest.mark.parametrize("place", ["corner", "middle"])
@@ -28,8 +36,10 @@ def test_origin_nodes_bit_identical(ls, oracle, place, aspect):
             h = np.array([1.0, 1.0, 1.0 / aspect]) * rng.choice([0.02, 1.0])
             x, y, z = (cases.F(c) for c in grid(n, at, h))
             phi = cases.F(rough(rng, n, at, h, off, amp))
-            pc = seed(phi)
-            ref, rids, _ = oracle.geometric_reinitialisation(g, p, phi, x, y, z, 0.0, pc)
-            out, ids, _ = ls.geometric_reinitialisation(G(g), P(p), *map(dev, (phi, x, y, z)), 0.0, dev(pc))
-            assert np.array_equal(host(ids), rids)
-            assert np.array_equal(host(out), ref)
+            check(ls, oracle, g, p, phi, x, y, z)
+
+
+@pytest.mark.parametrize("case", SEEDS[::3])
+def test_surfaces_that_decide_by_an_enclosure(ls, oracle, case):
+    n, _, xyz, phi = deciding(case)
+    check(ls, oracle, O.make_grid(n, n, n), O.make_params(), cases.F(phi), *(cases.F(c) for c in xyz))
