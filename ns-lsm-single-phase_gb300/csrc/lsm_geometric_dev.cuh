@@ -9,6 +9,11 @@
 #include "lsm_soft64.cuh"
 #include "lsm_volume_dev.cuh"
 
+// (the host tests count what fails it)
+#if !defined(LSM_CHAIN_CHECK)
+#define LSM_CHAIN_CHECK(ok) ((void)0)
+#endif
+
 namespace lsm {
 namespace {
 
@@ -929,6 +934,7 @@ __global__ void __launch_bounds__(32 * kChainWarps, 8) k_geo_sd(
                 } else {
                     if (rest > -2) sd = mag_step(sd, dp);   // its first tetrahedron, or a pnode between
                     rest = -2;
+                    LSM_CHAIN_CHECK(t1 > t0);
                     double m = Q.d[t0];
                     for (int q = t0 + 1; q < t1; ++q) m = dmin(m, Q.d[q]);
                     if (kind == kReset) {
@@ -961,7 +967,10 @@ __global__ void __launch_bounds__(32 * kChainWarps, 8) k_geo_sd(
                 const int o = ord + __popc(all & ((1u << b) - 1u));
                 Encl c = enclose(trif, tets, pent, s, n, P, lane);
                 if (c.lo > dhi) continue;
-                if (nt > kTasks - kMaxTri || nitem == kItems) flush();
+                if (nt > kTasks - kMaxTri || nitem == kItems) {
+                    flush();
+                    if (c.lo > dhi) continue;   // (dhi is tighter now: an item would have no task)
+                }
                 const bool exact = c.lo >= 0.50001f * shi && !box_only_near(c, dhi);
                 const int kind = !exact ? kFull : (c.hi < slo ? kReset : kSimple);
                 if (kind == kReset) nt = nitem = 0;
@@ -1167,6 +1176,7 @@ __global__ void __launch_bounds__(32 * kChainWarps, 8) k_geo_neigh(
                         for (int st = e & 3; st > 0; --st) av = mag_step(av, dp);
                     }
                 } else {
+                    LSM_CHAIN_CHECK(t1 > t0);
                     dp = Q.aux[it] >> 2 ? Q.d[t0] : run_min(dp, Q.d[t0]);
                     for (int q = t0 + 1; q < t1; ++q) dp = run_min(dp, Q.d[q]);   // exact_min: the least
                     av = kind == kReset ? dp : dmin(av, dp);

@@ -4,7 +4,8 @@ against the sequential loops, bit for bit, and its FP32 enclosures against the
 FP64 distances that they have to hold.  The surfaces pass close to a node at
 the coordinate origin (corner or middle of the grid), where the point's
 coordinates and its distance are small while the triangles are a cell wide, on
-cells of aspect 1 to 100, smooth and rough."""
+cells of aspect 1 to 100, smooth and rough; and layers of many nearly equal
+distances.  No queued item may be without tasks."""
 import ctypes as C
 import os
 import shutil
@@ -38,9 +39,9 @@ def ptr(a):
 
 
 def chains(lib, x, y, z, phi, pc, at, reach):
-    """(nodes, signed distances and |v| that differ, largest difference)"""
+    """(nodes, signed distances and |v| that differ, items without tasks, largest difference)"""
     x, y, z, phi, pc = (np.asfortranarray(a, dtype=np.float64) for a in (x, y, z, phi, pc))
-    n = np.zeros(4)
+    n = np.zeros(5)
     lib.geo_chains(*phi.shape, ptr(phi), ptr(x), ptr(y), ptr(z), ptr(pc), *at, reach, ptr(n))
     return n
 
@@ -62,7 +63,7 @@ def rough(rng, n, at, h, off, amp):
 @pytest.mark.parametrize("aspect", [1, 10, 100])
 def test_surfaces_near_an_origin_node(lib, place, aspect):
     n, at = (9, 0) if place == "corner" else (11, 5)
-    total = np.zeros(4)
+    total = np.zeros(5)
     for off in (0.3, 0.03, 0.003):
         for amp in (0.0, 0.3, 2.0):
             for s in range(4):
@@ -71,7 +72,26 @@ def test_surfaces_near_an_origin_node(lib, place, aspect):
                 pc = rng.standard_normal((n,) * 3) * rng.choice([20.0, 0.1, 9.9])
                 total += chains(lib, *grid(n, at, h), rough(rng, n, at, h, off, amp), pc, (at,) * 3, 1)
     assert total[0] > 200
-    assert (total[1:3] == 0).all(), total
+    assert (total[1:4] == 0).all(), total
+
+
+def layers(rng, n, h):
+    X, Y, Z = np.meshgrid(*(np.arange(n) - 0.3,) * 3, indexing="ij")
+    return np.sin(2.1 * Z + 0.02 * X) * 0.3 * min(h) + 0.01 * min(h) * rng.standard_normal((n,) * 3)
+
+
+@pytest.mark.parametrize("aspect", [1, 100])
+def test_many_nearly_equal_distances(lib, aspect):
+    """Flat and rippled layers, near and far from the origin: queues that fill."""
+    n, total = 11, np.zeros(5)
+    for s in range(10):
+        rng = np.random.default_rng([s, aspect])
+        h = np.array([1.0, 1.0, 1.0 / aspect])
+        shift = rng.choice([0.0, 3000.0]) * np.array([1.0, -0.3, 0.05])
+        f = layers(rng, n, h) if s % 2 else rough(rng, n, 5, h, 0.4, 0.02)
+        total += chains(lib, *grid(n, 5, h, shift), f, np.full((n,) * 3, -9.9), (5, 5, 5), 2)
+    assert total[0] > 300
+    assert (total[1:4] == 0).all(), total
 
 
 def deciding(seed):
@@ -88,7 +108,7 @@ def test_surfaces_that_decide_by_an_enclosure(lib, seed):
     its distance depend on triangles that an enclosure without the triangle's size loses."""
     n, at, xyz, phi = deciding(seed)
     c = chains(lib, *xyz, phi, np.full((n,) * 3, -9.9), (at,) * 3, 0)
-    assert c[0] == 1 and (c[1:3] == 0).all(), c
+    assert c[0] == 1 and (c[1:4] == 0).all(), c
 
 
 @pytest.mark.parametrize("seed", range(4))
