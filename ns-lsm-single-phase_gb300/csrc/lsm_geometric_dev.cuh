@@ -1189,9 +1189,10 @@ __global__ void __launch_bounds__(32 * kChainWarps, 8) k_geo_neigh(
         for (int q0 = 0; q0 < box.n; q0 += 32) {
             const int q = q0 + lane;
             const int m0 = q < box.n ? ids[box.node(g, q)] - 1 : -1;
-            // a |v| of 10 or more follows dp = 10 after any tetrahedron
+            // a |v| of 10 or more follows dp = 10 after any tetrahedron; one that
+            // is no number stays so: every test against 9.9999 fails for it
             const float lb = m0 >= 0 ? pnode_bound(m0, P, prad) : 3.0e38f;
-            const bool in = m0 >= 0 && (vhi >= 9.9999f || !beyond(lb, P.scale, vhi));
+            const bool in = m0 >= 0 && (!(vhi < 9.9999f) || !beyond(lb, P.scale, vhi));
             const int s0 = in ? pstart[m0] : 0, n0 = in ? pstart[m0 + 1] - s0 : 0, f0 = in ? lead[m0] : 0;
             unsigned near = __ballot_sync(FM, in);
             while (near) {
@@ -1227,7 +1228,7 @@ __global__ void __launch_bounds__(32 * kChainWarps, 8) k_geo_neigh(
                 }
                 ++nitem;
                 nt = push_tasks(Q, nt, c, t0, t1, lane);
-                if (vhi >= 9.9999f) {
+                if (!(vhi < 9.9999f)) {
                     flush();   // exact again at once: rare
                 } else {
                     // (kFull: the rounding of dp = 10 + (c - 10) stays below 1e-12)

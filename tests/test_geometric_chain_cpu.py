@@ -94,6 +94,19 @@ def test_many_nearly_equal_distances(lib, aspect):
     assert (total[1:4] == 0).all(), total
 
 
+def test_values_of_any_size_before(lib):
+    """|v| of the nodes without a distance: not a number, infinite, huge, about
+    10, tiny and zero, of either sign."""
+    total = np.zeros(5)
+    for s in range(6):
+        rng = np.random.default_rng(s)
+        n, h = 9, (1.0, 1.0, 1.0)
+        v = np.array([np.nan, -np.nan, np.inf, -np.inf, 1e300, -3e38, 10.0, 9.9999, -10.000001, 1e-300, 0.0, -0.0])
+        total += chains(lib, *grid(n, 4, h), rough(rng, n, 4, h, 0.4, 0.2), rng.choice(v, (n,) * 3), (4,) * 3, 2)
+    assert total[0] > 500
+    assert (total[1:4] == 0).all(), total
+
+
 def deciding(seed):
     rng = np.random.default_rng([seed, 5])
     n, at = ((5, 0), (9, 4))[seed & 1]
