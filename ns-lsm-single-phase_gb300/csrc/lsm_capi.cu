@@ -321,7 +321,10 @@ int reinit_device(lsm_context* c, const lsm_grid* g, const DevGrid& dg, const ls
 // reinitialisation_test2 (src/reinitialisation_test2.F90:1-221, non-hybrid)
 // from phizero into dn1 (dn: scratch); *iters = pseudo-time iterations run.
 // The convergence test (the reference's maxval/minval, then `exit`) is made
-// on the device: converged iterations leave the field alone.
+// on the device: converged iterations leave the field alone.  The host looks
+// after 16 iterations, after 32 more and so on (at most 128), so that decks of
+// up to 16 do not wait and the launches of a converged call stay below twice
+// those of the iterations that it ran, plus 16.
 int sussman_device(lsm_context* c, const DevGrid& dg, const lsm_params* p, const double* phizero,
                    const double* csi, const double* eta, const double* zet, double* dn1, double* dn, int* iters) {
     if (p->OrderReinitialisationBoundaries < 1 || p->OrderReinitialisationBoundaries > 3)
@@ -332,7 +335,8 @@ int sussman_device(lsm_context* c, const DevGrid& dg, const lsm_params* p, const
     double* sg = (double*)pool_get(c, "ss_sign", 8 * N, &e);
     double* B = sg ? (double*)pool_get(c, "ss_b", 8 * N, &e) : nullptr;
     auto* move = B ? (unsigned char*)pool_get(c, "ss_move", (size_t)N, &e) : nullptr;
-    auto* mm = move ? (unsigned long long*)pool_get(c, "ss_mm", 16 * ((size_t)R + 1), &e) : nullptr;
+    constexpr int kFirst = 16, kMost = 128;
+    auto* mm = move ? (unsigned long long*)pool_get(c, "ss_mm", 2 * 16 * (kMost + 1), &e) : nullptr;
     if (!mm) return cuda_fail(c, e, "cudaMalloc(reinitialisation_test2)");
     // the i-face blocks of calc_NormGrad_d take phizero at the last node of
     // the interior loop (src/calc_NormGrad_d.F90:41-56, 186-376)
@@ -340,22 +344,29 @@ int sussman_device(lsm_context* c, const DevGrid& dg, const lsm_params* p, const
     const int order = p->OrderReinitialisationBoundaries, enobc = p->ENOBCReinitialisation ? 1 : 0;
     lsm::launch_sign_phi0(N, phizero, p->epslsm, sg, c->stream);
     lsm::launch_copy(phizero, dn1, N, c->stream);
-    if (R > 0)
-        lsm::launch_sussman(dg, order, enobc, R, dn1, dn, B, move, sg, phizero, stale, csi, eta, zet, p->epslsm,
-                            p->epsReinitialisation, p->RNtimestep, mm, c->stream);
     LSM_TRY(after_launch(c));
-    if (iters) {
+    int ran = 0;
+    bool stop = false;
+    const unsigned long long* from = nullptr;
+    for (int it = 0, n = kFirst, k = 0; it < R && !stop; it += n, n = std::min(2 * n, kMost), ++k) {
+        n = std::min(n, R - it);
+        unsigned long long* m = mm + (k & 1) * 2 * (kMost + 1);
+        lsm::launch_sussman(dg, order, enobc, n, dn1, dn, B, move, sg, phizero, stale, csi, eta, zet, p->epslsm,
+                            p->epsReinitialisation, p->RNtimestep, m, from, c->stream);
+        LSM_TRY(after_launch(c));
+        from = m + 2 * n;
+        if (!iters && n == R - it) break;
         // iterations run: up to the first whose extrema had converged
-        std::vector<double> v(2 * (size_t)R + 2);
-        *iters = 0;
-        if (R > 0) {
-            LSM_CU(c, cudaMemcpyAsync(v.data(), mm, 16 * (size_t)R, cudaMemcpyDeviceToHost, c->stream));
-            LSM_CU(c, cudaStreamSynchronize(c->stream));
-            while (*iters < R && !(std::fabs(v[2 * *iters] - 1.0) < p->epsReinitialisation &&
-                                   std::fabs(v[2 * *iters + 1] - 1.0) < p->epsReinitialisation))
-                ++*iters;
+        double v[2 * kMost];
+        LSM_CU(c, cudaMemcpyAsync(v, m, 16 * (size_t)n, cudaMemcpyDeviceToHost, c->stream));
+        LSM_CU(c, cudaStreamSynchronize(c->stream));
+        for (int q = 0; q < n && !stop; ++q) {
+            stop = std::fabs(v[2 * q] - 1.0) < p->epsReinitialisation &&
+                   std::fabs(v[2 * q + 1] - 1.0) < p->epsReinitialisation;
+            if (!stop) ++ran;
         }
     }
+    if (iters) *iters = ran;
     return LSM_OK;
 }
 

@@ -46,7 +46,7 @@ void launch_normgrad_d(const DevGrid& g, int order, int enobc, const double* phi
 void launch_sussman(const DevGrid& g, int order, int enobc, int iters, double* d, double* A, double* B,
                     unsigned char* move, const double* sg, const double* phizero, long long stale, const double* csi,
                     const double* eta, const double* zet, double eps, double epsr, double dt, unsigned long long* mm,
-                    cudaStream_t s);
+                    const unsigned long long* from, cudaStream_t s);
 
 // ---- water volume, band and ghost-fluid list (lsm_volume.cu, --fmad=false)
 // Number of per-block partial slots the volume kernel needs for this grid.

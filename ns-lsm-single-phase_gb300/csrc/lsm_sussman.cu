@@ -307,12 +307,12 @@ __global__ void __launch_bounds__(256, 4) sussman_stage_kernel(DevGrid g, SussAr
     }
 }
 
-// extrema of no value yet, for n iterations
-__global__ void suss_init_kernel(u64* mm, int n) {
+// n pairs of extrema: the first as `from` has it, the others of no value yet
+__global__ void suss_init_kernel(u64* mm, int n, const u64* from) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q < n) {
-        mm[2 * q] = 0u;
-        mm[2 * q + 1] = 0x7FE1CCF385EBC8A0ull;
+        mm[2 * q] = q == 0 && from ? from[0] : 0u;
+        mm[2 * q + 1] = q == 0 && from ? from[1] : 0x7FE1CCF385EBC8A0ull;
     }
 }
 
@@ -333,17 +333,19 @@ void launch_normgrad_d(const DevGrid& g, int order, int enobc, const double* phi
 
 // `iters` iterations of reinitialisation_test2 on d (in place; A, B and move:
 // scratch fields); mm: iters + 1 pairs, the extrema at the start of each
-// iteration (the host counts those that had not converged)
+// iteration (the host counts those that had not converged).  from: the
+// extrema at the start of the first, of iterations run before (nullptr: it is
+// the first of all)
 void launch_sussman(const DevGrid& g, int order, int enobc, int iters, double* d, double* A, double* B,
                     unsigned char* move, const double* sg, const double* phizero, long long stale, const double* csi,
                     const double* eta, const double* zet, double eps, double epsr, double dt, unsigned long long* mm,
-                    cudaStream_t s) {
+                    const unsigned long long* from, cudaStream_t s) {
     const dim3 grid((g.ni + BX - 1) / BX, (g.nj + BY - 1) / BY, (g.nk + BZ - 1) / BZ), block(BX, BY, BZ);
     const double C[3][3] = {{1.0, 0.0, 1.0}, {3.0 / 4.0, 1.0 / 4.0, 1.0 / 4.0}, {1.0 / 3.0, 2.0 / 3.0, 2.0 / 3.0}};
     u64* m = reinterpret_cast<u64*>(mm);
     {
         ProfScope ps("suss_init_kernel", s);
-        suss_init_kernel<<<(iters + 256) / 256, 256, 0, s>>>(m, iters + 1);
+        suss_init_kernel<<<(iters + 256) / 256, 256, 0, s>>>(m, iters + 1, reinterpret_cast<const u64*>(from));
     }
     for (int it = 0; it < iters; ++it) {
         SussArgs a{d, d, A, sg, phizero, csi, eta, zet, move, stale, order, enobc, eps, 1.0 / (2.0 * eps), epsr, 0.0, 0.0,
@@ -362,7 +364,8 @@ void launch_sussman(const DevGrid& g, int order, int enobc, int iters, double* d
             else sussman_stage_kernel<3><<<grid, block, 0, s>>>(g, a);
         };
         // the first iteration's extrema are those of its own stage 1
-        stage(0, d, A, it ? m + 2 * it : nullptr, it ? nullptr : m);
+        const bool own = it == 0 && !from;
+        stage(0, d, A, own ? nullptr : m + 2 * it, own ? m : nullptr);
         stage(1, A, B, m + 2 * it, nullptr);
         stage(2, B, d, m + 2 * it, m + 2 * (it + 1));
     }
