@@ -6,8 +6,8 @@
 // instead of the reference's sequential k-j-i accumulation.
 //
 // Roofline: the algorithmic traffic is 4 words per node (phi, x, y, z), of
-// which x, y, z matter near the interface and the walls only; what bounds
-// the passes is the FP64 pipe, so comparisons run on the integer pipes.
+// which x, y, z matter in the water and at the interface; what bounds the
+// passes is the FP64 pipe, so comparisons run on the integer pipes.
 #include <cuda_runtime.h>
 
 #include "lsm_common.cuh"
@@ -160,36 +160,20 @@ __device__ double tet_water_ref(const double* __restrict__ x, const double* __re
     return r;
 }
 
-// 12 times the volume between the origin and the bilinear face a, b, c, d
-// (Davies and Salmond's face term), positive where the face, seen from the
-// side it faces, runs counter-clockwise
-__device__ __forceinline__ double face_flux(const double* __restrict__ x, const double* __restrict__ y,
-                                            const double* __restrict__ z, long long a, long long b, long long c,
-                                            long long d, double ox, double oy, double oz) {
-    const double ax = __ldg(x + a), ay = __ldg(y + a), az = __ldg(z + a);
-    const double bx = __ldg(x + b), by = __ldg(y + b), bz = __ldg(z + b);
-    const double u0 = __ldg(x + c) - ax, u1 = __ldg(y + c) - ay, u2 = __ldg(z + c) - az;
-    const double v0 = __ldg(x + d) - bx, v1 = __ldg(y + d) - by, v2 = __ldg(z + d) - bz;
-    return ((ax - ox) + (bx - ox)) * (u1 * v2 - u2 * v1) + ((ay - oy) + (by - oy)) * (u2 * v0 - u0 * v2) +
-           ((az - oz) + (bz - oz)) * (u0 * v1 - u1 * v0);
-}
-
 // Water volume of the base cells (TotalWaterVolume.F90:136-294) in chunks of
 // one cell per thread, block partials (K tetrahedra, second tetrahedra,
 // bulk) in a fixed order.
 //
-// Bulk cells: the Davies-Salmond volume is the sum of the cell's six face
-// terms, and the two cells of a face hold the same term with opposite
-// signs.  So the water cells' total is the sum over the faces between a
-// water cell and another cell or the wall (147 FP64 operations a water cell
-// before, 30 a face of the water's surface now).  With `cellvol` the cell's
-// own volume is formed as the reference does.
 // Interface cells: listed per chunk, and their 6 tetrahedra shared out over
 // the threads (before, a warp walked the tetrahedra of its few interface
 // cells one after the other); each cell's tetrahedra are added in order.
 // Bound by the FP64 work of the interface cells (~250 operations a
-// tetrahedron); 0.87 ms on 256 x 128 x 96 nodes before, 0.26 ms now (0.30 ms
-// with 128 registers and four blocks per SM).
+// tetrahedron) and of the water cells (147 each).  (The water cells' total
+// from the faces of the water's surface alone takes fewer, but the error of
+// such a sum grows with the distance to the point that its terms are taken
+// about: 2e-15 where the cells' own volumes give 1e-16.)  256 x 128 x 96
+// nodes: 0.87 ms before, 0.52 ms now, at eight blocks per SM as at four
+// (0.53 ms, without spills; five and six: 0.56 ms).
 __global__ void __launch_bounds__(VOL_THREADS, 8) volume_kernel(DevGrid g, CellBox cb,
         const double* __restrict__ phi, const double* __restrict__ x, const double* __restrict__ y,
         const double* __restrict__ z, double* __restrict__ partials, double* __restrict__ cellvol, unsigned* err) {
@@ -199,8 +183,6 @@ __global__ void __launch_bounds__(VOL_THREADS, 8) volume_kernel(DevGrid g, CellB
     __shared__ int wcut[VOL_THREADS / 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long ncell = (long long)cb.Ni * cb.Nj * cb.Nk;
-    const long long o0 = gid(g, cb.i0, cb.j0, cb.k0);
-    const double ox = __ldg(x + o0), oy = __ldg(y + o0), oz = __ldg(z + o0);
     double K = 0.0, S = 0.0, B = 0.0;
     for (long long base = blockIdx.x * (long long)VOL_THREADS; base < ncell;
          base += (long long)gridDim.x * VOL_THREADS) {
@@ -227,35 +209,13 @@ __global__ void __launch_bounds__(VOL_THREADS, 8) volume_kernel(DevGrid g, CellB
             }
             double vol = 0.0;
             if (allw) {
-                if (cellvol) {
-                    double C[8][3];
+                double C[8][3];
 #pragma unroll
-                    for (int v = 0; v < 8; ++v) {
-                        C[v][0] = __ldg(x + o[v]); C[v][1] = __ldg(y + o[v]); C[v][2] = __ldg(z + o[v]);
-                    }
-                    vol = hex_volume(C);
-                    B = B + vol;
-                } else {
-                    // a neighbour shares four water nodes: its other four decide
-                    auto open = [&](bool wall, long long s, long long p, long long q) {
-                        return wall || !(above_eps(__ldg(phi + s)) && above_eps(__ldg(phi + s + p)) &&
-                                         above_eps(__ldg(phi + s + q)) && above_eps(__ldg(phi + s + p + q)));
-                    };
-                    double F = 0.0;
-                    if (open(i == cb.i0, l - 1, g.sj, g.sk))
-                        F = F - face_flux(x, y, z, o[0], o[3], o[7], o[4], ox, oy, oz);
-                    if (open(i == cb.i0 + cb.Ni - 1, l + 2, g.sj, g.sk))
-                        F = F + face_flux(x, y, z, o[1], o[2], o[6], o[5], ox, oy, oz);
-                    if (open(j == cb.j0, l - g.sj, 1, g.sk))
-                        F = F - face_flux(x, y, z, o[0], o[4], o[5], o[1], ox, oy, oz);
-                    if (open(j == cb.j0 + cb.Nj - 1, l + 2 * g.sj, 1, g.sk))
-                        F = F + face_flux(x, y, z, o[3], o[7], o[6], o[2], ox, oy, oz);
-                    if (open(k == cb.k0, l - g.sk, 1, g.sj))
-                        F = F - face_flux(x, y, z, o[0], o[1], o[2], o[3], ox, oy, oz);
-                    if (open(k == cb.k0 + cb.Nk - 1, l + 2 * g.sk, 1, g.sj))
-                        F = F + face_flux(x, y, z, o[4], o[5], o[6], o[7], ox, oy, oz);
-                    B = B + F;
+                for (int v = 0; v < 8; ++v) {
+                    C[v][0] = __ldg(x + o[v]); C[v][1] = __ldg(y + o[v]); C[v][2] = __ldg(z + o[v]);
                 }
+                vol = hex_volume(C);
+                B = B + vol;
             } else if (!alla) {
                 // CellAnalysis: a vertex within eps of zero or a sign change
                 // (seen from vertex 0)
@@ -333,7 +293,6 @@ __global__ void __launch_bounds__(VOL_THREADS, 8) volume_kernel(DevGrid g, CellB
         }
         __syncthreads();
     }
-    if (!cellvol) B = B / 12.0;
     // fixed-order block reduction of (K, S, B)
     __shared__ double sh[3][VOL_THREADS / 32];
     K = warp_sum(K); S = warp_sum(S); B = warp_sum(B);
