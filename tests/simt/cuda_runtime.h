@@ -38,6 +38,12 @@ inline int min(int a, int b) { return a < b ? a : b; }
 inline double __longlong_as_double(long long v) { double d; std::memcpy(&d, &v, 8); return d; }
 inline float __double2float_rd(double d) { const float f = (float)d; return (double)f > d ? nextafterf(f, -INFINITY) : f; }
 inline float __double2float_ru(double d) { const float f = (float)d; return (double)f < d ? nextafterf(f, INFINITY) : f; }
+inline float __uint_as_float(unsigned v) { float f; std::memcpy(&f, &v, 4); return f; }
+inline unsigned __float_as_uint(float f) { unsigned v; std::memcpy(&v, &f, 4); return v; }
+inline double __hiloint2double(int h, int l) { return __longlong_as_double((long long)((uint64_t)(unsigned)h << 32 | (unsigned)l)); }
+inline int __double2hiint(double d) { uint64_t u; std::memcpy(&u, &d, 8); return (int)(u >> 32); }
+inline int __double2loint(double d) { uint64_t u; std::memcpy(&u, &d, 8); return (int)(unsigned)u; }
+using std::isfinite;
 inline float rsqrtf(float x) { return 1.0f / sqrtf(x); }
 inline unsigned atomicOr(unsigned* p, unsigned v) { const unsigned o = *p; *p |= v; return o; }
 
