@@ -453,10 +453,12 @@ __device__ __noinline__ double godunov_norm_ieee(bool plus, double m0, double m1
 // per direction.  The products and the root run on the integer pipes too,
 // beside the 20 additions left to the FP64 pipe (134 clocked operations
 // where both norms were formed with CUDA's root).  Each is exactly the value
-// of the written-out expression while every factor is 0 or within 2^+-240;
-// others take that expression, in a call (as in product_ieee).  0.79 ms a
-// pseudo-step before, 0.20 ms now on 256 x 128 x 96 nodes; at most 64
-// registers for four blocks per SM (86 and two blocks: 0.27 ms).
+// of the written-out expression while every factor is 0 or in 2^-200 .. 2^240
+// (products are then multiples of 2^-452, and so is a sum of them that
+// cancels: within usqr's range or 0); others take that expression, in a call
+// (as in product_ieee).  0.79 ms a pseudo-step before, 0.20 ms now on
+// 256 x 128 x 96 nodes; at most 64 registers for four blocks per SM (86 and
+// two blocks: 0.27 ms).
 __device__ __forceinline__ double godunov_norm(const DevGrid& g, const double* __restrict__ f,
                                                const double* __restrict__ csi, const double* __restrict__ eta,
                                                const double* __restrict__ zet, long long l, int i, int j, int k,
@@ -478,7 +480,7 @@ __device__ __forceinline__ double godunov_norm(const DevGrid& g, const double* _
         men[d] = first ? p : q;
     }
     const double* m[3] = {csi + 3 * l, eta + 3 * l, zet + 3 * l};
-    auto fits = [](double v) { return biased_exp(v) - 783u < 480u || mag(v) == 0u; };
+    auto fits = [](double v) { return biased_exp(v) - 823u < 440u || mag(v) == 0u; };
     bool ok = true;
 #pragma unroll
     for (int q = 0; q < 9; ++q) {

@@ -168,7 +168,8 @@ __device__ __forceinline__ double norm_grad(const DevGrid& g, int order, int eno
         if (!g.unit) d[m] = mul_ieee(dd[m], d[m]);
     }
     double M[9];
-    auto fits = [](double v) { return biased_exp(v) - 783u < 480u || mag(v) == 0u; };
+    // (the range as in godunov_norm)
+    auto fits = [](double v) { return biased_exp(v) - 823u < 440u || mag(v) == 0u; };
     bool ok = fits(d[0]) && fits(d[1]) && fits(d[2]);
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
