@@ -78,7 +78,7 @@ struct lsm_batch {
         int n = 0, len = 0, grid = 1;
         lsm::batch::Tiles tiles() const { return {d, n, len}; }
     } pmap, smap, cmap, jmap[2];
-    bool reinit_pair = true;    // FP32 pseudo-steps two at a time (reinit_pair) where two are left
+    bool reinit_pair = false;   // FP32 pseudo-steps two at a time (reinit_pair) where two are left
     bool reinit_march = true;   // plain pseudo-steps march in k (reinit_z) rather than walk the brick table
     unsigned long long* d_vacc = nullptr;   // volume accumulators, 4 per instance
     unsigned* d_ilist = nullptr;            // interface cells of a volume pass (N entries) and their count
@@ -791,11 +791,8 @@ int prepare(lsm_batch* b) {
         if (tune) {
             BTRY(autotune(b));
         } else {
-            // shape 0..4: that tile shape, pseudo-steps on the brick table;
-            // 5: tile shape 0, pseudo-steps marching in k and in pairs
             const int sh = std::min(std::max(b->cfg.shape, 0), 5);
             BTRY(build_bricks(b, sh == 5 ? 0 : sh));
-            b->reinit_march = b->reinit_pair = sh == 5;
             b->tma_stage = false;   // k_stage: the faster one on every shape measured
         }
         const int ov = stage_override();
@@ -1102,6 +1099,9 @@ int lsm_batch_create(lsm_batch_handle* out, int device, void* stream, int ninst,
     b->cfg = *cfg;
     b->prec = cfg->precision;
     b->esz = b->prec ? sizeof(double) : sizeof(float);
+    // without autotuning: shape 0..4 that tile shape, pseudo-steps on the brick
+    // table; 5 tile shape 0, pseudo-steps marching in k and in pairs
+    if (!cfg->autotune || b->prec) b->reinit_march = b->reinit_pair = cfg->shape >= 5;
     if (stream) {
         b->stream = (cudaStream_t)stream;
     } else {
