@@ -78,6 +78,7 @@ struct lsm_batch {
         int n = 0, len = 0, grid = 1;
         lsm::batch::Tiles tiles() const { return {d, n, len}; }
     } pmap, smap, cmap, jmap[2];
+    bool force_wide = false;    // LSM_BATCH_WIDE=1: 64-bit offsets whatever the size (tests)
     bool reinit_pair = false;   // FP32 pseudo-steps two at a time (reinit_pair) where two are left
     bool reinit_march = true;   // plain pseudo-steps march in k (reinit_z) rather than walk the brick table
     unsigned long long* d_vacc = nullptr;   // volume accumulators, 4 per instance
@@ -316,11 +317,8 @@ void march_lengths(const lsm_batch* b, int (&len)[lsm::batch::kMaps]) {
 }
 
 // The kernels on flat tiles take byte offsets from the arrays' bases, of 32
-// bits where they suffice (LSM_BATCH_WIDE=1: of 64 all the same, for tests)
-bool wide(const lsm_batch* b) {
-    static const bool forced = std::getenv("LSM_BATCH_WIDE") != nullptr;
-    return forced || b->N >= (1LL << 32) / (b->prec ? 8 : 4);
-}
+// bits where they suffice
+bool wide(const lsm_batch* b) { return b->force_wide || b->N >= (1LL << 32) / (b->prec ? 8 : 4); }
 bool pairs_on(const lsm_batch* b) { return b->reinit_pair && !b->prec; }
 
 // Columns of a flat tile on an instance: whole rows, or parts of a row of
@@ -1099,6 +1097,10 @@ int lsm_batch_create(lsm_batch_handle* out, int device, void* stream, int ninst,
     b->cfg = *cfg;
     b->prec = cfg->precision;
     b->esz = b->prec ? sizeof(double) : sizeof(float);
+    {
+        const char* e = std::getenv("LSM_BATCH_WIDE");
+        b->force_wide = e && *e && std::strcmp(e, "0") != 0;
+    }
     // without autotuning: shape 0..4 that tile shape, pseudo-steps on the brick
     // table; 5 tile shape 0, pseudo-steps marching in k and in pairs
     if (!cfg->autotune || b->prec) b->reinit_march = b->reinit_pair = cfg->shape >= 5;
