@@ -94,6 +94,29 @@ def test_many_nearly_equal_distances(lib, aspect):
     assert (total[1:4] == 0).all(), total
 
 
+@pytest.mark.parametrize("h", [1e-3, 1e-6, 1e-8])
+def test_short_edges(lib, h):
+    """Cells whose triangles' edges are too short for the enclosures: bounding boxes alone."""
+    total = np.zeros(5)
+    for s in range(6):
+        rng = np.random.default_rng(s)
+        n = 11
+        f = (layers(rng, n, (1, 1, 1)) if s % 2 else rough(rng, n, 5, (1, 1, 1), 0.4, 0.2)) * h
+        total += chains(lib, *grid(n, 5, (h, h, h)), f, np.full((n,) * 3, -9.9), (5, 5, 5), 2)
+    assert total[0] > 300
+    assert (total[1:4] == 0).all(), total
+
+
+@pytest.mark.parametrize("at", [(23, 0, 22), (27, 0, 21), (33, 0, 19), (35, 0, 18)])
+def test_flush_between_pnodes(lib, at):
+    """Nodes on a wall whose queue fills just before a pnode out of reach: an item
+    without tasks there changes the last bits."""
+    X, Y, Z = np.meshgrid(*(np.linspace(0, 1, m) for m in (64, 48, 40)), indexing="ij")
+    phi = (Z - 0.48 - 0.1 * np.sin(6 * X) * np.cos(4 * Y)) * 1e-5
+    c = chains(lib, X * 1e-5, Y * 1e-5, Z * 1e-5, phi, np.where(phi < 0, -9.9, 9.9), at, 0)
+    assert c[0] == 1 and (c[1:4] == 0).all(), c
+
+
 def test_values_of_any_size_before(lib):
     """|v| of the nodes without a distance: not a number, infinite, huge, about
     10, tiny and zero, of either sign."""
