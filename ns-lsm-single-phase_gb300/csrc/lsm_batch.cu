@@ -942,7 +942,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_reinit_pair(const Inst* __r
                 const O l = cb + sk * (O)(k - 1);
                 sto(dout, l, r);
                 if (dout2) sto(dout2, l, r);
-                if (err && !vfinite(r)) atomicOr(err, (O)kErrNonFinite);
+                if (err && !vfinite(r)) atomicOr(err, (unsigned)kErrNonFinite);
             }
             if (y < eh) E[me] = e1;
             em = ec;
