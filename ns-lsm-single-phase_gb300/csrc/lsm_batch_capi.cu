@@ -301,8 +301,7 @@ lsm::batch::Tiles tiles(const lsm_batch* b, int m) { return {b->d_amap[m], b->na
 // Measured, against 32 always: 128^3 (256 tiles of 32) k_reinit_rec_z 41 -> 35
 // us; two FP64 grids of about 40^3 k_adj_reinit 375 -> 70 us; 512 x 256 x 256
 // (4096 tiles of 32) loses 6 % at 8.
-void march_lengths(const lsm_batch* b, int (&len)[lsm::batch::kMaps]) {
-    const int sms = 152;
+void march_lengths(const lsm_batch* b, int sms, int (&len)[lsm::batch::kMaps]) {
     for (int m = 0; m < lsm::batch::kMaps; ++m) {
         const auto a = lsm::batch::adj_shape(m);
         const long long want = (m == 1 ? 6 : 3) * sms;
@@ -397,8 +396,10 @@ int build_bricks(lsm_batch* b, int shape) {
             for (int y = 0; y < by; ++y)
                 for (int x = 0; x < bx; ++x) v.push_back(Brick{q, x * sx, y * sy, z * sz});
     };
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
     int(&len)[lsm::batch::kMaps] = b->len;
-    march_lengths(b, len);
+    march_lengths(b, sms, len);
     long long face = 0, pre[3] = {0, 0, 0};
     for (int q = 0; q < b->ninst; ++q) {
         const auto& I = b->inst[q];
@@ -440,8 +441,6 @@ int build_bricks(lsm_batch* b, int shape) {
         pre[2] += (long long)I.ni * I.nj;
         add(brick, q, d.nbx, d.nby, nbz, 1, 1, 1);
     }
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
     b->nface = face;
     for (int a = 0; a < 3; ++a) b->nplane[a] = pre[a];
     b->nbricks = (int)brick.size();
