@@ -21,12 +21,9 @@ constexpr int kMaps = 2;   // tile maps (adj_shape)
 struct Inst {
     long long off;     // first node of the instance in the packed arrays
     int ni, nj, nk;
-    int brick0;        // first brick of the instance in the current brick map
-    int nbx, nby;      // bricks per row / per plane of the instance
     float dt;          // advection time step (multiplied into W)
     float dtau;        // reinitialisation pseudo time step
     float eps;         // smoothing half-width epslsm
-    int pad;
     long long face0;   // first boundary-face node of the instance (forward bc kernels)
     long long fpre[3]; // first node of the instance's i-, j-, k-face planes (adjoint face kernels)
     double dt64, dtau64, eps64;  // the same three parameters for the FP64 kernels

@@ -408,14 +408,9 @@ int build_bricks(lsm_batch* b, int shape) {
         d.ni = I.ni;
         d.nj = I.nj;
         d.nk = I.nk;
-        d.nbx = (I.ni + sh.tx - 1) / sh.tx;
-        d.nby = (I.nj + sh.ty - 1) / sh.ty;
-        const int nbz = (I.nk + sh.tz - 1) / sh.tz;
-        d.brick0 = (int)brick.size();
         d.dt = (float)I.dt;
         d.dtau = (float)I.dtau;
         d.eps = (float)I.eps;
-        d.pad = 0;
         flat_tile(I.ni, I.nj, lsm::batch::kPairThreads, 1, 1, &d.rw, &d.rh);
         flat_tile(I.ni, I.nj, lsm::batch::kStageThreads, 0, 0, &d.sw, &d.sh);
         flat_tile(I.ni, I.nj, lsm::batch::kAdjThreads, 2, 0, &d.xw, &d.xh);
@@ -439,7 +434,7 @@ int build_bricks(lsm_batch* b, int shape) {
         pre[0] += (long long)I.nj * I.nk;
         pre[1] += (long long)I.ni * I.nk;
         pre[2] += (long long)I.ni * I.nj;
-        add(brick, q, d.nbx, d.nby, nbz, 1, 1, 1);
+        add(brick, q, (I.ni + sh.tx - 1) / sh.tx, (I.nj + sh.ty - 1) / sh.ty, (I.nk + sh.tz - 1) / sh.tz, 1, 1, 1);
     }
     b->nface = face;
     for (int a = 0; a < 3; ++a) b->nplane[a] = pre[a];

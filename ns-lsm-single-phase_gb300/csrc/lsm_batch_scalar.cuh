@@ -12,8 +12,6 @@ namespace batch {
 namespace {
 
 // ------------------------------------------------------------ scalar helpers
-template <typename T> __device__ __forceinline__ T vmax(T a, T b) { return a > b ? a : b; }
-template <typename T> __device__ __forceinline__ T vmin(T a, T b) { return a < b ? a : b; }
 // 1 / (a sum of smoothness weights, at least 3e-12): FP32 by the hardware's
 // approximation without the general quotient's care for subnormal divisors,
 // FP64 on the integer pipes
