@@ -159,8 +159,8 @@ int lsm_batch_get_grad_phi0(lsm_batch_handle h, int inst, double* grad);
 /* dL/dq of one instance in the layout of q (4, ni, nj, nk); q(1) gets zero. */
 int lsm_batch_get_grad_velocity(lsm_batch_handle h, int inst, double* grad_q);
 
-/* Tile shape in use (index 0..5 as lsm_batch_config.shape, and the brick
-   table's TX, TY, TZ). */
+/* Tile shape in use (index 0..5 as lsm_batch_config.shape: 5 where the
+   pseudo-steps march in k or run in pairs; and the brick table's TX, TY, TZ). */
 int lsm_batch_shape(lsm_batch_handle h, int* index, int* tx, int* ty, int* tz);
 /* RK stage kernel in use after the first step: 1 plane tiles staged by TMA
    copies (FP32 batches of one instance with ni a multiple of 4, when the

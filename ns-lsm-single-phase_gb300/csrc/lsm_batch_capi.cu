@@ -1456,7 +1456,7 @@ int lsm_batch_mass_state(lsm_batch_handle b, double* out) {
 int lsm_batch_shape(lsm_batch_handle b, int* index, int* tx, int* ty, int* tz) {
     if (!b) return LSM_ERR_NULL;
     const auto sh = lsm::batch::kShapes[b->shape];
-    if (index) *index = b->reinit_march ? 5 : b->shape;
+    if (index) *index = b->reinit_march || pairs_on(b) ? 5 : b->shape;
     if (tx) *tx = sh.tx;
     if (ty) *ty = sh.ty;
     if (tz) *tz = sh.tz;
