@@ -210,10 +210,9 @@ int max_blocks_per_sm(int shape, int kernel);
 // Tile maps besides the forward brick table and the flat tiles (output nodes
 // per tile ox x oy x oz, adj_shape): 0 reverse pseudo-step recomputing its
 // coefficients (overlapped 32 x kReinRY tile marching in k), 1 the k marches
-// over 32 x 8 columns (pseudo-steps, volume scan, TMA stage, reverse
-// pseudo-step from stored coefficients).  The face and velocity adjoints walk
-// the packed nodes with one thread per node (instance found by binary search
-// over the node offsets `offs`).  The extent along the march is the longest;
+// over 32 x 8 columns (single pseudo-steps, volume scan, TMA stage, sums of
+// lam).  The face and velocity adjoints walk the packed nodes with one thread
+// per node (instance found by binary search over the node offsets `offs`).  The extent along the march is the longest;
 // a batch with few tiles takes shorter ones (Tiles::len).
 struct AdjShape { int ox, oy, oz; };
 constexpr int kReinRY = 12;

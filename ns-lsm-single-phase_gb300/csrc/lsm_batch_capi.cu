@@ -87,7 +87,7 @@ struct lsm_batch {
     double* d_vols = nullptr;
     // mass correction: per-instance target volumes (NaN: none) and the last
     // step's correction; adjoint scratch (N fixed-point weights, one partial
-    // per tile of adjoint map 2, one sum per instance)
+    // per tile of adjoint map 1, one sum per instance)
     double* d_target = nullptr;
     Mass* d_mass = nullptr;
     unsigned long long* wfix = nullptr;

@@ -174,10 +174,11 @@ __global__ void rk_upwind_kernel(DevGrid g, StageArgs a) {
 // six faces from there and evaluates for itself only an f- whose stored
 // choice is not its own (a sign change of the contravariant velocity).
 //
-// Bounded by the FP64 pipe (one warp operation in 16 clocks of an SM: 51 of
-// them a node here, six reconstructions with CUDA's divisions took 360) and,
-// nearly as much, by the issue of the integer work beside it: 1.81 ms before,
-// 0.33 ms now on 256 x 128 x 96 nodes.  A tile of 32 x 8 x 4 evaluates 3.4
+// Bounded by the FP64 pipe (one warp operation in 16 clocks of an SM: 40 of
+// them a node, counted on 192 x 96 x 72 nodes; six reconstructions with CUDA's
+// divisions took 360) and, nearly as much, by the issue of the integer work
+// beside it (62 % and 66 % of the time): 1.81 ms before, 0.33 ms now on 256 x
+// 128 x 96 nodes.  A tile of 32 x 8 x 4 evaluates 3.4
 // faces a node, 32 x 2 x 2 4.0.
 template <int TY, int TZ, int NT, bool RH>
 __global__ void __launch_bounds__(NT, 1280 / NT) weno_kernel(DevGrid g, StageArgs a) {
@@ -265,8 +266,11 @@ __global__ void __launch_bounds__(NT, 1280 / NT) weno_kernel(DevGrid g, StageArg
 
 // The largest tile that still fills the GPU: 32 x 8 x 4 from one full wave of
 // blocks on (5 on each of 152 SMs), 32 x 4 x 2 from two blocks per SM on,
-// 32 x 2 x 2 below.  Measured: 256 x 128 x 96 nodes 332 / 377 us with 8 x 4 /
-// 4 x 2, 64^3 49 / 42 us.
+// 32 x 2 x 2 below.  Measured (stage, 8 x 4 / 4 x 2 / 2 x 2, the event timer's
+// overhead included): 256 x 128 x 96 nodes 347 / 381 / 399 us, 128^3 250 / 265 /
+// 277, 112^3 199 / 205 / 214, 192 x 96 x 72 165 / 168 / 176, 96^3 126 / 120 /
+// 125, 88^3 109 / 103 / 107, 64^3 61 / 46 / 47, 48^3 45 / 33 / 32, 32^3 44 / 18 /
+// 17, 16^3 42 / 17 / 16: the lines cost 5 % next to them at most.
 template <bool RH>
 void launch_weno(const DevGrid& g, const StageArgs& a, cudaStream_t s) {
     auto grid = [&](int ty, int tz) { return dim3((g.ni + 31) / 32, (g.nj + ty - 1) / ty, (g.nk + tz - 1) / tz); };

@@ -2,22 +2,28 @@
 // integer pipes, bit for bit the IEEE 754 results (round to nearest even).
 //
 // What bounds the FP64 kernels on GB300 is the FP64 pipe: a multiply or add
-// takes it 19 clocks per warp and SM (measured with 32 warps per SM), and a
-// division or square root through CUDA's operators 143, while an integer
+// takes it 16 clocks per warp and SM by its two lanes (19 measured with 32
+// warps per SM), and a division or square root through CUDA's operators 143
+// (measured), while an integer
 // multiply-add with a 64-bit result takes its pipe 1.3 and a shift, add or
 // logical operation 0.3-0.5.  So quotients and roots are formed here in
 // 64-bit fixed point, beside the FP64 pipe's work.
 //
 // Method (Newton-Raphson on the reciprocal, then the exact remainder:
 // Muller et al., Handbook of Floating-Point Arithmetic, 2nd ed., sections
-// 4.7 and 5.3): a 23-bit seed from the FP32 reciprocal (rcp.approx, at most
-// 1 ulp), one Newton step in fixed point to 44 bits, the truncated quotient
+// 4.7 and 5.3): a 23-bit seed from the FP32 reciprocal or reciprocal root,
+// one Newton step in fixed point to 44 bits, the truncated quotient
 // Q0 = A R, its exact remainder A 2^k - Q0 B (64 bits suffice: Q0 is at most
 // 2^9 short), one more digit from the remainder, and the rounding decided
 // by the final remainder.  A quotient or root of two 53-bit significands
 // never lies half-way between two 53-bit numbers, so the comparison is
 // strict.  Operands or results outside the normal range (zeros, subnormals,
 // infinities, NaN) take CUDA's operator.
+//
+// The seeds may be two units in the last place from the correctly rounded
+// ones (with three some roots come out wrong, with four some quotients): the
+// tests move them by as many on the CPU and compare every argument that they
+// can get on the device.
 #pragma once
 
 #include <cstdint>
